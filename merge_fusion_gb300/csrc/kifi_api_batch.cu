@@ -251,7 +251,7 @@ kifi_status kifi_batch_step_device(kifi_batch* b, const void* const* depth_dev, 
             bj.pp_x = fmul(fsub(0.5f, cam.cx), bj.fl_inv_x);
             bj.pp_y = fmul(fsub(cam.cy, 0.5f), bj.fl_inv_y);
             bj.e2w = e2w;
-            if ((s = kifi_icp_batch_target(b->icp[i], &cam, e2w.m, &bj.out))) return s;
+            if ((s = kifi_icp_batch_target(b->icp[i], &cam, e2w.m, &bj.out, &bj.boxes))) return s;
             bjobs.push_back(bj);
             add_share(bmap, cdiv(P, 256 * 8));
         }

@@ -1,5 +1,6 @@
 // kifi_api_icp.cu -- C ABI of the ICP context and of Renderer::Bin
 // (include/kifi_gpu.h).  Host code; the kernels live in kifi_icp.cu.
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -9,6 +10,10 @@
 #include "kifi_api_util.h"
 
 using namespace kifi;
+
+// where the target's points come from, which decides what is known about
+// where they project (set_prune)
+enum class TargetKind { points, depth, bin };
 
 struct kifi_icp {
     int device = 0;
@@ -20,17 +25,24 @@ struct kifi_icp {
     size_t depth_bytes = 0;
     float4* synth = nullptr;  // target in the association's float4 layout
     size_t synth_cap = 0;     // bytes
+    float4* boxes = nullptr;  // its blocks' bounding boxes
+    size_t boxes_cap = 0;     // bytes
     void* staging = nullptr;  // host float3 targets on their way in
     size_t staging_cap = 0;
     int sw = 0, sh = 0;
     Mat4 synth_e2w{};
     bool have_target = false;
+    TargetKind kind = TargetKind::points;
+    kifi_camera target_cam{};  // depth: the camera that took it
+    Mat4 target_w2c{};         // bin: the matrix it was binned through
     int last_iters = 0;
     IcpState* head = nullptr;        // pinned host copy of the state's head (poses, statistics)
     bool record = false;             // keep the last iteration's association
     long long* pairs = nullptr;      // per source: target index, or -1
     float* pairs_len2 = nullptr;     // per source: len^2
     size_t pairs_cap = 0, pairs_n = 0;
+    unsigned int* winner = nullptr;  // per source: IcpArgs::winner
+    size_t winner_cap = 0;           // bytes
     void* zbuf = nullptr;            // Bin's z-buffer (8 bytes per target pixel)
     size_t zbuf_cap = 0;
     IcpPoseMail* mail = nullptr;     // page-locked, mapped: the last step's pose ...
@@ -59,8 +71,81 @@ kifi_status reserve_bytes(void** p, size_t* cap, size_t bytes, cudaStream_t st) 
     return KIFI_OK;
 }
 
+kifi_status reserve_sources(kifi_icp* c, const kifi_camera* cam) {
+    return reserve_bytes((void**)&c->winner, &c->winner_cap,
+                         (size_t)((cam->width + 3) / 4) * cam->height * sizeof(unsigned int), c->stream);
+}
+
 kifi_status reserve_target(kifi_icp* c, int w, int h) {
-    return reserve_bytes((void**)&c->synth, &c->synth_cap, (size_t)w * h * sizeof(float4), c->stream);
+    const kifi_status s = reserve_bytes((void**)&c->boxes, &c->boxes_cap, icp_box_count(w, h) * sizeof(float4),
+                                        c->stream);
+    return s ? s : reserve_bytes((void**)&c->synth, &c->synth_cap, (size_t)w * h * sizeof(float4), c->stream);
+}
+
+// What is known about where the target's points project through `proj`, for
+// the window search (kifi_icp.cu, Prune).  A back-projected frame aligned
+// with the camera that took it projects to its pixel centres, and a cloud
+// binned through this very matrix into its pixels; for points of the caller's
+// the device measures it before the first step.  Off where proj is no
+// projection of a rigid pose: the planes' distances would not be metric
+// (a = R e2w within 1e-4 of orthonormal), or where the reference's
+// EyeToClipRH shifts the image (a principal point off the centre).
+void set_prune(const kifi_icp& c, const kifi_camera& cam, const Mat4& proj, IcpArgs* a) {
+    a->prune = kPruneOff;
+    const float* e = c.synth_e2w.m;
+    double skew = 0.0, t = 0.0;
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 3; ++j) {
+            double d = i == j ? -1.0 : 0.0;
+            for (int k = 0; k < 3; ++k) d += (double)e[4 * i + k] * (double)e[4 * j + k];
+            skew = std::max(skew, std::fabs(d));
+        }
+    for (int k = 0; k < 3; ++k) t += std::fabs((double)e[12 + k]);
+    // (negated tests: a NaN fails them)
+    if (!(skew <= 1e-4) || !(t <= 1e4) || e[3] != 0.0f || e[7] != 0.0f || e[11] != 0.0f || e[15] != 1.0f) return;
+    // max over the target's columns (rows) c of |row_x - c row_w|: convex in c, so at the ends, and a little beyond
+    double nw = 0.0, n[2] = {0.0, 0.0};
+    for (int k = 0; k < 3; ++k) nw += (double)proj.m[4 * k + 3] * proj.m[4 * k + 3];
+    for (int r = 0; r < 2; ++r)
+        for (int s = -1; s <= 1; s += 2) {
+            double q = 0.0;
+            for (int k = 0; k < 3; ++k) {
+                const double x = (double)proj.m[4 * k + r] - s * 1.05 * (double)proj.m[4 * k + 3];
+                q += x * x;
+            }
+            n[r] = std::max(n[r], std::sqrt(q));
+        }
+    nw = std::sqrt(nw);
+    if (!(n[0] > 1e-3 && n[0] < 1e6 && n[1] > 1e-3 && n[1] < 1e6 && nw > 0.5 && nw < 2.0)) return;
+    a->kx = (float)(0.5 * c.sw * n[0] * 1.0001);
+    a->ky = (float)(0.5 * c.sh * n[1] * 1.0001);
+    a->w_min = (float)(0.12 * nw * 1.01);
+    a->eps = (float)(4e-6 + 4.0 * skew);
+    a->eps0 = (float)((4e-6 + 4.0 * skew) * (2.0 * t + 0.2));
+    switch (c.kind) {
+        case TargetKind::depth: {
+            const kifi_camera& k = c.target_cam;
+            if (k.width != cam.width || k.height != cam.height || k.fx != cam.fx || k.fy != cam.fy ||
+                k.cx != cam.cx || k.cy != cam.cy || 2.0f * cam.cx != (float)cam.width ||
+                2.0f * cam.cy != (float)cam.height) {
+                a->prune = kPruneMeasured;
+                return;
+            }
+            a->lo[0] = a->lo[1] = a->hi[0] = a->hi[1] = 0.5f;
+            a->prune = kPruneKnown;
+            return;
+        }
+        case TargetKind::bin:
+            if (std::memcmp(c.target_w2c.m, proj.m, sizeof proj.m) != 0) {
+                a->prune = kPruneMeasured;
+                return;
+            }
+            a->lo[0] = a->lo[1] = 0.0f;
+            a->hi[0] = a->hi[1] = 1.0f;
+            a->prune = kPruneKnown;
+            return;
+        case TargetKind::points: a->prune = kPruneMeasured; return;
+    }
 }
 
 kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const kifi_camera* cam,
@@ -69,7 +154,10 @@ kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const ki
     if (iterations < 0 || iterations > kIcpMaxStats)
         return fail(KIFI_ERR_INVALID_ARGUMENT, "iterations must be in [0, 64]");
     const size_t n_src = (size_t)((cam->width + 3) / 4) * cam->height;
+    kifi_status s = reserve_sources(c, cam);
+    if (s) return s;
     IcpArgs a{};
+    a.winner = c->winner;
     a.depth = depth_dev;
     a.depth_u16 = u16 ? 1 : 0;
     a.width = cam->width;
@@ -84,7 +172,9 @@ kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const ki
     a.synth = c->synth;
     a.synth_w = c->sw;
     a.synth_h = c->sh;
+    a.boxes = c->boxes;
     a.neg_zero = -0.0f;
+    set_prune(*c, *cam, proj, &a);
     if (c->record) {
         if (n_src > c->pairs_cap) {
             KIFI_CUDA(cudaStreamSynchronize(c->stream));
@@ -115,7 +205,10 @@ kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const ki
 kifi_status kifi_icp_batch_args(kifi_icp* c, const void* depth_dev, const kifi_camera* cam, IcpArgs* a,
                                 IcpState** st, int iterations) {
     if (!c->have_target) return fail(KIFI_ERR_INVALID_ARGUMENT, "ICP target not set");
+    kifi_status s = reserve_sources(c, cam);
+    if (s) return s;
     *a = IcpArgs{};
+    a->winner = c->winner;
     a->depth = depth_dev;
     a->depth_u16 = 1;
     a->width = cam->width;
@@ -129,7 +222,10 @@ kifi_status kifi_icp_batch_args(kifi_icp* c, const void* depth_dev, const kifi_c
     a->synth = c->synth;
     a->synth_w = c->sw;
     a->synth_h = c->sh;
+    a->boxes = c->boxes;
     a->neg_zero = -0.0f;
+    set_prune(*c, *cam, proj, a);
+    if (a->prune == kPruneMeasured) a->prune = kPruneOff;  // a batch measures no targets
     *st = c->st;
     c->last_iters = iterations;
     return KIFI_OK;
@@ -138,21 +234,26 @@ kifi_status kifi_icp_batch_args(kifi_icp* c, const void* depth_dev, const kifi_c
 // Room for a target of the camera's size; records that the next target is
 // this frame's back-projection (written by a batched launch) and returns
 // where it goes.
-kifi_status kifi_icp_batch_target(kifi_icp* c, const kifi_camera* cam, const float* eye_to_world, float4** out) {
+kifi_status kifi_icp_batch_target(kifi_icp* c, const kifi_camera* cam, const float* eye_to_world, float4** out,
+                                  float4** boxes) {
     kifi_status s = reserve_target(c, cam->width, cam->height);
     if (s) return s;
     c->sw = cam->width;
     c->sh = cam->height;
     c->synth_e2w = load_mat(eye_to_world);
+    c->kind = TargetKind::depth;
+    c->target_cam = *cam;
     c->have_target = true;
     *out = c->synth;
+    *boxes = c->boxes;
     return KIFI_OK;
 }
 
 // Everything an alignment against a target of the camera's size may need to
 // allocate, done ahead (outside any stream capture).
 kifi_status kifi_icp_prepare_frame(kifi_icp* c, const kifi_camera* cam) {
-    return reserve_target(c, cam->width, cam->height);
+    kifi_status s = reserve_sources(c, cam);
+    return s ? s : reserve_target(c, cam->width, cam->height);
 }
 
 extern "C" {
@@ -215,8 +316,10 @@ kifi_status kifi_icp_destroy(kifi_icp* c) {
     cudaFreeHost(c->mail);
     cudaFree(c->depth_dev);
     cudaFree(c->synth);
+    cudaFree(c->boxes);
     cudaFree(c->pairs);
     cudaFree(c->pairs_len2);
+    cudaFree(c->winner);
     cudaFree(c->staging);
     cudaFree(c->zbuf);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -256,12 +359,13 @@ kifi_status kifi_icp_set_target(kifi_icp* c, const float* points, int width, int
     const size_t bytes = (size_t)width * height * 12;
     if ((s = reserve_bytes(&c->staging, &c->staging_cap, bytes, c->stream))) return s;
     KIFI_CUDA(cudaMemcpyAsync(c->staging, points, bytes, cudaMemcpyHostToDevice, c->stream));
-    KIFI_CUDA(expand_target_enqueue((const float*)c->staging, width * height, c->synth,
+    KIFI_CUDA(expand_target_enqueue((const float*)c->staging, width, height, c->synth, c->boxes,
                                     c->ls.sms * 4, c->stream));
     KIFI_CUDA(cudaStreamSynchronize(c->stream));
     c->sw = width;
     c->sh = height;
     c->synth_e2w = load_mat(synth_eye_to_world);
+    c->kind = TargetKind::points;
     c->have_target = true;
     return KIFI_OK;
 }
@@ -282,12 +386,14 @@ kifi_status kifi_icp_set_target_from_depth(kifi_icp* c, const void* depth, int o
         src = c->depth_dev;
     }
     const Mat4 e2w = load_mat(eye_to_world);
-    KIFI_CUDA(backproject_enqueue(src, depth_is_u16 != 0, *cam, e2w, c->synth, c->ls.sms * 4,
+    KIFI_CUDA(backproject_enqueue(src, depth_is_u16 != 0, *cam, e2w, c->synth, c->boxes, c->ls.sms * 4,
                                   c->stream));
     if (!on_device) KIFI_CUDA(cudaStreamSynchronize(c->stream));
     c->sw = cam->width;
     c->sh = cam->height;
     c->synth_e2w = e2w;
+    c->kind = TargetKind::depth;
+    c->target_cam = *cam;
     c->have_target = true;
     return KIFI_OK;
 }
@@ -303,10 +409,12 @@ kifi_status kifi_icp_set_target_bin_device(kifi_icp* c, const float* points_dev,
     if (s) return s;
     if ((s = reserve_bytes(&c->zbuf, &c->zbuf_cap, (size_t)width * height * 8, c->stream))) return s;
     KIFI_CUDA(bin_target_enqueue(points_dev, (unsigned int)n, load_mat(world_to_clip), width, height,
-                                 (unsigned long long*)c->zbuf, c->synth, c->ls.sms * 4, c->stream));
+                                 (unsigned long long*)c->zbuf, c->synth, c->boxes, c->ls.sms * 4, c->stream));
     c->sw = width;
     c->sh = height;
     c->synth_e2w = load_mat(synth_eye_to_world);
+    c->kind = TargetKind::bin;
+    c->target_w2c = load_mat(world_to_clip);
     c->have_target = true;
     return KIFI_OK;
 }

@@ -10,9 +10,11 @@
 //                pixel: back-project it with the current pose estimate,
 //                project into the target camera, search the 21x21 window for
 //                the nearest valid target point within len^2 < 0.01
-//                (:100-131; the first minimum in scan order wins).  CTAs own
-//                tiles of sources and stage the union of their windows in
-//                shared memory.
+//                (:100-131; the first minimum in scan order wins).  Only the
+//                candidates that can win are read: a bound on the distance
+//                (the last step's winner, or a few probes) cuts the window to
+//                a rectangle, see Prune.  CTAs own tiles of sources and stage
+//                the part of the target they will read in shared memory.
 //  moments       the associated pairs are not stored: count, sum p, sum q,
 //                sum p q^T and the squared distances are accumulated per
 //                CTA in float-float, each product split exactly by an FMA.
@@ -32,6 +34,8 @@
 // out-of-range); the reference's 640x480 window clamp (:108-109) is kept,
 // with reads past the end of a smaller target buffer treated as invalid
 // points.
+#include <type_traits>
+
 #include "kifi_internal.h"
 
 namespace kifi {
@@ -85,14 +89,6 @@ __device__ __forceinline__ FF ff_div(FF a, FF b) {  // a / b, b != 0
     const FF r = a - b * q1;
     return ff_norm(q1, fdiv(r.hi, b.hi));
 }
-__device__ __forceinline__ FF warp_sum_ff(FF v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        FF w{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
-        v = ff_add(v, w);
-    }
-    return v;
-}
 __device__ __forceinline__ float load_depth(const void* depth, size_t i, bool u16) {
     if (u16) return fmul((float)(unsigned int)__ldg((const unsigned short*)depth + i), 0.001f);
     return __ldg((const float*)depth + i);
@@ -128,20 +124,20 @@ __device__ __forceinline__ bool last_cta(unsigned long long* counter, const unsi
 
 // Totals of the per-CTA float-float partials, by the whole (last) CTA.  The
 // partials are stored component-major (hi row, then lo row, each
-// kIcpMaxCtas long), so warp w reduces component w + 1 (the count, component
-// 0, comes with the last-CTA counter) with coalesced loads: lane l adds CTAs
+// kIcpMaxCtas long), so warp w reduces components w + 1 and w + 9 (the count,
+// component 0, comes with the last-CTA counter) with coalesced loads: lane l adds CTAs
 // l, l + 32, ... in float-float -- all of a lane's loads (up to 320 CTAs)
 // issued in one round -- then a shuffle tree.
 // Fixed order: independent of scheduling.  The loads bypass L1 (the partials
 // were written by other SMs during this launch).
 constexpr int kTotalsPerLane = 10;
-__device__ __forceinline__ FF lane_partials(const float* ph, int b0, int G) {
+__device__ __forceinline__ FF lane_partials(const float* ph, int b0, int n) {
     float h[kTotalsPerLane], l[kTotalsPerLane];
 #pragma unroll
     for (int k = 0; k < kTotalsPerLane; ++k) {
         const int b = b0 + 32 * k;
-        h[k] = b < G ? __ldcg(ph + b) : 0.0f;
-        l[k] = b < G ? __ldcg(ph + kIcpMaxCtas + b) : 0.0f;
+        h[k] = b < n ? __ldcg(ph + b) : 0.0f;
+        l[k] = b < n ? __ldcg(ph + kIcpMaxCtas + b) : 0.0f;
     }
     FF acc{h[0], l[0]};
 #pragma unroll
@@ -149,39 +145,93 @@ __device__ __forceinline__ FF lane_partials(const float* ph, int b0, int G) {
     return acc;
 }
 template <int NV>
-__device__ __forceinline__ void moments_total(const IcpState* st, unsigned int count, FF* out, int G) {
-    const int lane = threadIdx.x & 31, c = (threadIdx.x >> 5) + 1;
+__device__ __forceinline__ void moments_total(const IcpState* st, unsigned int count, FF* out, int n) {
+    constexpr int kPer = 2;  // moments w + 1 and w + 9 side by side
+    const int lane = threadIdx.x & 31, c0 = (threadIdx.x >> 5) + 1;
+    static_assert(NV == 17, "16 moments after the count");
     if (threadIdx.x == 0) out[0] = FF{(float)count, 0.0f};  // exact: at most 2^24 sources
-    if (c < NV) {
-        FF a{0.0f, 0.0f};
-        for (int b0 = lane; b0 < G; b0 += 32 * kTotalsPerLane)
-            a = ff_add(a, lane_partials(st->part + (size_t)(2 * c) * kIcpMaxCtas, b0, G));
-        a = warp_sum_ff(a);
-        if (lane == 0) out[c] = a;
-    }
+    FF a[kPer];
+#pragma unroll
+    for (int h = 0; h < kPer; ++h) a[h] = FF{0.0f, 0.0f};
+    for (int b0 = lane; b0 < n; b0 += 32 * kTotalsPerLane)
+#pragma unroll
+        for (int h = 0; h < kPer; ++h)
+            a[h] = ff_add(a[h], lane_partials(st->part + (size_t)(2 * (c0 + 8 * h)) * kIcpMaxCtas, b0, n));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int h = 0; h < kPer; ++h) {
+            const FF x{__shfl_xor_sync(0xffffffffu, a[h].hi, o), __shfl_xor_sync(0xffffffffu, a[h].lo, o)};
+            a[h] = ff_add(a[h], x);
+        }
+    if (lane < kPer) out[c0 + 8 * lane] = lane ? a[kPer - 1] : a[0];
     __syncthreads();
 }
 
 constexpr int kTileCols = 8, kTileRows = 32;
-constexpr int kSplitRow = 10;   // window rows [0, 10) to the lower half-warp set, [10, 21) to the upper
-constexpr int kStageBatch = 4;  // staging loads in flight per thread
-constexpr int kStagePixels = 5120;  // three float planes (x, y, z): 60 KB
-constexpr int kPredMargin = 2;      // pixels added around a predicted window box
+constexpr int kBlockW = 8, kBlockH = 4;  // target pixels per bounding box, a warp's worth
+constexpr int kTileThreads = kTileCols * kTileRows;  // one source per thread
+constexpr int kPredMargin = 4;  // pixels added around the rectangles that a tile searched in the last step,
+constexpr int kUseMargin = 4;   // and that the region so staged must leave around the projections to be used
+constexpr int kStagePixels = 5120;  // float4 target points staged per tile: 80 KB, two tiles per SM
 
-// Row pitch of a staged region `w` pixels wide: even, so that a pair of
-// adjacent pixels is one aligned 64-bit load, with pitch/2 odd, so that the
-// 64-bit loads of lanes whose windows sit one row apart hit distinct banks.
-__host__ __device__ constexpr int stage_pitch(int w) {
-    return ((w + 1) & ~1) + ((((w + 1) & ~1) >> 1) & 1 ? 0 : 2);
+// Row pitch of a staged region `w` pixels wide: odd, so that the 16-byte
+// loads of eight lanes one row apart cover all banks.
+__host__ __device__ constexpr int stage_pitch(int w) { return w | 1; }
+
+// The target pixels [x0, x0 + w) x [y0, y0 + h) (linear index y * synth_w + x,
+// as the reference reads them) into `stage` with row pitch `pitch`, by the
+// tile's eight warps, as 16-byte asynchronous copies (stage_wait, then a
+// barrier, before they are read).  Points that are none (ICP.cpp:112) hold NaN in the
+// target buffer; indices past the buffer's end are none too.
+__device__ __forceinline__ void stage_region(float4* stage, const float4* __restrict__ synth, size_t n_synth,
+                                             int synth_w, int x0, int y0, int w, int h, int pitch) {
+    // warps take rows, lanes take columns
+    const int warp = threadIdx.x >> 5 & 7, lane = threadIdx.x & 31;
+    for (int ry = warp; ry < h; ry += 8) {
+        for (int rx = lane; rx < w; rx += 32) {
+            const size_t at = (size_t)(y0 + ry) * synth_w + (x0 + rx);
+            float4* dst = stage + ry * pitch + rx;
+            if (at < n_synth) {
+                const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(synth + at) : "memory");
+            } else {
+                *dst = make_float4(__int_as_float(0x7fffffff), 0.f, 0.f, 0.f);
+            }
+        }
+    }
 }
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Packed float pairs (f32x2): each half is rounded exactly as the scalar
-// __fsub_rn / __fadd_rn of that half.  Products are formed as
-// fma(a, a, -0) with the -0 a kernel parameter: that is the rounded product
-// for every input (x + -0 = x, also for x = -0), and unlike a packed
-// multiply it cannot be fused into the add that consumes it -- ptxas does
-// fuse mul.rn.f32x2 into a following add.rn.f32x2, which would round the
-// sum of squares once instead of the reference's separate roundings.
+// Which candidates of a source's window can win.
+//
+// A target point q at pixel x has a projected column X(q) in [x + lo, x + hi]
+// (lo = hi = 1/2 for a back-projected frame, [0, 1] for a binned cloud), and
+// the points whose column is X lie in a plane through the eye.  A source p at
+// distance |n . p + n3| / |n| from that plane -- |X(p) - X| w / (W/2) over at
+// most max |n| -- cannot be nearer than that to q, nor to a point whose
+// column lies further out.  So once some candidate of the window is at
+// distance r, only candidates within
+//     m = r (W/2) max|n| / w
+// columns of X(p) can be as near; likewise for rows.  The first strict
+// minimum of that rectangle is the first strict minimum of the window: the
+// candidates left out are strictly further away.  kx, ky hold (W/2) max|n| and
+// (H/2) max|n| over the target's columns and rows; r is widened by 1e-5 (the
+// rounding of len^2) and by eps |p|_1 + eps0 (metres: the roundings of the
+// target's points, of proj and of p's projection), m by 0.1% and a fiftieth of
+// a pixel.  Sources nearer than w_min to the eye plane (points behind the eye
+// project too), windows that wrap past the target's width into the next row
+// (:110) and targets without the property search the whole window.
+struct Prune {
+    float kx, ky, eps, eps0, w_min;
+    float lo_x, hi_x, lo_y, hi_y;
+    bool on;
+};
+
+// A point as two packed float pairs (x, y), (z, w); target points have w = 1.
+struct alignas(16) Packed {
+    unsigned long long xy, zw;
+};
 __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
     unsigned long long d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
@@ -190,152 +240,284 @@ __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
 __device__ __forceinline__ void f2_unpack(unsigned long long v, float& lo, float& hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long f2_sq(unsigned long long a, unsigned long long neg_zero) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(a), "l"(neg_zero));
-    return d;
-}
-__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
+// Squared distance of a candidate and a source in the reference's order,
+// (dx^2 + dy^2) + (dz^2 + dw^2): two packed subtractions and two packed
+// squares (f32x2: each half rounded as the scalar operation), three adds.  A
+// square is fma(d, d, -0) with the -0 a kernel parameter: the rounded product
+// for every input (x + -0 = x, also for x = -0), which unlike a packed
+// multiply ptxas does not fuse into the add that consumes it.
+__device__ __forceinline__ float len2(const Packed& q, const Packed& p, unsigned long long nz) {
+    unsigned long long a, b;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(q.xy), "l"(p.xy));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(b) : "l"(q.zw), "l"(p.zw));
+    asm("fma.rn.f32x2 %0, %0, %0, %1;" : "+l"(a) : "l"(nz));
+    asm("fma.rn.f32x2 %0, %0, %0, %1;" : "+l"(b) : "l"(nz));
+    float xx, yy, zz, ww;
+    f2_unpack(a, xx, yy);
+    f2_unpack(b, zz, ww);
+    return fadd(fadd(xx, yy), fadd(zz, ww));
 }
 
-// The staging buffer: planes of x, y and z, kStagePixels floats each.
-struct Stage {
-    float* x;
-    float* y;
-    float* z;
+// A tile while its sources' windows are searched: the sources whose rectangles
+// are searched by all threads, and their rows.
+struct Rect {
+    long long first;  // its first candidate's index in the staging buffer or the target
+    int stride;       // of its rows there; negative in the target
+    int number;       // the first candidate's number r * 32 + c << 8 | columns
+};
+constexpr int kItems = 21 * kTileThreads;  // every row of every window
+struct SearchSmem {
+    struct List {
+        Packed p[kTileThreads];                // per source: world point
+        Rect rect[kTileThreads];
+        unsigned long long key[kTileThreads];  // best so far: len^2 bits << 32 | candidate number
+        unsigned short item[kItems];           // rows to search: source << 5 | row
+    };
+    union {
+        List list;
+        float rec[7][kTileThreads];  // per source: p xyz, q xyz, len^2 (0 when no pair)
+    };
+    unsigned int n_items;
+    int box[4];      // the tile's rectangles: x0, y0, x1, y1
+    int cbox[4];     // and projections
+    int pred[4];     // the region staged ahead: x0, y0, w, h
+    FF acc[17];      // the CTA's moments (index 0 unused: count)
+    unsigned int count;
+};
+// What part of the target a tile has staged: pixels [x0, x1) x [y0, y1).
+struct Region {
+    int buf;  // its first pixel's index in the CTA's staging buffer
+    int x0, y0, x1, y1, pitch;
+    __device__ __forceinline__ int at(int x, int y) const { return buf + (y - y0) * pitch + (x - x0); }
+    __device__ __forceinline__ bool holds(int x, int y, int cols, int rows) const {
+        return x >= x0 && y >= y0 && x + cols <= x1 && y + rows <= y1;
+    }
 };
 
-// The target pixels [x0, x0 + w) x [y0, y0 + h) (linear index y * synth_w + x,
-// as the reference reads them) into the planes of `stage` with row pitch
-// `pitch`, by the whole CTA: kStageBatch independent loads in flight per
-// thread, then the stores.  (0,0,0) is no point (ICP.cpp:112) and is staged
-// with x = NaN; indices past the buffer's end are invalid points too.
-__device__ __forceinline__ void stage_region(const Stage& stage, const float4* __restrict__ synth,
-                                             size_t n_synth, int synth_w, int x0, int y0, int w, int h,
-                                             int pitch) {
-    // warps take rows (kStageBatch rows in flight each), lanes take columns
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
-    for (int ry0 = warp; ry0 < h; ry0 += kStageBatch * n_warps) {
-        for (int rx = lane; rx < w; rx += 32) {
-            float4 q[kStageBatch];
+constexpr unsigned long long kNoPair = (unsigned long long)0x3c23d70au << 32;  // len^2 = 0.01f, candidate 0
+
+// The tile's staged region (dynamic shared memory).
+extern __shared__ float4 stage_all[];
+
+// A target point in the staging buffer or in the target itself.
+template <bool kStaged>
+__device__ __forceinline__ Packed target_at(const float4* __restrict__ synth, long long i) {
+    if (kStaged) return *reinterpret_cast<const Packed*>(stage_all + (int)i);
+    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(synth + i));
+    return Packed{v.x, v.y};
+}
+
+// The first strict minimum of `cols` candidates from index i on: four at a
+// time, then the rest three at a time (past the row's end its last one again,
+// which cannot win).
+template <bool kStaged>
+__device__ __forceinline__ void scan_row(const float4* __restrict__ synth, long long i, int cols, const Packed& p,
+                                         unsigned long long nz, float& best, int& at, int number) {
+    int c = 0;
+    for (; c + 8 <= cols; c += 4) {
+        float l2[4];
 #pragma unroll
-            for (int k = 0; k < kStageBatch; ++k) {
-                const int ry = ry0 + k * n_warps;
-                q[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (ry < h) {
-                    const size_t at = (size_t)(y0 + ry) * synth_w + (x0 + rx);
-                    if (at < n_synth) q[k] = __ldg(synth + at);
-                }
-            }
+        for (int k = 0; k < 4; ++k) l2[k] = len2(target_at<kStaged>(synth, i + c + k), p, nz);
 #pragma unroll
-            for (int k = 0; k < kStageBatch; ++k) {
-                const int ry = ry0 + k * n_warps;
-                if (ry < h) {
-                    if (q[k].x == 0.0f && q[k].y == 0.0f && q[k].z == 0.0f) q[k].x = __int_as_float(0x7fffffff);
-                    const int at = ry * pitch + rx;
-                    stage.x[at] = q[k].x;
-                    stage.y[at] = q[k].y;
-                    stage.z[at] = q[k].z;
-                }
+        for (int k = 0; k < 4; ++k)
+            if (l2[k] < best) {
+                best = l2[k];
+                at = number + c + k;
             }
-        }
+    }
+    for (; c < cols; c += 3) {
+        float l2[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) l2[k] = len2(target_at<kStaged>(synth, i + min(c + k, cols - 1)), p, nz);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (l2[k] < best) {
+                best = l2[k];
+                at = number + c + k;
+            }
     }
 }
 
-// Scan of one thread's window in the staged region (`base` = its first
-// candidate's plane index, even pitch).  Invalid target points were staged
-// with x = NaN, which never passes `l2 < best`.  A full 21-wide row is ten
-// aligned pairs of adjacent candidates, whose squared distances are formed
-// two at a time in packed float pairs (each half with the reference's
-// operations and rounding), plus the one candidate left over: the first when
-// the window starts on an odd plane index, else the last.  Three chains --
-// the pairs' first halves, their second halves and the leftovers -- keep
-// their own first strict minimum; the lexicographic (l2, candidate) minimum
-// of the chains is the first strict minimum of the row-major scan.  Returns
-// the best squared distance (0.01 when none) and its candidate number
-// r * 32 + c (-1 when none).
-template <bool kW>
-__device__ __forceinline__ float scan_staged(const Stage& sp, int base, int pitch, int nr, int nc, float px,
-                                             float py, float pz, float dw2, float neg_zero, int* best_rc) {
-    float b0 = 0.01f, b1 = 0.01f, b2 = 0.01f;
-    int i0 = 0x7fffffff, i1 = 0x7fffffff, i2 = 0x7fffffff;
-    // one candidate in scalar float, the reference's order: (dx^2 + dy^2) + (dz^2 + dw^2)
-    auto cand = [&](int at, int c, float& b, int& bc) {
-        const float dx = fsub(sp.x[at], px), dy = fsub(sp.y[at], py), dz = fsub(sp.z[at], pz);
-        const float zz = kW ? fadd(fmul(dz, dz), dw2) : fmul(dz, dz);
-        const float l2 = fadd(fadd(fmul(dx, dx), fmul(dy, dy)), zz);
-        if (l2 < b) {
-            b = l2;
-            bc = c;
-        }
+// The search of a source's window [nr x nc] (first candidate: target pixel
+// (u, v)) by its own thread.  It bounds the distance to the nearest candidate,
+// cuts the window down to the rectangle that can win and, where that is still
+// large (fast motion, a depth edge), to the blocks of 8 x 4 target pixels
+// whose bounding boxes are near enough; it scans the rectangle in the
+// reference's row-major order, in the staged region where that holds it, else
+// in the target itself.  A rectangle far above its warp's average goes onto
+// the tile's list row by row, for all threads (search_items).  (cr, cc): the
+// candidate the source projects to; X, Y, w: its projected column and row
+// coordinate (upwards) and clip w; (hr, hc): a candidate likely to be near
+// (-1: none).  Returns the best key so far; by whole warps.  Measured at
+// 640x480: 10-40 candidates per source instead of 441 after the first two
+// steps, an alignment of 15 steps 335 us (433 us with the whole windows); the
+// step is then held by its serial parts -- the projection, the moments, the
+// last CTA's totals and Horn solve, about 11 of 16 us -- and by the tile with
+// the most candidates.
+constexpr int kOwnArea = 32;    // rectangles up to this, and up to 1.5 times the warp's average, are scanned by their thread
+constexpr int kBoxArea = 72;    // rectangles above this are cut down by the blocks' boxes
+__device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const Region& reg, int nr, int nc, int cr,
+                                                         int cc, int hr, int hc, bool first, int u, int v, float X,
+                                                         float Y, float w, const Prune& pr, const float (&p)[4],
+                                                         SearchSmem& ss, bool& listed) {
+    const int W = a.synth_w, H = a.synth_h;
+    const Packed pp{f2_pack(p[0], p[1]), f2_pack(p[2], p[3])};
+    const unsigned long long nz = f2_pack(a.neg_zero, a.neg_zero);
+    auto pixel_len2 = [&](int x, int y) {
+        const Packed q = reg.holds(x, y, 1, 1) ? target_at<true>(nullptr, reg.at(x, y))
+                                               : target_at<false>(a.synth, (long long)y * W + x);
+        return len2(q, pp, nz);
     };
-    if (nc == 21) {
-        const int o = base & 1;       // the pairs start at an even plane index
-        const int cs = o ? 0 : 20;    // the leftover candidate's column
-        const unsigned long long PX = f2_pack(px, px), PY = f2_pack(py, py), PZ = f2_pack(pz, pz);
-        const unsigned long long DW = f2_pack(dw2, dw2), NZ = f2_pack(neg_zero, neg_zero);
-        for (int r = 0; r < nr; ++r, base += pitch) {
-            // a candidate records only its pair number (a constant of the
-            // unrolled row); the row and the parity are folded in once per row
-            int c0 = -1, c1 = -1;
-            bool moved = false;
-            const int pb = base + o;
+    // the distance bound.  From the second step on the pixel that won the
+    // step before is usually within a pixel of the new winner; in the first
+    // one, the 3 x 3 candidates around the projection and, when the source is
+    // still five pixels' distance and more from them, every fifth candidate of
+    // the window's rows and columns.
+    const int nrt = min(nr, H - v), nct = min(nc, W - u);  // the window's part inside the target
+    float b = 0.01f;
+    if (hr >= 0 && hr < nrt && hc < nct) {
+        const float l2 = pixel_len2(u + hc, v + hr);
+        if (l2 < b) b = l2;
+    }
+    if (first) {
+        float l2[9];
 #pragma unroll
-            for (int k = 0; k < 10; ++k) {
-                const int at = pb + 2 * k;
-                const unsigned long long X = *(const unsigned long long*)(sp.x + at);
-                const unsigned long long Y = *(const unsigned long long*)(sp.y + at);
-                const unsigned long long Z = *(const unsigned long long*)(sp.z + at);
-                const unsigned long long dx = f2_sub(X, PX), dy = f2_sub(Y, PY), dz = f2_sub(Z, PZ);
-                unsigned long long zz = f2_sq(dz, NZ);
-                if (kW) zz = f2_add(zz, DW);
-                const unsigned long long l2 = f2_add(f2_add(f2_sq(dx, NZ), f2_sq(dy, NZ)), zz);
-                float lo, hi;
-                f2_unpack(l2, lo, hi);
-                if (lo < b0) {
-                    b0 = lo;
-                    c0 = 2 * k;
-                }
-                if (hi < b1) {
-                    b1 = hi;
-                    c1 = 2 * k;
-                }
-            }
-            {
-                int cl = -1;
-                cand(base + cs, 0, b2, cl);
-                moved = cl >= 0;
-            }
-            const int r32 = r * 32;
-            if (c0 >= 0) i0 = r32 + o + c0;
-            if (c1 >= 0) i1 = r32 + o + c1 + 1;
-            if (moved) i2 = r32 + cs;
+        for (int k = 0; k < 9; ++k) {
+            const int r = cr + k / 3 - 1, c = cc + k % 3 - 1;
+            l2[k] = 1.0f;
+            if (r >= 0 && c >= 0 && r < nrt && c < nct) l2[k] = pixel_len2(u + c, v + r);
         }
-    } else {
-        for (int r = 0; r < nr; ++r, base += pitch) {
-            int c0 = -1;
-            for (int c = 0; c < nc; ++c) cand(base + c, c, b0, c0);
-            if (c0 >= 0) i0 = r * 32 + c0;
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+            if (l2[k] < b) b = l2[k];
+        if (b * pr.kx * pr.kx > 25.0f * w * w) {
+            const int rs = cr >= 10 ? cr - 10 : 0, cs = cc >= 10 ? cc - 10 : 0;
+            const bool all = reg.holds(u + cs, v + rs, max(nct - cs, 0), max(nrt - rs, 0));
+            for (int r = rs; r < nrt; r += 5)
+                for (int c = cs; c < nct; c += 5) {
+                    const float g = all ? len2(target_at<true>(nullptr, reg.at(u + c, v + r)), pp, nz)
+                                        : pixel_len2(u + c, v + r);
+                    if (g < b) b = g;
+                }
         }
     }
-    if (b1 < b0 || (b1 == b0 && i1 < i0)) {
-        b0 = b1;
-        i0 = i1;
+    int r0 = 0, rows = nr, c0 = 0, cols = nc;
+    if (pr.on && w > pr.w_min && nr > 0) {
+        const float r = sqrtf(b) * 1.00001f + (pr.eps * (fabsf(p[0]) + fabsf(p[1]) + fabsf(p[2])) + pr.eps0);
+        const float s = __fdividef(r * 1.001f, w);
+        const float mx = fmaf(pr.kx, s, 0.02f + 1e-5f * fabsf(X)), my = fmaf(pr.ky, s, 0.02f + 1e-5f * fabsf(Y));
+        // a window past the target's width reads on in the next row, whose
+        // first columns are the ones to exclude then
+        const int wrap = u + nc - W;
+        if (wrap <= 0 || X - mx - pr.hi_x > (float)wrap) {
+            const int nc1 = wrap > 0 ? nc - wrap : nc;
+            // columns x + lo <= X + mx, x + hi >= X - mx; column 0 also takes what truncates to it from below
+            const int x0 = (int)ceilf(fminf(fmaxf(X - mx - pr.hi_x, (float)u), (float)(u + nc)));
+            const int x1 = max((int)floorf(fmaxf(fminf(X + mx - pr.lo_x, (float)(u + nc1 - 1)), (float)u - 1.0f)), 0);
+            // rows count downwards: row y has coordinate t = H - 1 - y
+            const float tv0 = (float)(H - 1 - (v + nr - 1)), tv1 = (float)(H - 1 - v);
+            const int t0 = (int)ceilf(fminf(fmaxf(Y - my - pr.hi_y, tv0), tv1 + 1.0f));
+            const int t1 = max((int)floorf(fmaxf(fminf(Y + my - pr.lo_y, tv1), tv0 - 1.0f)), 0);
+            c0 = x0 - u;
+            cols = min(x1 - u, nc1 - 1) - c0 + 1;
+            r0 = max(H - 1 - t1 - v, 0);
+            rows = min(H - 1 - t0 - v, nr - 1) - r0 + 1;
+        }
     }
-    if (b2 < b0 || (b2 == b0 && i2 < i0)) {
-        b0 = b2;
-        i0 = i2;
+    rows = min(rows, H - v - r0);  // past the target's last row there is nothing
+    if (rows <= 0 || cols <= 0) rows = cols = 0;
+    const bool wraps = u + c0 + cols > W;
+    if (rows * cols > kBoxArea && !wraps) {  // (blocks do not follow a window into the next row)
+        // the rectangle of the blocks no further than the bound (with the roundings covered)
+        const int nbx = (W + kBlockW - 1) / kBlockW;
+        const int x0 = u + c0, y0 = v + r0, bx1 = (x0 + cols - 1) >> 3, by1 = (y0 + rows - 1) >> 2;
+        const float far = b * 1.00001f;
+        int mx0 = bx1 + 1, mx1 = -1, my0 = by1 + 1, my1 = -1;
+        for (int by = y0 >> 2; by <= by1; ++by)
+            for (int bx = x0 >> 3; bx <= bx1; ++bx) {
+                const float4* q = a.boxes + 2 * ((size_t)by * nbx + bx);
+                const float4 lo = __ldg(q), hi = __ldg(q + 1);
+                const float dx = fmaxf(fmaxf(lo.x - p[0], p[0] - hi.x), 0.0f);
+                const float dy = fmaxf(fmaxf(lo.y - p[1], p[1] - hi.y), 0.0f);
+                const float dz = fmaxf(fmaxf(lo.z - p[2], p[2] - hi.z), 0.0f);
+                if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= far) {
+                    mx0 = min(mx0, bx);
+                    mx1 = max(mx1, bx);
+                    my0 = min(my0, by);
+                    my1 = max(my1, by);
+                }
+            }
+        const int nx0 = max(x0, mx0 * kBlockW), nx1 = min(x0 + cols, (mx1 + 1) * kBlockW);
+        const int ny0 = max(y0, my0 * kBlockH), ny1 = min(y0 + rows, (my1 + 1) * kBlockH);
+        c0 = nx0 - u;
+        cols = nx1 - nx0;
+        r0 = ny0 - v;
+        rows = ny1 - ny0;
+        if (rows <= 0 || cols <= 0) rows = cols = 0;  // no block near enough
     }
-    *best_rc = i0 == 0x7fffffff ? -1 : i0;
-    return b0;
+    const int n = rows * cols, x0 = u + c0, y0 = v + r0;
+    {  // the region the next step will want
+        const int bx0 = (int)__reduce_min_sync(0xffffffffu, n ? (unsigned)x0 : 0x7fffffffu);
+        const int by0 = (int)__reduce_min_sync(0xffffffffu, n ? (unsigned)y0 : 0x7fffffffu);
+        const int bx1 = __reduce_max_sync(0xffffffffu, n ? x0 + cols : -1);
+        const int by1 = __reduce_max_sync(0xffffffffu, n ? y0 + rows : -1);
+        if ((threadIdx.x & 31) == 0 && bx1 >= 0) {
+            atomicMin(&ss.box[0], bx0);
+            atomicMin(&ss.box[1], by0);
+            atomicMax(&ss.box[2], bx1);
+            atomicMax(&ss.box[3], by1);
+        }
+    }
+    // (a warp's own rectangles, of vertical neighbours, read shared memory
+    // without conflicts; the list's rows do not)
+    const int total = (int)__reduce_add_sync(0xffffffffu, (unsigned int)n);
+    const int most = max(kOwnArea, total * 3 >> 6);
+    const bool in = reg.holds(x0, y0, cols, rows);
+    const int number = r0 * 32 + c0;
+    if (n > most && !wraps) {
+        const int me = threadIdx.x;
+        ss.list.p[me] = pp;
+        ss.list.rect[me] = in ? Rect{reg.at(x0, y0), reg.pitch, number << 8 | cols}
+                              : Rect{(long long)y0 * W + x0, -W, number << 8 | cols};
+        ss.list.key[me] = kNoPair;
+        const unsigned int i0 = atomicAdd(&ss.n_items, (unsigned int)rows);
+        for (int r = 0; r < rows; ++r) ss.list.item[i0 + r] = (unsigned short)(me << 5 | r);
+        listed = true;
+        return kNoPair;
+    }
+    float best = 0.01f;
+    int brc = -1;
+    if (in) {  // (a staged region has no points past the target's end)
+        int i = reg.at(x0, y0);
+        for (int r = 0; r < rows; ++r, i += reg.pitch) scan_row<true>(nullptr, i, cols, pp, nz, best, brc, number + r * 32);
+    } else {  // (a wrapped window's last columns may lie past the target's end)
+        long long i = (long long)y0 * W + x0;
+        for (int r = 0; r < rows; ++r, i += W)
+            scan_row<false>(a.synth, i, (int)min((long long)cols, (long long)W * H - i), pp, nz, best, brc,
+                            number + r * 32);
+    }
+    return brc < 0 ? kNoPair : (unsigned long long)__float_as_uint(best) << 32 | (unsigned int)brc;
+}
+
+// The listed rows, dealt out to the CTA's threads; a source's key takes the
+// lexicographic (len^2, candidate number) minimum, the first strict minimum
+// in row-major order.
+__device__ __forceinline__ void search_items(const float4* __restrict__ synth, unsigned int n_items, float neg_zero,
+                                             SearchSmem& ss) {
+    const unsigned long long nz = f2_pack(neg_zero, neg_zero);
+    for (unsigned int i = threadIdx.x; i < n_items; i += kTileThreads) {
+        const int it = ss.list.item[i], s = it >> 5, row = it & 31;
+        const Packed p = ss.list.p[s];
+        const Rect rect = ss.list.rect[s];
+        float best = 0.01f;
+        int at = -1;
+        const int cols = rect.number & 0xff, number = (rect.number >> 8) + row * 32;
+        if (rect.stride > 0)
+            scan_row<true>(nullptr, (int)rect.first + row * rect.stride, cols, p, nz, best, at, number);
+        else
+            scan_row<false>(synth, rect.first - (long long)row * rect.stride, cols, p, nz, best, at, number);
+        if (at >= 0) atomicMin(&ss.list.key[s], (unsigned long long)__float_as_uint(best) << 32 | (unsigned int)at);
+    }
 }
 
 __device__ __noinline__ void finish_step(IcpState* __restrict__ st, const FF* __restrict__ tot,
@@ -344,20 +526,12 @@ __device__ __noinline__ void finish_step(IcpState* __restrict__ st, const FF* __
 // One ICP::AlignStep (ICP.cpp:35-265) as one kernel.
 //
 // Association (:66-131): a CTA owns a tile of 8 source columns x 32 source
-// rows.  Warp w takes source column w/2 of the tile and lane l source row l,
-// so a warp's lanes are vertically adjacent sources whose windows sit about
-// one image row apart; the two warps of a column split each 21x21 window
-// into rows 0-10 and 11-20.  Each thread back-projects and projects its
-// source, the CTA stages the bounding box of the tile's windows in shared
-// memory (planes of x, y and z; an even row pitch with pitch/2 odd: pairs of
-// pixels are aligned 64-bit loads, lanes hit distinct banks) and each
-// thread scans its rows in the reference's loop order, two candidates at a
-// time in packed float pairs; the halves are merged
-// by (len^2, scan position), so the first strict minimum wins as in the
-// reference.  A region too large for the staging buffer (fast motion) is
-// read from global memory instead.  Target pixel (y1, x1) is linear index
-// y1 * synth_w + x1 as in the reference; indices past the buffer's end are
-// invalid points.
+// rows, a thread one source, a warp 32 vertically adjacent ones.  Each thread
+// back-projects and projects its source, the CTA stages the part of the
+// target that the tile's searches will mostly read in shared memory, and
+// search_own and search_items find each source's nearest candidate, the
+// reference's first strict minimum.  Target pixel (y1, x1) is linear index y1 * synth_w + x1 as
+// in the reference; indices past the buffer's end are invalid points.
 //
 // Horn's sums: instead of a second pass over the pairs for the centred
 // cross-covariance (:169-197), the kernel accumulates the raw moments --
@@ -367,15 +541,21 @@ __device__ __noinline__ void finish_step(IcpState* __restrict__ st, const FF* __
 // and S = sum p q^T - (sum p) mu_q^T in float-float, and runs the Horn
 // solve.  Algebraically this is the reference's two-pass sum; numerically it
 // is more accurate than the reference's float Kahan sums.
-constexpr int kAssocThreads = 512;
 constexpr int kMoments = 17;  // n, p xyz, q xyz, p q^T (9), len^2
-static_assert(kAssocThreads / 32 == kMoments - 1, "one warp per moment after the count");
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+
+// floats as integers of the same order (atomicMin / atomicMax of any sign)
+__device__ __forceinline__ int to_ordered(float f) {
+    const int b = __float_as_int(f);
+    return b >= 0 ? b : b ^ 0x7fffffff;
+}
+__device__ __forceinline__ float from_ordered(int b) { return __int_as_float(b >= 0 ? b : b ^ 0x7fffffff); }
+constexpr float kMaxRange = 4.0f;  // pixels: a target whose points scatter further is searched whole
 
 __device__ __forceinline__ FF two_prod(float a, float b) {
     const float p = fmul(a, b);
@@ -385,34 +565,28 @@ __device__ __forceinline__ FF two_prod(float a, float b) {
 // One AlignStep of one frame pair; `blk` / `nblk`: this CTA's index among
 // the nblk CTAs that work on the pair (the launch's own grid, or a share of
 // a batched launch over several pairs).
-__device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __restrict__ st, unsigned int blk,
-                                              unsigned int nblk) {
-    extern __shared__ float4 stage_mem[];  // three planes of kStagePixels floats
-    const Stage stage{(float*)stage_mem, (float*)stage_mem + kStagePixels, (float*)stage_mem + 2 * kStagePixels};
-    __shared__ int s_box[4];
-    __shared__ float s_hb[kTileCols][32];  // lower half's best len^2 per source
-    __shared__ int s_hi[kTileCols][32];    // and its candidate number
-    __shared__ FF s_acc[kMoments];             // this CTA's moments (index 0 unused: s_count)
-    __shared__ float s_rec[7][kTileCols * 32];  // per source: p xyz, q xyz, len^2 (0 when no pair)
-    __shared__ unsigned int s_count;
+__device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __restrict__ st, bool first,
+                                              unsigned int blk, unsigned int nblk) {
+    static_assert(2 * kTileThreads / 32 == kMoments - 1, "two moments after the count per warp");
+    __shared__ SearchSmem ss;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // Steps are launched programmatically behind one another: this grid may
     // start while the previous step's last CTA still updates the pose.  Wait
     // for that grid (and its memory) before touching the ICP state.
     const int n_cols = (a.width + 3) / 4;
     const int tiles_x = (n_cols + kTileCols - 1) / kTileCols;
-    const int tiles_y = (a.height + kTileRows - 1) / kTileRows;
+    const int tiles = tiles_x * ((a.height + kTileRows - 1) / kTileRows);
     const size_t n_synth = (size_t)a.synth_w * a.synth_h;
-    // While the previous step may still be finishing: stage the box this
-    // CTA's first tile covered then, plus a margin -- windows move little
-    // between steps.  The box is read by one thread (it may be stale or
-    // half-updated; any box is only a guess) and shared, so every thread
-    // stages the same region; after the wait the guess is used only if it
-    // holds every window.
-    __shared__ int s_pred[4];
+    // While the previous step may still be finishing: stage the box that the
+    // tile searched then, plus a margin -- little moves between steps.  The
+    // box is read by one thread (it may be stale or half-updated; any box is
+    // only a guess) and shared, so every thread stages the same region; after
+    // the wait the guess is used if it holds every projection with a margin.
+    const int tile0 = (int)blk;
     if (threadIdx.x == 0) {
         int p[4] = {0, 0, 0, 0};
-        if (blk < tiles_x * tiles_y) {
-            const volatile int* tb = st->tile_box + 4 * blk;
+        if (!first && tile0 < tiles && tile0 < kIcpMaxCtas) {  // (the first step's windows are searched widely)
+            const volatile int* tb = st->tile_box + 4 * tile0;
             const int b0 = tb[0], b1 = tb[1], b2 = tb[2], b3 = tb[3];
             if (b2 > b0 && b3 > b1 && b0 >= 0 && b1 >= 0) {
                 const int x0 = max(b0 - kPredMargin, 0), y0 = max(b1 - kPredMargin, 0);
@@ -425,214 +599,228 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
                 }
             }
         }
-        s_pred[0] = p[0];
-        s_pred[1] = p[1];
-        s_pred[2] = p[2];
-        s_pred[3] = p[3];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            ss.pred[k] = p[k];
+            ss.box[k] = ss.cbox[k] = k < 2 ? 0x7fffffff : -1;
+        }
+        ss.n_items = ss.count = 0u;
     }
+    if (threadIdx.x < kMoments) ss.acc[threadIdx.x] = FF{0.0f, 0.0f};
     __syncthreads();
-    const int px0 = s_pred[0], py0 = s_pred[1], pw = s_pred[2], ph = s_pred[3];
-    if (pw > 0) stage_region(stage, a.synth, n_synth, a.synth_w, px0, py0, pw, ph, stage_pitch(pw));
-    // this thread's source of the first tile in eye space (no pose needed yet)
-    const int lane0 = threadIdx.x & 31, wcol0 = (threadIdx.x >> 5) >> 1;
+    const int px0 = ss.pred[0], py0 = ss.pred[1], pw = ss.pred[2], ph = ss.pred[3];
+    if (pw > 0) stage_region(stage_all, a.synth, n_synth, a.synth_w, px0, py0, pw, ph, stage_pitch(pw));
+    // this thread's depth and last winner (a hint: it may be older, any pixel will do)
     float pre_d = 0.0f;
-    {
-        const int t0 = blk;
-        if (t0 < tiles_x * tiles_y) {
-            const int col = (t0 % tiles_x) * kTileCols + wcol0, y = (t0 / tiles_x) * kTileRows + lane0;
-            if (col < n_cols && y < a.height) pre_d = load_depth(a.depth, (size_t)y * a.width + col * 4, a.depth_u16);
+    unsigned int pre_hint = ~0u;
+    if (tile0 < tiles) {
+        const int col = (tile0 % tiles_x) * kTileCols + warp, y = (tile0 / tiles_x) * kTileRows + lane;
+        if (col < n_cols && y < a.height) {
+            pre_d = load_depth(a.depth, (size_t)y * a.width + col * 4, a.depth_u16);
+            if (!first) pre_hint = __ldcg(a.winner + (size_t)y * n_cols + col);
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wcol = warp >> 1, half = warp & 1;
     const float half_w = fmul((float)a.synth_w, 0.5f), half_h = fmul((float)a.synth_h, 0.5f);
-    if (threadIdx.x < kMoments) s_acc[threadIdx.x] = FF{0.0f, 0.0f};
-    if (threadIdx.x == 0) s_count = 0u;
+    Prune pr;
+    pr.kx = a.kx;
+    pr.ky = a.ky;
+    pr.eps = a.eps;
+    pr.eps0 = a.eps0;
+    pr.w_min = a.w_min;
+    pr.lo_x = a.lo[0];
+    pr.hi_x = a.hi[0];
+    pr.lo_y = a.lo[1];
+    pr.hi_y = a.hi[1];
+    pr.on = a.prune != kPruneOff;
+    if (a.prune == kPruneMeasured) {  // measured by k_target_range before the first step
+        pr.lo_x = from_ordered(st->range[0]);
+        pr.hi_x = from_ordered(st->range[1]);
+        pr.lo_y = from_ordered(st->range[2]);
+        pr.hi_y = from_ordered(st->range[3]);
+        // (an empty target leaves lo > hi: nothing to find either way); within 2% of
+        // their pixels, so that kx and ky, taken over 105% of the image, hold
+        pr.on = pr.hi_x - pr.lo_x <= kMaxRange && pr.hi_y - pr.lo_y <= kMaxRange &&
+                pr.lo_x >= -0.02f * a.synth_w && pr.hi_x <= 1.0f + 0.02f * a.synth_w &&
+                pr.lo_y >= -0.02f * a.synth_h && pr.hi_y <= 1.0f + 0.02f * a.synth_h;
+    }
     if (threadIdx.x == 0) atomicMin(&st->t_start, global_ns());
-    for (int tile = blk; tile < tiles_x * tiles_y; tile += nblk) {
-        const int tx = tile % tiles_x, ty = tile / tiles_x;
-        const int col = tx * kTileCols + wcol, y = ty * kTileRows + lane;
+    float pose[16];  // four 16-byte loads of the new pose
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 c = reinterpret_cast<const float4*>(st->pose_f)[i];
+        pose[4 * i] = c.x; pose[4 * i + 1] = c.y; pose[4 * i + 2] = c.z; pose[4 * i + 3] = c.w;
+    }
+    for (int tile = (int)blk; tile < tiles; tile += (int)nblk) {
+        const bool ahead = tile == tile0;  // its region, depths and hints were loaded above
+        const int col = (tile % tiles_x) * kTileCols + warp, y = (tile / tiles_x) * kTileRows + lane;
         const bool mine = col < n_cols && y < a.height;
         float wp[4] = {0.f, 0.f, 0.f, 0.f};
-        int u = 0, v = 0, nr = 0, nc = 0;
+        float X = 0.f, Y = 0.f, w = 0.f;
+        unsigned int hint = ~0u;
+        if (ahead) hint = pre_hint;
+        else if (mine && !first) hint = a.winner[(size_t)y * n_cols + col];
+        int u = 0, v = 0, nr = 0, nc = 0, cc = 0, cr = 0;
         if (mine) {
             const int x = col * 4;
-            const float d = tile == (int)blk ? pre_d : load_depth(a.depth, (size_t)y * a.width + x, a.depth_u16);
+            const float d = ahead ? pre_d : load_depth(a.depth, (size_t)y * a.width + x, a.depth_u16);
             if (0.0f != d) {
                 float pt[4], cl[4];
                 pt[0] = fmul(fadd(fmul((float)x, a.fl_inv_x), a.pp_x), d);
                 pt[1] = fmul(fadd(fmul(-(float)y, a.fl_inv_y), a.pp_y), d);
                 pt[2] = fmul(fadd(fmul(-1.0f, 1.0f), 0.0f), d);
                 pt[3] = 1.0f;
-                mat_vec(st->pose_f, pt, wp);
+                mat_vec(pose, pt, wp);
                 mat_vec(a.proj, wp, cl);
                 const float ux = fdiv(cl[0], cl[3]), uy = fdiv(cl[1], cl[3]);
-                u = wrap_sub(cvt_i32_x86(fadd(fmul(ux, half_w), half_w)), 10);
-                v = wrap_sub(wrap_sub(a.synth_h - 1, cvt_i32_x86(fadd(fmul(uy, half_h), half_h))), 10);
-                u = max(0, u);
-                v = max(0, v);
+                X = fadd(fmul(ux, half_w), half_w);
+                Y = fadd(fmul(uy, half_h), half_h);
+                w = cl[3];
+                const int cx = cvt_i32_x86(X), cy = wrap_sub(a.synth_h - 1, cvt_i32_x86(Y));
+                u = max(0, wrap_sub(cx, 10));
+                v = max(0, wrap_sub(cy, 10));
                 nr = (int)min(480ll, (long long)v + 21) - v;
                 nc = (int)min(640ll, (long long)u + 21) - u;
                 if (nr <= 0 || nc <= 0) nr = nc = 0;
+                cc = wrap_sub(cx, u);
+                cr = wrap_sub(cy, v);
             }
         }
-        // bounding box of the tile's windows
-        if (threadIdx.x == 0) {
-            s_box[0] = 0x7fffffff; s_box[1] = 0x7fffffff; s_box[2] = -1; s_box[3] = -1;
-        }
-        __syncthreads();
-        if (half == 0) {  // warp-uniform; one shared atomic per warp and bound
+        stage_wait();  // the region staged ahead
+        {  // the projections inside their windows; one shared atomic per warp and bound
             const bool has = nr > 0;
-            const int mu0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)u : 0x7fffffffu);
-            const int mv0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)v : 0x7fffffffu);
-            const int mu1 = __reduce_max_sync(0xffffffffu, has ? u + nc : -1);
-            const int mv1 = __reduce_max_sync(0xffffffffu, has ? v + nr : -1);
+            const int px = min(max(cc, 0), nc - 1) + u, py = min(max(cr, 0), nr - 1) + v;
+            const int mu0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)px : 0x7fffffffu);
+            const int mv0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)py : 0x7fffffffu);
+            const int mu1 = __reduce_max_sync(0xffffffffu, has ? px + 1 : -1);
+            const int mv1 = __reduce_max_sync(0xffffffffu, has ? py + 1 : -1);
             if (lane == 0 && mu1 >= 0) {
-                atomicMin(&s_box[0], mu0);
-                atomicMin(&s_box[1], mv0);
-                atomicMax(&s_box[2], mu1);
-                atomicMax(&s_box[3], mv1);
+                atomicMin(&ss.cbox[0], mu0);
+                atomicMin(&ss.cbox[1], mv0);
+                atomicMax(&ss.cbox[2], mu1);
+                atomicMax(&ss.cbox[3], mv1);
             }
         }
         __syncthreads();
-        const int ax0 = s_box[0], ay0 = s_box[1], ax1 = s_box[2], ay1 = s_box[3];
-        // the prefetched region if it holds every window of the tile, else stage the box now
-        const bool use_pred = tile == (int)blk && pw > 0 && ax1 >= 0 && ax0 >= px0 && ay0 >= py0 &&
-                              ax1 <= px0 + pw && ay1 <= py0 + ph;
-        int bx0 = ax0, by0 = ay0, pitch = stage_pitch(ax1 - ax0);
-        bool staged;
-        if (use_pred) {
-            bx0 = px0;
-            by0 = py0;
-            pitch = stage_pitch(pw);
-            staged = true;
-        } else {
-            staged = ax1 >= 0 && pitch * (ay1 - ay0) <= kStagePixels;
-            if (staged) stage_region(stage, a.synth, n_synth, a.synth_w, ax0, ay0, ax1 - ax0, ay1 - ay0, pitch);
+        const int ax0 = ss.cbox[0], ay0 = ss.cbox[1], ax1 = ss.cbox[2], ay1 = ss.cbox[3];
+        // the region staged ahead if it holds every projection of the tile with a
+        // margin, else the projections with as much of the windows around them as fits
+        Region reg{0, 0, 0, 0, 0, 1};
+        if (ahead && pw > 0 && max(ax0 - kUseMargin, 0) >= px0 && max(ay0 - kUseMargin, 0) >= py0 &&
+            min(ax1 + kUseMargin, 640) <= px0 + pw && min(ay1 + kUseMargin, 480) <= py0 + ph) {
+            reg = Region{0, px0, py0, px0 + pw, py0 + ph, stage_pitch(pw)};
+        } else if (ax1 >= 0) {
+            for (int m = 10; m >= 0; m -= m > 4 ? 3 : 1) {
+                const int x0 = max(ax0 - m, 0), y0 = max(ay0 - m, 0);
+                const int w0 = min(ax1 + m, 640) - x0, h0 = min(ay1 + m, 480) - y0;
+                if (stage_pitch(w0) * h0 > kStagePixels) continue;
+                reg = Region{0, x0, y0, x0 + w0, y0 + h0, stage_pitch(w0)};
+                stage_region(stage_all, a.synth, n_synth, a.synth_w, x0, y0, w0, h0, reg.pitch);
+                stage_wait();
+                __syncthreads();
+                break;
+            }
         }
-        if (threadIdx.x == 0 && tile < kIcpMaxCtas && ax1 >= 0) {
+        int hr = (int)(hint >> 16) - v, hc = (int)(hint & 0xffffu) - u;
+        if ((unsigned)hr >= (unsigned)nr || (unsigned)hc >= (unsigned)nc) hr = hc = -1;
+        bool listed = false;
+        unsigned long long key = search_own(a, reg, nr, nc, cr, cc, hr, hc, first, u, v, X, Y, w, pr, wp, ss, listed);
+        __syncthreads();
+        const unsigned int n_items = ss.n_items;
+        if (threadIdx.x == 0 && tile < kIcpMaxCtas && ss.box[2] >= 0) {
             int* tb = st->tile_box + 4 * tile;
-            tb[0] = ax0;
-            tb[1] = ay0;
-            tb[2] = ax1;
-            tb[3] = ay1;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) tb[k] = ss.box[k];
         }
-        __syncthreads();
-        // this thread's rows of the window
-        const int r0 = half ? kSplitRow : 0, r1 = half ? nr : min(nr, kSplitRow);
-        float best = 0.01f;
-        int rc = -1;
-        float3 bq = make_float3(0.f, 0.f, 0.f);
-        if (r1 > r0) {
-            const float dw = fsub(1.0f, wp[3]);
-            const float dw2 = fmul(dw, dw);
-            if (staged) {
-                const int base = (v + r0 - by0) * pitch + (u - bx0);
-                // dz^2 + dw^2 == dz^2 exactly when dw == 0 (dz^2 >= 0)
-                best = dw2 != 0.0f
-                           ? scan_staged<true>(stage, base, pitch, r1 - r0, nc, wp[0], wp[1], wp[2], dw2,
-                                               a.neg_zero, &rc)
-                           : scan_staged<false>(stage, base, pitch, r1 - r0, nc, wp[0], wp[1], wp[2], dw2,
-                                                a.neg_zero, &rc);
-                if (rc >= 0) {
-                    const int at = base + (rc >> 5) * pitch + (rc & 31);
-                    bq = make_float3(stage.x[at], stage.y[at], stage.z[at]);
-                    rc += r0 * 32;
-                }
-            } else {
-                for (int r = r0; r < r1; ++r) {
-                    for (int c = 0; c < nc; ++c) {
-                        const size_t at = (size_t)(v + r) * a.synth_w + (u + c);
-                        if (at >= n_synth) continue;
-                        const float4 q = __ldg(a.synth + at);
-                        if (q.x == 0.0f && q.y == 0.0f && q.z == 0.0f) continue;
-                        const float dx = fsub(q.x, wp[0]), dy = fsub(q.y, wp[1]), dz = fsub(q.z, wp[2]);
-                        const float l2 = fadd(fadd(fmul(dx, dx), fmul(dy, dy)), fadd(fmul(dz, dz), dw2));
-                        if (l2 < best) {
-                            best = l2;
-                            rc = r * 32 + c;
-                            bq = make_float3(q.x, q.y, q.z);
-                        }
-                    }
-                }
-            }
+        if (n_items) {
+            search_items(a.synth, n_items, a.neg_zero, ss);
+            __syncthreads();
+            if (listed) key = ss.list.key[threadIdx.x];
+            __syncthreads();  // the records take the list's place
         }
-        // merge the halves: the upper rows come earlier in scan order
-        if (half == 1) {
-            s_hb[wcol][lane] = best;
-            s_hi[wcol][lane] = rc;
+        const bool hit = mine && key < kNoPair;
+        const float best = __uint_as_float((unsigned int)(key >> 32));
+        const int rc = (int)(unsigned int)key;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (hit) {
+            const int x = u + (rc & 31), yy = v + (rc >> 5);
+            q = reg.holds(x, yy, 1, 1) ? stage_all[reg.at(x, yy)] : __ldg(a.synth + (size_t)yy * a.synth_w + x);
         }
-        __syncthreads();
-        if (half == 0) {
-            const float ob = s_hb[wcol][lane];
-            const int oi = s_hi[wcol][lane];
-            if (oi >= 0 && (rc < 0 || ob < best)) {
-                best = ob;
-                rc = oi;
-                if (staged) {
-                    const int at = (v + (oi >> 5) - by0) * pitch + (u + (oi & 31) - bx0);
-                    bq = make_float3(stage.x[at], stage.y[at], stage.z[at]);
-                } else {
-                    const float4 q = __ldg(a.synth + (size_t)(v + (oi >> 5)) * a.synth_w + (u + (oi & 31)));
-                    bq = make_float3(q.x, q.y, q.z);
-                }
-            }
-            const bool hit = mine && rc >= 0;
-            if (a.pairs && mine) {
-                const size_t k = (size_t)y * n_cols + col;
-                a.pairs[k] = hit ? (long long)(v + (rc >> 5)) * a.synth_w + (u + (rc & 31)) : -1ll;
-                a.pairs_len2[k] = hit ? best : 0.01f;
-            }
-            // this source's pair for the tile's moments (zeros when none)
-            const int sidx = wcol * 32 + lane;
-            s_rec[0][sidx] = hit ? wp[0] : 0.f;
-            s_rec[1][sidx] = hit ? wp[1] : 0.f;
-            s_rec[2][sidx] = hit ? wp[2] : 0.f;
-            s_rec[3][sidx] = hit ? bq.x : 0.f;
-            s_rec[4][sidx] = hit ? bq.y : 0.f;
-            s_rec[5][sidx] = hit ? bq.z : 0.f;
-            s_rec[6][sidx] = hit ? best : 0.f;
+        if (mine) a.winner[(size_t)y * n_cols + col] = hit ? (unsigned int)(v + (rc >> 5)) << 16 | (u + (rc & 31)) : ~0u;
+        if (a.pairs && mine) {
+            const size_t k = (size_t)y * n_cols + col;
+            a.pairs[k] = hit ? (long long)(v + (rc >> 5)) * a.synth_w + (u + (rc & 31)) : -1ll;
+            a.pairs_len2[k] = hit ? best : 0.01f;
+        }
+        // this source's pair for the tile's moments (zeros when none)
+        {
+            const int sidx = threadIdx.x;
+            ss.rec[0][sidx] = hit ? wp[0] : 0.f;
+            ss.rec[1][sidx] = hit ? wp[1] : 0.f;
+            ss.rec[2][sidx] = hit ? wp[2] : 0.f;
+            ss.rec[3][sidx] = q.x;
+            ss.rec[4][sidx] = q.y;
+            ss.rec[5][sidx] = q.z;
+            ss.rec[6][sidx] = hit ? best : 0.f;
             const unsigned int nh = __popc(__ballot_sync(0xffffffffu, hit));
-            if (lane == 0 && nh) atomicAdd(&s_count, nh);
+            if (lane == 0 && nh) atomicAdd(&ss.count, nh);
         }
         __syncthreads();
-        // the tile's raw moments: warp w reduces moment w + 1 over the 256
+        if (threadIdx.x == 0) {  // for the next tile
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ss.box[k] = ss.cbox[k] = k < 2 ? 0x7fffffff : -1;
+            ss.n_items = 0u;
+        }
+        // the tile's raw moments: each warp reduces two of the 16 over all
         // sources (lane l takes sources l, l + 32, ...), in float-float
         {
-            const int c = warp + 1;
-            FF acc{0.0f, 0.0f};
+            constexpr int kPer = 2;
+            FF acc[kPer];
 #pragma unroll
-            for (int k = 0; k < kTileCols; ++k) {
-                const int sidx = lane + 32 * k;
-                FF m;
-                if (c < 7) m = FF{s_rec[c - 1][sidx], 0.0f};
-                else if (c < 16) m = two_prod(s_rec[(c - 7) / 3][sidx], s_rec[3 + (c - 7) % 3][sidx]);
-                else m = FF{s_rec[6][sidx], 0.0f};
-                acc = ff_add(acc, m);
+            for (int h = 0; h < kPer; ++h) {
+                const int c = warp + 1 + 8 * h;
+                acc[h] = FF{0.0f, 0.0f};
+#pragma unroll
+                for (int k = 0; k < kTileCols; ++k) {
+                    const int sidx = lane + 32 * k;
+                    FF m;
+                    if (c < 7) m = FF{ss.rec[c - 1][sidx], 0.0f};
+                    else if (c < 16) m = two_prod(ss.rec[(c - 7) / 3][sidx], ss.rec[3 + (c - 7) % 3][sidx]);
+                    else m = FF{ss.rec[6][sidx], 0.0f};
+                    acc[h] = ff_add(acc[h], m);
+                }
             }
-            acc = warp_sum_ff(acc);
-            if (lane == 0) s_acc[c] = ff_add(s_acc[c], acc);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)  // the trees side by side
+#pragma unroll
+                for (int h = 0; h < kPer; ++h) {
+                    const FF x{__shfl_xor_sync(0xffffffffu, acc[h].hi, o), __shfl_xor_sync(0xffffffffu, acc[h].lo, o)};
+                    acc[h] = ff_add(acc[h], x);
+                }
+            if (lane < kPer) {
+                const int c = warp + 1 + 8 * lane;
+                ss.acc[c] = ff_add(ss.acc[c], lane ? acc[kPer - 1] : acc[0]);
+            }
         }
-        __syncthreads();  // staging buffer, half results and records are reused by the next tile
+        __syncthreads();  // staging buffer and records are reused by the next tile
     }
     // association done: the next step's grid may be scheduled (it waits above)
     asm volatile("griddepcontrol.launch_dependents;");
     if (threadIdx.x >= 1 && threadIdx.x < kMoments) {
-        const FF t = s_acc[threadIdx.x];
+        const FF t = ss.acc[threadIdx.x];
         st->part[(size_t)(2 * threadIdx.x) * kIcpMaxCtas + blk] = t.hi;
         st->part[(size_t)(2 * threadIdx.x + 1) * kIcpMaxCtas + blk] = t.lo;
     }
     if (threadIdx.x == 0) atomicMax(&st->t_body, global_ns());
     unsigned int n_total;
-    if (!last_cta(&st->done, s_count, &n_total, nblk)) return;
+    if (!last_cta(&st->done, ss.count, &n_total, nblk)) return;
     __shared__ FF tot[kMoments];
     moments_total<kMoments>(st, n_total, tot, (int)nblk);
     if (threadIdx.x < 32) finish_step(st, tot, a.mail, a.mail_seq);
 }
 
-__global__ void __launch_bounds__(kAssocThreads, 2) k_icp_step(IcpArgs a, IcpState* __restrict__ st) {
-    icp_step_body(a, st, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(kTileThreads, 2) k_icp_step(IcpArgs a, IcpState* __restrict__ st, bool first) {
+    icp_step_body(a, st, first, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------- Horn solve
@@ -818,6 +1006,16 @@ __device__ __noinline__ void finish_step(IcpState* __restrict__ st, const FF* __
         t_start = __ldcg(&st->t_start);
         t_body = __ldcg(&st->t_body);
     }
+    const int pk = lane < 12 ? lane : 0, pc = pk / 3, pr = pk - 3 * pc;  // the pose entry it will update ...
+    FF P[4];                                                            // ... and its column, likewise read now
+    {
+        const float4 hi = __ldcg(reinterpret_cast<const float4*>(st->pose_f) + pc);
+        const float4 lo = __ldcg(reinterpret_cast<const float4*>(st->pose_lo) + pc);
+        P[0] = FF{hi.x, lo.x};
+        P[1] = FF{hi.y, lo.y};
+        P[2] = FF{hi.z, lo.z};
+        P[3] = FF{hi.w, lo.w};
+    }
     // 1. centroids (lanes 0-5), S (lanes 0-8), N (lanes 0-9) in FF
     const float n = fadd(tot[0].hi, tot[0].lo);  // an exact count below 2^24
     FF my_mu{0.0f, 0.0f};
@@ -973,10 +1171,6 @@ __device__ __noinline__ void finish_step(IcpState* __restrict__ st, const FF* __
     const FF my_t = mud - (shfl_ff(my_r, 3 * tr3) * mu0 + shfl_ff(my_r, 3 * tr3 + 1) * mu1 +
                            shfl_ff(my_r, 3 * tr3 + 2) * mu2);
     // pose <- [R t; 0 1] pose (:259-263, :20-28): lane k < 12 takes row r = k % 3 of column c = k / 3
-    const int pk = lane < 12 ? lane : 0, pc = pk / 3, pr = pk - 3 * pc;
-    FF P[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) P[i] = FF{st->pose_f[4 * pc + i], st->pose_lo[4 * pc + i]};
     const FF v = shfl_ff(my_r, 3 * pr) * P[0] + shfl_ff(my_r, 3 * pr + 1) * P[1] + shfl_ff(my_r, 3 * pr + 2) * P[2] +
                  shfl_ff(my_t, pr) * P[3];
     __syncwarp();  // every lane has read its column before any entry is replaced
@@ -1025,6 +1219,8 @@ __device__ __forceinline__ void icp_begin_body(IcpState* st, const Mat4& guess) 
         st->pose_lo[i] = 0.0f;
     }
     st->iter = 0;
+    st->range[0] = st->range[2] = to_ordered(INFINITY);
+    st->range[1] = st->range[3] = to_ordered(-INFINITY);
     st->done = 0ull;
     st->t_start = ~0ull;
     st->t_body = 0ull;
@@ -1035,41 +1231,124 @@ __global__ void k_icp_begin(IcpState* st, Mat4 guess) {
     icp_begin_body(st, guess);
 }
 
+// Where the points of a caller's target project within their pixels: the
+// smallest and largest X(q) - x and Y(q) - (H - 1 - y) over the points in
+// front of the eye (a point nearer than w_far to the eye plane, or behind
+// it, is further than 0.1 m from every source that prunes).
+__global__ void __launch_bounds__(kThreads) k_target_range(IcpArgs a, float w_far, IcpState* __restrict__ st) {
+    const int n = a.synth_w * a.synth_h;
+    const float hw = fmul((float)a.synth_w, 0.5f), hh = fmul((float)a.synth_h, 0.5f);
+    float lx = INFINITY, hx = -INFINITY, ly = INFINITY, hy = -INFINITY;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 q = __ldg(a.synth + i);
+        const float p[4] = {q.x, q.y, q.z, 1.0f};
+        float c[4];
+        mat_vec(a.proj, p, c);
+        if (!(isfinite(q.x) && isfinite(q.y) && isfinite(q.z)) || !(c[3] > w_far)) continue;
+        const int y = i / a.synth_w, x = i - y * a.synth_w;
+        const float dx = c[0] / c[3] * hw + hw - (float)x;
+        const float dy = c[1] / c[3] * hh + hh - (float)(a.synth_h - 1 - y);
+        lx = fminf(lx, dx);
+        hx = fmaxf(hx, dx);
+        ly = fminf(ly, dy);
+        hy = fmaxf(hy, dy);
+    }
+    int r[4] = {to_ordered(lx), to_ordered(hx), to_ordered(ly), to_ordered(hy)};
+    r[0] = __reduce_min_sync(0xffffffffu, r[0]);
+    r[1] = __reduce_max_sync(0xffffffffu, r[1]);
+    r[2] = __reduce_min_sync(0xffffffffu, r[2]);
+    r[3] = __reduce_max_sync(0xffffffffu, r[3]);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&st->range[0], r[0]);
+        atomicMax(&st->range[1], r[1]);
+        atomicMin(&st->range[2], r[2]);
+        atomicMax(&st->range[3], r[3]);
+    }
+}
+
+// The target's producers walk it in blocks of 8 x 4 pixels, a warp each (lane
+// 8 r + c: the block's row r and column c), so that a block's bounding box is
+// six warp reductions.
+struct TargetPixel {
+    int x, y, block;
+    bool in;  // inside the target (blocks at its edges stick out)
+};
+__device__ __forceinline__ TargetPixel target_pixel(int block, int width, int height) {
+    const int nbx = (width + kBlockW - 1) / kBlockW, by = block / nbx, lane = threadIdx.x & 31;
+    TargetPixel t;
+    t.x = (block - by * nbx) * kBlockW + (lane & 7);
+    t.y = by * kBlockH + (lane >> 3);
+    t.block = block;
+    t.in = t.x < width && t.y < height;
+    return t;
+}
+__device__ __forceinline__ int target_blocks(int width, int height) {
+    return ((width + kBlockW - 1) / kBlockW) * ((height + kBlockH - 1) / kBlockH);
+}
+
+// Writes a target point as the association reads it -- (0,0,0) is no point
+// (ICP.cpp:112) and gets x = NaN, which no distance test passes -- and, by
+// the whole warp, its block's bounding box (inverted where there is no point).
+__device__ __forceinline__ void put_target(const TargetPixel& t, float x, float y, float z, int width,
+                                           float4* __restrict__ out, float4* __restrict__ boxes) {
+    const bool point = t.in && !(x == 0.0f && y == 0.0f && z == 0.0f);
+    if (t.in) out[(size_t)t.y * width + t.x] = make_float4(point ? x : __int_as_float(0x7fffffff), y, z, 1.0f);
+    // a point with a NaN is nearest to nothing; infinite ones leave a box that excludes nothing wrongly
+    const bool use = point && x == x && y == y && z == z;
+    const float big = INFINITY;
+    const float lx = from_ordered(__reduce_min_sync(0xffffffffu, to_ordered(use ? x : big)));
+    const float ly = from_ordered(__reduce_min_sync(0xffffffffu, to_ordered(use ? y : big)));
+    const float lz = from_ordered(__reduce_min_sync(0xffffffffu, to_ordered(use ? z : big)));
+    const float hx = from_ordered(__reduce_max_sync(0xffffffffu, to_ordered(use ? x : -big)));
+    const float hy = from_ordered(__reduce_max_sync(0xffffffffu, to_ordered(use ? y : -big)));
+    const float hz = from_ordered(__reduce_max_sync(0xffffffffu, to_ordered(use ? z : -big)));
+    if ((threadIdx.x & 31) == 0) {
+        boxes[2 * (size_t)t.block] = make_float4(lx, ly, lz, 0.0f);
+        boxes[2 * (size_t)t.block + 1] = make_float4(hx, hy, hz, 0.0f);
+    }
+}
+
 // World points of a depth frame: the back-projection of
 // DepthMap2PointCloud (Integrator.cpp:121-144) without the voxel step;
 // pixels without depth get (0,0,0), the reference's "invalid" target value.
 __device__ __forceinline__ void backproject_body(const void* __restrict__ depth, int u16, int width, int height,
                                                  float fl_inv_x, float fl_inv_y, float pp_x, float pp_y,
-                                                 const Mat4& e2w, float4* __restrict__ out, unsigned int blk,
-                                                 unsigned int nblk) {
-    const int n = width * height;
-    for (int i = blk * blockDim.x + threadIdx.x; i < n; i += nblk * blockDim.x) {
-        const int v = i / width, u = i - v * width;
-        const float d = load_depth(depth, i, u16 != 0);
+                                                 const Mat4& e2w, float4* __restrict__ out,
+                                                 float4* __restrict__ boxes, unsigned int blk, unsigned int nblk) {
+    const int n = target_blocks(width, height), warps = blockDim.x >> 5;
+    for (int b = blk * warps + (threadIdx.x >> 5); b < n; b += nblk * warps) {
+        const TargetPixel t = target_pixel(b, width, height);
+        const float d = t.in ? load_depth(depth, (size_t)t.y * width + t.x, u16 != 0) : 0.0f;
         float w[4] = {0.f, 0.f, 0.f, 0.f};
         if (d > 0.0f) {
             float p[4];
-            p[0] = fadd(fmul(fadd(fmul((float)u, fl_inv_x), pp_x), d), 0.0f);
-            p[1] = fadd(fmul(fadd(fmul(fadd(0.0f, -(float)v), fl_inv_y), pp_y), d), 0.0f);
+            p[0] = fadd(fmul(fadd(fmul((float)t.x, fl_inv_x), pp_x), d), 0.0f);
+            p[1] = fadd(fmul(fadd(fmul(fadd(0.0f, -(float)t.y), fl_inv_y), pp_y), d), 0.0f);
             p[2] = fadd(fmul(fadd(fmul(-1.0f, 1.0f), 0.0f), d), 0.0f);
             p[3] = fadd(fmul(fadd(fmul(0.0f, 1.0f), 0.0f), d), 1.0f);
             mat_vec(e2w.m, p, w);
         }
-        out[i] = make_float4(w[0], w[1], w[2], 0.0f);
+        put_target(t, w[0], w[1], w[2], width, out, boxes);
     }
 }
 
 __global__ void k_backproject(const void* __restrict__ depth, int u16, int width, int height,
                               float fl_inv_x, float fl_inv_y, float pp_x, float pp_y, Mat4 e2w,
-                              float4* __restrict__ out) {
-    backproject_body(depth, u16, width, height, fl_inv_x, fl_inv_y, pp_x, pp_y, e2w, out, blockIdx.x, gridDim.x);
+                              float4* __restrict__ out, float4* __restrict__ boxes) {
+    backproject_body(depth, u16, width, height, fl_inv_x, fl_inv_y, pp_x, pp_y, e2w, out, boxes, blockIdx.x,
+                     gridDim.x);
 }
 
 // host float3 target -> the float4 layout the association reads (one
 // 16-byte load per candidate)
-__global__ void k_expand_target(const float* __restrict__ in, int n, float4* __restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = make_float4(in[3 * i], in[3 * i + 1], in[3 * i + 2], 0.0f);
+__global__ void k_expand_target(const float* __restrict__ in, int width, int height, float4* __restrict__ out,
+                                float4* __restrict__ boxes) {
+    const int n = target_blocks(width, height), warps = blockDim.x >> 5;
+    for (int b = blockIdx.x * warps + (threadIdx.x >> 5); b < n; b += gridDim.x * warps) {
+        const TargetPixel t = target_pixel(b, width, height);
+        const size_t i = t.in ? (size_t)t.y * width + t.x : 0;
+        put_target(t, in[3 * i], in[3 * i + 1], in[3 * i + 2], width, out, boxes);
+    }
 }
 
 // Renderer::Bin: a z-buffered splat.  The first point (in input order) with
@@ -1120,43 +1399,56 @@ __global__ void k_icp_begin_batch(const IcpJob* __restrict__ jobs, int n) {
     if (v < n) icp_begin_body(jobs[v].st, jobs[v].guess);
 }
 
-__global__ void __launch_bounds__(kAssocThreads, 2) k_icp_step_batch(const IcpJob* __restrict__ jobs, BlockMap m) {
+__global__ void __launch_bounds__(kTileThreads, 2) k_icp_step_batch(const IcpJob* __restrict__ jobs, BlockMap m,
+                                                                   bool first) {
     const int v = block_owner(m, blockIdx.x);
     const unsigned int b0 = m.first[v];
-    icp_step_body(jobs[v].a, jobs[v].st, blockIdx.x - b0, m.first[v + 1] - b0);
+    icp_step_body(jobs[v].a, jobs[v].st, first, blockIdx.x - b0, m.first[v + 1] - b0);
 }
 
 __global__ void k_backproject_batch(const BackprojectJob* __restrict__ jobs, BlockMap m) {
     const int v = block_owner(m, blockIdx.x);
     const BackprojectJob& j = jobs[v];
     const unsigned int b0 = m.first[v];
-    backproject_body(j.depth, 1, j.width, j.height, j.fl_inv_x, j.fl_inv_y, j.pp_x, j.pp_y, j.e2w, j.out,
+    backproject_body(j.depth, 1, j.width, j.height, j.fl_inv_x, j.fl_inv_y, j.pp_x, j.pp_y, j.e2w, j.out, j.boxes,
                      blockIdx.x - b0, m.first[v + 1] - b0);
 }
 
 // the same resolve into the association's float4 target layout
 __global__ void k_bin_resolve_target(const float* __restrict__ pts, const unsigned long long* __restrict__ zbuf,
-                                     int n_pix, float4* __restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_pix; i += gridDim.x * blockDim.x) {
-        const unsigned long long z = zbuf[i];
-        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+                                     int width, int height, float4* __restrict__ out, float4* __restrict__ boxes) {
+    const int n = target_blocks(width, height), warps = blockDim.x >> 5;
+    for (int b = blockIdx.x * warps + (threadIdx.x >> 5); b < n; b += gridDim.x * warps) {
+        const TargetPixel t = target_pixel(b, width, height);
+        const unsigned long long z = t.in ? zbuf[(size_t)t.y * width + t.x] : ~0ull;
+        float x = 0.f, y = 0.f, w = 0.f;
         if (z != ~0ull) {
             const unsigned int j = (unsigned int)(z & 0xffffffffu);
-            o = make_float4(pts[3 * j], pts[3 * j + 1], pts[3 * j + 2], 0.f);
+            x = pts[3 * (size_t)j];
+            y = pts[3 * (size_t)j + 1];
+            w = pts[3 * (size_t)j + 2];
         }
-        out[i] = o;
+        put_target(t, x, y, w, width, out, boxes);
     }
 }
 
 }  // namespace
 
+// CTAs of one pair's association (its tiles, at most kIcpMaxCtas)
+int icp_tiles(int width, int height) {
+    const int n_cols = (width + 3) / 4;
+    const int tiles = ((n_cols + kTileCols - 1) / kTileCols) * ((height + kTileRows - 1) / kTileRows);
+    return tiles < kIcpMaxCtas ? tiles : kIcpMaxCtas;
+}
+
 cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess, int iterations,
                               int /*ctas*/, cudaStream_t stream, IcpPoseMail* mail, unsigned long long seq) {
     k_icp_begin<<<1, 32, 0, stream>>>(st, guess);
-    const int n_cols = (a.width + 3) / 4;
-    const int tiles = ((n_cols + kTileCols - 1) / kTileCols) * ((a.height + kTileRows - 1) / kTileRows);
-    const int ctas = tiles < kIcpMaxCtas ? tiles : kIcpMaxCtas;
-    const size_t smem = 3 * kStagePixels * sizeof(float);
+    if (a.prune == kPruneMeasured && iterations > 0)
+        k_target_range<<<(a.synth_w * a.synth_h + kThreads * 4 - 1) / (kThreads * 4), kThreads, 0, stream>>>(
+            a, a.w_min * 0.125f, st);
+    const int ctas = icp_tiles(a.width, a.height);
+    const size_t smem = kStagePixels * sizeof(float4);
     // programmatic dependent launch: each step's grid is scheduled as soon as
     // every CTA of the one before has finished its association, overlapping
     // its launch with the previous finisher (k_icp_step waits for it)
@@ -1165,7 +1457,7 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(kAssocThreads);
+    cfg.blockDim = dim3(kTileThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;
@@ -1176,7 +1468,7 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
     IcpArgs other = a;
     other.mail = nullptr;
     for (int it = 0; it < iterations; ++it) {
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_icp_step, it + 1 == iterations ? last : other, st);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_icp_step, it + 1 == iterations ? last : other, st, it == 0);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
@@ -1186,10 +1478,10 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
 // once per device, outside any stream capture.
 cudaError_t icp_init_device() {
     cudaError_t e = cudaFuncSetAttribute(k_icp_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(3 * kStagePixels * sizeof(float)));
+                                         (int)(kStagePixels * sizeof(float4)));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_icp_step_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(3 * kStagePixels * sizeof(float)));
+                                 (int)(kStagePixels * sizeof(float4)));
     return e;
 }
 
@@ -1197,7 +1489,7 @@ cudaError_t icp_align_batch_enqueue(const IcpJob* jobs, int n, const BlockMap& m
                                     cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     k_icp_begin_batch<<<(n + 63) / 64, 64, 0, stream>>>(jobs, n);
-    const size_t smem = 3 * kStagePixels * sizeof(float);
+    const size_t smem = kStagePixels * sizeof(float4);
     // programmatic dependent launch, as for a single pair: each step's grid
     // is scheduled once every CTA of the step before has finished its association
     cudaLaunchAttribute attr[1];
@@ -1205,13 +1497,13 @@ cudaError_t icp_align_batch_enqueue(const IcpJob* jobs, int n, const BlockMap& m
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(map.grid);
-    cfg.blockDim = dim3(kAssocThreads);
+    cfg.blockDim = dim3(kTileThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     for (int it = 0; it < iterations; ++it) {
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_icp_step_batch, jobs, map);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_icp_step_batch, jobs, map, it == 0);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
@@ -1223,24 +1515,23 @@ cudaError_t backproject_batch_enqueue(const BackprojectJob* jobs, int n, const B
     return cudaGetLastError();
 }
 
-// CTAs of one pair's association (its tiles, at most kIcpMaxCtas)
-int icp_tiles(int width, int height) {
-    const int n_cols = (width + 3) / 4;
-    const int tiles = ((n_cols + kTileCols - 1) / kTileCols) * ((height + kTileRows - 1) / kTileRows);
-    return tiles < kIcpMaxCtas ? tiles : kIcpMaxCtas;
+// float4s of a target's block boxes
+size_t icp_box_count(int width, int height) {
+    return 2 * (size_t)((width + kBlockW - 1) / kBlockW) * ((height + kBlockH - 1) / kBlockH);
 }
 
-cudaError_t expand_target_enqueue(const float* in, int n, float4* out, int ctas, cudaStream_t st) {
-    k_expand_target<<<ctas, kThreads, 0, st>>>(in, n, out);
+cudaError_t expand_target_enqueue(const float* in, int width, int height, float4* out, float4* boxes, int ctas,
+                                  cudaStream_t st) {
+    k_expand_target<<<ctas, kThreads, 0, st>>>(in, width, height, out, boxes);
     return cudaGetLastError();
 }
 
 cudaError_t backproject_enqueue(const void* depth, bool u16, const kifi_camera& cam,
-                                const Mat4& eye_to_world, float4* out, int ctas, cudaStream_t st) {
+                                const Mat4& eye_to_world, float4* out, float4* boxes, int ctas, cudaStream_t st) {
     const float fix = fdiv(1.0f, cam.fx), fiy = fdiv(1.0f, cam.fy);
     const float ppx = fmul(fsub(0.5f, cam.cx), fix), ppy = fmul(fsub(cam.cy, 0.5f), fiy);
     k_backproject<<<ctas, kThreads, 0, st>>>(depth, u16 ? 1 : 0, cam.width, cam.height, fix, fiy,
-                                             ppx, ppy, eye_to_world, out);
+                                             ppx, ppy, eye_to_world, out, boxes);
     return cudaGetLastError();
 }
 
@@ -1254,11 +1545,11 @@ cudaError_t bin_enqueue(const float* pts, unsigned int n, const Mat4& w2c, int w
 }
 
 cudaError_t bin_target_enqueue(const float* pts, unsigned int n, const Mat4& w2c, int width, int height,
-                               unsigned long long* zbuf, float4* out, int ctas, cudaStream_t st) {
+                               unsigned long long* zbuf, float4* out, float4* boxes, int ctas, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(zbuf, 0xff, (size_t)width * height * 8, st);
     if (e) return e;
     if (n) k_bin_splat<<<ctas, kThreads, 0, st>>>(pts, n, w2c, width, height, zbuf);
-    k_bin_resolve_target<<<ctas, kThreads, 0, st>>>(pts, zbuf, width * height, out);
+    k_bin_resolve_target<<<ctas, kThreads, 0, st>>>(pts, zbuf, width, height, out, boxes);
     return cudaGetLastError();
 }
 

@@ -253,14 +253,22 @@ struct IcpPoseMail {
     unsigned long long seq;
 };
 
+constexpr int kPruneOff = 0, kPruneKnown = 1, kPruneMeasured = 2;
+
 struct IcpArgs {
     const void* depth;      // source frame (float metres or uint16 mm)
     int depth_u16;
     int width, height;
     float fl_inv_x, fl_inv_y, pp_x, pp_y;
     float proj[16];         // EyeToClipRH * inverse(synth eye-to-world), kifi order
-    const float4* synth;    // target world points (w unused), synth_w * synth_h
+    const float4* synth;    // target world points (x = NaN: none; w = 1), synth_w * synth_h
     int synth_w, synth_h;
+    const float4* boxes;    // per block of 8 x 4 target pixels (row-major): its points' bounds, lower then upper
+    // which candidates of a window can win (kifi_icp.cu, Prune)
+    int prune;              // kPruneOff, kPruneKnown (lo, hi below) or kPruneMeasured (IcpState::range)
+    float kx, ky, eps, eps0, w_min;
+    float lo[2], hi[2];
+    unsigned int* winner;   // per source: the pixel that won the last step (row << 16 | column), or ~0
     long long* pairs;       // optional: per source the winner's target index (-1: none) ...
     float* pairs_len2;      // ... and its len^2, overwritten by every iteration
     float neg_zero;         // -0.0f, a value the device code cannot see at compile time
@@ -277,12 +285,13 @@ struct IcpIterStats {
 };
 
 struct IcpState {
-    float pose_f[16];   // eye-to-world estimate, kifi order (float-float high part)
+    alignas(16) float pose_f[16];   // eye-to-world estimate, kifi order (float-float high part)
     float pose_lo[16];  // and its low part
     unsigned long long done;  // CTAs finished (high 32 bits) and their associations (low 32 bits)
     float mu_s[4], mu_d[4];
     int n_assoc;
     int iter;
+    int range[4];  // kPruneMeasured: the target's lo x, hi x, lo y, hi y as ordered integers
     unsigned long long t_start, t_body;  // globaltimer stamps of the running step
     IcpIterStats stats[kIcpMaxStats];
     float part[34 * kIcpMaxCtas];   // per-CTA float-float partials: hi, lo rows of 17 components
@@ -310,6 +319,7 @@ struct BackprojectJob {
     float fl_inv_x, fl_inv_y, pp_x, pp_y;
     Mat4 e2w;
     float4* out;
+    float4* boxes;
 };
 cudaError_t backproject_batch_enqueue(const BackprojectJob* jobs, int n, const BlockMap& map, cudaStream_t st);
 // CTAs of one frame pair's association (one per tile)
@@ -320,14 +330,17 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
                               int ctas, cudaStream_t stream, IcpPoseMail* mail = nullptr,
                               unsigned long long seq = 0);
 cudaError_t backproject_enqueue(const void* depth, bool u16, const kifi_camera& cam,
-                                const Mat4& eye_to_world, float4* out, int ctas, cudaStream_t st);
-cudaError_t expand_target_enqueue(const float* in, int n, float4* out, int ctas, cudaStream_t st);
+                                const Mat4& eye_to_world, float4* out, float4* boxes, int ctas, cudaStream_t st);
+// float4s of a width x height target's block boxes (IcpArgs::boxes)
+size_t icp_box_count(int width, int height);
+cudaError_t expand_target_enqueue(const float* in, int width, int height, float4* out, float4* boxes, int ctas,
+                                  cudaStream_t st);
 
 cudaError_t bin_enqueue(const float* pts, unsigned int n, const Mat4& w2c, int width, int height,
                         unsigned long long* zbuf, float* out, int ctas, cudaStream_t st);
 // Bin straight into an ICP target (float4 per pixel, w unused)
 cudaError_t bin_target_enqueue(const float* pts, unsigned int n, const Mat4& w2c, int width, int height,
-                               unsigned long long* zbuf, float4* out, int ctas, cudaStream_t st);
+                               unsigned long long* zbuf, float4* out, float4* boxes, int ctas, cudaStream_t st);
 
 // Optional epilogue of gemm_bf16_enqueue: C = acc + bias[n] (FP32), or with
 // out_bf16 set, out_bf16 = bf16(relu?(acc + bias[n])) (row stride ldc) in
