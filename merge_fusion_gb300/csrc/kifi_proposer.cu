@@ -24,7 +24,8 @@
 // pre-activation gradient [M x Cout]:
 //   dW    [Cout x Kp] = dY^T col      A = dY^T, B = col^T (inner M, split K)
 //   dcol  [M x Kp]    = dY W          A = dY,   B = W^T
-//   dX                = col2im(dcol)  a gather over the <= 4 taps per input
+//   dX                = col2im(dcol)  a gather over the <= 4 taps per input, in
+//                                     the pass that forms the next dY (k_grad)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -97,38 +98,115 @@ __global__ void k_downsample(const void* __restrict__ da, const void* __restrict
     out[i] = __float2half_rn(n ? sum / (float)n : 0.0f);
 }
 
-// im2col of a 3x3, stride 2, pad 1 convolution: col[m][k], m = (b, oy, ox),
-// k = (ky * 3 + kx) * C + c, zero outside the input and for k >= 9C
-template <typename T>
-__global__ void k_im2col(const T* __restrict__ x, int batch, int H, int W, int C, int Ho, int Wo, int Kp,
-                         bf16* __restrict__ col) {
-    const size_t n = (size_t)batch * Ho * Wo * Kp;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int k = (int)(i % Kp);
-        const size_t m = i / Kp;
-        const int ox = (int)(m % Wo), oy = (int)((m / Wo) % Ho), b = (int)(m / ((size_t)Wo * Ho));
-        float v = 0.0f;
-        if (k < 9 * C) {
-            const int c = k % C, tap = k / C, ky = tap / 3, kx = tap % 3;
-            const int iy = 2 * oy - 1 + ky, ix = 2 * ox - 1 + kx;
-            if (iy >= 0 && iy < H && ix >= 0 && ix < W) v = (float)x[(((size_t)b * H + iy) * W + ix) * C + c];
+// im2col of the first convolution (3x3, stride 2, pad 1, C = 2): col[m][k],
+// m = (b, oy, ox), k = (ky * 3 + kx) * 2 + c, zero outside the input and for
+// k >= 18; with kTrain its transpose colT[k][m] too, which the weight
+// gradient reads.  A thread takes one m: nine 4-byte loads, one 64-byte row,
+// and 32 columns that its warp writes as 64-byte runs.  Bound by its bytes
+// (20 MB read and written per 256 inputs): 11 us, 80 with a thread per element
+// and a transpose pass after it before.
+template <bool kTrain>
+__global__ void __launch_bounds__(kThreads) k_im2col_first(const __half* __restrict__ x, int batch,
+                                                           bf16* __restrict__ col, bf16* __restrict__ colT) {
+    constexpr int H = kHin[0], W = kWin[0], Ho = kHout[0], Wo = kWout[0], Kp = kKp[0];
+    const int M = batch * Ho * Wo;
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
+        const int ox = m % Wo, oy = m / Wo % Ho, b = m / (Wo * Ho);
+        __align__(16) bf16 v[Kp];
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {
+            const int iy = 2 * oy - 1 + t / 3, ix = 2 * ox - 1 + t % 3;
+            __half2 h = __floats2half2_rn(0.0f, 0.0f);
+            if (iy >= 0 && iy < H && ix >= 0 && ix < W)
+                h = reinterpret_cast<const __half2*>(x)[((size_t)b * H + iy) * W + ix];
+            v[2 * t] = __float2bfloat16_rn(__low2float(h));
+            v[2 * t + 1] = __float2bfloat16_rn(__high2float(h));
         }
-        col[i] = __float2bfloat16_rn(v);
+#pragma unroll
+        for (int k = 18; k < Kp; ++k) v[k] = __float2bfloat16_rn(0.0f);
+        uint4* row = reinterpret_cast<uint4*>(col + (size_t)m * Kp);
+#pragma unroll
+        for (int q = 0; q < Kp / 8; ++q) row[q] = reinterpret_cast<const uint4*>(v)[q];
+        if (kTrain)
+#pragma unroll
+            for (int k = 0; k < Kp; ++k) colT[(size_t)k * M + m] = v[k];
     }
 }
 
-// out[c][r] = in[r][c], 32x32 tiles through shared memory
-__global__ void k_transpose(const bf16* __restrict__ in, int R, int Cc, bf16* __restrict__ out) {
+constexpr int kTileM = 64;        // rows of a transposing tile
+constexpr int kTileP = kTileM + 8;  // its pitch: 16-byte vectors, a quarter of the banks apart
+
+// A [rows of C][kTileM] tile in shared memory out to out[c][m0 ..], 16 bytes
+// at a time (M is a multiple of 8: batches are).
+template <int C>
+__device__ __forceinline__ void put_transposed(const bf16 (*t)[kTileP], int m0, int M, bf16* __restrict__ out) {
+    for (int i = threadIdx.x; i < C * (kTileM / 8); i += kThreads) {
+        const int c = i / (kTileM / 8), q = i % (kTileM / 8) * 8;
+        if (m0 + q < M)
+            *reinterpret_cast<uint4*>(out + (size_t)c * M + m0 + q) = *reinterpret_cast<const uint4*>(&t[c][q]);
+    }
+}
+
+// The transposed im2col matrix colT[k][m] of convolution L > 0, straight from
+// the activation x [b][H][W][C] it convolves: per tap a tile of 64 output
+// pixels' channel vectors goes through shared memory.  The matrix itself is
+// not formed (the forward pass gathers its windows by TMA).  Bound by its
+// writes: 74 MB for the three layers at batch 256, where the im2col matrix was
+// written, read and written transposed (about 420 us, now 40).
+template <int L>
+__global__ void __launch_bounds__(kThreads) k_im2col_t(const bf16* __restrict__ x, int batch,
+                                                       bf16* __restrict__ colT) {
+    constexpr int H = kHin[L], W = kWin[L], C = kCin[L], Ho = kHout[L], Wo = kWout[L];
+    constexpr int kVec = C / 8;  // 16-byte vectors per pixel
+    __shared__ __align__(16) bf16 t[C][kTileP];
+    const int M = batch * Ho * Wo, tap = blockIdx.y, ky = tap / 3, kx = tap % 3;
+    for (int m0 = blockIdx.x * kTileM; m0 < M; m0 += gridDim.x * kTileM) {
+        for (int i = threadIdx.x; i < kTileM * kVec; i += kThreads) {
+            const int r = i / kVec, q = i % kVec, m = m0 + r;
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (m < M) {
+                const int ox = m % Wo, oy = m / Wo % Ho, b = m / (Wo * Ho);
+                const int iy = 2 * oy - 1 + ky, ix = 2 * ox - 1 + kx;
+                if (iy >= 0 && iy < H && ix >= 0 && ix < W)
+                    v = *reinterpret_cast<const uint4*>(x + (((size_t)b * H + iy) * W + ix) * C + q * 8);
+            }
+            const bf16* e = reinterpret_cast<const bf16*>(&v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) t[q * 8 + k][r] = e[k];
+        }
+        __syncthreads();
+        put_transposed<C>(t, m0, M, colT + (size_t)tap * C * M);
+        __syncthreads();
+    }
+}
+
+// out[c][r] = in[r][c] for several small matrices in one launch, 32x32 tiles
+// through shared memory
+struct TransposeJob {
+    const bf16* in;
+    bf16* out;
+    int R, C, first;  // first: the launch's first tile of this matrix
+};
+constexpr int kMaxTransposes = 7;
+struct TransposeJobs {
+    TransposeJob j[kMaxTransposes];
+    int n;
+};
+__global__ void k_transpose(TransposeJobs jobs) {
     __shared__ bf16 t[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+    int k = 0;
+    while (k + 1 < jobs.n && (int)blockIdx.x >= jobs.j[k + 1].first) ++k;
+    const TransposeJob& q = jobs.j[k];
+    const int tile = (int)blockIdx.x - q.first, tc = (q.C + 31) / 32;
+    const int c0 = tile % tc * 32, r0 = tile / tc * 32;
     for (int j = threadIdx.y; j < 32; j += 8) {
         const int r = r0 + j, c = c0 + threadIdx.x;
-        if (r < R && c < Cc) t[j][threadIdx.x] = in[(size_t)r * Cc + c];
+        if (r < q.R && c < q.C) t[j][threadIdx.x] = q.in[(size_t)r * q.C + c];
     }
     __syncthreads();
     for (int j = threadIdx.y; j < 32; j += 8) {
         const int c = c0 + j, r = r0 + threadIdx.x;
-        if (r < R && c < Cc) out[(size_t)c * R + r] = t[threadIdx.x][j];
+        if (r < q.R && c < q.C) q.out[(size_t)c * q.R + r] = t[threadIdx.x][j];
     }
 }
 
@@ -163,63 +241,78 @@ __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ 
     if ((threadIdx.x & 31) == 0 && l != 0.0f) atomicAdd(loss, l / (float)(batch * kOut));
 }
 
-// column sums of g [M][C] (FP32) into db[C] (+=)
-__global__ void k_colsum(const float* __restrict__ g, int M, int C, float* __restrict__ db) {
-    const int c = blockIdx.x;
-    float s = 0.0f;
-    for (int m = threadIdx.x; m < M; m += blockDim.x) s += g[(size_t)m * C + c];
-    __shared__ float red[kThreads / 32];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-        db[c] += t;
-    }
-}
-
-// ReLU backward: g = act > 0 ? g : 0 (in place, FP32) and a BF16 copy
-__global__ void k_relu_back(float* __restrict__ g, const bf16* __restrict__ act, size_t n, bf16* __restrict__ gb) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float v = __bfloat162float(act[i]) > 0.0f ? g[i] : 0.0f;
-        g[i] = v;
-        gb[i] = __float2bfloat16_rn(v);
-    }
-}
-
-// global average pool backward: d[B][P][C] = dg[B][C] / P
-__global__ void k_gap_back(const float* __restrict__ dg, int batch, int P, int C, float* __restrict__ d) {
-    const size_t n = (size_t)batch * P * C;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        const int b = (int)(i / ((size_t)P * C));
-        d[i] = dg[(size_t)b * C + c] / (float)P;
-    }
-}
-
-// col2im of the 3x3 / stride 2 / pad 1 convolution as a gather: input
-// element (b, iy, ix, c) collects dcol[(b, oy, ox)][(ky, kx, c)] over the taps
-// with iy = 2 oy - 1 + ky, ix = 2 ox - 1 + kx
-__global__ void k_col2im(const float* __restrict__ dcol, int batch, int H, int W, int C, int Ho, int Wo, int Kp,
-                         float* __restrict__ dx) {
-    const size_t n = (size_t)batch * H * W * C;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        const int ix = (int)((i / C) % W), iy = (int)((i / ((size_t)C * W)) % H);
-        const int b = (int)(i / ((size_t)C * W * H));
-        float s = 0.0f;
-        for (int ky = 0; ky < 3; ++ky) {
-            const int ty = iy + 1 - ky;
-            if (ty < 0 || (ty & 1) || (ty >> 1) >= Ho) continue;
-            for (int kx = 0; kx < 3; ++kx) {
-                const int tx = ix + 1 - kx;
-                if (tx < 0 || (tx & 1) || (tx >> 1) >= Wo) continue;
-                const size_t m = ((size_t)b * Ho + (ty >> 1)) * Wo + (tx >> 1);
-                s += dcol[m * Kp + (ky * 3 + kx) * C + c];
+// The gradient of a layer's pre-activation, in one pass: its value from the
+// layer above, through the ReLU (act > 0, where there is one), as BF16 [M][C]
+// and its transpose [C][M] for the two products that read it, and its column
+// sums (the bias gradient, added to db).  A thread keeps one column; a tile
+// of 64 rows is transposed in shared memory.  Values:
+//   kPlain   src[m][c]
+//   kPool    src[b][c] / P: the global average pool's gradient
+//   kConv    the gather form of col2im over src = dcol [M'][Kp] of the
+//            convolution above (3x3, stride 2, pad 1; taps in order): input
+//            pixel (iy, ix) collects the outputs with iy = 2 oy - 1 + ky,
+//            ix = 2 ox - 1 + kx
+// Bound by its bytes and the gathers' latency: the lowest layer's pass moves
+// 150 MB in 61 us.  Before, col2im, the ReLU, the column sums (one strided
+// column per CTA, 830 of 2080 us at batch 256) and the transpose were passes of
+// their own; a gradient step 1750 -> 677 us.
+// L is the convolution above for kConv.
+enum class GradSrc { kPlain, kPool, kConv };
+template <int C, GradSrc kSrc, int L = 0>
+__global__ void __launch_bounds__(kThreads) k_grad(const float* __restrict__ src, const bf16* __restrict__ act, int M,
+                                                   bf16* __restrict__ gb, bf16* __restrict__ gbT,
+                                                   float* __restrict__ db) {
+    constexpr int H = kHin[L], W = kWin[L], Ho = kHout[L], Wo = kWout[L], Kp = kKp[L], P = kHout[3] * kWout[3];
+    constexpr int kGroups = kThreads / C;  // rows taken side by side
+    __shared__ __align__(16) bf16 t[C][kTileP];
+    __shared__ float red[kGroups][C];
+    const int c = threadIdx.x % C, rg = threadIdx.x / C;
+    float sum = 0.0f;
+    for (int m0 = blockIdx.x * kTileM; m0 < M; m0 += gridDim.x * kTileM) {
+#pragma unroll 8
+        for (int r = rg; r < kTileM; r += kGroups) {
+            const int m = m0 + r;
+            bf16 o = __float2bfloat16_rn(0.0f);
+            if (m < M) {
+                float v;
+                if (kSrc == GradSrc::kPlain) {
+                    v = src[(size_t)m * C + c];
+                } else if (kSrc == GradSrc::kPool) {
+                    v = src[(size_t)(m / P) * C + c] / (float)P;
+                } else {
+                    const int ix = m % W, iy = m / W % H, b = m / (W * H);
+                    v = 0.0f;
+#pragma unroll
+                    for (int ky = 0; ky < 3; ++ky) {
+                        const int ty = iy + 1 - ky;
+                        if (ty < 0 || (ty & 1) || (ty >> 1) >= Ho) continue;
+#pragma unroll
+                        for (int kx = 0; kx < 3; ++kx) {
+                            const int tx = ix + 1 - kx;
+                            if (tx < 0 || (tx & 1) || (tx >> 1) >= Wo) continue;
+                            const size_t q = ((size_t)b * Ho + (ty >> 1)) * Wo + (tx >> 1);
+                            v += src[q * Kp + (ky * 3 + kx) * C + c];
+                        }
+                    }
+                }
+                if (act && !(__bfloat162float(act[(size_t)m * C + c]) > 0.0f)) v = 0.0f;
+                sum += v;
+                o = __float2bfloat16_rn(v);
+                if (gb) gb[(size_t)m * C + c] = o;
             }
+            t[c][r] = o;
         }
-        dx[i] = s;
+        __syncthreads();
+        put_transposed<C>(t, m0, M, gbT);
+        __syncthreads();
+    }
+    red[rg][c] = sum;
+    __syncthreads();
+    if (rg == 0) {
+        float s = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kGroups; ++k) s += red[k][c];
+        atomicAdd(db + c, s);
     }
 }
 
@@ -262,16 +355,16 @@ struct kifi_proposer {
     long long step = 0;
     // activations and scratch
     __half* x = nullptr;                 // the network input [B][60][80][2]
-    bf16* col[kConvs] = {};              // im2col [M][Kp]
-    bf16* colT[kConvs] = {};             // its transpose [Kp][M] (training)
-    float* y = nullptr;                  // GEMM output / gradient scratch, FP32 (largest [M][C])
-    float* y2 = nullptr;                 // second FP32 scratch (dcol, dX)
+    bf16* col = nullptr;                 // convolution 1's im2col [M][Kp]
+    bf16* colT[kConvs] = {};             // transposed im2col matrices [Kp][M] (training)
+    float* y = nullptr;                  // the hidden layer's gradient, FP32 [B][64]
+    float* y2 = nullptr;                 // FP32 scratch: dout, dgap, dcol
     bf16* act[kConvs] = {};              // conv activations [M][Cout]
     bf16 *gap = nullptr, *gapT = nullptr;   // [B][128], [128][B]
     bf16 *h1 = nullptr, *h1T = nullptr;     // [B][64], [64][B]
     float* out = nullptr;                   // [B][16]
     bf16 *dbf = nullptr, *dbfT = nullptr;   // BF16 gradient [M][C] and transpose
-    bf16* wT = nullptr;                     // transposed weights
+    bf16* wT[12] = {};                      // transposed weights (those whose layer passes a gradient on)
 };
 
 namespace {
@@ -283,41 +376,38 @@ kifi_status gemm(kifi_proposer* pr, const void* A, const void* B, float* C, int 
     KIFI_CUDA(gemm_bf16_enqueue(A, B, C, M, N, K, lda, ldb, ldc, k_split, acc, pr->status, pr->stream, epi));
     return KIFI_OK;
 }
-kifi_status transpose(kifi_proposer* pr, const bf16* in, int R, int Cc, bf16* out) {
-    dim3 grid((Cc + 31) / 32, (R + 31) / 32);
-    k_transpose<<<grid, dim3(32, 8), 0, pr->stream>>>(in, R, Cc, out);
-    KIFI_CUDA(cudaGetLastError());
-    return KIFI_OK;
-}
+// CTAs of a gradient pass, 64 rows a tile, at most eight per SM
+int tile_grid(int M) { return std::min((M + kTileM - 1) / kTileM, 8 * 152); }
 
 const bf16* wb(const kifi_proposer* pr, int t) { return pr->pb + kLayout.off[t]; }
 const float* pf(const kifi_proposer* pr, int t) { return pr->p + kLayout.off[t]; }
 float* gf(kifi_proposer* pr, int t) { return pr->g + kLayout.off[t]; }
 
-// forward pass; with `train` the transposed im2col matrices are kept for the
-// weight gradients.  Convolutions 2-4 run as implicit GEMMs over the previous
+// forward pass; with `train` the transposed im2col matrices are written for
+// the weight gradients.  Convolutions 2-4 run as implicit GEMMs over the previous
 // activation; convolution 1 (Cin = 2) through its im2col matrix.  Bias and
 // ReLU are applied in the GEMM epilogue, which writes the BF16 activation.
 kifi_status forward(kifi_proposer* pr, int batch, bool train) {
     kifi_status s;
     cudaStream_t st = pr->stream;
-    const int grid = pr->max_batch > 0 ? 4 * 152 : 1;
     for (int l = 0; l < kConvs; ++l) {
         const int M = (int)conv_m(l, batch);
-        if (l == 0)
-            k_im2col<__half><<<grid, kThreads, 0, st>>>(pr->x, batch, kHin[0], kWin[0], kCin[0], kHout[0],
-                                                        kWout[0], kKp[0], pr->col[0]);
-        else if (train)
-            k_im2col<bf16><<<grid, kThreads, 0, st>>>(pr->act[l - 1], batch, kHin[l], kWin[l], kCin[l], kHout[l],
-                                                      kWout[l], kKp[l], pr->col[l]);
+        if (l == 0) {
+            if (train) k_im2col_first<true><<<blocks(M), kThreads, 0, st>>>(pr->x, batch, pr->col, pr->colT[0]);
+            else k_im2col_first<false><<<blocks(M), kThreads, 0, st>>>(pr->x, batch, pr->col, nullptr);
+        } else if (train) {
+            const dim3 tiles((M + kTileM - 1) / kTileM, 9);
+            if (l == 1) k_im2col_t<1><<<tiles, kThreads, 0, st>>>(pr->act[0], batch, pr->colT[1]);
+            else if (l == 2) k_im2col_t<2><<<tiles, kThreads, 0, st>>>(pr->act[1], batch, pr->colT[2]);
+            else k_im2col_t<3><<<tiles, kThreads, 0, st>>>(pr->act[2], batch, pr->colT[3]);
+        }
         KIFI_CUDA(cudaGetLastError());
-        if (train && (s = transpose(pr, pr->col[l], M, kKp[l], pr->colT[l]))) return s;
         GemmEpilogue epi;
         epi.bias = pf(pr, 2 * l + 1);
         epi.relu = true;
         epi.out_bf16 = pr->act[l];
         if (l == 0) {
-            if ((s = gemm(pr, pr->col[0], wb(pr, 0), nullptr, M, kCout[0], kKp[0], kKp[0], kKp[0], kCout[0], 0, false,
+            if ((s = gemm(pr, pr->col, wb(pr, 0), nullptr, M, kCout[0], kKp[0], kKp[0], kKp[0], kCout[0], 0, false,
                           &epi)))
                 return s;
         } else {
@@ -343,40 +433,48 @@ kifi_status forward(kifi_proposer* pr, int batch, bool train) {
 kifi_status backward(kifi_proposer* pr, int batch) {
     kifi_status s;
     cudaStream_t st = pr->stream;
-    const int grid = 4 * 152;
     KIFI_CUDA(cudaMemsetAsync(pr->g, 0, kLayout.total * sizeof(float), st));
-    // fc2: dW2 [16 x 64] = dout^T h1, db2 = colsum(dout), dh1 = dout W2
-    if ((s = transpose(pr, pr->dbf, batch, kOutPad, pr->dbfT))) return s;
-    if ((s = transpose(pr, pr->h1, batch, kFc1, pr->h1T))) return s;
+    {  // every transpose that waits for nothing of the backward pass
+        TransposeJobs tj{};
+        int tiles = 0;
+        auto add = [&](const bf16* in, int R, int C, bf16* out) {
+            tj.j[tj.n++] = TransposeJob{in, out, R, C, tiles};
+            tiles += ((R + 31) / 32) * ((C + 31) / 32);
+        };
+        add(pr->h1, batch, kFc1, pr->h1T);
+        add(pr->gap, batch, 128, pr->gapT);
+        add(wb(pr, 10), kOutPad, kFc1, pr->wT[10]);
+        add(wb(pr, 8), kFc1, 128, pr->wT[8]);
+        for (int l = 1; l < kConvs; ++l) add(wb(pr, 2 * l), kCout[l], kKp[l], pr->wT[2 * l]);
+        k_transpose<<<tiles, dim3(32, 8), 0, st>>>(tj);
+    }
+    // fc2: db2 = colsum(dout), dW2 [16 x 64] = dout^T h1, dh1 = dout W2
+    k_grad<kOutPad, GradSrc::kPlain><<<tile_grid(batch), kThreads, 0, st>>>(pr->y2, nullptr, batch, nullptr,
+                                                                          pr->dbfT, gf(pr, 11));
     if ((s = gemm(pr, pr->dbfT, pr->h1T, gf(pr, 10), kOutPad, kFc1, batch, batch, batch, kFc1, batch, true)))
         return s;
-    k_colsum<<<kOutPad, kThreads, 0, st>>>(pr->y2, batch, kOutPad, gf(pr, 11));
-    if ((s = transpose(pr, wb(pr, 10), kOutPad, kFc1, pr->wT))) return s;
-    if ((s = gemm(pr, pr->dbf, pr->wT, pr->y, batch, kFc1, kOutPad, kOutPad, kOutPad, kFc1, 0, false))) return s;
-    k_relu_back<<<blocks((size_t)batch * kFc1), kThreads, 0, st>>>(pr->y, pr->h1, (size_t)batch * kFc1, pr->dbf);
-    // fc1: dW1 [64 x 128] = dh^T gap, db1, dgap = dh W1
-    if ((s = transpose(pr, pr->dbf, batch, kFc1, pr->dbfT))) return s;
-    if ((s = transpose(pr, pr->gap, batch, 128, pr->gapT))) return s;
+    if ((s = gemm(pr, pr->dbf, pr->wT[10], pr->y, batch, kFc1, kOutPad, kOutPad, kOutPad, kFc1, 0, false))) return s;
+    // fc1: through its ReLU; db1, dW1 [64 x 128] = dh^T gap, dgap = dh W1
+    k_grad<kFc1, GradSrc::kPlain><<<tile_grid(batch), kThreads, 0, st>>>(pr->y, pr->h1, batch, pr->dbf,
+                                                                       pr->dbfT, gf(pr, 9));
     if ((s = gemm(pr, pr->dbfT, pr->gapT, gf(pr, 8), kFc1, 128, batch, batch, batch, 128, batch, true))) return s;
-    k_colsum<<<kFc1, kThreads, 0, st>>>(pr->y, batch, kFc1, gf(pr, 9));
-    if ((s = transpose(pr, wb(pr, 8), kFc1, 128, pr->wT))) return s;
-    if ((s = gemm(pr, pr->dbf, pr->wT, pr->y2, batch, 128, kFc1, kFc1, kFc1, 128, 0, false))) return s;
-    // pool backward into the last conv's gradient
-    k_gap_back<<<grid, kThreads, 0, st>>>(pr->y2, batch, kHout[3] * kWout[3], 128, pr->y);
+    if ((s = gemm(pr, pr->dbf, pr->wT[8], pr->y2, batch, 128, kFc1, kFc1, kFc1, 128, 0, false))) return s;
     for (int l = kConvs - 1; l >= 0; --l) {
-        const int M = (int)conv_m(l, batch), Co = kCout[l], Kp = kKp[l];
-        // pr->y holds dL/d(act l) [M][Co]: through the ReLU
-        k_relu_back<<<grid, kThreads, 0, st>>>(pr->y, pr->act[l], (size_t)M * Co, pr->dbf);
-        k_colsum<<<Co, kThreads, 0, st>>>(pr->y, M, Co, gf(pr, 2 * l + 1));
-        if ((s = transpose(pr, pr->dbf, M, Co, pr->dbfT))) return s;
+        const int M = (int)conv_m(l, batch), Co = kCout[l], Kp = kKp[l], grid = tile_grid(M);
+        // the pre-activation's gradient, from the pool (y2 [B][128]) or from
+        // the convolution above (y2 = its dcol)
+        bf16* const db = pr->dbf;
+        bf16* const dt = pr->dbfT;
+        float* const bias = gf(pr, 2 * l + 1);
+        if (l == 3) k_grad<128, GradSrc::kPool><<<grid, kThreads, 0, st>>>(pr->y2, pr->act[3], M, db, dt, bias);
+        else if (l == 2) k_grad<64, GradSrc::kConv, 3><<<grid, kThreads, 0, st>>>(pr->y2, pr->act[2], M, db, dt, bias);
+        else if (l == 1) k_grad<64, GradSrc::kConv, 2><<<grid, kThreads, 0, st>>>(pr->y2, pr->act[1], M, db, dt, bias);
+        else k_grad<32, GradSrc::kConv, 1><<<grid, kThreads, 0, st>>>(pr->y2, pr->act[0], M, nullptr, dt, bias);
         // dW [Co x Kp] = dY^T col, inner M split across CTAs
         if ((s = gemm(pr, pr->dbfT, pr->colT[l], gf(pr, 2 * l), Co, Kp, M, M, M, Kp, 4096, true))) return s;
         if (l == 0) break;
-        // dcol = dY W, then col2im into dL/d(act l-1)
-        if ((s = transpose(pr, wb(pr, 2 * l), Co, Kp, pr->wT))) return s;
-        if ((s = gemm(pr, pr->dbf, pr->wT, pr->y2, M, Kp, Co, Co, Co, Kp, 0, false))) return s;
-        k_col2im<<<grid, kThreads, 0, st>>>(pr->y2, batch, kHin[l], kWin[l], kCin[l], kHout[l], kWout[l], Kp,
-                                            pr->y);
+        // dcol = dY W for the layer below
+        if ((s = gemm(pr, pr->dbf, pr->wT[2 * l], pr->y2, M, Kp, Co, Co, Co, Kp, 0, false))) return s;
     }
     KIFI_CUDA(cudaGetLastError());
     return KIFI_OK;
@@ -407,13 +505,13 @@ kifi_status kifi_proposer_destroy(kifi_proposer* pr) {
     if (!pr) return KIFI_OK;
     if (pr->stream) cudaStreamSynchronize(pr->stream);
     void* bufs[] = {pr->status, pr->loss, pr->p, pr->g, pr->m1, pr->m2, pr->pb, pr->mask, pr->x, pr->y, pr->y2,
-                    pr->gap, pr->gapT, pr->h1, pr->h1T, pr->out, pr->dbf, pr->dbfT, pr->wT};
+                    pr->gap, pr->gapT, pr->h1, pr->h1T, pr->out, pr->dbf, pr->dbfT, pr->col};
     for (void* b : bufs) cudaFree(b);
     for (int l = 0; l < kConvs; ++l) {
-        cudaFree(pr->col[l]);
         cudaFree(pr->colT[l]);
         cudaFree(pr->act[l]);
     }
+    for (bf16* w : pr->wT) cudaFree(w);
     if (pr->stream) cudaStreamDestroy(pr->stream);
     delete pr;
     return KIFI_OK;
@@ -441,18 +539,16 @@ kifi_status kifi_proposer_create(int device, int max_batch, kifi_proposer** out)
     alloc(&pr->pb, P * 2);
     alloc(&pr->mask, P);
     alloc(&pr->x, B * kInH * kInW * kInC * 2);
-    size_t ymax = 0, colmax = 0, dmax = 0;
+    size_t colmax = 0, dmax = 0;
     for (int l = 0; l < kConvs; ++l) {
         const size_t M = conv_m(l, max_batch);
-        alloc(&pr->col[l], M * kKp[l] * 2);
+        if (l == 0) alloc(&pr->col, M * kKp[0] * 2);
         alloc(&pr->colT[l], M * kKp[l] * 2);
         alloc(&pr->act[l], M * kCout[l] * 2);
-        ymax = std::max(ymax, M * (size_t)kCout[l]);
         colmax = std::max(colmax, M * (size_t)kKp[l]);
         dmax = std::max(dmax, M * (size_t)kCout[l]);
-        if (l > 0) ymax = std::max(ymax, (size_t)max_batch * kHin[l] * kWin[l] * kCin[l]);
     }
-    alloc(&pr->y, ymax * 4);
+    alloc(&pr->y, B * kFc1 * 4);
     alloc(&pr->y2, std::max(colmax, B * 128) * 4);
     alloc(&pr->gap, B * 128 * 2);
     alloc(&pr->gapT, B * 128 * 2);
@@ -461,7 +557,7 @@ kifi_status kifi_proposer_create(int device, int max_batch, kifi_proposer** out)
     alloc(&pr->out, B * kOutPad * 4);
     alloc(&pr->dbf, dmax * 2);
     alloc(&pr->dbfT, dmax * 2);
-    alloc(&pr->wT, 128 * 576 * 2);
+    for (int t = 2; t <= 10; t += 2) alloc(&pr->wT[t], kLayout.size[t] * 2);
     if (!e) e = cudaMemsetAsync(pr->status, 0, 16, pr->stream);
     if (!e) e = cudaMemsetAsync(pr->p, 0, P * 4, pr->stream);
     if (!e) e = cudaMemsetAsync(pr->m1, 0, P * 4, pr->stream);
