@@ -226,7 +226,7 @@ kifi_status kifi_batch_step_device(kifi_batch* b, const void* const* depth_dev, 
         add_share(g.splat, cdiv(P, 1024));
         add_share(g.hist, cdiv(P, 4096));
         add_share(g.pass, cdiv(P, 2048));
-        add_share(g.part, cdiv(j.max_tiles + 1, 256));
+        add_share(g.part, cdiv(j.max_tiles + 1, 32));
         // the merge's CTAs: about four 2048-voxel tiles each, of the resident bound
         add_share(g.merge, cdiv(std::min(v->n_upper + 8 * P, v->vb.cap), 8192));
         v->n_upper += 8 * P;

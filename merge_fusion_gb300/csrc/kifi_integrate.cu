@@ -1,10 +1,9 @@
 // kifi_integrate.cu -- one Integrator::Integrate (KinectFission/kifi/
 // Integrator.cpp:26-71) on sm_103a, as four kernels on one stream:
 //
-//  k_frame_setup   derive eyeToWorld / worldToClip and the projection
-//                  constants from the pose (Integrator.cpp:41-42), reset the
-//                  per-frame counters (k_frame_setup_sort for 30-bit keys also
-//                  prepares the sort's digit histograms and tile counters).
+//  k_frame_setup_sort  reset the per-frame counters and prepare the sort's
+//                  digit histograms and tile counters (the pose's constants,
+//                  Integrator.cpp:41-42, are formed on the host).
 //  k_splat_emit    DepthMap2PointCloud (Integrator.cpp:76-183) fused with
 //                  ExpandChunks (:186-250) and the de-duplication of
 //                  std::unique (:50-55): every valid pixel's voxel key and its
@@ -12,8 +11,7 @@
 //                  occupancy bitmap (one bit per voxel of the res^3 grid); the
 //                  thread whose atomicOr flips a bit owns that key and appends
 //                  it to the frame's list of keys NEW to the volume.
-//                  For 30-bit keys (k_splat_emit_hist) it also counts the
-//                  three 10-bit digits of every key it stores.
+//                  It also counts the sort digits of every key it stores.
 //  (radix sort)    the new keys are sorted (kifi_sort.cu): three 10-bit
 //                  digit passes for 30-bit keys.
 //  k_merge_update  flat_map::insert (flat_map.h:164-197) as a merge-path
@@ -61,19 +59,13 @@ template <typename K>
 __host__ __device__ constexpr int merge_tile() { return sizeof(K) == 4 ? kMergeTile : kMergeTile / 2; }
 constexpr uint16_t kFromB = 0x8000u;
 
-__global__ void k_frame_setup(DeviceCtl* ctl) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        ctl->n_new = 0u;
-        ctl->excluded_key = 0ull;
-    }
-}
-
-// The same for 30-bit keys, plus the set-up of the frame's sort: its digit
-// histograms (filled by the splat) zeroed, its passes' tile counters at the
-// first tile and a new look-back generation.
-__global__ void k_frame_setup_sort(DeviceCtl* ctl, SortScratch ss) {
+// The frame's counters, plus the set-up of its sort: the digit histograms
+// (filled by the splat) zeroed, the passes' tile counters at the first tile
+// and a new look-back generation.
+__global__ void k_frame_setup_sort(DeviceCtl* ctl, SortScratch ss, int passes) {
+    chain_begin();
     for (int i = threadIdx.x; i < kSortHistWords; i += blockDim.x) ss.hist[i] = 0u;
-    if (threadIdx.x < kFrameSortPasses) ss.tile_counter[threadIdx.x] = ss.first_tile;
+    if (threadIdx.x < passes) ss.tile_counter[threadIdx.x] = ss.first_tile;
     if (threadIdx.x == 0) {
         ctl->n_new = 0u;
         ctl->excluded_key = 0ull;
@@ -162,9 +154,9 @@ __device__ __forceinline__ bool splat_pixel(const FrameConst& fc, const float (&
 
 // Splat + dilation + new-key emission of one frame; `blk` / `nblk` are the
 // CTA's index and the CTA count working on this frame (the launch's own, or
-// a share of a batched launch over several volumes).  With kHist (30-bit
-// keys) the CTA also counts the three 10-bit digits of every key it stores,
-// in shared memory, and adds its counts to the sort's histograms `hist`.
+// a share of a batched launch over several volumes).  With kHist the CTA also
+// counts the sort digits of every key it stores, in shared memory, and adds
+// its counts to the sort's histograms `hist`.
 constexpr int kEmitWarps = kEmitThreads / 32;
 struct SplatSmem {
     unsigned long long ex;
@@ -180,13 +172,14 @@ __device__ __forceinline__ void splat_emit_body(DeviceCtl* __restrict__ ctl, con
                                                 K* __restrict__ new_keys, unsigned int new_cap,
                                                 const FrameConst& fc, unsigned int blk, unsigned int nblk,
                                                 SplatSmemHist<kHist>& sm, unsigned int* __restrict__ hist = nullptr) {
-    static_assert(!kHist || sizeof(K) == 4, "digit counts of 30-bit keys");
+    constexpr int kRadix = 1 << kFrameDigitBits<K>;
+    const int passes = frame_sort_passes<K>(sizeof(K) == 4 ? 10 : g.kb);  // digits counted
     unsigned int* s_hist = nullptr;
     if constexpr (kHist) {
         // a CTA without pixels has nothing to count
         if ((size_t)blk * kEmitThreads >= (size_t)fc.width * fc.height) return;
         s_hist = sm.counts;
-        for (int i = threadIdx.x; i < kSortHistWords; i += blockDim.x) s_hist[i] = 0u;
+        for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) s_hist[i] = 0u;
         __syncthreads();
     }
     const Codec<K> cd(g.kb);
@@ -295,10 +288,12 @@ __device__ __forceinline__ void splat_emit_body(DeviceCtl* __restrict__ ctl, con
                         const K key_out = cd.pack(bx + (b & 3u), by + ((b >> 2) & 3u), bz + (b >> 4));
                         new_keys[at] = key_out;
                         if constexpr (kHist) {
-                            const uint32_t ku = (uint32_t)key_out;
-                            atomicAdd(&s_hist[ku & (kFrameRadix - 1)], 1u);
-                            atomicAdd(&s_hist[kFrameRadix + ((ku >> kFrameDigitBits) & (kFrameRadix - 1))], 1u);
-                            atomicAdd(&s_hist[2 * kFrameRadix + (ku >> (2 * kFrameDigitBits))], 1u);
+#pragma unroll
+                            for (int p = 0; p < (sizeof(K) == 4 ? 3 : kFrameMaxPasses); ++p)
+                                if (sizeof(K) == 4 || p < passes)
+                                    atomicAdd(&s_hist[p * kRadix +
+                                                      ((uint32_t)(key_out >> (p * kFrameDigitBits<K>)) & (kRadix - 1))],
+                                              1u);
                         }
                     } else {
                         atomicOr(&ctl->status, KIFI_DEV_ERR_CAPACITY);
@@ -311,7 +306,7 @@ __device__ __forceinline__ void splat_emit_body(DeviceCtl* __restrict__ ctl, con
     __syncthreads();
     if (threadIdx.x == 0 && s_ex) atomicMax(&ctl->excluded_key, s_ex);
     if constexpr (kHist) {
-        for (int i = threadIdx.x; i < kSortHistWords; i += blockDim.x) {
+        for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) {
             const unsigned int c = s_hist[i];
             if (c) atomicAdd(&hist[i], c);
         }
@@ -322,24 +317,11 @@ template <bool kU16, typename K>
 __global__ void __launch_bounds__(kEmitThreads) k_splat_emit(DeviceCtl* __restrict__ ctl, Geom g,
                                                              const void* __restrict__ depth,
                                                              uint32_t* __restrict__ bitmap,
-                                                             K* __restrict__ new_keys,
-                                                             unsigned int new_cap,
-                                                             const FrameConst fc) {
-    __shared__ SplatSmemHist<false> sm;
-    splat_emit_body<kU16, K>(ctl, g, depth, bitmap, new_keys, new_cap, fc, blockIdx.x, gridDim.x, sm);
-}
-
-// 30-bit keys: the splat also fills the frame sort's digit histograms
-template <bool kU16>
-__global__ void __launch_bounds__(kEmitThreads) k_splat_emit_hist(DeviceCtl* __restrict__ ctl, Geom g,
-                                                                  const void* __restrict__ depth,
-                                                                  uint32_t* __restrict__ bitmap,
-                                                                  uint32_t* __restrict__ new_keys,
-                                                                  unsigned int new_cap, const FrameConst fc,
-                                                                  unsigned int* __restrict__ hist) {
+                                                             K* __restrict__ new_keys, unsigned int new_cap,
+                                                             const FrameConst fc, unsigned int* __restrict__ hist) {
     __shared__ SplatSmemHist<true> sm;
-    splat_emit_body<kU16, uint32_t, true>(ctl, g, depth, bitmap, new_keys, new_cap, fc, blockIdx.x, gridDim.x,
-                                          sm, hist);
+    chain_begin();
+    splat_emit_body<kU16, K, true>(ctl, g, depth, bitmap, new_keys, new_cap, fc, blockIdx.x, gridDim.x, sm, hist);
 }
 
 // Packed float pairs (f32x2): one instruction, each half rounded as the
@@ -490,19 +472,26 @@ __device__ __forceinline__ void update4(const K (&key)[4], float2 (&val)[4],
         if (ix[q] >= 0) apply_depth(val[q], d[q], w[q], g);
 }
 
-// number of A elements among the first d outputs of merge(A, B); A and B
-// are sorted and disjoint.
+// number of A elements among the first d outputs of merge(A, B), by a whole
+// warp; A and B are sorted and disjoint.  A 32-way search: a round tests 32
+// places of the range (at most |B| long), so that a frame's hundred thousand
+// new keys take four dependent reads instead of seventeen (the partition of a
+// 640x480 frame 12 -> 5 us).
 template <typename K>
-__device__ __forceinline__ unsigned long long merge_path(const K* __restrict__ A,
-                                                         unsigned long long na,
-                                                         const K* __restrict__ B,
+__device__ __forceinline__ unsigned long long merge_path(const K* A, unsigned long long na, const K* B,
                                                          unsigned long long nb,
                                                          unsigned long long d) {
+    const unsigned int lane = threadIdx.x & 31u;
     unsigned long long lo = d > nb ? d - nb : 0, hi = d < na ? d : na;
     while (lo < hi) {
-        unsigned long long mid = (lo + hi) >> 1;
-        if (A[mid] < B[d - 1 - mid]) lo = mid + 1;
-        else hi = mid;
+        // A[mid] < B[d - 1 - mid] holds for mid below the answer, and not from it on
+        const unsigned long long n = hi - lo, step = (n + 31) / 32, mid = lo + lane * step;
+        const bool below = mid < hi && sort_detail::ld_l2(A + mid) < sort_detail::ld_l2(B + (d - 1 - mid));
+        const unsigned int c = (unsigned int)__popc(__ballot_sync(0xffffffffu, below));
+        if (c == 0) break;
+        const unsigned long long next = lo + c * step;  // the first place tested that does not hold, if any
+        lo += (c - 1) * step + 1;
+        if (next < hi) hi = next;
     }
     return lo;
 }
@@ -523,7 +512,7 @@ struct PartitionSmem {
 
 // Merge set-up and partition.  Thread 0 settles the merge: drops the
 // dilation's excluded key when it is the largest new key (clearing its
-// occupancy bit), checks the capacity and publishes (e, N1).  Every thread t
+// occupancy bit), checks the capacity and publishes (e, N1).  Every warp t
 // then computes the merge-path split of output tile t: the number of resident
 // keys among the first t*kMergeTile outputs.  The binary searches of all
 // tiles run in parallel here instead of serialising the merge kernel's tiles.
@@ -538,19 +527,23 @@ __device__ __forceinline__ void merge_partition_body(DeviceCtl* __restrict__ ctl
     unsigned long long& s_e = sm.e;
     unsigned long long& s_n1 = sm.n1;
     int& s_ok = sm.ok;
+    // (independent reads: one memory latency)
     const unsigned int cur = ctl->cur;
-    const unsigned long long N0 = ctl->n[cur];
+    const unsigned long long n0 = ctl->n[0], n1 = ctl->n[1];
+    const unsigned int status = ctl->status;
+    const K excluded = (K)ctl->excluded_key;
+    const unsigned long long e0 = *in.b_count;
+    const unsigned long long N0 = cur ? n1 : n0;
     // select rather than index: a runtime index into a parameter array
     // would force the array into local memory
-    const K* __restrict__ A = (const K*)(cur ? vb.keys[1] : vb.keys[0]);
-    const K* __restrict__ B = in.b_keys;
+    const K* A = (const K*)(cur ? vb.keys[1] : vb.keys[0]);
+    const K* B = in.b_keys;
     // a sort that gave up on a bounded wait leaves its keys unordered: the
     // volume stays as it was (the host rebuilds the occupancy bits)
-    const bool timed_out = (ctl->status & KIFI_DEV_ERR_TIMEOUT) != 0u;
+    const bool timed_out = (status & KIFI_DEV_ERR_TIMEOUT) != 0u;
     if (threadIdx.x == 0) {
-        unsigned long long e = *in.b_count;
-        const K excluded = (K)ctl->excluded_key;
-        const bool drop = !timed_out && e > 0 && excluded != 0 && B[e - 1] == excluded;
+        unsigned long long e = e0;
+        const bool drop = !timed_out && e > 0 && excluded != 0 && sort_detail::ld_l2(B + (e - 1)) == excluded;
         if (drop) --e;
         const bool ok = !timed_out && N0 + e <= vb.cap;
         s_e = e;
@@ -575,16 +568,18 @@ __device__ __forceinline__ void merge_partition_body(DeviceCtl* __restrict__ ctl
         // of the occupancy bitmap; the host grows the buffers and retries.
         for (unsigned long long i = (unsigned long long)blk * blockDim.x + threadIdx.x; i < e;
              i += (unsigned long long)nblk * blockDim.x) {
-            size_t b = bit_index(B[i], cd, g.res);
+            size_t b = bit_index(sort_detail::ld_l2(B + i), cd, g.res);
             atomicAnd(vb.bitmap + (b >> 5), ~(1u << (b & 31)));
         }
         return;
     }
     const unsigned long long n_tiles = (N1 + kTile - 1) / kTile;
-    for (unsigned long long t = (unsigned long long)blk * blockDim.x + threadIdx.x;
-         t <= n_tiles && t < max_tiles; t += (unsigned long long)nblk * blockDim.x) {
+    const unsigned int warps = blockDim.x >> 5;
+    for (unsigned long long t = (unsigned long long)blk * warps + (threadIdx.x >> 5);
+         t <= n_tiles && t < max_tiles; t += (unsigned long long)nblk * warps) {
         const unsigned long long d = t * kTile < N1 ? t * kTile : N1;
-        splits[t] = merge_path(A, N0, B, e, d);
+        const unsigned long long a = merge_path(A, N0, B, e, d);
+        if ((threadIdx.x & 31u) == 0) splits[t] = a;
     }
 }
 
@@ -594,6 +589,7 @@ __global__ void __launch_bounds__(256) k_merge_partition(DeviceCtl* __restrict__
                                                           unsigned long long* __restrict__ splits,
                                                           unsigned int max_tiles) {
     __shared__ PartitionSmem sm;
+    chain_begin();
     merge_partition_body<K>(ctl, g, vb, in, splits, max_tiles, blockIdx.x, gridDim.x, sm);
 }
 
@@ -627,7 +623,7 @@ template <bool kU16, typename K>
 __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, const Geom& g,
                                                   const VolumeBuffers& vb, const MergeInputs<K>& in,
                                                   const void* __restrict__ depth,
-                                                  const unsigned long long* __restrict__ splits,
+                                                  const unsigned long long* splits,
                                                   const FrameConst& fc, unsigned int blk, unsigned int nblk,
                                                   MergeSmem<K>& sm) {
     constexpr int kTile = merge_tile<K>();
@@ -637,14 +633,17 @@ __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, c
     K* const sB_k = sm.sB_k;
     uint16_t* const sSrc = sm.sSrc;
 
-    if (!ctl->merge_ok) return;
+    // (independent reads: one memory latency)
+    const unsigned int ok = ctl->merge_ok;
     const unsigned int cur = ctl->cur, out = cur ^ 1u;
-    const unsigned long long N0 = ctl->n[cur];
+    const unsigned long long n0 = ctl->n[0], n1 = ctl->n[1];
     const unsigned long long e = ctl->merge_e;
     const unsigned long long N1 = ctl->merge_n1;
-    const K* __restrict__ A = (const K*)(cur ? vb.keys[1] : vb.keys[0]);
-    const float2* __restrict__ Av = cur ? vb.vals[1] : vb.vals[0];
-    const K* __restrict__ B = in.b_keys;
+    if (!ok) return;
+    const unsigned long long N0 = cur ? n1 : n0;
+    const K* A = (const K*)(cur ? vb.keys[1] : vb.keys[0]);
+    const float2* Av = cur ? vb.vals[1] : vb.vals[0];
+    const K* B = in.b_keys;
     const unsigned long long upd_end = in.update ? (N1 / 4 * 4) : 0ull;
     K* __restrict__ outK = (K*)(out ? vb.keys[1] : vb.keys[0]);
     float2* __restrict__ outV = out ? vb.vals[1] : vb.vals[0];
@@ -657,7 +656,7 @@ __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, c
         const unsigned long long d0 = t * kTile;
         const unsigned long long d1 = (d0 + kTile < N1) ? d0 + kTile : N1;
         const int len = (int)(d1 - d0);
-        const unsigned long long a0 = splits[t], a1 = splits[t + 1];
+        const unsigned long long a0 = __ldcg(splits + t), a1 = __ldcg(splits + t + 1);
         const int na = (int)(a1 - a0), nb = len - na;
         if (nb == 0) {
             // only resident voxels in this tile: straight streaming, no
@@ -728,7 +727,7 @@ __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, c
             const unsigned long long ka = a0 & ~3ull;
             const int koff = (int)(a0 - ka);
             const unsigned long long b0 = d0 - a0;
-            if ((int)threadIdx.x < nb) sB_k[threadIdx.x] = B[b0 + threadIdx.x];
+            if ((int)threadIdx.x < nb) sB_k[threadIdx.x] = sort_detail::ld_l2(B + (b0 + threadIdx.x));
             K kk[2][4];
             float2 vv[2][4];
             int li0[2];
@@ -821,7 +820,7 @@ __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, c
         const int voff = (int)(a0 - va);
         for (int i = threadIdx.x * 2; i < voff + na; i += kMergeThreads * 2)
             *(float4*)&sA_v[i] = __ldcs((const float4*)(Av + va + i));
-        for (int i = threadIdx.x; i < nb; i += kMergeThreads) sB_k[i] = B[b0 + i];
+        for (int i = threadIdx.x; i < nb; i += kMergeThreads) sB_k[i] = sort_detail::ld_l2(B + (b0 + i));
         __syncthreads();
         {
             const int dd = threadIdx.x * kItems;
@@ -905,18 +904,20 @@ template <bool kU16, typename K>
 __global__ void __launch_bounds__(kMergeThreads) k_merge_update(DeviceCtl* __restrict__ ctl, Geom g,
                                                                 VolumeBuffers vb, MergeInputs<K> in,
                                                                 const void* __restrict__ depth,
-                                                                const unsigned long long* __restrict__ splits,
+                                                                const unsigned long long* splits,
                                                                 const FrameConst fc) {
     __shared__ MergeSmem<K> sm;
+    chain_begin();
     merge_update_body<kU16, K>(ctl, g, vb, in, depth, splits, fc, blockIdx.x, gridDim.x, sm);
 }
 template <bool kU16, typename K>
 __global__ void __launch_bounds__(kMergeThreads, 4) k_merge_update_alone(DeviceCtl* __restrict__ ctl, Geom g,
                                                                          VolumeBuffers vb, MergeInputs<K> in,
                                                                          const void* __restrict__ depth,
-                                                                         const unsigned long long* __restrict__ splits,
+                                                                         const unsigned long long* splits,
                                                                          const FrameConst fc) {
     __shared__ MergeSmem<K> sm;
+    chain_begin();
     merge_update_body<kU16, K>(ctl, g, vb, in, depth, splits, fc, blockIdx.x, gridDim.x, sm);
 }
 
@@ -1155,25 +1156,20 @@ size_t merge_max_tiles(const VolumeBuffers& vb, size_t cap) {
 template <typename K>
 static cudaError_t merge_enqueue(DeviceCtl* ctl, const Geom& g, VolumeBuffers& vb,
                                  const MergeInputs<K>& in, const void* depth, bool u16,
-                                 const FrameConst& fc, const LaunchShape& ls, cudaStream_t st,
+                                 const FrameConst& fc, const LaunchShape& ls, bool chained, cudaStream_t st,
                                  cudaEvent_t after_partition = nullptr) {
     const unsigned int mt = max_tiles_of<K>(vb);
-    k_merge_partition<K><<<(mt + 255) / 256, 256, 0, st>>>(ctl, g, vb, in, vb.splits, mt);
+    // one warp per tile boundary, two CTAs per SM (the boundaries' number is not known here)
+    const unsigned int part_ctas = std::min((mt + 7) / 8, (unsigned int)ls.sms * 2u);
+    cudaError_t e = chain_launch(chained, dim3(part_ctas), dim3(256), st, k_merge_partition<K>, ctl, g, vb, in, vb.splits,
+                                 mt);
+    if (e != cudaSuccess) return e;
     if (after_partition) cudaEventRecord(after_partition, st);
-    if (ls.beside_tracking) {
-        if (u16)
-            k_merge_update<true, K><<<ls.merge_ctas, kMergeThreads, 0, st>>>(ctl, g, vb, in, depth, vb.splits, fc);
-        else
-            k_merge_update<false, K><<<ls.merge_ctas, kMergeThreads, 0, st>>>(ctl, g, vb, in, depth, vb.splits, fc);
-    } else {
-        if (u16)
-            k_merge_update_alone<true, K><<<ls.merge_ctas, kMergeThreads, 0, st>>>(ctl, g, vb, in, depth, vb.splits,
-                                                                                   fc);
-        else
-            k_merge_update_alone<false, K><<<ls.merge_ctas, kMergeThreads, 0, st>>>(ctl, g, vb, in, depth, vb.splits,
-                                                                                    fc);
-    }
-    return cudaGetLastError();
+    auto kernel = ls.beside_tracking ? (u16 ? k_merge_update<true, K> : k_merge_update<false, K>)
+                                     : (u16 ? k_merge_update_alone<true, K> : k_merge_update_alone<false, K>);
+    e = chain_launch(chained, dim3(ls.merge_ctas), dim3(kMergeThreads), st, kernel, ctl, g, vb, in, depth,
+                     (const unsigned long long*)vb.splits, fc);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <typename K>
@@ -1187,40 +1183,30 @@ static cudaError_t integrate_enqueue_t(DeviceCtl* ctl, const Geom& g, VolumeBuff
     if (events) cudaEventRecord(events[0], st);
     const unsigned int new_cap = (unsigned int)vb.new_cap;
     K* nk = (K*)vb.new_keys;
-    const K* sorted = nk;
-    cudaError_t e;
-    if constexpr (sizeof(K) == 4) {
-        // 30-bit keys: set-up and digit counts ride on the set-up and splat
-        // kernels; the sort is its three digit passes.  The splat takes at
-        // most one CTA per kEmitThreads pixels (a CTA without pixels would
-        // only launch and leave).
-        const size_t pix_ctas = ((size_t)cam.width * cam.height + kEmitThreads - 1) / kEmitThreads;
-        const int splat_ctas = (int)std::min<size_t>((size_t)ls.splat_ctas, std::max<size_t>(pix_ctas, 1));
-        sort_limits(&ss);
-        k_frame_setup_sort<<<1, 256, 0, st>>>(ctl, ss);
-        if (depth_u16)
-            k_splat_emit_hist<true><<<splat_ctas, kEmitThreads, 0, st>>>(ctl, g, depth_dev, vb.bitmap, nk, new_cap,
-                                                                          fc, ss.hist);
-        else
-            k_splat_emit_hist<false><<<splat_ctas, kEmitThreads, 0, st>>>(ctl, g, depth_dev, vb.bitmap, nk, new_cap,
-                                                                           fc, ss.hist);
-        if (events) cudaEventRecord(events[1], st);
-        e = sort_frame_keys(nk, &ctl->n_new, ss, &ctl->status, ls.sort_ctas, st, &sorted);
-    } else {
-        k_frame_setup<<<1, 32, 0, st>>>(ctl);
-        if (depth_u16)
-            k_splat_emit<true, K><<<ls.splat_ctas, kEmitThreads, 0, st>>>(ctl, g, depth_dev, vb.bitmap, nk, new_cap,
-                                                                          fc);
-        else
-            k_splat_emit<false, K><<<ls.splat_ctas, kEmitThreads, 0, st>>>(ctl, g, depth_dev, vb.bitmap, nk,
-                                                                           new_cap, fc);
-        if (events) cudaEventRecord(events[1], st);
-        e = sort_keys(vb.new_keys, sizeof(K), 3 * g.kb, nullptr, &ctl->n_new, ss, &ctl->status, ls.sort_ctas, st);
-    }
+    // stage events would stand between the kernels, and a captured frame's graph is updated in place: plain launches
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+    const bool chained = !ls.beside_tracking && !events && capture == cudaStreamCaptureStatusNone;
+    // set-up and digit counts of the sort ride on the set-up and splat
+    // kernels; the sort is its digit passes.  The splat takes at most one CTA
+    // per kEmitThreads pixels (a CTA without pixels would only launch and leave).
+    const size_t pix_ctas = ((size_t)cam.width * cam.height + kEmitThreads - 1) / kEmitThreads;
+    const int splat_ctas = (int)std::min<size_t>((size_t)ls.splat_ctas, std::max<size_t>(pix_ctas, 1));
+    sort_limits(&ss);
+    const int kb = sizeof(K) == 4 ? 10 : g.kb;
+    cudaError_t e = chain_launch(chained, dim3(1), dim3(256), st, k_frame_setup_sort, ctl, ss, frame_sort_passes<K>(kb));
+    if (!e)
+        e = chain_launch(chained, dim3(splat_ctas), dim3(kEmitThreads), st,
+                         depth_u16 ? k_splat_emit<true, K> : k_splat_emit<false, K>, ctl, g, depth_dev, vb.bitmap, nk,
+                         new_cap, fc, ss.hist);
+    if (events) cudaEventRecord(events[1], st);
+    const void* sorted = nullptr;
+    if (!e)
+        e = sort_frame_keys(nk, (int)sizeof(K), kb, &ctl->n_new, ss, &ctl->status, ls.sort_ctas, chained, st, &sorted);
     if (e != cudaSuccess) return e;
     if (events) cudaEventRecord(events[2], st);
-    MergeInputs<K> in{sorted, nullptr, nullptr, &ctl->n_new, true};
-    e = merge_enqueue<K>(ctl, g, vb, in, depth_dev, depth_u16, fc, ls, st, events ? events[3] : nullptr);
+    MergeInputs<K> in{(const K*)sorted, nullptr, nullptr, &ctl->n_new, true};
+    e = merge_enqueue<K>(ctl, g, vb, in, depth_dev, depth_u16, fc, ls, chained, st, events ? events[3] : nullptr);
     if (events) cudaEventRecord(events[4], st);
     return e;
 }
@@ -1297,10 +1283,10 @@ cudaError_t insert_merge_enqueue(DeviceCtl* ctl, const Geom& g, VolumeBuffers& v
     FrameConst fc{};
     if (vb.key_bytes == 8) {
         MergeInputs<uint64_t> in{(const uint64_t*)vb.new_keys, vb.new_idx, vals_dev, &ctl->n_new, false};
-        return merge_enqueue<uint64_t>(ctl, g, vb, in, nullptr, false, fc, ls, st);
+        return merge_enqueue<uint64_t>(ctl, g, vb, in, nullptr, false, fc, ls, false, st);
     }
     MergeInputs<uint32_t> in{(const uint32_t*)vb.new_keys, vb.new_idx, vals_dev, &ctl->n_new, false};
-    return merge_enqueue<uint32_t>(ctl, g, vb, in, nullptr, false, fc, ls, st);
+    return merge_enqueue<uint32_t>(ctl, g, vb, in, nullptr, false, fc, ls, false, st);
 }
 
 }  // namespace kifi

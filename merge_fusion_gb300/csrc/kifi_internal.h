@@ -11,18 +11,57 @@
 
 namespace kifi {
 
+// ------------------------------------------------- chained launches
+// The kernels of a frame's fusion follow one another on one stream, each a
+// few microseconds long.  Launched as programmatic dependents (chained), a
+// kernel's CTAs are placed as the last CTAs of the one before leave, and wait
+// (chain_begin, the first thing they do) for its memory to be visible: the
+// launch no longer stands between them (a 320x240 frame 75 -> 59 us; letting
+// them in when the kernel before had started, so that they held SM slots while
+// it ran, gave 65).  Beside a tracking stream launches are plain: waiting CTAs
+// would hold the SMs that tracking's next step needs.  To a chained kernel,
+// what the ones before write is not read-only data (ld.global.nc, which const
+// __restrict__ pointers invite, may find stale lines): such pointers are not
+// restrict, and the arrays are read in L2.  The few words that every CTA
+// starts with are plain loads: every warp of a grid reading them in L2 queues
+// at one slice (7 us of a 320x240 frame's merge).
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... Params, typename... Args>
+inline cudaError_t chain_launch(bool chained, dim3 grid, dim3 block, cudaStream_t st, void (*kernel)(Params...),
+                                Args&&... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 // ------------------------------------------------------------ radix sort
 // up to 8 digit passes: keys of up to 64 bits
 constexpr int kSortMaxPasses = 8;
-// A frame's 30-bit new keys sort in three 10-bit digit passes.  The frame's
-// set-up kernel zeroes their histograms and tile counters, and the splat
-// counts the digits of every key it stores, so the sort itself is the three
-// passes (its result lands in SortScratch::alt_keys).
-constexpr int kFrameDigitBits = 10;
-constexpr int kFrameRadix = 1 << kFrameDigitBits;
-constexpr int kFrameSortPasses = 3;
-// counters of the largest digit set: 3 x 1024 (frame keys) or 8 x 256
-constexpr int kSortHistWords = kFrameSortPasses * kFrameRadix;
+// A frame's 30-bit new keys sort in three 10-bit digit passes, 64-bit ones in
+// as many 8-bit passes as their bits need (five beyond 10 bits per axis: their
+// frames have more tiles, and 10-bit digits' look-back words, 8 KB a tile, would
+// be half the traffic).  The frame's set-up kernel zeroes the passes' histograms
+// and tile counters, and the splat counts the digits of every key it stores,
+// so the sort itself is its passes (after an odd number the result lies in
+// SortScratch::alt_keys).
+template <typename K>
+constexpr int kFrameDigitBits = sizeof(K) == 4 ? 10 : 8;
+template <typename K>
+__host__ __device__ constexpr int frame_sort_passes(int kb) {
+    return (3 * kb + kFrameDigitBits<K> - 1) / kFrameDigitBits<K>;
+}
+constexpr int kFrameMaxPasses = 5;
+// counters of the largest digit set: 3 x 1024 (30-bit frame keys) or 8 x 256
+constexpr int kSortHistWords = 3 * 1024;
 static_assert(kSortHistWords >= kSortMaxPasses * 256, "histogram sized for both digit sets");
 struct SortScratch {
     unsigned int* hist = nullptr;           // [passes][radix] digit counts
@@ -55,8 +94,8 @@ cudaError_t sort_keys(void* keys, int key_bytes, int key_bits, uint32_t* vals, c
 // the frame path's three 10-bit passes over 30-bit keys whose histograms and
 // pass counters are already set (see kFrameDigitBits); *sorted receives the
 // buffer holding the result
-cudaError_t sort_frame_keys(uint32_t* keys, const unsigned int* n_dev, SortScratch& s, unsigned int* status,
-                            int grid_ctas, cudaStream_t st, const uint32_t** sorted);
+cudaError_t sort_frame_keys(void* keys, int key_bytes, int kb, const unsigned int* n_dev, SortScratch& s,
+                            unsigned int* status, int grid_ctas, bool chained, cudaStream_t st, const void** sorted);
 
 // ------------------------------------------------------------- integrate
 struct VolumeBuffers {

@@ -51,24 +51,22 @@ __global__ void __launch_bounds__(kThreads) k_sort_histogram(const K* __restrict
 }
 
 template <bool kWithValues, typename K>
-__global__ void __launch_bounds__(kThreads) k_sort_pass(const K* __restrict__ keys_in,
-                                                        K* __restrict__ keys_out,
-                                                        const uint32_t* __restrict__ vals_in,
-                                                        uint32_t* __restrict__ vals_out,
-                                                        const unsigned int* __restrict__ n_ptr,
+__global__ void __launch_bounds__(kThreads) k_sort_pass(const K* keys_in, K* __restrict__ keys_out,
+                                                        const uint32_t* vals_in, uint32_t* __restrict__ vals_out,
+                                                        const unsigned int* n_ptr,
                                                         SortScratch s, int pass) {
     __shared__ SortPassSmem<8> sm;
     sort_pass_body<kWithValues, K, 8>(keys_in, keys_out, vals_in, vals_out, n_ptr, s, pass, blockIdx.x, sm);
 }
 
-// a pass of the frame keys' 10-bit digits
-__global__ void __launch_bounds__(kThreads) k_sort_pass_frame(const uint32_t* __restrict__ keys_in,
-                                                              uint32_t* __restrict__ keys_out,
-                                                              const unsigned int* __restrict__ n_ptr,
+// a pass of a frame's new keys
+template <typename K>
+__global__ void __launch_bounds__(kThreads) k_sort_pass_frame(const K* keys_in, K* __restrict__ keys_out,
+                                                              const unsigned int* n_ptr,
                                                               SortScratch s, int pass) {
-    __shared__ SortPassSmem<kFrameDigitBits> sm;
-    sort_pass_body<false, uint32_t, kFrameDigitBits>(keys_in, keys_out, nullptr, nullptr, n_ptr, s, pass,
-                                                     blockIdx.x, sm);
+    __shared__ SortPassSmem<kFrameDigitBits<K>> sm;
+    chain_begin();
+    sort_pass_body<false, K, kFrameDigitBits<K>>(keys_in, keys_out, nullptr, nullptr, n_ptr, s, pass, blockIdx.x, sm);
 }
 
 // ---- batched: every volume of a batch sorts its frame's new keys, one
@@ -166,16 +164,27 @@ void sort_limits(SortScratch* s) {
     s->first_tile = g_first_tile.load();
 }
 
-// keys -> alt -> keys -> alt: the sorted keys end in s.alt_keys
-cudaError_t sort_frame_keys(uint32_t* keys, const unsigned int* n_dev, SortScratch& s, unsigned int* status,
-                            int grid_ctas, cudaStream_t st, const uint32_t** sorted) {
+// keys -> alt -> keys ...: the sorted keys end in s.alt_keys after an odd number of passes
+template <typename K>
+static cudaError_t sort_frame_t(K* keys, int passes, const unsigned int* n_dev, SortScratch& s,
+                                unsigned int* status, int grid_ctas, bool chained, cudaStream_t st,
+                                const void** sorted) {
     s.status = status;
-    uint32_t* alt = (uint32_t*)s.alt_keys;
-    for (int pass = 0; pass < kFrameSortPasses; ++pass)
-        k_sort_pass_frame<<<grid_ctas, kThreads, 0, st>>>(pass & 1 ? alt : keys, pass & 1 ? keys : alt, n_dev, s,
-                                                          pass);
-    *sorted = kFrameSortPasses & 1 ? alt : keys;
+    K* alt = (K*)s.alt_keys;
+    for (int pass = 0; pass < passes; ++pass) {
+        const cudaError_t e = chain_launch(chained, dim3(grid_ctas), dim3(kThreads), st, k_sort_pass_frame<K>,
+                                           (const K*)(pass & 1 ? alt : keys), pass & 1 ? keys : alt, n_dev, s, pass);
+        if (e != cudaSuccess) return e;
+    }
+    *sorted = passes & 1 ? alt : keys;
     return cudaGetLastError();
+}
+
+cudaError_t sort_frame_keys(void* keys, int key_bytes, int kb, const unsigned int* n_dev, SortScratch& s,
+                            unsigned int* status, int grid_ctas, bool chained, cudaStream_t st, const void** sorted) {
+    if (key_bytes == 8)
+        return sort_frame_t((uint64_t*)keys, frame_sort_passes<uint64_t>(kb), n_dev, s, status, grid_ctas, chained, st, sorted);
+    return sort_frame_t((uint32_t*)keys, frame_sort_passes<uint32_t>(kb), n_dev, s, status, grid_ctas, chained, st, sorted);
 }
 
 template <typename K>

@@ -57,6 +57,11 @@ __device__ __forceinline__ unsigned int lanemask_lt() {
     return m;
 }
 
+// Reads of what the kernels before wrote go to L2: a chained kernel's life
+// begins before those writes, so they are no read-only data to it and L1 may
+// hold older lines.
+__device__ __forceinline__ uint32_t ld_l2(const uint32_t* p) { return __ldcg(p); }
+__device__ __forceinline__ uint64_t ld_l2(const uint64_t* p) { return __ldcg((const unsigned long long*)p); }
 __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long* p) {
     unsigned long long v;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -78,9 +83,9 @@ struct SortPassSmem {
     unsigned int tile_id;
 };
 template <bool kWithValues, typename K, int kBits>
-__device__ __forceinline__ void sort_pass_body(const K* __restrict__ keys_in, K* __restrict__ keys_out,
-                                               const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ vals_out,
-                                               const unsigned int* __restrict__ n_ptr, const SortScratch& s,
+__device__ __forceinline__ void sort_pass_body(const K* keys_in, K* __restrict__ keys_out,
+                                               const uint32_t* vals_in, uint32_t* __restrict__ vals_out,
+                                               const unsigned int* n_ptr, const SortScratch& s,
                                                int pass, unsigned int blk, SortPassSmem<kBits>& sm) {
     constexpr int R = 1 << kBits;
     constexpr int D = R / kThreads;
@@ -117,7 +122,7 @@ __device__ __forceinline__ void sort_pass_body(const K* __restrict__ keys_in, K*
             unsigned int c[D], sum = 0;
 #pragma unroll
             for (int q = 0; q < D; ++q) {
-                c[q] = s.hist[pass * R + threadIdx.x * D + q];
+                c[q] = __ldcg(s.hist + pass * R + threadIdx.x * D + q);
                 sum += c[q];
             }
             unsigned int x = sum;
@@ -147,8 +152,8 @@ __device__ __forceinline__ void sort_pass_body(const K* __restrict__ keys_in, K*
         for (int j = 0; j < kKeysPerThread; ++j) {
             unsigned int i = base + j * 32 + lane;
             bool ok = i < n;
-            k[j] = ok ? keys_in[i] : (K)0;
-            if (kWithValues) v[j] = ok ? vals_in[i] : 0u;
+            k[j] = ok ? ld_l2(keys_in + i) : (K)0;
+            if (kWithValues) v[j] = ok ? __ldcg(vals_in + i) : 0u;
             dig[j] = ok ? (int)((unsigned int)(k[j] >> shift) & (unsigned int)(R - 1)) : R;
         }
         // stable warp-local ranks: lanes with equal digits, in (j, lane) order
