@@ -703,13 +703,24 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         }
         __syncthreads();
         const int ax0 = ss.cbox[0], ay0 = ss.cbox[1], ax1 = ss.cbox[2], ay1 = ss.cbox[3];
+        // a tile whose windows are all empty (most of a frame wider than the
+        // reference's 640 columns projects past them) has no pairs to search or sum
+        if (ax1 < 0) {
+            if (a.pairs && mine) {
+                const size_t k = (size_t)y * n_cols + col;
+                a.pairs[k] = -1ll;
+                a.pairs_len2[k] = 0.01f;
+            }
+            __syncthreads();  // every thread has read the box before the next tile writes it
+            continue;
+        }
         // the region staged ahead if it holds every projection of the tile with a
         // margin, else the projections with as much of the windows around them as fits
         Region reg{0, 0, 0, 0, 0, 1};
         if (ahead && pw > 0 && max(ax0 - kUseMargin, 0) >= px0 && max(ay0 - kUseMargin, 0) >= py0 &&
             min(ax1 + kUseMargin, 640) <= px0 + pw && min(ay1 + kUseMargin, 480) <= py0 + ph) {
             reg = Region{0, px0, py0, px0 + pw, py0 + ph, stage_pitch(pw)};
-        } else if (ax1 >= 0) {
+        } else {
             for (int m = 10; m >= 0; m -= m > 4 ? 3 : 1) {
                 const int x0 = max(ax0 - m, 0), y0 = max(ay0 - m, 0);
                 const int w0 = min(ax1 + m, 640) - x0, h0 = min(ay1 + m, 480) - y0;
