@@ -63,9 +63,11 @@ WORKLOAD = ("room 4x3x4 m, 40 boxes + 20 spheres, 640x480 uint16 depth, res 1024
 # kernels launched per frame: frame set-up (with the sort's set-up), splat+emit
 # (with the digit counts), three digit passes, merge partition, merge+update;
 # tracking: ICP begin, one step per iteration, the next target's
-# back-projection; per mesh: snapshot, row directory, tile ranges, status
-# bytes, classification, tile-sum scan, two emission passes
+# back-projection; per mesh: snapshot, count and build of the words,
+# classification, emission.  LAUNCHES_MESH is a mesh's count when it searched per
+# voxel and emitted twice, which recorded lines were counted with
 LAUNCHES_FUSION, LAUNCHES_TRACKING, LAUNCHES_MESH = 7, ICP_ITERS + 2, 8
+KERNELS_PER_MESH = 5
 # bytes the host reads back per tracked frame: the head of the ICP state
 # (float and float-float pose, counters, 64 iteration records of 20 bytes)
 ICP_HEAD_BYTES = 192 + 64 * 20
@@ -627,14 +629,14 @@ def run_gpu(args, rank, world, local):
             {"traffic": traffic,
              "isolated": {"ms_per_launch": iso_stage[3] / iso_per,
                           "frac": gbs(iso_merge_bytes, iso_stage[3] / iso_per) / peak}}),
-        "mesher (row directory, classify, scan, emit)": roofline_entry(
+        "mesher (words, classify, emit)": roofline_entry(
             "hbm", gbs(mesh_bytes, pipe_ms[1]), peak, "GB/s",
             {"bytes_per_launch": mesh_bytes, "bytes_rule": "12 B per voxel + 12 B per vertex + 12 B per triangle",
              "per": "mesh"}, pipe_ms[1], peak_kind,
             {"meshes": int(pipe_n[1]),
              "isolated": {"ms_per_launch": iso_mesh_ms.value, "voxels": n_mesh_vox.value,
                           "frac": gbs(iso_mesh_bytes, iso_mesh_ms.value) / peak,
-                          "stage_ms": {"row_directory": iso_mesh[0], "classification": iso_mesh[1],
+                          "stage_ms": {"words": iso_mesh[0], "classification": iso_mesh[1],
                                        "scan": iso_mesh[2], "emission": iso_mesh[3]}}}),
         "k_icp_step": roofline_entry(
             "fp32", icp_flops / (track_step_ms * 1e-3) / 1e12 if track_step_ms > 0 else 0.0, fp32_peak, "TFLOP/s",
@@ -646,7 +648,7 @@ def run_gpu(args, rank, world, local):
                           "finisher_us_median": float(np.median(tail[:min(nit.value, 64)]))}}),
     }
     value = job_throughput(world, KF, ms / 1e3)
-    steps_launches = K * (FS * (LAUNCHES_FUSION + LAUNCHES_TRACKING) + LAUNCHES_MESH)
+    steps_launches = K * (FS * (LAUNCHES_FUSION + LAUNCHES_TRACKING) + KERNELS_PER_MESH)
     # `config` names the workload (the reference arm prints the same dict); `run` describes this run
     cfg = workload_config(Fp, FS)
     run = {"resident_voxels_start": n_start, "resident_voxels_end": int(n1[-1]) if m else None,

@@ -632,7 +632,8 @@ static kifi_status mesh_to_device(kifi_volume* v, int with_indices, size_t* n_ve
     if (n < 2) return KIFI_OK;  // the reference's loop starts at size-2
     if (n >= ((size_t)1 << 28)) return fail(KIFI_ERR_UNSUPPORTED, "mesh of more than 2^28 voxels");
     const unsigned int cur = v->ctl_host->cur;
-    KIFI_CUDA(mesh_scratch_reserve(&v->ms, n, v->g.kb));
+    // with headroom: a growing volume's next meshes still fit
+    if (v->ms.cap < n) KIFI_CUDA(mesh_scratch_reserve(&v->ms, n + n / 4, v->g.kb));
     const unsigned int n32 = (unsigned int)n;
     KIFI_CUDA(cudaMemcpyAsync(v->ms.n_dev, &n32, sizeof n32, cudaMemcpyHostToDevice, v->stream));
     std::array<cudaEvent_t, 5> ev{};
@@ -649,11 +650,11 @@ static kifi_status mesh_to_device(kifi_volume* v, int with_indices, size_t* n_ve
         KIFI_CUDA(cudaEventRecord(ev[0], v->stream));
     }
     KIFI_CUDA(mesh_count_enqueue(v->vb.keys[cur], v->vb.key_bytes, v->vb.vals[cur], n, v->g.kb,
-                                 with_indices ? 1 : 0, v->ms, v->ls.sms, v->stream, ev[0] ? &ev[1] : nullptr));
+                                 with_indices ? 1 : 0, v->ms, v->stream, ev[0] ? &ev[1] : nullptr));
     if (ev[0]) KIFI_CUDA(cudaEventRecord(ev[3], v->stream));
     MeshCounts* mc = &v->ctl_host_mesh;
     for (int attempt = 0; attempt < 2; ++attempt) {
-        KIFI_CUDA(mesh_emit_enqueue(v->g, v->vb.keys[cur], v->vb.key_bytes, v->vb.vals[cur], n,
+        KIFI_CUDA(mesh_emit_enqueue(v->g, v->vb.key_bytes, v->vb.vals[cur], n,
                                     with_indices ? 1 : 0, v->ms, v->mesh_verts_cap, v->mesh_idx_cap, v->mesh_verts,
                                     v->mesh_idx, v->ls.sms, v->stream));
         if (attempt == 0 && ev[0]) {
@@ -662,7 +663,6 @@ static kifi_status mesh_to_device(kifi_volume* v, int with_indices, size_t* n_ve
         }
         KIFI_CUDA(cudaMemcpyAsync(mc, v->ms.counts, sizeof(MeshCounts), cudaMemcpyDeviceToHost, v->stream));
         KIFI_CUDA(cudaStreamSynchronize(v->stream));
-        if (mc->error) return fail(KIFI_ERR_TIMEOUT, "mesh classification: a bounded wait gave up");
         if (!mc->overflow) break;
         if (attempt == 1) return fail(KIFI_ERR_CUDA, "mesh emission overflowed buffers sized to its counts");
         const size_t nv = (size_t)mc->n_verts, ni = with_indices ? (size_t)mc->n_idx : 0;

@@ -155,7 +155,7 @@ kifi_status span_end(std::vector<std::array<cudaEvent_t, 2>>& pending, std::arra
 
 // emission of the snapshot into the current buffers, then its counts to the host
 kifi_status mesh_emit(kifi_pipeline* p, std::array<cudaEvent_t, 2>* ev) {
-    KIFI_CUDA(mesh_emit_enqueue(p->vol->g, p->snap_keys, p->vol->vb.key_bytes, p->snap_vals, p->snap_n,
+    KIFI_CUDA(mesh_emit_enqueue(p->vol->g, p->vol->vb.key_bytes, p->snap_vals, p->snap_n,
                                 p->desc.mesh_with_indices, p->mscr, p->mverts_cap, p->midx_cap, p->mverts, p->midx,
                                 p->vol->ls.sms, p->ms));
     if (ev) {
@@ -182,10 +182,6 @@ kifi_status mesh_poll(kifi_pipeline* p, bool wait) {
             if (q != cudaSuccess) return cuda_fail(q, "mesh counts");
         }
         const MeshCounts& c = *p->counts_host;
-        if (c.error) {  // the classification gave up on a bounded wait: no mesh
-            p->counting = false;
-            return fail(KIFI_ERR_TIMEOUT, "mesh classification: a bounded wait gave up");
-        }
         const size_t nv = (size_t)c.n_verts, ni = p->desc.mesh_with_indices ? (size_t)c.n_idx : 0;
         if (!c.overflow) {
             p->mesh_verts = nv;
@@ -245,7 +241,7 @@ kifi_status mesh_begin(kifi_pipeline* p) {
     std::array<cudaEvent_t, 2> ev;
     if ((s = span_begin(p, ev, p->ms))) return s;
     KIFI_CUDA(mesh_count_enqueue(p->snap_keys, v->vb.key_bytes, p->snap_vals, p->snap_n, v->g.kb,
-                                 p->desc.mesh_with_indices, p->mscr, v->ls.sms, p->ms));
+                                 p->desc.mesh_with_indices, p->mscr, p->ms));
     return mesh_emit(p, &ev);
 }
 

@@ -70,8 +70,8 @@ struct kifi_volume {
     bool profiling = false;
     std::vector<cudaEvent_t> event_pool;
     std::vector<std::array<cudaEvent_t, kStageEvents>> pending;
-    // kifi_mesh* timers: before the row directory, after it, after the
-    // classification, after the scan, after the emission
+    // kifi_mesh* timers: before the words are built, after, after the
+    // classification (twice), after the emission
     std::vector<std::array<cudaEvent_t, 5>> mesh_pending;
 };
 

@@ -228,55 +228,46 @@ struct MeshCounts {
     unsigned long long n_idx;
     unsigned long long missing_min;  // smallest triangle edge id without a vertex (or ~0)
     unsigned long long overflow;     // emission skipped: the output buffers were too small
-    unsigned long long n_flagged;    // voxels with output (vertices or triangles)
-    unsigned long long error;        // non-zero: a bounded wait of the classification gave up
+    unsigned int runs_done;          // classification CTAs that have finished
 };
 
-// per classification tile: the voxels staged for its lookups -- region A,
-// from the tile's first voxel on (the tile itself and its +y lookups), and
-// region B (the +z and +yz lookups) in up to two ranges (lo, len), the second
-// for the tile's voxels from `split` on (split = the tile's end when there is
-// one range)
-struct MeshTileRange {
-    unsigned int a_len, b_lo[2], b_len[2], split;
+// The volume as words: runs of 32 consecutive keys (key >> 5) with at least
+// one resident voxel, ascending; at most one per voxel.
+struct MeshWords {
+    void* key = nullptr;           // key >> 5 << 4 | the state of its key 0 (bits of the four masks below)
+    uint4* a = nullptr;            // first voxel; masks: resident, weight != 0, weight > 0
+    uint2* b = nullptr;            // masks: Distance() < 0, operands in the sign rule's range
+    uint4* v = nullptr;            // vertex masks of the +x, +y and +z edges; the first vertex within the run
+    uint4* link = nullptr;         // words with output: the +y, +z and +yz words; an index offset within the run
+    unsigned int* count = nullptr;
 };
 
 struct MeshScratch {
-    // per voxel: vertex axes | triangle count << 3 | marching-cubes case << 6 |
-    // the voxel's first vertex within its classification tile << 14
-    unsigned int* vflags = nullptr;
-    unsigned char* vstatus = nullptr;      // per voxel: the status byte classification reads
-    // per voxel with output: indices of its +y, +z, +yz lookups and its first
-    // index within its classification tile
-    uint4* corners = nullptr;
-    // per classification tile: packed (index count << 32 | vertex count),
-    // then (after the scan) their exclusive prefix
-    unsigned long long* tile_sums = nullptr;
-    // per tile: its voxels with output, then (after the scan) their exclusive
-    // prefix, with the total at [tiles]
-    unsigned int* tile_nflag = nullptr;
-    unsigned int* flagged = nullptr;       // per tile, a slot per voxel: those voxels, ascending
-    unsigned int* rows = nullptr;          // start index of each (z, y) key row
-    MeshTileRange* tile_ranges = nullptr;  // per classification tile: the staged regions
+    void* block = nullptr;  // the allocation that holds the arrays below
+    MeshWords words;
+    uint2* flagged = nullptr;            // a slot per voxel: those with output, run by run, ascending --
+                                         // word within the run << 13 | bit << 8 | case; first index, from the word's link
+    unsigned int* run_words = nullptr;  // per run of voxels: words that start in it
+    uint4* run_out = nullptr;           // per run of words: vertices, indices and voxels with output before it, their list
+    unsigned int* rows = nullptr;         // first word of each (z, y) key row
     MeshCounts* counts = nullptr;
-    unsigned int* n_dev = nullptr;         // the voxel count the passes read
+    unsigned int* n_dev = nullptr;        // the voxel count the passes read
     size_t cap = 0, rows_cap = 0;
 };
 
 cudaError_t mesh_scratch_reserve(MeshScratch* m, size_t n, int kb);
 void mesh_scratch_free(MeshScratch* m);
-// stage_events (optional, 2 entries): recorded after the row directory and
+// stage_events (optional, 2 entries): recorded after the words are built and
 // after the classification
 cudaError_t mesh_count_enqueue(const void* keys, int key_bytes, const float2* vals, size_t n_cap, int kb,
-                               int with_indices, MeshScratch& ms, int sms, cudaStream_t st,
-                               cudaEvent_t* stage_events = nullptr);
-// Emission reads the counts on the device (ms.counts, written by the
-// counting passes), so it can be enqueued right behind them.  The buffers
+                               int with_indices, MeshScratch& ms, cudaStream_t st, cudaEvent_t* stage_events = nullptr);
+// Emission sums up the counting passes' totals on the device and writes them
+// to ms.counts, so it can be enqueued right behind them.  The buffers
 // hold vert_cap vertices and idx_cap indices; when the mesh needs more, the
-// emission writes nothing and sets ms.counts->overflow instead.
-cudaError_t mesh_emit_enqueue(const Geom& g, const void* keys, int key_bytes, const float2* vals, size_t n_cap,
-                              int with_indices, MeshScratch& ms, size_t vert_cap, size_t idx_cap,
-                              float* verts_dev, uint32_t* idx_dev, int sms, cudaStream_t st);
+// emission writes nothing else and sets ms.counts->overflow.
+cudaError_t mesh_emit_enqueue(const Geom& g, int key_bytes, const float2* vals, size_t n_cap, int with_indices,
+                              MeshScratch& ms, size_t vert_cap, size_t idx_cap, float* verts_dev, uint32_t* idx_dev,
+                              int sms, cudaStream_t st);
 cudaError_t mesh_snapshot_enqueue(const DeviceCtl* ctl, const VolumeBuffers& vb, void* keys, float2* vals,
                                   size_t cap, unsigned int* n_dev, int sms, cudaStream_t st);
 

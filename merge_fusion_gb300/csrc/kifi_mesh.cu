@@ -6,29 +6,31 @@
 // three neighbour pointers (+y, +z, +yz) that start at n-2 and only move down.
 // After the walk for voxel i each pointer sits at
 //     min(n-2, upper_bound(keys, key_i + delta) - 1),
-// a closed form that depends on voxel i alone, so every voxel is handled by
-// its own thread:
+// a closed form that depends on voxel i alone: the voxel at key_i + delta when
+// it is resident and not the last one, else a voxel of another key; and the
+// pointer plus one is the voxel at key_i + delta + 1 exactly when that is
+// resident.  So what a cube reads is decided by which keys are resident, and
+// 32 voxels are handled at once: a word is a run of 32 consecutive keys (key >>
+// 5; the bits per axis are at least 10, so +y and +z move by whole words) of
+// which at least one is resident, with a bit per key in a few masks.  Sorted
+// keys give sorted words, and there are 10 to 20 times fewer of them.
 //
-//  k_row_directory  start index of every (y, z) key row (key >> b, b key bits
-//                   per axis); a neighbour search then only scans one row,
-//                   starting where the searching voxel sits in its own row.
-//  k_mesh_tile_ranges  per tile of 1024 voxels and neighbour offset, the
-//                   ranges of positions its voxels' lookups fall in.
-//  k_mesh_status    one status byte per voxel (weight, distance sign).
-//  k_mesh_classify_tiled  per voxel i in [0, n-2] with weight > 0: which of its
-//                   +x/+y/+z edges carry a vertex (Mesher.cpp:140-168) and,
-//                   for Mesh(verts, indices), the cube's marching-cubes case
-//                   and triangle count (:172-226); a voxel with any output
-//                   keeps its +y, +z and +yz lookups for emission.  Per tile
-//                   it also scans the vertex and index counts (a voxel's
-//                   first vertex within the tile goes into its flags, its
-//                   first index beside its lookups), lists the tile's voxels
-//                   with output and writes the tile's packed (index, vertex)
-//                   totals.
-//  k_scan_tile_sums one CTA turns the tile totals into tile offsets.
-//  k_mesh_emit      per tile, over its list of voxels with output: writes the
-//                   vertices (by the voxel's lane) and the triangle indices
-//                   (spread over the warp's lanes).
+//  k_word_count     counts the words that start in each of kVoxelRuns runs of voxels.
+//  k_word_build     writes the words: first voxel, masks (resident, weight != 0,
+//                   weight > 0, Distance() < 0, operands in the sign rule's
+//                   range), and the first word of every (y, z) key row.
+//  k_word_classify  a word per thread: finds the +y, +z and +yz words through
+//                   the row table, and from the masks which +x/+y/+z edges
+//                   carry a vertex (Mesher.cpp:140-168) and which cubes have
+//                   triangles (:172-226), 32 at a time.  Lists the voxels with
+//                   output, and totals vertices and indices per run of words.
+//  k_mesh_emit      over the listed voxels: writes the vertices (by the voxel's
+//                   lane) and the triangle indices (spread over the warp's lanes).
+//
+// (14.6 M voxels of a 640 x 480 room scan at 4 mm in 1.36 M words, 4.6 M
+// vertices and 21 M indices: a mesh call 440 us, of it count and build 100,
+// classification 107, emission 139.  A thread per voxel that searched among
+// staged keys and a second emission for the stop rule: 728.)
 //
 // Output order equals the reference's:
 //  * Mesh(verts): vertices in generation order -- voxels descending, axes
@@ -37,10 +39,9 @@
 //    which is ascending voxel order; triangles in generation order (voxels
 //    descending, table order), each index mapped to its vertex's rank
 //    (:28-44).  That mapping walk stops at the first index id that has no
-//    vertex; every index id at or above it keeps its raw id.  k_mesh_emit
-//    reproduces this: its first pass records the smallest missing id, and a
-//    second pass reads that bound on the device and rewrites the indices at
-//    or above it (it returns at once when no id was missing).
+//    vertex; every index id at or above it keeps its raw id.  The smallest
+//    such id is found by the classification, so one emission writes the
+//    indices as they end up.
 #include "kifi_internal.h"
 #include "mc_table.cuh"
 
@@ -49,74 +50,7 @@ namespace {
 
 constexpr int kThreads = 256;
 
-template <typename K>
-__device__ __forceinline__ unsigned long long lower_bound_key(const K* __restrict__ k, unsigned long long n, K t) {
-    unsigned long long lo = 0, hi = n;
-    while (lo < hi) {
-        unsigned long long mid = (lo + hi) >> 1;
-        if (k[mid] < t) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// row_start[r] = first index whose (z, y) row (key >> b) >= r, for r in [0, 2^2b]
-template <typename K>
-__global__ void k_row_directory(const K* __restrict__ keys, const unsigned int* __restrict__ n_dev, int b,
-                                unsigned int* __restrict__ row_start) {
-    const unsigned long long n = *n_dev;
-    const unsigned int rows = 1u << (2 * b);
-    for (unsigned int r = blockIdx.x * blockDim.x + threadIdx.x; r <= rows; r += gridDim.x * blockDim.x)
-        row_start[r] = (unsigned int)lower_bound_key<K>(keys, n, (K)r << b);
-}
-
-// upper_bound(keys, t) using the row directory: keys of t's row lie in
-// [row_start[r], row_start[r+1]) sorted by x.  `hint` is where t probably
-// sits within its row -- the searching voxel's own offset within its row,
-// since neighbouring rows of a surface hold similar runs of x.  Two probes
-// around the guess settle most lookups; otherwise a binary search of the
-// side the probes leave.  The result does not depend on the hint.
-template <typename K>
-__device__ __forceinline__ unsigned int upper_bound_row(const K* __restrict__ keys,
-                                                        const unsigned int* __restrict__ rs,
-                                                        K t, unsigned int n, const Codec<K>& cd,
-                                                        unsigned int hint) {
-    const unsigned long long r = cd.row(t);
-    // a neighbour of a voxel on the last z slice lies past every key
-    if (r >= (1ull << (2 * cd.b))) return n;
-    unsigned int lo = rs[r], hi = rs[r + 1];
-    if (lo == hi) return lo;
-    const unsigned int g = hint < hi - lo ? lo + hint : hi;
-    const bool right = g < hi && keys[g] <= t;   // the answer lies above g
-    const bool left = g > lo && keys[g - 1] > t;  // ... or below g
-    if (right) lo = g + 1;
-    else if (left) hi = g - 1;  // keys[g - 1] > t: the answer is at most g - 1
-    else return g;
-    while (lo < hi) {
-        unsigned int mid = (lo + hi) >> 1;
-        if (keys[mid] <= t) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// neighbour pointer position after the reference's walk (see file comment)
-template <typename K>
-__device__ __forceinline__ unsigned int walk_ptr(const K* keys, const unsigned int* rs, K t, unsigned int n,
-                                                 const Codec<K>& cd, unsigned int hint) {
-    unsigned int p = upper_bound_row<K>(keys, rs, t, n, cd, hint) - 1u;
-    return p < n - 2 ? p : n - 2;
-}
-
 __device__ __forceinline__ float vdist(float2 v) { return fdiv(v.x, v.y); }  // Voxel::Distance
-
-// Packed per-voxel flags: bits 0-2 the vertex axes, 3-5 the triangle count,
-// 6-13 the marching-cubes case, 14-24 the voxel's first vertex within its
-// classification tile (at most 3 x 1024 = 3072).
-__device__ __forceinline__ unsigned int f_axes(unsigned int f) { return f & 7u; }
-__device__ __forceinline__ unsigned int f_tris(unsigned int f) { return (f >> 3) & 7u; }
-__device__ __forceinline__ unsigned int f_case(unsigned int f) { return (f >> 6) & 0xffu; }
-__device__ __forceinline__ unsigned int f_vofs(unsigned int f) { return f >> 14; }
 
 // exclusive scan of one 64-bit value per thread over a CTA of kT threads;
 // the CTA's total to *total
@@ -144,47 +78,6 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long
     return before + inc - x;
 }
 
-struct Cube {
-    unsigned int idx[8];  // voxel index of each corner (valid where found)
-    float2 val[8];        // Voxel() = (0,0) where not found
-};
-
-// Corner lookups of Mesher.cpp:122-132 (corners 0,1,2,4) and, when
-// kTris, :174-181 (corners 3,5,6,7).  Corner c = (c&1, c>>1&1, c>>2) in the
-// reference's voxels[] numbering: self, +x, +y, +xy, +z, +xz, +yz, +xyz.
-template <bool kTris, typename K>
-__device__ __forceinline__ void load_cube(const K* __restrict__ keys,
-                                          const float2* __restrict__ vals,
-                                          const unsigned int* __restrict__ rs, unsigned int n,
-                                          unsigned int i, Cube& c, const Codec<K>& cd) {
-    const K key = keys[i];
-    const float2 zero = make_float2(0.0f, 0.0f);
-    // this voxel's offset within its row, where its neighbours likely sit in theirs
-    const unsigned int hint = i - rs[cd.row(key)];
-    c.idx[0] = i;
-    c.val[0] = vals[i];
-    c.idx[1] = i + 1;
-    c.val[1] = keys[i + 1] == key + cd.pack(1, 0, 0) ? vals[i + 1] : zero;
-    const unsigned int iTop = walk_ptr<K>(keys, rs, key + cd.pack(0, 1, 0), n, cd, hint);
-    const unsigned int iFront = walk_ptr<K>(keys, rs, key + cd.pack(0, 0, 1), n, cd, hint);
-    c.idx[2] = iTop;
-    c.val[2] = keys[iTop] == key + cd.pack(0, 1, 0) ? vals[iTop] : zero;
-    c.idx[4] = iFront;
-    c.val[4] = keys[iFront] == key + cd.pack(0, 0, 1) ? vals[iFront] : zero;
-    if (kTris) {
-        const unsigned int iFT = walk_ptr<K>(keys, rs, key + cd.pack(0, 1, 1), n, cd, hint);
-        c.idx[6] = iFT;
-        c.val[6] = keys[iFT] == key + cd.pack(0, 1, 1) ? vals[iFT] : zero;
-        c.idx[3] = iTop + 1;
-        c.val[3] = keys[iTop + 1] == key + cd.pack(1, 1, 0) ? vals[iTop + 1] : zero;
-        c.idx[5] = iFront + 1;
-        c.val[5] = keys[iFront + 1] == key + cd.pack(1, 0, 1) ? vals[iFront + 1] : zero;
-        c.idx[7] = iFT + 1;
-        c.val[7] = keys[iFT + 1] == key + cd.pack(1, 1, 1) ? vals[iFT + 1] : zero;
-    }
-}
-
-// vertex axes of a voxel: bit a set when edge +a carries a vertex
 // Mesher.cpp:140-168's test Distance(self) * Distance(neighbour) <= 0
 // without the divisions where its outcome is certain: for 2^-30 <= |x|, |w|
 // <= 2^30 (both voxels) each quotient x / w is a float of magnitude in
@@ -207,500 +100,6 @@ __device__ __forceinline__ bool dist_negative(float2 v) {
     return vdist(v) < 0.0f;
 }
 
-// Classification reads a voxel through one status byte, computed once per
-// staged voxel: E weight != 0 (the reference's skip test, :172-181), P
-// weight > 0 (the vertex test's neighbour condition, :140-168), N
-// Distance() < 0 (the case bit, :191-199, exact through dist_negative), R
-// operands in in_sign_range, S the quotient's sign (x < 0 != w < 0).  A
-// voxel that is not found reads as status 0, as Voxel() = (0, 0) does.
-constexpr unsigned int kStE = 1, kStP = 2, kStN = 4, kStR = 8, kStS = 16;
-__device__ __forceinline__ unsigned int voxel_status(float2 v) {
-    unsigned int s = 0;
-    if (v.y != 0.0f) s |= kStE;
-    if (v.y > 0.0f) s |= kStP;
-    if (dist_negative(v)) s |= kStN;
-    if (in_sign_range(v)) s |= kStR;
-    if ((v.x < 0.0f) != (v.y < 0.0f)) s |= kStS;
-    return s;
-}
-
-// the status of every voxel (one byte each, four per 32-bit store)
-__global__ void __launch_bounds__(kThreads) k_mesh_status(const float2* __restrict__ vals,
-                                                          const unsigned int* __restrict__ n_dev,
-                                                          unsigned int* __restrict__ status4) {
-    const unsigned int n = *n_dev;
-    const float4* v2 = reinterpret_cast<const float4*>(vals);  // two voxels per vector
-    for (unsigned int q = blockIdx.x * blockDim.x + threadIdx.x; q < (n + 3u) / 4u; q += gridDim.x * blockDim.x) {
-        const unsigned int i = 4u * q;
-        unsigned int word = 0;
-        if (i + 4u <= n) {
-            const float4 a = __ldg(v2 + 2 * q), b = __ldg(v2 + 2 * q + 1);
-            word = voxel_status(make_float2(a.x, a.y)) | voxel_status(make_float2(a.z, a.w)) << 8 |
-                   voxel_status(make_float2(b.x, b.y)) << 16 | voxel_status(make_float2(b.z, b.w)) << 24;
-        } else {
-            for (unsigned int k = 0; i + k < n; ++k) word |= voxel_status(vals[i + k]) << (8u * k);
-        }
-        status4[q] = word;
-    }
-}
-
-// One live voxel's flags without the tile offset -- vertex axes, triangle
-// count, case -- from its corners' statuses st and indices idx (corner c =
-// (c&1, c>>1&1, c>>2): self, +x, +y, +xy, +z, +xz, +yz, +xyz).  A vertex
-// test whose operands are out of in_sign_range takes the reference's
-// divisions on the voxels themselves.
-template <bool kTris>
-__device__ __forceinline__ unsigned int classify_status(const unsigned int (&st)[8], const unsigned int (&idx)[8],
-                                                        const float2* __restrict__ vals, const uint64_t* s_mc) {
-    unsigned int f = 0;
-    const unsigned int s0 = st[0];
-    const int nb[3] = {1, 2, 4};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const unsigned int o = st[nb[a]];
-        if (!(o & kStP)) continue;
-        bool cross;
-        if (s0 & o & kStR) cross = ((s0 ^ o) & kStS) != 0u;
-        else cross = fmul(vdist(vals[idx[0]]), vdist(vals[idx[nb[a]]])) <= 0.0f;
-        if (cross) f |= 1u << a;
-    }
-    if (kTris) {
-        const unsigned int all = st[1] & st[2] & st[3] & st[4] & st[5] & st[6] & st[7];
-        if (all & kStE) {
-            // the reference's corner bit order (Mesher.cpp:191-199)
-            auto neg = [&](int q) { return (st[q] & kStN) ? 1u : 0u; };
-            const unsigned int lut = neg(0) << 2 | neg(1) << 3 | neg(2) << 6 | neg(3) << 7 | neg(4) << 1 |
-                                     neg(5) << 0 | neg(6) << 5 | neg(7) << 4;
-            const unsigned int tris = mc_tri_count_of(s_mc[lut]);
-            if (tris) f |= tris << 3 | lut << 6;
-        }
-    }
-    return f;
-}
-
-// Classification by tiles of kClassTile consecutive voxels.  For a
-// neighbour offset d (+y, +z, +yz) the lookup positions walk_ptr(key_i + d)
-// are non-decreasing in i, so the positions of a run of voxels all lie
-// between those of its first and last voxel.  The +y positions start at the
-// voxel itself, so the tile and its +y lookups are one region (A) from the
-// tile's first voxel on; the +yz positions start at or after the +z ones,
-// so those two offsets share region B.  A tile that spans two z slices gets
-// region B in two ranges, one per slice, since the lookups of the two parts
-// land a whole slice apart.  k_mesh_tile_ranges finds the regions of every
-// tile at once (one thread per tile, searches through the row directory).
-// The classification stages both regions in shared memory with independent
-// coalesced loads -- keys, and the status byte k_mesh_status wrote per voxel
-// in place of its value -- and builds every cube from the staging: one
-// search in the staged keys for a thread's first voxel in a range, a
-// forward walk for its next.  A tile whose regions are longer than the
-// staging holds searches per voxel (load_cube).  Results are identical.
-constexpr int kClassItems = 4;
-constexpr int kClassTile = kThreads * kClassItems;  // 1024 voxels
-constexpr int kStageA = 2048, kStageB = 2048;        // staged keys per region
-// One staging buffer: keys of region A, keys of region B (two ranges), then
-// the status bytes alike.  Copies start on 16-byte boundaries, so each part
-// has room for the alignment shifts and round-ups; every part starts on a
-// 16-byte boundary.  Two buffers: the next tile's copies land in one while
-// the current tile is classified from the other.
-constexpr int kKeyA = kStageA + 8, kKeyB = kStageB + 16, kStA = kStageA + 32, kStB = kStageB + 64;
-template <typename K>
-__host__ __device__ constexpr size_t class_buf_bytes() {
-    return (size_t)(kKeyA + kKeyB) * sizeof(K) + kStA + kStB;
-}
-template <typename K>
-__host__ __device__ constexpr size_t class_smem() {
-    return 2 * class_buf_bytes<K>();
-}
-static_assert(class_buf_bytes<uint32_t>() % 16 == 0 && class_buf_bytes<uint64_t>() % 16 == 0, "16-byte parts");
-static_assert((kKeyA * 4) % 16 == 0 && (kKeyA * 8) % 16 == 0 && kStA % 16 == 0, "16-byte parts");
-
-constexpr unsigned int kStageSpinLimit = 1u << 24;  // polls before a staging wait gives up
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init1(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
-    for (unsigned int i = 0; i < kStageSpinLimit; ++i)
-        if (mbar_try(bar, parity)) return true;
-    return false;
-}
-// `bytes` (a multiple of 16) from global `src` to shared `dst`, both 16-byte
-// aligned, completing on `bar` by transaction bytes
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-
-// Where a tile's staged regions sit in its buffer: per part, the element
-// offset of the aligned copy's start and of the range's first element.
-struct StagedTile {
-    unsigned int ka0, ka;        // region A keys
-    unsigned int sa0, sa;        // region A statuses
-    unsigned int kb0[2], kb[2];  // region B keys, per range
-    unsigned int sb0[2], sb[2];  // region B statuses, per range
-};
-__device__ __forceinline__ unsigned int up_to(unsigned int x, unsigned int m) { return (x + m - 1) / m * m; }
-template <typename K>
-__device__ __forceinline__ StagedTile staged_tile(const MeshTileRange& r, unsigned int i0) {
-    constexpr unsigned int kv = 16 / sizeof(K);  // keys per 16 bytes
-    StagedTile L;
-    L.ka0 = 0;
-    L.ka = i0 % kv;
-    L.sa0 = 0;
-    L.sa = i0 % 16u;
-    unsigned int ko = 0, so = 0;
-#pragma unroll
-    for (int sg = 0; sg < 2; ++sg) {
-        L.kb0[sg] = ko;
-        L.kb[sg] = ko + r.b_lo[sg] % kv;
-        L.sb0[sg] = so;
-        L.sb[sg] = so + r.b_lo[sg] % 16u;
-        if (r.b_len[sg]) {
-            ko = up_to(L.kb[sg] + r.b_len[sg], kv);
-            so = up_to(L.sb[sg] + r.b_len[sg], 16u);
-        }
-    }
-    return L;
-}
-// thread 0: the copies of tile (r, i0) into buffer `buf`, announced on `bar`
-template <typename K>
-__device__ __forceinline__ void stage_tile_async(unsigned char* buf, const K* keys, const unsigned char* status,
-                                                 const MeshTileRange& r, unsigned int i0, uint64_t* bar) {
-    const StagedTile L = staged_tile<K>(r, i0);
-    K* kA = (K*)buf;
-    K* kB = kA + kKeyA;
-    unsigned char* sA = (unsigned char*)(kB + kKeyB);
-    unsigned char* sB = sA + kStA;
-    // the buffer's earlier contents were read through the generic proxy
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    const uint32_t bka = up_to((L.ka + r.a_len) * (unsigned int)sizeof(K), 16u);
-    const uint32_t bsa = up_to(L.sa + r.a_len, 16u);
-    uint32_t bkb[2], bsb[2];
-    uint32_t total = bka + bsa;
-#pragma unroll
-    for (int sg = 0; sg < 2; ++sg) {
-        bkb[sg] = r.b_len[sg] ? up_to((L.kb[sg] - L.kb0[sg] + r.b_len[sg]) * (unsigned int)sizeof(K), 16u) : 0u;
-        bsb[sg] = r.b_len[sg] ? up_to(L.sb[sg] - L.sb0[sg] + r.b_len[sg], 16u) : 0u;
-        total += bkb[sg] + bsb[sg];
-    }
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(total)
-                 : "memory");
-    bulk_g2s(kA + L.ka0, keys + (i0 - L.ka), bka, bar);
-    bulk_g2s(sA + L.sa0, status + (i0 - L.sa), bsa, bar);
-#pragma unroll
-    for (int sg = 0; sg < 2; ++sg)
-        if (r.b_len[sg]) {
-            const unsigned int lo = r.b_lo[sg];
-            bulk_g2s(kB + L.kb0[sg], keys + (lo - (L.kb[sg] - L.kb0[sg])), bkb[sg], bar);
-            bulk_g2s(sB + L.sb0[sg], status + (lo - (L.sb[sg] - L.sb0[sg])), bsb[sg], bar);
-        }
-}
-__device__ __forceinline__ bool tile_fits(const MeshTileRange& r) {
-    return r.a_len <= (unsigned int)kStageA && r.b_len[0] + r.b_len[1] <= (unsigned int)kStageB;
-}
-
-typedef MeshTileRange TileRange;
-
-// Eight lanes per tile.  The z-slice split needs no search: the first key of
-// slice z0 + 1 starts row (z0 + 1) << b of the row directory.  The tile's up
-// to seven neighbour searches are independent and run one per lane.
-constexpr int kRangeLanes = 8;
-
-template <typename K>
-__global__ void k_mesh_tile_ranges(const K* __restrict__ keys, int kb, const unsigned int* __restrict__ rs,
-                                   const unsigned int* __restrict__ n_dev, int with_yz,
-                                   TileRange* __restrict__ ranges, unsigned int max_tiles) {
-    const unsigned int n = *n_dev;
-    const unsigned int tiles = min((n + kClassTile - 1) / kClassTile, max_tiles);
-    const Codec<K> cd(kb);
-    const K dy = cd.pack(0, 1, 0), dz = cd.pack(0, 0, 1), dyz = cd.pack(0, 1, 1);
-    const unsigned int lane = threadIdx.x & (kRangeLanes - 1);
-    const unsigned int gmask = 0xFFu << ((threadIdx.x & 31u) & ~(unsigned int)(kRangeLanes - 1));
-    const unsigned int groups = gridDim.x * blockDim.x / kRangeLanes;
-    for (unsigned int t = (blockIdx.x * blockDim.x + threadIdx.x) / kRangeLanes; t < tiles; t += groups) {
-        const unsigned int i0 = t * kClassTile;
-        const unsigned int last = min(min(i0 + (unsigned int)kClassTile, n), n - 1u);  // voxels with a cube: < last
-        TileRange r;
-        r.b_lo[0] = r.b_lo[1] = r.b_len[0] = r.b_len[1] = 0u;
-        // region A: the tile and the one after, and every +y position plus one
-        r.a_len = min(i0 + (unsigned int)kClassTile + 1u, n) - i0;
-        r.split = last;
-        if (last > i0) {
-            const K k0 = keys[i0], kl = keys[last - 1];
-            unsigned int split = last;
-            const unsigned int z0 = cd.z(k0), zl = cd.z(kl);
-            if (z0 != zl) {  // a range per z slice when the tile spans exactly two
-                const unsigned int a = rs[cd.row(cd.pack(0, 0, z0 + 1))];  // keys[i0] < keys[a] <= keys[last - 1]
-                if (cd.z(keys[a]) == zl) split = a;
-            }
-            const bool two = split < last;
-            // region B per slice: from the first +z position (clamped) to the
-            // last +z or +yz position plus one
-            K q = kl + dy;
-            bool active = true;
-            switch (lane) {
-                case 1: q = k0 + dz; break;
-                case 2: q = keys[split - 1] + dz; break;
-                case 3: q = keys[split - 1] + dyz; active = with_yz; break;
-                case 4: q = keys[split] + dz; active = two; break;
-                case 5: q = kl + dz; active = two; break;
-                case 6: q = kl + dyz; active = two && with_yz; break;
-                case 7: active = false; break;
-                default: break;
-            }
-            const unsigned int p = active ? upper_bound_row<K>(keys, rs, q, n, cd, 0u) - 1u : 0u;
-            unsigned int w[7];
-#pragma unroll
-            for (int j = 0; j < 7; ++j) w[j] = __shfl_sync(gmask, p, j, kRangeLanes);
-            r.a_len = max(r.a_len, min(w[0] + 1u, n - 1u) + 1u - i0);
-            r.b_lo[0] = min(w[1], n - 2u);
-            r.b_len[0] = min((with_yz ? max(w[2], w[3]) : w[2]) + 1u, n - 1u) - r.b_lo[0] + 1u;
-            if (two) {
-                r.b_lo[1] = min(w[4], n - 2u);
-                r.b_len[1] = min((with_yz ? max(w[5], w[6]) : w[5]) + 1u, n - 1u) - r.b_lo[1] + 1u;
-            }
-            r.split = split;
-        }
-        if (lane == 0) ranges[t] = r;
-    }
-}
-
-template <bool kTris, typename K>
-__global__ void __launch_bounds__(kThreads, 4) k_mesh_classify_tiled(const K* __restrict__ keys, int kb,
-                                                                     const float2* __restrict__ vals,
-                                                                     const unsigned char* __restrict__ status,
-                                                                     const unsigned int* __restrict__ rs,
-                                                                     const unsigned int* __restrict__ n_dev,
-                                                                     const TileRange* __restrict__ ranges,
-                                                                     unsigned int max_tiles,
-                                                                     unsigned int* __restrict__ flags,
-                                                                     unsigned long long* __restrict__ tile_sums,
-                                                                     unsigned int* __restrict__ tile_nflag,
-                                                                     unsigned int* __restrict__ flagged,
-                                                                     uint4* __restrict__ corners,
-                                                                     unsigned long long* __restrict__ error) {
-    constexpr int kD = kTris ? 3 : 2;  // offsets looked up: +y, +z (and +yz)
-    extern __shared__ __align__(16) unsigned char class_mem[];
-    __shared__ __align__(8) uint64_t s_bar[2];  // a staging buffer's copies have landed
-    __shared__ int s_fail;
-    __shared__ uint64_t s_mc[256];
-    if (kTris) mc_table_to_shared(s_mc);
-    const unsigned int n = *n_dev;
-    const Codec<K> cd(kb);
-    const K delta[3] = {cd.pack(0, 1, 0), cd.pack(0, 0, 1), cd.pack(0, 1, 1)};
-    const unsigned int tiles = min((n + kClassTile - 1) / kClassTile, max_tiles);
-    unsigned int issued0 = 0u, issued1 = 0u;  // thread 0: batches of copies issued per buffer
-    if (threadIdx.x == 0) {
-        mbar_init1(&s_bar[0]);
-        mbar_init1(&s_bar[1]);
-        s_fail = 0;
-        // the first tile's copies
-        if (blockIdx.x < tiles && tile_fits(ranges[blockIdx.x])) {
-            stage_tile_async<K>(class_mem, keys, status, ranges[blockIdx.x], blockIdx.x * kClassTile, &s_bar[0]);
-            ++issued0;
-        }
-    }
-    __syncthreads();
-    uint32_t phase0 = 0u, phase1 = 0u;  // per buffer: the parity of its next batch of copies
-    unsigned int it = 0;
-    for (unsigned int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
-        const unsigned int i0 = t * kClassTile;
-        const unsigned int i1 = min(i0 + (unsigned int)kClassTile, n);
-        const TileRange r = ranges[t];
-        const bool fits = tile_fits(r);
-        const unsigned int b = it & 1u;
-        unsigned char* buf = class_mem + b * class_buf_bytes<K>();
-        // the next tile's copies into the other buffer (free: every thread has
-        // passed the previous tile's closing barrier)
-        const unsigned int tn = t + gridDim.x;
-        if (threadIdx.x == 0 && tn < tiles) {
-            const TileRange rn = ranges[tn];
-            if (tile_fits(rn)) {
-                stage_tile_async<K>(class_mem + (b ^ 1u) * class_buf_bytes<K>(), keys, status, rn, tn * kClassTile,
-                                    &s_bar[b ^ 1u]);
-                if (b) ++issued0;
-                else ++issued1;
-            }
-        }
-        if (fits) {
-            const bool ok = mbar_wait_bounded(&s_bar[b], b ? phase1 : phase0);
-            if (!ok) s_fail = 1;
-            if (b) phase1 ^= 1u;
-            else phase0 ^= 1u;
-        }
-        if (__syncthreads_or(s_fail)) break;  // a wait gave up: leave the tile loop (reported below)
-        const StagedTile L = staged_tile<K>(r, i0);
-        const K* s_ka = (const K*)buf + L.ka;                                   // key i0 of region A
-        const unsigned char* s_sa = buf + (kKeyA + kKeyB) * sizeof(K) + L.sa;   // its status
-        const K* kbase = (const K*)buf + kKeyA;
-        const unsigned char* sbase = buf + (kKeyA + kKeyB) * sizeof(K) + kStA;
-        const unsigned int tb = threadIdx.x * kClassItems;  // this thread's first voxel in the tile
-        unsigned int pos[kD], seg[kD];  // running count of a range's staged keys <= key + d; its range
-#pragma unroll
-        for (int d = 0; d < kD; ++d) {
-            pos[d] = 0u;
-            seg[d] = 2u;  // none yet: search
-        }
-        unsigned int fl[kClassItems];
-        uint3 look[kClassItems];  // the +y, +z, +yz lookups, kept for emission
-#pragma unroll
-        for (int j = 0; j < kClassItems; ++j) {
-            fl[j] = 0u;
-            look[j] = make_uint3(0u, 0u, 0u);
-        }
-#pragma unroll
-        for (int j = 0; j < kClassItems; ++j) {
-            const unsigned int i = i0 + tb + j;
-            if (i >= i1) break;
-            unsigned int st[8], idx[8];
-            bool live;
-            if (!fits) {
-                live = i + 1 < n && vals[i].y != 0.0f;
-                if (live) {
-                    Cube c;
-                    load_cube<kTris, K>(keys, vals, rs, n, i, c, cd);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        idx[q] = c.idx[q];
-                        st[q] = (kTris || q == 0 || q == 1 || q == 2 || q == 4) ? voxel_status(c.val[q]) : 0u;
-                    }
-                }
-            } else {
-                const unsigned int s0 = s_sa[tb + j];
-                live = i + 1 < n && (s0 & kStE);
-                if (live) {
-                    const K key = s_ka[tb + j];
-                    idx[0] = i;
-                    st[0] = s0;
-                    idx[1] = i + 1;
-                    st[1] = s_ka[tb + j + 1] == key + cd.pack(1, 0, 0) ? s_sa[tb + j + 1] : 0u;
-                    unsigned int w[kD];  // each lookup's position within its staged range
-                    // region B's range of this voxel (+z, +yz): its keys and statuses
-                    const unsigned int sgb = i >= r.split ? 1u : 0u;
-                    const K* s_kbr = kbase + (sgb ? L.kb[1] : L.kb[0]);
-                    const unsigned char* s_sbr = sbase + (sgb ? L.sb[1] : L.sb[0]);
-#pragma unroll
-                    for (int d = 0; d < kD; ++d) {
-                        // region A for +y (one range, from i0); region B for +z, +yz
-                        const unsigned int sg = d == 0 ? 0u : sgb;
-                        const unsigned int Ln = d == 0 ? r.a_len : (sg ? r.b_len[1] : r.b_len[0]);
-                        const unsigned int lod = d == 0 ? i0 : (sg ? r.b_lo[1] : r.b_lo[0]);
-                        const K* sk = d == 0 ? s_ka : s_kbr;
-                        const K tk = key + delta[d];
-                        unsigned int p = pos[d];
-                        if (seg[d] != sg) {  // the thread's first live voxel in this range: search
-                            unsigned int a = 0, e = Ln;
-                            while (a < e) {
-                                const unsigned int mid = (a + e) >> 1;
-                                if (sk[mid] <= tk) a = mid + 1;
-                                else e = mid;
-                            }
-                            p = a;
-                            seg[d] = sg;
-                        } else {  // later voxels: the positions only move forward
-                            while (p < Ln && sk[p] <= tk) ++p;
-                        }
-                        pos[d] = p;
-                        // walk_ptr = min(n - 2, upper_bound - 1), upper_bound = lo + p
-                        const unsigned int gp = min(lod + p - 1u, n - 2u);
-                        idx[d == 0 ? 2 : (d == 1 ? 4 : 6)] = gp;
-                        w[d] = gp - lod;
-                    }
-                    // corners: +y, +z (+yz) at the lookups, +xy, +xz (+xyz) one past
-                    st[2] = s_ka[w[0]] == key + delta[0] ? s_sa[w[0]] : 0u;
-                    st[4] = s_kbr[w[1]] == key + delta[1] ? s_sbr[w[1]] : 0u;
-                    idx[3] = idx[2] + 1;
-                    idx[5] = idx[4] + 1;
-                    if (kTris) {
-                        st[6] = s_kbr[w[2]] == key + delta[2] ? s_sbr[w[2]] : 0u;
-                        idx[7] = idx[6] + 1;
-                        st[3] = s_ka[w[0] + 1] == key + cd.pack(1, 1, 0) ? s_sa[w[0] + 1] : 0u;
-                        st[5] = s_kbr[w[1] + 1] == key + cd.pack(1, 0, 1) ? s_sbr[w[1] + 1] : 0u;
-                        st[7] = s_kbr[w[2] + 1] == key + cd.pack(1, 1, 1) ? s_sbr[w[2] + 1] : 0u;
-                    } else {
-                        idx[6] = idx[7] = 0u;
-                        st[3] = st[5] = st[6] = st[7] = 0u;
-                    }
-                }
-            }
-            if (live) {
-                fl[j] = classify_status<kTris>(st, idx, vals, s_mc);
-                look[j] = make_uint3(idx[2], idx[4], kTris ? idx[6] : 0u);
-            }
-        }
-        // in-tile offsets of the vertices (into the flags), of the indices
-        // (beside the lookups) and of the voxels with output (their list),
-        // one CTA scan of (output voxels << 48 | indices << 24 | vertices)
-        unsigned int nv = 0, ni = 0, nf = 0;
-#pragma unroll
-        for (int j = 0; j < kClassItems; ++j) {
-            nv += __popc(f_axes(fl[j]));
-            ni += 3u * f_tris(fl[j]);
-            nf += fl[j] ? 1u : 0u;
-        }
-        unsigned long long total;
-        // (no trailing barrier: the next tile's first barrier orders the reuse)
-        const unsigned long long ex = block_exclusive_scan<kThreads, false>(
-            (unsigned long long)nf << 48 | (unsigned long long)ni << 24 | nv, &total);
-        unsigned int vo = (unsigned int)(ex & 0xffffffu), io = (unsigned int)((ex >> 24) & 0xffffffu);
-        unsigned int fo = (unsigned int)(ex >> 48);
-#pragma unroll
-        for (int j = 0; j < kClassItems; ++j) {
-            const unsigned int i = i0 + tb + j;
-            if (i < i1) {
-                flags[i] = fl[j] | vo << 14;
-                if (fl[j]) {
-                    // emission reuses the lookups instead of searching again
-                    corners[i] = make_uint4(look[j].x, look[j].y, look[j].z, io);
-                    flagged[i0 + fo] = i;
-                    ++fo;
-                }
-            }
-            vo += __popc(f_axes(fl[j]));
-            io += 3u * f_tris(fl[j]);
-        }
-        if (threadIdx.x == 0) {
-            tile_sums[t] = (total >> 24 & 0xffffffull) << 32 | (total & 0xffffffull);
-            tile_nflag[t] = (unsigned int)(total >> 48);
-        }
-    }
-    if (s_fail && threadIdx.x == 0) {
-        // a staging wait gave up: report it (the mesh is not emitted) and wait,
-        // bounded, for the copies still in flight before the CTA exits
-        atomicExch(error, 1ull);
-        if (issued0) mbar_wait_bounded(&s_bar[0], (issued0 - 1u) & 1u);
-        if (issued1) mbar_wait_bounded(&s_bar[1], (issued1 - 1u) & 1u);
-    }
-}
-
-// The corners of a flagged voxel from its stored lookups: +x, +xy, +xz and
-// +xyz sit one index past self, +y, +z and +yz (load_cube's walk).  Values
-// are loaded where emission reads them.
-__device__ __forceinline__ void stored_cube(unsigned int i, uint4 cr, unsigned int* idx) {
-    idx[0] = i;
-    idx[1] = i + 1;
-    idx[2] = cr.x;
-    idx[3] = cr.x + 1;
-    idx[4] = cr.y;
-    idx[5] = cr.y + 1;
-    idx[6] = cr.z;
-    idx[7] = cr.z + 1;
-}
-
 // edge e of the cube -> (corner, axis), from localToGlobal (Mesher.cpp:206-218):
 // corners {4, 0, 0, 1, 6, 2, 2, 3, 5, 4, 0, 1} (4 bits each) and axes
 // {0, 2, 0, 2, 0, 2, 0, 2, 1, 1, 1, 1} (2 bits each), decoded in registers
@@ -709,120 +108,773 @@ constexpr unsigned int kEdgeAxes = 0x558888u;
 __device__ __forceinline__ int edge_corner(int e) { return (int)((kEdgeCorners >> (4 * e)) & 15u); }
 __device__ __forceinline__ int edge_axis(int e) { return (int)((kEdgeAxes >> (2 * e)) & 3u); }
 
-// Emission over the voxels with output in ascending order (the tiles'
-// lists end to end), 32 per warp step.  A voxel's first vertex is its
-// tile's vertex offset plus the in-tile offset in its flags, its first index
-// slot its tile's index offset plus the in-tile offset kept beside its
-// lookups.
-template <bool kTris, typename K>
-__global__ void __launch_bounds__(kThreads) k_mesh_emit(const K* __restrict__ keys, int kb,
-                                                        const float2* __restrict__ vals,
-                                                        const unsigned int* __restrict__ n_dev, Geom g,
-                                                        const unsigned int* __restrict__ flags,
-                                                        const uint4* __restrict__ corners,
-                                                        const unsigned long long* __restrict__ tile_ofs,
-                                                        const unsigned int* __restrict__ tile_nflag,
-                                                        const unsigned int* __restrict__ flagged,
-                                                        MeshCounts* __restrict__ mc,
-                                                        unsigned long long vert_cap,
-                                                        unsigned long long idx_cap,
-                                                        unsigned long long missing_bound,
-                                                        const unsigned long long* __restrict__ missing_bound_dev,
-                                                        float* __restrict__ verts,
-                                                        uint32_t* __restrict__ idx,
-                                                        unsigned long long* __restrict__ missing_min) {
-    __shared__ uint64_t s_mc[256];
-    if (kTris) {
-        mc_table_to_shared(s_mc);
-        __syncthreads();
+
+// Distance(a) * Distance(b) <= 0 with the reference's divisions
+__device__ __noinline__ bool cross_exact(const float2* vals, unsigned int a, unsigned int b) {
+    return fmul(vdist(vals[a]), vdist(vals[b])) <= 0.0f;
+}
+
+// Voxels, and then words, are cut into contiguous runs, one per CTA (2048
+// voxels or more to a run of either).  Of voxels, the runs' counts are summed up by every
+// CTA of the next kernel for itself; of words, the last CTA to finish turns the
+// runs' totals into offsets.  Up to 4 and 3 rounds of resident CTAs: runs differ
+// in what they hold, and in one round the longest sets the time (at the size
+// above, build 98 us in one round, 82 in four; classification 130 and 107).
+constexpr unsigned int kVoxelRuns = 2432, kWordRuns = 3648;
+constexpr int kClassThreads = 128;
+constexpr unsigned int kNoWord = 0xffffffffu;
+constexpr unsigned int kBuildGroups = 64, kBuildTile = 32 * kBuildGroups;  // voxels taken at a time
+__device__ __forceinline__ unsigned int run_length(unsigned int n, unsigned int runs, unsigned int whole) {
+    return ((n + runs - 1) / runs + whole - 1u) / whole * whole;
+}
+
+// words that start in each run of voxels; and the row table cleared
+template <typename K>
+__global__ void __launch_bounds__(kThreads) k_word_count(const K* __restrict__ keys,
+                                                         const unsigned int* __restrict__ n_dev,
+                                                         unsigned int* __restrict__ run_words,
+                                                         uint4* __restrict__ rows, unsigned int row_vecs,
+                                                         MeshCounts* __restrict__ mc) {
+    const unsigned int n = *n_dev;
+    for (unsigned int r = blockIdx.x * kThreads + threadIdx.x; r < row_vecs; r += gridDim.x * kThreads)
+        rows[r] = make_uint4(kNoWord, kNoWord, kNoWord, kNoWord);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        mc->missing_min = ~0ull;
+        mc->runs_done = 0u;
     }
+    const unsigned int len = run_length(n, gridDim.x, kBuildTile);
+    const unsigned int lo = min(blockIdx.x * len, n), hi = min(lo + len, n);
+    const unsigned int lane = threadIdx.x & 31u;
+    unsigned int cnt = 0;
+#pragma unroll 4
+    for (unsigned int i0 = lo; i0 < hi; i0 += 4 * kThreads) {
+        const unsigned int i = i0 + 4 * threadIdx.x;
+        K k[4] = {};
+        if (i < hi) {  // (reads up to 3 keys past the run: the buffers are padded)
+            const uint4* p = reinterpret_cast<const uint4*>(keys + i);
+#pragma unroll
+            for (int q = 0; q < (int)sizeof(K) / 4; ++q) reinterpret_cast<uint4*>(k)[q] = __ldg(p + q);
+        }
+        K before = __shfl_up_sync(0xffffffffu, k[3], 1);
+        if (lane == 0 && i < hi && i > 0) before = keys[i - 1];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const K b = q ? k[q - 1] : before;
+            if (i + q < hi && (i + q == 0 || (k[q] ^ b) >> 5)) ++cnt;
+        }
+    }
+    __shared__ unsigned int s_cnt[kThreads / 32];
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) s_cnt[threadIdx.x >> 5] = cnt;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned int all = 0;
+        for (int w = 0; w < kThreads / 32; ++w) all += s_cnt[w];
+        run_words[blockIdx.x] = all;
+    }
+}
+
+// Tiles of 2048 voxels (and the 32 after them, where the last word may end),
+// 4 consecutive voxels per thread and load: bits for "a word starts", "keys
+// leave a gap" and the voxel's state, in the order of position, 32 to a group;
+// then a thread per word moves its stretch of those to the keys' bits, one
+// shift per gap-free run of keys.  Reads 12 B
+// per voxel; bound by instructions (100 per 32 voxels) more than by memory: 82
+// us at the size above, of which the reads take 26.
+template <typename K>
+__global__ void __launch_bounds__(kThreads, 4) k_word_build(const K* __restrict__ keys, int kb,
+                                                            const float2* __restrict__ vals,
+                                                            const unsigned int* __restrict__ n_dev,
+                                                            const unsigned int* __restrict__ run_words,
+                                                            unsigned int* __restrict__ rows, MeshWords words) {
+    constexpr unsigned int kWarps = kThreads / 32, kSteps = kBuildTile / (4 * kThreads);  // 128 voxels per warp step
+    __shared__ __align__(16) K s_key[kBuildTile + 32];
+    __shared__ unsigned short s_list[kBuildTile + 1];  // positions where words start, then the last one's end
+    __shared__ unsigned int s_gap[kBuildGroups + 2], s_neg[kBuildGroups + 2];
+    __shared__ unsigned int s_e[kBuildGroups + 2], s_p[kBuildGroups + 2], s_r[kBuildGroups + 2];
+    __shared__ unsigned int s_cnt[kWarps];
+    __shared__ K s_before;
     const unsigned int n = *n_dev;
     const Codec<K> cd(kb);
-    // the counts of the counting passes; outputs that do not fit are not written
-    // (every CTA sees the same counts and returns alike; the host grows and re-emits)
-    const unsigned long long n_verts = mc->n_verts, n_idx = mc->n_idx;
-    if (mc->error) return;  // the classification gave up: nothing to emit (the host reports it)
-    const bool overflow = n_verts > vert_cap || (kTris && n_idx > idx_cap);
-    // the flag describes this emission (an earlier one into smaller buffers may have set it)
-    if (blockIdx.x == 0 && threadIdx.x == 0) mc->overflow = overflow ? 1ull : 0ull;
-    if (overflow) return;
-    // a re-run for the index mapping's stop rule takes its bound from the first run, and only
-    // when that run found a missing vertex
-    if (missing_bound_dev) {
-        missing_bound = *missing_bound_dev;
-        if (missing_bound == ~0ull) return;
+    const unsigned int len = run_length(n, gridDim.x, kBuildTile);
+    const unsigned int lo = min(blockIdx.x * len, n), hi = min(lo + len, n);
+    const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    // words before this run, and all of them
+    unsigned int base;
+    {
+        unsigned int before = 0, all = 0;
+        for (unsigned int c = threadIdx.x; c < gridDim.x; c += kThreads) {
+            const unsigned int w = run_words[c];
+            all += w;
+            if (c < blockIdx.x) before += w;
+        }
+        unsigned long long total;
+        block_exclusive_scan<kThreads>((unsigned long long)all << 32 | before, &total);
+        base = (unsigned int)total;
+        if (blockIdx.x == 0 && threadIdx.x == 0) *words.count = (unsigned int)(total >> 32);
     }
-    // Indices are emitted warp-cooperatively: the warp's 32 voxels stage their
-    // case word, corner indices and first output slot in shared memory, and
-    // all lanes walk the warp's indices together (a lane finds its voxel by a
-    // search over the prefix of the voxels' index counts), so a warp does
-    // not wait on its lane with the most triangles.
+    K* wkey = (K*)words.key;
+    // four bits per lane, eight lanes to a group's 32: to every lane of the group
+    auto join = [&](unsigned int nibble) {
+        unsigned int m = nibble << (4u * (lane & 7u));
+        m |= __shfl_xor_sync(0xffffffffu, m, 1);
+        m |= __shfl_xor_sync(0xffffffffu, m, 2);
+        m |= __shfl_xor_sync(0xffffffffu, m, 4);
+        return m;
+    };
+    const unsigned int p0 = warp * (kSteps * 128u) + 4u * lane;  // this thread's first position in a tile
+    // a tile's loads, issued while the tile before is turned into words
+    K key[kSteps][4], carry = 0, tail_key = 0, tail_prev = 0;
+    float2 v[kSteps][4], tail_val = make_float2(0.0f, 0.0f);
+    auto load = [&](unsigned int t0) {
+#pragma unroll
+        for (int u = 0; u < (int)kSteps; ++u) {
+            const unsigned int i = t0 + p0 + 128u * u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                key[u][q] = 0;
+                v[u][q] = make_float2(0.0f, 0.0f);
+            }
+            if (i < n) {  // (reads up to 3 voxels past the last: the buffers are padded)
+                const uint4* kp = reinterpret_cast<const uint4*>(keys + i);
+#pragma unroll
+                for (int q = 0; q < (int)sizeof(K) / 4; ++q) reinterpret_cast<uint4*>(key[u])[q] = __ldg(kp + q);
+                const float4* vp = reinterpret_cast<const float4*>(vals + i);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) reinterpret_cast<float4*>(v[u])[q] = __ldg(vp + q);
+            }
+        }
+        carry = 0;  // the key before the warp's first
+        const unsigned int i0 = t0 + warp * (kSteps * 128u);
+        if (lane == 0 && i0 > 0 && i0 < n) carry = keys[i0 - 1];
+        if (warp == 0) {  // the group after the tile, a voxel per lane
+            const unsigned int i = t0 + (min(kBuildTile, hi - t0) + 31u) / 32u * 32u + lane;
+            tail_key = tail_prev = 0;
+            tail_val = make_float2(0.0f, 0.0f);
+            if (i < n) {
+                tail_key = keys[i];
+                tail_prev = keys[i - 1];
+                tail_val = vals[i];
+            }
+        }
+    };
+    if (lo < hi) load(lo);
+    for (unsigned int t0 = lo; t0 < hi; t0 += kBuildTile) {
+        const unsigned int t1 = min(t0 + kBuildTile, hi);
+        const unsigned int ng = (t1 - t0 + 31u) / 32u;  // the tile's groups; group ng is the one after
+        if (threadIdx.x == 0) s_before = carry;
+        unsigned int starts[kSteps], gmask[kSteps], words_here = 0;
+#pragma unroll
+        for (int u = 0; u < (int)kSteps; ++u) {
+            const unsigned int pos = p0 + 128u * u, i = t0 + pos;
+            K prev = __shfl_up_sync(0xffffffffu, key[u][3], 1);
+            if (lane == 0) prev = carry;
+            carry = __shfl_sync(0xffffffffu, key[u][3], 31);
+            unsigned int st = 0, gp = 0, ng_ = 0;
+            bool plain = true;  // both operands in the sign rule's range and the weight positive: the usual case
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const K b = q ? key[u][q - 1] : prev;
+                const unsigned int xb = __float_as_uint(v[u][q].x), wb = __float_as_uint(v[u][q].y);
+                st |= (key[u][q] ^ b) >> 5 ? 1u << q : 0u;
+                gp |= key[u][q] != b + 1 ? 1u << q : 0u;
+                ng_ |= xb >> 31 << q;
+                const bool r = (xb & 0x7fffffffu) - 0x30800000u <= 0x4e800000u - 0x30800000u &&
+                               wb - 0x30800000u <= 0x4e800000u - 0x30800000u;
+                plain = plain && (r || i + q >= n);
+            }
+            if (i == 0) st |= 1u;
+            const unsigned int left = i < t1 ? min(t1 - i, 4u) : 0u;  // the tile's voxels among the four
+            starts[u] = st & ((1u << left) - 1u);
+            words_here += __popc(starts[u]);
+            gmask[u] = join(starts[u]);
+            const unsigned int g = pos >> 5;
+            const bool put = (lane & 7u) == 0u && g < ng;
+            const unsigned int gpm = join(gp);
+            unsigned int e = ~0u, p = ~0u, r = ~0u;  // (positions past the last voxel are not read)
+            if (!__all_sync(0xffffffffu, plain)) {
+                unsigned int eb = 0, pb = 0, rb = 0;
+                ng_ = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    eb |= v[u][q].y != 0.0f ? 1u << q : 0u;
+                    pb |= v[u][q].y > 0.0f ? 1u << q : 0u;
+                    rb |= in_sign_range(v[u][q]) ? 1u << q : 0u;
+                    ng_ |= dist_negative(v[u][q]) ? 1u << q : 0u;
+                }
+                e = join(eb);
+                p = join(pb);
+                r = join(rb);
+            }
+            const unsigned int nm = join(ng_);
+            if (put) {
+                s_gap[g] = gpm;
+                s_neg[g] = nm;
+                s_e[g] = e;
+                s_p[g] = p;
+                s_r[g] = r;
+            }
+            if (g < ng)
+#pragma unroll
+                for (int q = 0; q < (int)sizeof(K) / 4; ++q)
+                    reinterpret_cast<uint4*>(s_key + pos)[q] = reinterpret_cast<const uint4*>(key[u])[q];
+        }
+        words_here = __reduce_add_sync(0xffffffffu, words_here);
+        if (lane == 0) s_cnt[warp] = words_here;
+        unsigned int tail_start = 0;  // warp 0: where words start in the group after the tile
+        if (warp == 0) {
+            tail_start = __ballot_sync(0xffffffffu, t0 + 32u * ng + lane >= n || (tail_key ^ tail_prev) >> 5);
+            const unsigned int gp = __ballot_sync(0xffffffffu, tail_key != tail_prev + 1);
+            const unsigned int e = __ballot_sync(0xffffffffu, tail_val.y != 0.0f);
+            const unsigned int p = __ballot_sync(0xffffffffu, tail_val.y > 0.0f);
+            const unsigned int r = __ballot_sync(0xffffffffu, in_sign_range(tail_val));
+            const unsigned int nm = __ballot_sync(0xffffffffu, dist_negative(tail_val));
+            s_key[32u * ng + lane] = tail_key;
+            if (lane == 0) {
+                s_gap[ng] = gp;
+                s_neg[ng] = nm;
+                s_e[ng] = e;
+                s_p[ng] = p;
+                s_r[ng] = r;
+            }
+        }
+        if (t0 + kBuildTile < hi) load(t0 + kBuildTile);
+        __syncthreads();
+        unsigned int slot0 = 0, total = 0;  // words of the warps before; of the tile
+#pragma unroll
+        for (unsigned int w = 0; w < kWarps; ++w) {
+            const unsigned int c = s_cnt[w];
+            if (w < warp) slot0 += c;
+            total += c;
+        }
+#pragma unroll
+        for (int u = 0; u < (int)kSteps; ++u) {
+            const unsigned int gc = __popc(gmask[u]);
+            unsigned int slot = slot0 + __popc(gmask[u] & ((1u << (4u * (lane & 7u))) - 1u));
+#pragma unroll
+            for (int o = 0; o < 4; ++o) {
+                const unsigned int c = __shfl_sync(0xffffffffu, gc, 8 * o);
+                if (o < (int)(lane >> 3)) slot += c;
+                slot0 += c;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (starts[u] >> q & 1u) s_list[slot++] = (unsigned short)(p0 + 128u * u + q);
+        }
+        if (threadIdx.x == 0)  // where the last word ends: the first start after the tile
+            s_list[total] = (unsigned short)(t1 == n ? n - t0 : t1 - t0 + (unsigned int)__ffs(tail_start) - 1u);
+        __syncthreads();
+        for (unsigned int w = threadIdx.x; w < total; w += kThreads) {
+            const unsigned int pos = s_list[w], cnt = s_list[w + 1] - pos;
+            const unsigned int g = pos >> 5, sh = pos & 31u;
+            const unsigned int ones = 0xffffffffu >> (32u - cnt);
+            auto stretch = [&](const unsigned int* s) { return __funnelshift_r(s[g], s[g + 1], sh) & ones; };
+            unsigned int gap = stretch(s_gap) | 1u;
+            const unsigned int e = stretch(s_e), p = stretch(s_p), ng_ = stretch(s_neg), r = stretch(s_r);
+            unsigned int M = 0, E = 0, P = 0, N = 0, R = 0;
+            while (gap) {
+                const unsigned int a = __ffs(gap) - 1u;  // the run [a, next gap) of positions
+                gap &= gap - 1u;
+                const unsigned int run = ones & (0xffffffffu << a) & (gap ? (gap & (0u - gap)) - 1u : 0xffffffffu);
+                const unsigned int up = ((unsigned int)s_key[pos + a] & 31u) - a;
+                M |= run << up;
+                E |= (e & run) << up;
+                P |= (p & run) << up;
+                N |= (ng_ & run) << up;
+                R |= (r & run) << up;
+            }
+            const unsigned int j = base + w;
+            const K k = s_key[pos], before = pos ? s_key[pos - 1] : s_before;
+            // beside the word's number, the state of its key 0, which the word before looks at
+            wkey[j] = (k >> 5) << 4 | (K)((E & 1u) | (P & 1u) << 1 | (N & 1u) << 2 | (R & 1u) << 3);
+            words.a[j] = make_uint4(t0 + pos, M, E, P);
+            words.b[j] = make_uint2(N, R);
+            if (t0 + pos == 0 || cd.row(k) != cd.row(before)) rows[cd.row(k)] = j;
+        }
+        base += total;
+        __syncthreads();  // the staging is rewritten by the next tile
+    }
+}
+
+// The position in the sorted words of word `t` (a key >> 5), where it is or
+// would be.  `s` is the first word of its row, of which four words from the
+// guess g on (w[], loaded by the caller beside other lookups') mostly settle it.
+template <typename K>
+__device__ __forceinline__ unsigned int find_word(const K* __restrict__ wkey, K t, unsigned int s, unsigned int g,
+                                                  const K (&w)[4], unsigned int n_words, int kb) {
+    unsigned int c = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c += w[q] < t ? 1u : 0u;
+    if (c < 4u && (c > 0u || g == s)) return g + c;
+    unsigned int lo = c ? g + 4u : s, hi = c ? min(s + (1u << (kb - 5)), n_words) : g;  // a row's words: 2^(kb - 5)
+    while (lo < hi) {
+        const unsigned int mid = (lo + hi) >> 1;
+        if ((wkey[mid] >> 4) < t) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// A row of cubes' corners: a word's masks, and those at key + 1
+struct CornerRow {
+    unsigned int start, M, E, P, N, R;  // the word (0 when it is not resident)
+    unsigned int En, Pn, Nn, Rn;
+};
+template <typename K>
+__device__ __forceinline__ CornerRow corner_row(const MeshWords& words, K t, unsigned int q, bool found,
+                                                unsigned int n_words) {
+    CornerRow c = {};
+    const unsigned int q1 = found ? q + 1u : q;
+    K next = 0;
+    if (q1 < n_words) next = ((const K*)words.key)[q1];
+    if (found) {
+        const uint4 a = words.a[q];
+        const uint2 b = words.b[q];
+        c.start = a.x;
+        c.M = a.y;
+        c.E = a.z;
+        c.P = a.w;
+        c.N = b.x;
+        c.R = b.y;
+    }
+    const unsigned int low = next >> 4 == t + 1 ? (unsigned int)next : 0u;  // the next word's key 0
+    c.En = __funnelshift_r(c.E, low, 1u);
+    c.Pn = __funnelshift_r(c.P, low >> 1, 1u);
+    c.Nn = __funnelshift_r(c.N, low >> 2, 1u);
+    c.Rn = __funnelshift_r(c.R, low >> 3, 1u);
+    return c;
+}
+__device__ __forceinline__ unsigned int top_bit(unsigned int m) { return 0x80000000u >> __clz(m); }  // m != 0
+
+// One cube's triangle edges without a vertex: the smallest of their ids into *missing.  Corner c =
+// (c&1, c>>1&1, c>>2), Distance() < 0 in bit c of `neg`; its row is c >> 1, at words q[row].  All
+// corners are resident, and the triangles use the edges whose corners differ in sign.  An edge
+// carries a vertex when its corner is not the last voxel (the walk starts at n - 2), the
+// neighbour has weight > 0 and is not the last voxel unless along +x, and the distances do not
+// have the same sign.
+__device__ __noinline__ void missing_edges(const MeshWords words, const float2* vals, unsigned int n, uint4 q,
+                                           unsigned int bit, unsigned int neg, unsigned long long key,
+                                           unsigned long long dy, unsigned long long dz,
+                                           unsigned long long* missing) {
+    const unsigned int qs[4] = {q.x, q.y, q.z, q.w};
+    unsigned int idx[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const unsigned int b = bit + (c & 1);
+        const uint4 a = words.a[qs[c >> 1] + (b >> 5)];
+        idx[c] = a.x + __popc(a.y & ((1u << (b & 31u)) - 1u));
+    }
+    float d[8], w[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float2 v = vals[idx[c]];
+        d[c] = vdist(v);
+        w[c] = v.y;
+    }
+    unsigned long long first = ~0ull;
+#pragma unroll
+    for (int e = 0; e < 12; ++e) {
+        const int c = edge_corner(e), axis = edge_axis(e), o = c | 1 << axis;
+        if (!((neg >> c ^ neg >> o) & 1u)) continue;
+        const bool has = idx[c] != n - 1u && w[o] > 0.0f && (axis == 0 || idx[o] != n - 1u) &&
+                         fmul(d[c], d[o]) <= 0.0f;
+        if (!has)
+            first = min(first, 3ull * (key + (c & 1) + (c & 2 ? dy : 0ull) + (c & 4 ? dz : 0ull)) +
+                                   (unsigned long long)axis);
+    }
+    if (first != ~0ull) atomicMin(missing, first);
+}
+
+// the reference's corner bit order (Mesher.cpp:191-199), from bit 0 of each corner's mask
+__device__ __forceinline__ unsigned int lut_of(unsigned int c0, unsigned int c1, unsigned int c2, unsigned int c3,
+                                               unsigned int c4, unsigned int c5, unsigned int c6, unsigned int c7) {
+    return (c0 & 1u) << 2 | (c1 & 1u) << 3 | (c2 & 1u) << 6 | (c3 & 1u) << 7 | (c4 & 1u) << 1 | (c5 & 1u) |
+           (c6 & 1u) << 5 | (c7 & 1u) << 4;
+}
+
+// A word per thread.  Of a corner looked up as "at the pointer" the last voxel
+// is never found (the pointers stay at or below n - 2); of one looked up as
+// "pointer plus one" it is.  Bound by latency and by
+// instructions (1000 per 32 words): 107 us at the size above; the voxel per
+// thread before it took 330, with 79 for the passes that prepared it.
+template <bool kTris, typename K>
+__global__ void __launch_bounds__(kClassThreads, 8) k_word_classify(int kb, const float2* __restrict__ vals,
+                                                               const unsigned int* __restrict__ n_dev,
+                                                               const unsigned int* __restrict__ rows, MeshWords words,
+                                                               uint4* __restrict__ run_out,
+                                                               uint2* __restrict__ flagged,
+                                                               MeshCounts* __restrict__ mc) {
+    constexpr int kWarps = kClassThreads / 32;
+    __shared__ uint64_t s_mc[256];
+    __shared__ unsigned int s_nx[kWarps][8][32], s_tri[kWarps][32];
+    __shared__ unsigned int s_sum[kWarps], s_ind[kWarps];
+    __shared__ unsigned short s_item[kWarps][1024];  // lane << 5 | bit
+    if (kTris) mc_table_to_shared(s_mc);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned int n = *n_dev, n_words = *words.count;
+    const K* wkey = (const K*)words.key;
+    const unsigned int len = run_length(n_words, gridDim.x, 32u);
+    const unsigned int lo = min(blockIdx.x * len, n_words), hi = min(lo + len, n_words);
+    const K dy = (K)1 << (kb - 5), dz = (K)1 << (2 * kb - 5);
+    unsigned int verts = 0, inds = 0, flags = 0;  // this run's so far
+    // the run's list of voxels with output starts at its first voxel's slot
+    const unsigned int list0 = lo < hi ? words.a[lo].x : 0u;
+    for (unsigned int j0 = lo; j0 < hi; j0 += kClassThreads) {
+        const unsigned int j = j0 + threadIdx.x;
+        unsigned int vx = 0, vy = 0, vz = 0, tri = 0;
+        unsigned int q2 = 0, q4 = 0, q6 = 0;
+        unsigned int nx[8] = {};  // Distance() < 0 of the eight corners
+        K key = 0;
+        if (j < hi) {
+            key = wkey[j] >> 4;
+            constexpr int kD = kTris ? 3 : 2;  // +y, +z (and +yz)
+            const K t[3] = {key + dy, key + dz, key + dy + dz};
+            // every row's first word, then every row's four words about the guess -- this word's offset
+            // in its own row, as neighbouring rows of a surface hold similar runs -- at once
+            const unsigned int own = rows[key >> (kb - 5)];
+            unsigned int s[kD], g[kD], q[kD];
+            bool f[3] = {};
+            K w[kD][4];
+#pragma unroll
+            for (int d = 0; d < kD; ++d) {
+                const K r = t[d] >> (kb - 5);
+                s[d] = r >> (2 * kb) ? kNoWord : rows[r];
+            }
+            const unsigned int back = j - own > 1u ? j - own - 1u : 0u;
+#pragma unroll
+            for (int d = 0; d < kD; ++d) {
+                g[d] = s[d] == kNoWord ? 0u : min(s[d] + back, n_words - 1u);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    w[d][k] = s[d] != kNoWord && g[d] + k < n_words ? wkey[g[d] + k] >> 4 : ~(K)0;
+            }
+#pragma unroll
+            for (int d = 0; d < kD; ++d) {
+                if (s[d] == kNoWord) {
+                    // an empty row: after it only the next row's first key matters, to the row's last key
+                    const K r1 = (t[d] >> (kb - 5)) + 1;
+                    const bool last = ((t[d] + 1) & (((K)1 << (kb - 5)) - 1)) == 0;
+                    q[d] = last && !(r1 >> (2 * kb)) ? min(rows[r1], n_words) : n_words;
+                } else {
+                    q[d] = find_word<K>(wkey, t[d], s[d], g[d], w[d], n_words, kb);
+                    // (a word beyond the window: looked at again)
+                    f[d] = q[d] < n_words && wkey[q[d]] >> 4 == t[d];
+                }
+            }
+            q2 = q[0];
+            q4 = q[1];
+            if (kTris) q6 = q[kD - 1];
+            const bool f2 = f[0], f4 = f[1], f6 = kTris && f[kD - 1];
+            const CornerRow c0 = corner_row<K>(words, key, j, true, n_words);
+            CornerRow c2 = corner_row<K>(words, key + dy, q2, f2, n_words);
+            CornerRow c4 = corner_row<K>(words, key + dz, q4, f4, n_words);
+            CornerRow c6 = {};
+            if (kTris) c6 = corner_row<K>(words, key + dy + dz, q6, f6, n_words);
+            unsigned int live = c0.E;
+            if (j + 1 == n_words) live &= ~top_bit(c0.M);
+            auto no_last = [&](CornerRow& c, unsigned int q, bool f) {
+                if (f && q + 1 == n_words) {
+                    const unsigned int m = ~top_bit(c.M);
+                    c.E &= m;
+                    c.P &= m;
+                }
+            };
+            no_last(c2, q2, f2);
+            no_last(c4, q4, f4);
+            if (kTris) no_last(c6, q6, f6);
+            // vertices: neighbour weight > 0 and a change of sign; by the divisions where an
+            // operand is out of the sign rule's range
+            auto axis = [&](unsigned int P, unsigned int N, unsigned int R, unsigned int start, unsigned int M,
+                            bool self) {
+                const unsigned int may = live & P;
+                unsigned int v = may & c0.R & R & (c0.N ^ N);
+                unsigned int slow = may & ~(c0.R & R);
+                while (slow) {
+                    const unsigned int b = __ffs(slow) - 1u;
+                    slow &= slow - 1u;
+                    const unsigned int i = c0.start + __popc(c0.M & ((1u << b) - 1u));
+                    const unsigned int o = self ? i + 1u : start + __popc(M & ((1u << b) - 1u));
+                    if (cross_exact(vals, i, o)) v |= 1u << b;
+                }
+                return v;
+            };
+            vx = axis(c0.Pn, c0.Nn, c0.Rn, 0u, 0u, true);
+            vy = axis(c2.P, c2.N, c2.R, c2.start, c2.M, false);
+            vz = axis(c4.P, c4.N, c4.R, c4.start, c4.M, false);
+            if (kTris) {
+                nx[0] = c0.N;
+                nx[1] = c0.Nn;
+                nx[2] = c2.N;
+                nx[3] = c2.Nn;
+                nx[4] = c4.N;
+                nx[5] = c4.Nn;
+                nx[6] = c6.N;
+                nx[7] = c6.Nn;
+                const unsigned int all = live & c0.En & c2.E & c2.En & c4.E & c4.En & c6.E & c6.En;
+                const unsigned int any = nx[0] | nx[1] | nx[2] | nx[3] | nx[4] | nx[5] | nx[6] | nx[7];
+                const unsigned int every = nx[0] & nx[1] & nx[2] & nx[3] & nx[4] & nx[5] & nx[6] & nx[7];
+                tri = all & any & ~every;
+                // A cube whose corners all have weight > 0 and operands in range, and whose last corner
+                // is not the last voxel, has a vertex on every edge its triangles use (the table uses
+                // exactly the edges whose corners differ in sign); the others are looked at edge by edge.
+                const unsigned int good = c0.Pn & c2.P & c2.Pn & c4.P & c4.Pn & c6.P & c6.Pn & c0.R & c0.Rn & c2.R &
+                                          c2.Rn & c4.R & c4.Rn & c6.R & c6.Rn;
+                unsigned int odd = tri & ~good;
+                if (f6 && q6 + 1 == n_words) odd |= tri & top_bit(c6.M) >> 1;
+                if (f6 && q6 + 2 == n_words) odd |= tri & 0x80000000u;  // key + 1 may be the last word's only voxel
+                while (odd) {
+                    const unsigned int b = __ffs(odd) - 1u;
+                    odd &= odd - 1u;
+                    unsigned int neg = 0;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) neg |= (nx[c] >> b & 1u) << c;
+                    missing_edges(words, vals, n, make_uint4(j, q2, q4, q6), b, neg,
+                                  (unsigned long long)key << 5 | b, (unsigned long long)dy << 5,
+                                  (unsigned long long)dz << 5, &mc->missing_min);
+                }
+            }
+        }
+        unsigned int out = vx | vy | vz | tri;  // voxels with output
+        const bool any_out = out != 0u;
+        const unsigned int nv = __popc(vx) + __popc(vy) + __popc(vz);
+        // the run's positions: vertices and listed voxels before this word (both below 2^16 here)
+        const unsigned int mine = (unsigned int)__popc(out) << 16 | nv;
+        unsigned int inc = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (lane == 31) s_sum[warp] = inc;
+        __syncthreads();
+        unsigned int ex = inc - mine, total = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const unsigned int c = s_sum[w];
+            if (w < warp) ex += c;
+            total += c;
+        }
+        // The warp's voxels with output are listed in shared memory and then taken 32 at a time: a
+        // loop over each word's own would wait on the word with the most.
+        const unsigned int at = ex >> 16, at0 = __shfl_sync(0xffffffffu, at, 0);
+        const unsigned int items = __shfl_sync(0xffffffffu, at + __popc(out), 31) - at0;
+        if (kTris) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) s_nx[warp][c][lane] = nx[c];
+            s_tri[warp][lane] = tri;
+        }
+        for (unsigned int o = at - at0; out; ++o) {
+            s_item[warp][o] = (unsigned short)(lane << 5 | (__ffs(out) - 1u));
+            out &= out - 1u;
+        }
+        __syncwarp();
+        unsigned int n_ind = 0;  // the warp's indices so far
+        uint2* list = flagged + list0 + flags + at0;
+        for (unsigned int k0 = 0; k0 < items; k0 += 32u) {
+            const bool valid = k0 + lane < items;
+            const unsigned int it = valid ? s_item[warp][k0 + lane] : 0u, w = it >> 5, b = it & 31u;
+            unsigned int lut = 0, ni = 0;
+            if (kTris) {
+                if (valid && (s_tri[warp][w] >> b & 1u)) {
+                    lut = lut_of(s_nx[warp][0][w] >> b, s_nx[warp][1][w] >> b, s_nx[warp][2][w] >> b,
+                                 s_nx[warp][3][w] >> b, s_nx[warp][4][w] >> b, s_nx[warp][5][w] >> b,
+                                 s_nx[warp][6][w] >> b, s_nx[warp][7][w] >> b);
+                    ni = 3u * mc_tri_count_of(s_mc[lut]);
+                }
+                unsigned int inc = ni;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned int y = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += y;
+                }
+                ni = n_ind + inc - ni;  // the voxel's first index, from the warp's first
+                n_ind += __shfl_sync(0xffffffffu, inc, 31);
+            }
+            if (valid) list[k0 + lane] = make_uint2((j0 + 32u * warp + w - lo) << 13 | b << 8 | lut, ni);
+        }
+        if (j < hi) words.v[j] = make_uint4(vx, vy, vz, verts + (ex & 0xffffu));
+        verts += total & 0xffffu;
+        flags += total >> 16;
+        if (kTris) {
+            if (lane == 0) s_ind[warp] = n_ind;
+            __syncthreads();
+            unsigned int before = inds;
+#pragma unroll
+            for (int w = 0; w < kClassThreads / 32; ++w) {
+                const unsigned int c = s_ind[w];
+                if (w < warp) before += c;
+                inds += c;
+            }
+            if (any_out) words.link[j] = make_uint4(q2, q4, q6, before);
+        } else {
+            if (vy | vz) words.link[j] = make_uint4(q2, q4, 0u, 0u);
+            __syncthreads();  // s_sum is rewritten by the next step
+        }
+    }
+    __shared__ bool s_last;
+    if (threadIdx.x == 0) {
+        run_out[blockIdx.x] = make_uint4(verts, inds, flags, list0);
+        __threadfence();
+        s_last = atomicAdd(&mc->runs_done, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    // totals to offsets, in place; the sums after the last (the loads of a thread's stretch all in flight)
+    __threadfence();
+    constexpr unsigned int kEach = (kWordRuns + kClassThreads - 1) / kClassThreads;
+    const unsigned int each = (gridDim.x + kClassThreads - 1u) / kClassThreads, k0 = each * threadIdx.x;
+    const unsigned int mine = k0 < gridDim.x ? min(each, gridDim.x - k0) : 0u;
+    unsigned long long vi = 0, f = 0, vi_all, f_all;  // indices << 32 | vertices: each below 2^32 under 2^28 voxels
+#pragma unroll
+    for (unsigned int k = 0; k < kEach; ++k) {
+        const uint4 c = k < mine ? __ldcg(run_out + k0 + k) : make_uint4(0u, 0u, 0u, 0u);
+        vi += (unsigned long long)c.y << 32 | c.x;
+        f += c.z;
+    }
+    vi = block_exclusive_scan<kClassThreads>(vi, &vi_all);
+    f = block_exclusive_scan<kClassThreads>(f, &f_all);
+#pragma unroll 8
+    for (unsigned int k = 0; k < mine; ++k) {
+        const uint4 c = __ldcg(run_out + k0 + k);
+        __stcg(run_out + k0 + k, make_uint4((unsigned int)vi, (unsigned int)(vi >> 32), (unsigned int)f, c.w));
+        vi += (unsigned long long)c.y << 32 | c.x;
+        f += c.z;
+    }
+    if (threadIdx.x == 0)
+        run_out[gridDim.x] = make_uint4((unsigned int)vi_all, (unsigned int)(vi_all >> 32), (unsigned int)f_all, 0u);
+}
+
+// Emission over the voxels with output in ascending order (the runs' lists
+// end to end), 32 per warp step.  A voxel's first vertex, and that of each
+// corner of its cube, is counted from the corner's word: the word's first
+// vertex plus the set bits below in its three vertex masks.  139 us at the size
+// above, of it 43 for the bytes; bound by instructions (560 per 32 voxels).  With
+// flags and lookups kept per voxel: 103 us, but run twice for the stop rule.
+template <bool kTris, typename K>
+__global__ void __launch_bounds__(kThreads) k_mesh_emit(int kb, const float2* __restrict__ vals, Geom g,
+                                                        MeshWords words, const uint4* __restrict__ run_out,
+                                                        unsigned int runs,
+                                                        const uint2* __restrict__ flagged,
+                                                        MeshCounts* __restrict__ mc, unsigned long long vert_cap,
+                                                        unsigned long long idx_cap, float* __restrict__ verts,
+                                                        uint32_t* __restrict__ idx) {
+    __shared__ uint64_t s_mc[256];
+    if (kTris) mc_table_to_shared(s_mc);
+    __shared__ unsigned int s_cf[kWordRuns + 1];  // the runs' first listed voxels
+    for (unsigned int k = threadIdx.x; k <= runs; k += kThreads) s_cf[k] = run_out[k].z;
+    __syncthreads();
+    const unsigned int n_verts = run_out[runs].x, n_idx = run_out[runs].y, n_out = s_cf[runs];
+    // outputs that do not fit are not written (every CTA returns alike; the host grows and re-emits)
+    const bool overflow = n_verts > vert_cap || (kTris && n_idx > idx_cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        mc->n_verts = n_verts;
+        mc->n_idx = n_idx;
+        mc->overflow = overflow ? 1ull : 0ull;
+    }
+    if (overflow) return;
+    const unsigned long long bound = kTris ? mc->missing_min : ~0ull;  // ids from here on stay ids
+    // Triangles are emitted warp-cooperatively: the warp's 32 voxels stage their
+    // case word, the vertices of their cubes' 12 edges, their first output slot
+    // and a list of their triangles in shared memory, and all lanes walk the
+    // triangles together, so a warp does not wait on its lane with the most.
     constexpr int kWarps = kThreads / 32;
-    __shared__ unsigned int s_cidx[kWarps][8][32];  // corner voxel
-    __shared__ unsigned int s_cvb[kWarps][8][32];   // corner voxel's first vertex
-    __shared__ unsigned char s_cax[kWarps][8][32];  // corner voxel's vertex axes
+    __shared__ unsigned int s_vert[kWarps][12][32];  // each edge's vertex
     __shared__ uint64_t s_mcw[kWarps][32];
     __shared__ unsigned int s_first[kWarps][32];
-    __shared__ unsigned int s_excl[kWarps][33];
+    __shared__ unsigned char s_map[kWarps][160];  // voxel's lane << 3 | triangle (at most 5)
+    const Codec<K> cd(kb);
+    const K* wkey = (const K*)words.key;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned int warps = gridDim.x * kWarps;
-    const unsigned int tiles = (n + kClassTile - 1) / kClassTile;
-    // The voxels with output, counted across tiles (tile_nflag holds each tile's
-    // first position), are cut into chunks of 32; each warp takes a contiguous
-    // run of chunks and finds the tile of each position by walking forward.
-    const unsigned int n_out = (unsigned int)mc->n_flagged;
-    const unsigned int chunks = (n_out + 31u) / 32u;
+    const unsigned int len = run_length(*words.count, runs, 32u);
+    const unsigned int inv = len > 1u ? (unsigned int)(0x100000000ull / len) : 0xffffffffu;
+    auto run_of = [&](unsigned int j) {  // j / len: the estimate is at most one short
+        unsigned int c = __umulhi(j, inv);
+        if (j - c * len >= len) ++c;
+        return c;
+    };
+    // the listed voxels are cut into steps of 32; each warp takes a contiguous run of steps
+    const unsigned int steps = (n_out + 31u) / 32u;
     const unsigned int wid = blockIdx.x * kWarps + warp;
-    const unsigned int cbeg = (unsigned int)((unsigned long long)chunks * wid / warps);
-    const unsigned int cend = (unsigned int)((unsigned long long)chunks * (wid + 1) / warps);
-    unsigned int tile = 0;
-    if (cbeg < cend) {  // the warp's first tile: the last with a first position <= 32 cbeg
-        unsigned int a = 0, b = tiles;
+    const unsigned int cbeg = (unsigned int)((unsigned long long)steps * wid / warps);
+    const unsigned int cend = (unsigned int)((unsigned long long)steps * (wid + 1) / warps);
+    unsigned int run = 0;
+    if (cbeg < cend) {  // the warp's first run of words: the last with a first position <= 32 cbeg
+        unsigned int a = 0, b = runs;
         while (a + 1 < b) {
             const unsigned int mid = (a + b) >> 1;
-            if (tile_nflag[mid] <= 32u * cbeg) a = mid;
+            if (s_cf[mid] <= 32u * cbeg) a = mid;
             else b = mid;
         }
-        tile = a;
+        run = a;
     }
-    for (unsigned int ch = cbeg; ch < cend; ++ch) {
+    // a step's listed voxels, loaded a step ahead
+    unsigned int rl_next = 0;
+    uint2 item_next = make_uint2(0u, 0u);
+    auto next_items = [&](unsigned int ch) {
         const unsigned int gpos = 32u * ch + lane;
-        const bool valid = gpos < n_out;
-        unsigned int tl = tile;
-        if (valid)
-            while (tile_nflag[tl + 1] <= gpos) ++tl;  // tile_nflag[tiles] = n_out > gpos
-        tile = __shfl_sync(0xffffffffu, tl, 31);      // positions only move forward
-        const unsigned int i = valid ? flagged[tl * kClassTile + (gpos - tile_nflag[tl])] : 0u;
-        const unsigned int f = valid ? flags[i] : 0u;
-        const unsigned long long tofs = valid ? tile_ofs[tl] : 0ull;
-        unsigned int cidx[8];
-        uint4 cr = make_uint4(0u, 0u, 0u, 0u);
-        if (f) {
-            cr = corners[i];
-            stored_cube(i, cr, cidx);
+        const bool valid = ch < cend && gpos < n_out;
+        rl_next = run;
+        if (valid) {
+            while (s_cf[rl_next + 1] <= gpos) ++rl_next;  // s_cf[runs] = n_out > gpos
+            item_next = flagged[run_out[rl_next].w + (gpos - s_cf[rl_next])];
         }
-        const unsigned int axes = f_axes(f);
+        run = __shfl_sync(0xffffffffu, rl_next, 31);  // positions only move forward
+    };
+    next_items(cbeg);
+    for (unsigned int ch = cbeg; ch < cend; ++ch) {
+        const bool valid = 32u * ch + lane < n_out;
+        const unsigned int rl = rl_next;
+        const uint2 item = valid ? item_next : make_uint2(0u, 0u);
+        next_items(ch + 1u);
+        const unsigned int j = rl * len + (item.x >> 13), bit = item.x >> 8 & 31u, lut = item.x & 0xffu;
+        const unsigned int lt = (1u << bit) - 1u;
+        uint4 v0 = make_uint4(0u, 0u, 0u, 0u), a0 = v0, link = v0;
+        K key = 0;
+        uint4 ofs = make_uint4(0u, 0u, 0u, 0u);
+        if (valid) {
+            ofs = run_out[rl];
+            v0 = words.v[j];
+            a0 = words.a[j];
+            key = wkey[j] >> 4 << 5 | (K)bit;
+            link = words.link[j];
+        }
+        const unsigned int axes = (v0.x >> bit & 1u) | (v0.y >> bit & 1u) << 1 | (v0.z >> bit & 1u) << 2;
+        // a voxel's first vertex: its word's, plus those of the word's voxels below
+        auto rank = [](const uint4& v, unsigned int below) {
+            return v.w + __popc(v.x & below) + __popc(v.y & below) + __popc(v.z & below);
+        };
         // vertices (Mesher.cpp:134-168): at most three per voxel, by the voxel's lane
         if (axes) {
-            const K key = keys[i];
-            const unsigned int vbase = (unsigned int)(tofs & 0xffffffffu) + f_vofs(f);
+            const unsigned int vbase = ofs.x + rank(v0, lt);
             const unsigned int nv = __popc(axes);
-            const unsigned long long first =
-                kTris ? vbase : n_verts - vbase - nv;  // ascending ids / generation order
+            const unsigned int first = kTris ? vbase : n_verts - vbase - nv;  // ascending ids / generation order
             const float cx = fadd(fmul((float)(int)cd.x(key), g.vlen), g.center_off);
             const float cy = fadd(fmul((float)(int)cd.y(key), g.vlen), g.center_off);
             const float cz = fadd(fmul((float)(int)cd.z(key), g.vlen), g.center_off);
-            const float dself = vdist(vals[i]);
-            const int nb[3] = {1, 2, 4};
+            const unsigned int self = a0.x + __popc(a0.y & lt);
+            unsigned int nb[3];  // the neighbours' voxels (a flagged axis: the neighbour exists)
+            nb[0] = self + 1u;
+            uint4 ay = make_uint4(0u, 0u, 0u, 0u), az = ay;
+            if (axes & 2u) ay = words.a[link.x];
+            if (axes & 4u) az = words.a[link.y];
+            nb[1] = ay.x + __popc(ay.y & lt);
+            nb[2] = az.x + __popc(az.y & lt);
+            const float dself = vdist(vals[self]);
+            float2 vn[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                if (axes >> a & 1u) vn[a] = vals[nb[a]];
             unsigned int r = 0;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (!(axes >> a & 1u)) continue;
-                const float dn = vdist(vals[cidx[nb[a]]]);  // a flagged axis: the neighbour exists
+                const float dn = vdist(vn[a]);
                 const float t = fmul(fdiv(fabsf(dself), fadd(fabsf(dself), fabsf(dn))), g.vlen);
                 float p[3] = {cx, cy, cz};
                 p[a] = fadd(p[a], t);
-                float* o = verts + 3 * (first + r);
+                float* o = verts + 3 * (unsigned long long)(first + r);
                 o[0] = p[0];
                 o[1] = p[1];
                 o[2] = p[2];
@@ -830,8 +882,9 @@ __global__ void __launch_bounds__(kThreads) k_mesh_emit(const K* __restrict__ ke
             }
         }
         if constexpr (kTris) {
-            const unsigned int ni = 3u * f_tris(f);
-            unsigned int inc = ni;
+            const uint64_t mcw = s_mc[lut];
+            const unsigned int nt = valid ? mc_tri_count_of(mcw) : 0u;
+            unsigned int inc = nt;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const unsigned int y = __shfl_up_sync(0xffffffffu, inc, o);
@@ -840,248 +893,166 @@ __global__ void __launch_bounds__(kThreads) k_mesh_emit(const K* __restrict__ ke
             const unsigned int total = __shfl_sync(0xffffffffu, inc, 31);
             if (total == 0u) continue;  // warp-uniform
             __syncwarp();  // the previous round's readers are done with the staging
-            s_excl[warp][lane] = inc - ni;
-            if (lane == 31) s_excl[warp][32] = inc;
-            if (ni) {
-                s_mcw[warp][lane] = s_mc[f_case(f)];  // the case's triangle edges
+            if (nt) {
+                for (unsigned int t = 0; t < nt; ++t) s_map[warp][inc - nt + t] = (unsigned char)(lane << 3 | t);
+                s_mcw[warp][lane] = mcw;  // the case's triangle edges
                 // generation order: voxels descending
-                s_first[warp][lane] = (unsigned int)(n_idx - ((tofs >> 32) + cr.w) - ni);
-                // each corner voxel's vertex axes and first vertex: independent loads
-                unsigned int cf[8];
-                unsigned long long co[8];
+                s_first[warp][lane] = n_idx - (ofs.y + link.w + item.y) - 3u * nt;
+                // The corners' first vertices and axes, by rows along x: corner 2k and, along x from it,
+                // 2k + 1 (in the next word when the voxel is its word's last key)
+                const unsigned int q[4] = {j, link.x, link.y, link.z};
+                uint4 v[4];
+                unsigned int first[8], ax[8];
+                v[0] = v0;
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    cf[k] = flags[cidx[k]];
-                    co[k] = tile_ofs[cidx[k] / kClassTile];
+                for (int k = 1; k < 4; ++k) v[k] = words.v[q[k]];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    ax[2 * k] = (v[k].x >> bit & 1u) | (v[k].y >> bit & 1u) << 1 | (v[k].z >> bit & 1u) << 2;
+                    first[2 * k] = (k ? run_out[run_of(q[k])].x : ofs.x) + rank(v[k], lt);
+                    if (bit == 31u) {
+                        const uint4 w = words.v[q[k] + 1u];
+                        ax[2 * k + 1] = (w.x & 1u) | (w.y & 1u) << 1;
+                        first[2 * k + 1] = run_out[run_of(q[k] + 1u)].x + w.w;
+                    } else {
+                        ax[2 * k + 1] = (v[k].x >> bit >> 1 & 1u) | (v[k].y >> bit >> 1 & 1u) << 1;
+                        first[2 * k + 1] = first[2 * k] + __popc(ax[2 * k]);
+                    }
                 }
+                // each edge's vertex: its corner's first, plus the corner's axes before the edge's
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    s_cidx[warp][k][lane] = cidx[k];
-                    s_cax[warp][k][lane] = (unsigned char)f_axes(cf[k]);
-                    s_cvb[warp][k][lane] = (unsigned int)(co[k] & 0xffffffffu) + f_vofs(cf[k]);
+                for (int e = 0; e < 12; ++e)
+                    s_vert[warp][e][lane] =
+                        first[edge_corner(e)] + __popc(ax[edge_corner(e)] & ((1u << edge_axis(e)) - 1u));
+                // edge ids 3 * key + axis from the stop rule's bound on stay ids: 32 bits wide for
+                // 30-bit keys (as in the reference); for 64-bit keys the rule compares full ids and
+                // an id written in place of a missing vertex keeps its low 32 bits
+                if (3ull * (unsigned long long)(key + cd.pack(1, 1, 1)) + 2ull >= bound) {
+#pragma unroll
+                    for (int e = 0; e < 12; ++e) {
+                        const int c = edge_corner(e);
+                        const unsigned long long id = 3ull * (unsigned long long)(key + cd.pack(c & 1, c >> 1 & 1, c >> 2)) +
+                                                      (unsigned long long)edge_axis(e);
+                        if (id >= bound) s_vert[warp][e][lane] = (unsigned int)id;
+                    }
                 }
             }
             __syncwarp();
-            unsigned long long local_min = ~0ull;
-            for (unsigned int j = lane; j < total; j += 32u) {
-                // v = the last voxel whose exclusive prefix is <= j (it has ni > 0)
-                int v = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1)
-                    if (s_excl[warp][v + step] <= j) v += step;
-                const unsigned int t = j - s_excl[warp][v];
-                const int e = mc_tri_edge_of(s_mcw[warp][v], (int)t);
-                const int corner = edge_corner(e), axis = edge_axis(e);
-                const unsigned int cax = s_cax[warp][corner][v];
-                const bool has = (cax >> axis & 1u) != 0u;
-                // the edge id 3 * key + axis, needed for a missing vertex and on the
-                // stop rule's re-run: 32 bits wide for 30-bit keys (as in the reference);
-                // for 64-bit keys the stop rule compares full ids and an id written in
-                // place of a missing vertex keeps its low 32 bits
-                const bool need_id = !has || missing_bound != ~0ull;
-                const unsigned long long id =
-                    need_id ? 3ull * (unsigned long long)keys[s_cidx[warp][corner][v]] + (unsigned long long)axis
-                            : 0ull;
-                uint32_t outv;
-                if (has) {
-                    outv = s_cvb[warp][corner][v] + __popc(cax & ((1u << axis) - 1u));
-                } else {
-                    outv = (uint32_t)id;
-                    local_min = min(local_min, id);
-                }
-                if (need_id && id >= missing_bound) outv = (uint32_t)id;
-                idx[(unsigned long long)s_first[warp][v] + t] = outv;
+            for (unsigned int o = lane; o < total; o += 32u) {
+                const unsigned int u = s_map[warp][o] >> 3, t = s_map[warp][o] & 7u;
+                const unsigned int e3 = (unsigned int)(s_mcw[warp][u] >> (12u * t));
+                uint32_t* d = idx + (unsigned long long)(s_first[warp][u] + 3u * t);
+                d[0] = s_vert[warp][e3 & 15u][u];
+                d[1] = s_vert[warp][e3 >> 4 & 15u][u];
+                d[2] = s_vert[warp][e3 >> 8 & 15u][u];
             }
-            if (local_min != ~0ull && missing_min) atomicMin(missing_min, local_min);
         }
-    }
-}
-
-// single CTA: exclusive scans (in place) of the classification tiles' packed
-// (index count << 32 | vertex count) and of their counts of voxels with
-// output (the total after the last), the totals to *counts; the packed
-// halves stay below 2^32 for volumes under 2^28 voxels
-constexpr int kSumThreads = 1024, kSumItems = 8, kSumRound = kSumThreads * kSumItems;
-// dynamic shared memory of k_scan_tile_sums: one round of both arrays
-constexpr size_t kSumSmem = (size_t)kSumRound * (sizeof(unsigned long long) + sizeof(unsigned int));
-__global__ void __launch_bounds__(kSumThreads) k_scan_tile_sums(unsigned long long* __restrict__ sums,
-                                                                unsigned int* __restrict__ nflag,
-                                                                const unsigned int* __restrict__ n_dev,
-                                                                MeshCounts* __restrict__ counts) {
-    extern __shared__ __align__(16) unsigned char sum_mem[];
-    unsigned long long* s_v = (unsigned long long*)sum_mem;  // [kSumRound]
-    unsigned int* s_f = (unsigned int*)(s_v + kSumRound);    // [kSumRound]
-    const unsigned int n_tiles = (*n_dev + kClassTile - 1) / kClassTile;
-    unsigned long long carry = 0, fcarry = 0;
-    for (unsigned int b = 0; b < n_tiles; b += kSumRound) {
-        // coalesced loads of the round into shared memory, then each thread
-        // takes kSumItems consecutive entries from there
-        for (unsigned int j = threadIdx.x; j < (unsigned int)kSumRound; j += kSumThreads) {
-            const bool in = b + j < n_tiles;
-            s_v[j] = in ? sums[b + j] : 0ull;
-            s_f[j] = in ? nflag[b + j] : 0u;
-        }
-        __syncthreads();
-        const unsigned int l0 = threadIdx.x * kSumItems;
-        unsigned long long v[kSumItems], s = 0, fs = 0;
-        unsigned int fv[kSumItems];
-#pragma unroll
-        for (int q = 0; q < kSumItems; ++q) {
-            v[q] = s_v[l0 + q];
-            fv[q] = s_f[l0 + q];
-            s += v[q];
-            fs += fv[q];
-        }
-        unsigned long long total, ftotal;
-        unsigned long long run = carry + block_exclusive_scan<kSumThreads>(s, &total);
-        unsigned long long frun = fcarry + block_exclusive_scan<kSumThreads>(fs, &ftotal);
-#pragma unroll
-        for (int q = 0; q < kSumItems; ++q) {
-            s_v[l0 + q] = run;
-            s_f[l0 + q] = (unsigned int)frun;
-            run += v[q];
-            frun += fv[q];
-        }
-        __syncthreads();
-        for (unsigned int j = threadIdx.x; j < (unsigned int)kSumRound; j += kSumThreads)
-            if (b + j < n_tiles) {
-                sums[b + j] = s_v[j];
-                nflag[b + j] = s_f[j];
-            }
-        carry += total;
-        fcarry += ftotal;
-        __syncthreads();  // the staging is reused by the next round
-    }
-    if (threadIdx.x == 0) {
-        nflag[n_tiles] = (unsigned int)fcarry;
-        counts->n_verts = carry & 0xffffffffull;
-        counts->n_idx = carry >> 32;
-        counts->missing_min = ~0ull;
-        counts->overflow = 0ull;
-        counts->n_flagged = fcarry;
     }
 }
 
 }  // namespace
 
 cudaError_t mesh_scratch_reserve(MeshScratch* m, size_t n, int kb) {
-    const size_t rows = ((size_t)1 << (2 * kb)) + 1;
-    if (m->cap >= n && m->vflags && m->rows_cap >= rows) return cudaSuccess;
+    const size_t rows = (size_t)1 << (2 * kb);
+    if (m->cap >= n && m->block && m->rows_cap >= rows) return cudaSuccess;
     if (n < m->cap) n = m->cap;
     mesh_scratch_free(m);
-    size_t cap = n < 1024 ? 1024 : n;
-    const size_t tiles = (cap + kClassTile - 1) / kClassTile + 1;
-    cudaError_t e;
-    if ((e = cudaMalloc(&m->vflags, cap * sizeof(unsigned int)))) return e;
-    if ((e = cudaMalloc(&m->vstatus, (cap + 4) / 4 * 4 + 32))) return e;  // 16-byte copies read past the end
-    if ((e = cudaMalloc(&m->corners, cap * sizeof(uint4)))) return e;
-    if ((e = cudaMalloc(&m->tile_sums, tiles * sizeof(unsigned long long)))) return e;
-    if ((e = cudaMalloc(&m->tile_nflag, tiles * sizeof(unsigned int)))) return e;
-    if ((e = cudaMalloc(&m->flagged, tiles * kClassTile * sizeof(unsigned int)))) return e;
-    if ((e = cudaMalloc(&m->rows, rows * sizeof(unsigned int)))) return e;
-    if ((e = cudaMalloc(&m->tile_ranges, tiles * sizeof(MeshTileRange)))) return e;
+    const size_t cap = n < 1024 ? 1024 : n;
+    const size_t key_words = (size_t)1 << (3 * kb - 5);
+    const size_t words = (cap < key_words ? cap : key_words) + 1;
+    // one allocation, cut into 256-byte aligned arrays
+    size_t size = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = size;
+        size += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t key = take(words * sizeof(uint64_t)), a = take(words * sizeof(uint4)), b = take(words * sizeof(uint2)),
+                 v = take(words * sizeof(uint4)), link = take(words * sizeof(uint4)), flagged = take(cap * sizeof(uint2)),
+                 run_words = take(kVoxelRuns * sizeof(unsigned int)), run_out = take((kWordRuns + 1) * sizeof(uint4)),
+                 row = take(rows * sizeof(unsigned int)), counts = take(sizeof(MeshCounts)),
+                 single = take(2 * sizeof(unsigned int));
+    const cudaError_t e = cudaMalloc(&m->block, size);
+    if (e) return e;
+    unsigned char* p = (unsigned char*)m->block;
+    m->words.key = p + key;
+    m->words.a = (uint4*)(p + a);
+    m->words.b = (uint2*)(p + b);
+    m->words.v = (uint4*)(p + v);
+    m->words.link = (uint4*)(p + link);
+    m->words.count = (unsigned int*)(p + single) + 1;
+    m->flagged = (uint2*)(p + flagged);
+    m->run_words = (unsigned int*)(p + run_words);
+    m->run_out = (uint4*)(p + run_out);
+    m->rows = (unsigned int*)(p + row);
+    m->counts = (MeshCounts*)(p + counts);
+    m->n_dev = (unsigned int*)(p + single);
     m->rows_cap = rows;
-    if ((e = cudaMalloc(&m->counts, sizeof(MeshCounts)))) return e;
-    if ((e = cudaMalloc(&m->n_dev, sizeof(unsigned int)))) return e;
     m->cap = cap;
     return cudaSuccess;
 }
 
 void mesh_scratch_free(MeshScratch* m) {
-    cudaFree(m->vflags);
-    cudaFree(m->vstatus);
-    cudaFree(m->corners);
-    cudaFree(m->tile_sums);
-    cudaFree(m->tile_nflag);
-    cudaFree(m->flagged);
-    cudaFree(m->rows);
-    cudaFree(m->tile_ranges);
-    cudaFree(m->counts);
-    cudaFree(m->n_dev);
+    cudaFree(m->block);
     *m = MeshScratch{};
-}
-
-static int grid_for(size_t n, int sms) {
-    size_t b = (n + kThreads - 1) / kThreads;
-    size_t cap = (size_t)sms * 8;
-    return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
 // The voxel count is read on the device from ms.n_dev (<= n_cap, which sizes
 // the grids), so the passes can be enqueued before the count is known.
-template <typename K>
-static void mesh_count_t(const K* keys, const float2* vals, size_t n_cap, int kb, int with_indices, MeshScratch& ms,
-                         int sms, cudaStream_t st, cudaEvent_t* stage_events) {
-    cudaMemsetAsync(&ms.counts->error, 0, sizeof(unsigned long long), st);  // set by a staging wait that gives up
-    k_row_directory<K><<<grid_for(((size_t)1 << (2 * kb)) + 1, sms), kThreads, 0, st>>>(keys, ms.n_dev, kb, ms.rows);
-    if (stage_events) cudaEventRecord(stage_events[0], st);
-    // tile ranges, then the classification (its grid: up to 8 CTAs per SM, each walking tiles)
-    const unsigned int max_tiles = (unsigned int)((n_cap + kClassTile - 1) / kClassTile);
-    k_mesh_tile_ranges<K><<<grid_for((size_t)max_tiles * kRangeLanes, sms), kThreads, 0, st>>>(
-        keys, kb, ms.rows, ms.n_dev, with_indices, ms.tile_ranges, max_tiles);
-    const int class_grid = (int)(max_tiles < (unsigned int)(sms * 8) ? (max_tiles ? max_tiles : 1) : sms * 8);
-    k_mesh_status<<<grid_for((n_cap + 3) / 4, sms), kThreads, 0, st>>>(vals, ms.n_dev, (unsigned int*)ms.vstatus);
-    if (with_indices) {
-        const size_t smem = class_smem<K>();
-        cudaFuncSetAttribute(k_mesh_classify_tiled<true, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_mesh_classify_tiled<true, K><<<class_grid, kThreads, smem, st>>>(keys, kb, vals, ms.vstatus, ms.rows, ms.n_dev,
-                                                                          ms.tile_ranges, max_tiles, ms.vflags,
-                                                                          ms.tile_sums, ms.tile_nflag, ms.flagged,
-                                                                          ms.corners, &ms.counts->error);
-    } else {
-        const size_t smem = class_smem<K>();
-        cudaFuncSetAttribute(k_mesh_classify_tiled<false, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_mesh_classify_tiled<false, K><<<class_grid, kThreads, smem, st>>>(keys, kb, vals, ms.vstatus, ms.rows, ms.n_dev,
-                                                                           ms.tile_ranges, max_tiles, ms.vflags,
-                                                                           ms.tile_sums, ms.tile_nflag, ms.flagged,
-                                                                           ms.corners, &ms.counts->error);
-    }
-    if (stage_events) cudaEventRecord(stage_events[1], st);
-    cudaFuncSetAttribute(k_scan_tile_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSumSmem);
-    k_scan_tile_sums<<<1, kSumThreads, kSumSmem, st>>>(ms.tile_sums, ms.tile_nflag, ms.n_dev, ms.counts);
+static unsigned int mesh_runs(size_t n_cap, unsigned int most) {
+    const size_t r = (n_cap + kBuildTile - 1) / kBuildTile;
+    return (unsigned int)(r < 1 ? 1 : (r < most ? r : most));
 }
 
-cudaError_t mesh_count_enqueue(const void* keys, int key_bytes, const float2* vals, size_t n_cap, int kb,
-                               int with_indices, MeshScratch& ms, int sms, cudaStream_t st, cudaEvent_t* stage_events) {
+template <typename K>
+static void mesh_count_t(const K* keys, const float2* vals, size_t n_cap, int kb, int with_indices, MeshScratch& ms,
+                         cudaStream_t st, cudaEvent_t* stage_events) {
+    const unsigned int vruns = mesh_runs(n_cap, kVoxelRuns), wruns = mesh_runs(n_cap, kWordRuns);
+    const unsigned int row_vecs = (unsigned int)(((size_t)1 << (2 * kb)) / 4);
+    k_word_count<K><<<vruns, kThreads, 0, st>>>(keys, ms.n_dev, ms.run_words, (uint4*)ms.rows, row_vecs, ms.counts);
+    k_word_build<K><<<vruns, kThreads, 0, st>>>(keys, kb, vals, ms.n_dev, ms.run_words, ms.rows, ms.words);
+    if (stage_events) cudaEventRecord(stage_events[0], st);
+    if (with_indices)
+        k_word_classify<true, K><<<wruns, kClassThreads, 0, st>>>(kb, vals, ms.n_dev, ms.rows, ms.words, ms.run_out,
+                                                              ms.flagged, ms.counts);
+    else
+        k_word_classify<false, K><<<wruns, kClassThreads, 0, st>>>(kb, vals, ms.n_dev, ms.rows, ms.words, ms.run_out,
+                                                               ms.flagged, ms.counts);
+    if (stage_events) cudaEventRecord(stage_events[1], st);
+}
+
+cudaError_t mesh_count_enqueue(const void* keys, int key_bytes, const float2* vals, size_t n_cap, int kb, int with_indices,
+                               MeshScratch& ms, cudaStream_t st, cudaEvent_t* stage_events) {
     if (key_bytes == 8)
-        mesh_count_t<uint64_t>((const uint64_t*)keys, vals, n_cap, kb, with_indices, ms, sms, st, stage_events);
-    else mesh_count_t<uint32_t>((const uint32_t*)keys, vals, n_cap, 10, with_indices, ms, sms, st, stage_events);
+        mesh_count_t<uint64_t>((const uint64_t*)keys, vals, n_cap, kb, with_indices, ms, st, stage_events);
+    else mesh_count_t<uint32_t>((const uint32_t*)keys, vals, n_cap, 10, with_indices, ms, st, stage_events);
     return cudaGetLastError();
 }
 
-// Both emit passes: the first records the smallest edge id without a vertex
-// in ms.counts->missing_min; the second (the index mapping's stop rule)
-// re-emits with that bound and does nothing when the first found none.
+// up to 4 CTAs per SM (all resident), each with 2048 voxels of the volume or more
 template <typename K>
-static void mesh_emit_t(const Geom& g, const K* keys, const float2* vals, size_t n_cap, int with_indices,
-                        MeshScratch& ms, size_t vert_cap, size_t idx_cap, float* verts_dev, uint32_t* idx_dev,
-                        int sms, cudaStream_t st) {
-    unsigned long long* mm = &ms.counts->missing_min;
+static void mesh_emit_t(const Geom& g, const float2* vals, size_t n_cap, int with_indices, MeshScratch& ms,
+                        size_t vert_cap, size_t idx_cap, float* verts_dev, uint32_t* idx_dev, int sms,
+                        cudaStream_t st) {
     const int kb = sizeof(K) == 4 ? 10 : g.kb;
-    const int grid = grid_for(n_cap, sms);
-    if (with_indices) {
-        k_mesh_emit<true, K><<<grid, kThreads, 0, st>>>(keys, kb, vals, ms.n_dev, g, ms.vflags, ms.corners,
-                                                          ms.tile_sums, ms.tile_nflag, ms.flagged, ms.counts, vert_cap, idx_cap, ~0ull, nullptr,
-                                                          verts_dev, idx_dev, mm);
-        k_mesh_emit<true, K><<<grid, kThreads, 0, st>>>(keys, kb, vals, ms.n_dev, g, ms.vflags, ms.corners,
-                                                          ms.tile_sums, ms.tile_nflag, ms.flagged, ms.counts, vert_cap, idx_cap, 0ull, mm,
-                                                          verts_dev, idx_dev, nullptr);
-    } else {
-        k_mesh_emit<false, K><<<grid, kThreads, 0, st>>>(keys, kb, vals, ms.n_dev, g, ms.vflags, ms.corners,
-                                                           ms.tile_sums, ms.tile_nflag, ms.flagged, ms.counts, vert_cap, idx_cap, ~0ull, nullptr,
-                                                           verts_dev, idx_dev, mm);
-    }
+    const size_t want = (n_cap + 2047) / 2048;
+    const unsigned int runs = mesh_runs(n_cap, kWordRuns);  // as the classification's
+    const int grid = (int)(want < 1 ? 1 : (want > (size_t)sms * 4 ? (size_t)sms * 4 : want));
+    if (with_indices)
+        k_mesh_emit<true, K><<<grid, kThreads, 0, st>>>(kb, vals, g, ms.words, ms.run_out, runs, ms.flagged, ms.counts,
+                                                       vert_cap, idx_cap, verts_dev, idx_dev);
+    else
+        k_mesh_emit<false, K><<<grid, kThreads, 0, st>>>(kb, vals, g, ms.words, ms.run_out, runs, ms.flagged, ms.counts,
+                                                        vert_cap, idx_cap, verts_dev, idx_dev);
 }
 
-cudaError_t mesh_emit_enqueue(const Geom& g, const void* keys, int key_bytes, const float2* vals, size_t n_cap,
-                              int with_indices, MeshScratch& ms, size_t vert_cap, size_t idx_cap,
-                              float* verts_dev, uint32_t* idx_dev, int sms, cudaStream_t st) {
+cudaError_t mesh_emit_enqueue(const Geom& g, int key_bytes, const float2* vals, size_t n_cap, int with_indices,
+                              MeshScratch& ms, size_t vert_cap, size_t idx_cap, float* verts_dev, uint32_t* idx_dev,
+                              int sms, cudaStream_t st) {
     if (key_bytes == 8)
-        mesh_emit_t<uint64_t>(g, (const uint64_t*)keys, vals, n_cap, with_indices, ms, vert_cap, idx_cap, verts_dev,
-                              idx_dev, sms, st);
+        mesh_emit_t<uint64_t>(g, vals, n_cap, with_indices, ms, vert_cap, idx_cap, verts_dev, idx_dev, sms, st);
     else
-        mesh_emit_t<uint32_t>(g, (const uint32_t*)keys, vals, n_cap, with_indices, ms, vert_cap, idx_cap, verts_dev,
-                              idx_dev, sms, st);
+        mesh_emit_t<uint32_t>(g, vals, n_cap, with_indices, ms, vert_cap, idx_cap, verts_dev, idx_dev, sms, st);
     return cudaGetLastError();
 }
 
