@@ -444,11 +444,12 @@ __device__ __forceinline__ void apply_depth(float2& val, float d, float w, const
     }
 }
 
-// The TSDF update of four output voxels: the voxels at positions >= upd_end
-// (outside the reference's update range, or no voxel) keep their values.
+// The TSDF update of four output voxels, at positions within their tile: those
+// from upd_end on (outside the reference's update range, or no voxel) keep
+// their values.
 template <bool kU16, typename K>
 __device__ __forceinline__ void update4(const K (&key)[4], float2 (&val)[4],
-                                        const unsigned long long (&pos)[4], unsigned long long upd_end,
+                                        const unsigned int (&pos)[4], unsigned int upd_end,
                                         const FrameConst& fc, const float (&w2c)[16], const Geom& g,
                                         const void* depth) {
     int ix[4];
@@ -603,14 +604,6 @@ __device__ __forceinline__ void ld4(const uint64_t* p, uint64_t (&k)[4]) {
     const ulonglong2 a = __ldcs((const ulonglong2*)p), b = __ldcs((const ulonglong2*)(p + 2));
     k[0] = a.x; k[1] = a.y; k[2] = b.x; k[3] = b.y;
 }
-__device__ __forceinline__ void st4(uint32_t* p, const uint32_t (&k)[4]) {
-    __stcs((uint4*)p, make_uint4(k[0], k[1], k[2], k[3]));
-}
-__device__ __forceinline__ void st4(uint64_t* p, const uint64_t (&k)[4]) {
-    __stcs((ulonglong2*)p, make_ulonglong2(k[0], k[1]));
-    __stcs((ulonglong2*)(p + 2), make_ulonglong2(k[2], k[3]));
-}
-
 template <typename K>
 struct MergeSmem {
     alignas(16) K sA_k[merge_tile<K>() + 8];
@@ -658,133 +651,95 @@ __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, c
         const int len = (int)(d1 - d0);
         const unsigned long long a0 = __ldcg(splits + t), a1 = __ldcg(splits + t + 1);
         const int na = (int)(a1 - a0), nb = len - na;
-        if (nb == 0) {
-            // only resident voxels in this tile: straight streaming, no
-            // barrier.  Each thread loads all its groups of four first, then
-            // projects them, reads their depth pixels together and stores.
-            constexpr int kGroups = kItems / 4;
-            const bool vec = (a0 & 3ull) == 0;
+        // positions within the tile that the update takes (it ends at N1's last whole four)
+        const unsigned int upd = upd_end > d0 ? (unsigned int)min(upd_end - d0, (unsigned long long)kTile) : 0u;
+        // Thread i of the CTA takes entries i, i + 256, ... of a tile: a tile starts at any element of the
+        // resident arrays and its outputs shift by the new keys between them, and single elements side
+        // by side fill whole sectors wherever they start (four consecutive per thread with 128-bit
+        // accesses where both ends are aligned, which one tile in four is, and strided elements
+        // else: the merge of a 640x480 frame 36 us against 31, of a 512x424 frame with 64-bit keys 111
+        // against 77).
+        constexpr int kGroups = kItems / 4;
+        if (nb <= kMergeThreads) {
             K kk[kGroups][4];
             float2 vv[kGroups][4];
 #pragma unroll
-            for (int r = 0; r < kGroups; ++r) {
-                const int j0 = threadIdx.x * 4 + r * kMergeThreads * 4;
-                const unsigned long long ia = a0 + j0;
-                if (j0 >= len) {
+            for (int r = 0; r < kGroups; ++r)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        kk[r][q] = (K)0;
-                        vv[r][q] = make_float2(0.0f, 0.0f);
-                    }
-                } else if (vec && j0 + 4 <= len) {
-                    ld4(A + ia, kk[r]);
-                    const float4 va = __ldcs((const float4*)(Av + ia));
-                    const float4 vb4 = __ldcs((const float4*)(Av + ia + 2));
-                    vv[r][0] = make_float2(va.x, va.y); vv[r][1] = make_float2(va.z, va.w);
-                    vv[r][2] = make_float2(vb4.x, vb4.y); vv[r][3] = make_float2(vb4.z, vb4.w);
-                } else {
-                    const int m = len - j0;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        kk[r][q] = q < m ? __ldcs(A + ia + q) : (K)0;
-                        vv[r][q] = q < m ? __ldcs(Av + ia + q) : make_float2(0.0f, 0.0f);
-                    }
+                for (int q = 0; q < 4; ++q) {
+                    const int li = (int)threadIdx.x + (4 * r + q) * kMergeThreads;
+                    kk[r][q] = li < na ? __ldcs(A + a0 + li) : (K)0;
+                    vv[r][q] = li < na ? __ldcs(Av + a0 + li) : make_float2(0.0f, 0.0f);
                 }
-            }
+            if (nb == 0) {
+                // only resident voxels in this tile: straight streaming, no barrier
 #pragma unroll
-            for (int r = 0; r < kGroups; ++r) {
-                const int j0 = threadIdx.x * 4 + r * kMergeThreads * 4;
-                if (j0 >= len) break;
-                const unsigned long long p = d0 + j0;
-                // positions past the tile are past the update range too
-                // (only the last tile is ragged, and upd_end <= N1)
-                const unsigned long long pos[4] = {p, p + 1, p + 2, p + 3};
-                update4<kU16, K>(kk[r], vv[r], pos, upd_end, fc, w2c, g, depth);
-                if (j0 + 4 <= len) {
-                    st4(outK + p, kk[r]);
-                    __stcs((float4*)(outV + p), make_float4(vv[r][0].x, vv[r][0].y, vv[r][1].x, vv[r][1].y));
-                    __stcs((float4*)(outV + p + 2), make_float4(vv[r][2].x, vv[r][2].y, vv[r][3].x, vv[r][3].y));
-                } else {
-                    const int m = len - j0;
+                for (int r = 0; r < kGroups; ++r) {
+                    unsigned int pos[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) pos[q] = threadIdx.x + (4 * r + q) * kMergeThreads;
+                    if (pos[0] >= (unsigned int)len) break;
+                    // (positions past a ragged last tile are past the update range too)
+                    update4<kU16, K>(kk[r], vv[r], pos, upd, fc, w2c, g, depth);
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
-                        if (q < m) {
-                            outK[p + q] = kk[r][q];
-                            outV[p + q] = vv[r][q];
+                        if (pos[q] < (unsigned int)len) {
+                            __stcs(outK + d0 + pos[q], kk[r][q]);
+                            __stcs(outV + d0 + pos[q], vv[r][q]);
                         }
                 }
+                continue;
             }
-            continue;
-        }
-        if (nb <= kMergeThreads && (int)(a0 & 3ull) + na <= kTile) {
             // Few new keys (the common mixed tile: a median of 16-25 per
-            // 2048 outputs).  Each thread keeps its resident entries in
-            // registers (aligned 128-bit loads from a0 rounded down to 4) and
-            // places each at its A index plus the number of new keys below
-            // it, found in the tile's staged new keys; a new key goes to its
-            // B index plus the number of resident keys below it.  Resident
-            // keys are staged too, for that second search.
-            const unsigned long long ka = a0 & ~3ull;
-            const int koff = (int)(a0 - ka);
+            // 2048 outputs).  A resident key goes to its A index plus the
+            // number of new keys below it, found in the tile's staged new keys: the
+            // numbers at the first and last of each 32 consecutive entries by
+            // one search of the warp's lanes, and within them, where they
+            // differ, by a walk; a new key goes to its B index plus the number
+            // of resident keys below it, which are staged too, for that search.
             const unsigned long long b0 = d0 - a0;
             if ((int)threadIdx.x < nb) sB_k[threadIdx.x] = sort_detail::ld_l2(B + (b0 + threadIdx.x));
-            K kk[2][4];
-            float2 vv[2][4];
-            int li0[2];
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const int ls = (int)threadIdx.x * 4 + r * kMergeThreads * 4;
-                li0[r] = ls - koff;
-                if (ka + (unsigned long long)ls < a1) {  // reads at most 3 entries past a1 (array padding)
-                    ld4(A + ka + ls, kk[r]);
-                    const float4 x0 = __ldcs((const float4*)(Av + ka + ls));
-                    const float4 x1 = __ldcs((const float4*)(Av + ka + ls + 2));
-                    vv[r][0] = make_float2(x0.x, x0.y); vv[r][1] = make_float2(x0.z, x0.w);
-                    vv[r][2] = make_float2(x1.x, x1.y); vv[r][3] = make_float2(x1.z, x1.w);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        kk[r][q] = (K)0;
-                        vv[r][q] = make_float2(0.0f, 0.0f);
-                    }
-                }
+            for (int r = 0; r < kGroups; ++r)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const int li = li0[r] + q;
-                    if (li >= 0 && li < na) sA_k[li] = kk[r][q];
+                    const int li = (int)threadIdx.x + (4 * r + q) * kMergeThreads;
+                    if (li < na) sA_k[li] = kk[r][q];
                 }
-            }
             __syncthreads();
+            const int lane = (int)threadIdx.x & 31, warp0 = (int)threadIdx.x & ~31;
+            int bound = 0;  // lane i: new keys below entry 0 (i < kItems) or entry 31 (i + 16) of the warp's i-th 32
+            {
+                const int li = (lane & 15) * kMergeThreads + warp0 + (lane < 16 ? 0 : 31);
+                if ((lane & 15) < kItems && na > 0) {
+                    const K a = sA_k[min(li, na - 1)];
+                    int lo = 0, hi = nb;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (sB_k[mid] < a) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    bound = lo;
+                }
+                __syncwarp();
+            }
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                unsigned long long pos[4];
-                int rank = -1;  // new keys below the current resident key
+            for (int r = 0; r < kGroups; ++r) {
+                unsigned int pos[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const int li = li0[r] + q;
-                    pos[q] = ~0ull;  // not this tile's: never updated or stored
-                    if (li >= 0 && li < na) {
-                        const K a = kk[r][q];
-                        if (rank < 0) {
-                            int lo = 0, hi = nb;
-                            while (lo < hi) {
-                                const int mid = (lo + hi) >> 1;
-                                if (sB_k[mid] < a) lo = mid + 1;
-                                else hi = mid;
-                            }
-                            rank = lo;
-                        } else {
-                            while (rank < nb && sB_k[rank] < a) ++rank;
-                        }
-                        pos[q] = d0 + (unsigned long long)(li + rank);
-                    }
+                    const int li = (int)threadIdx.x + (4 * r + q) * kMergeThreads;
+                    int rank = __shfl_sync(0xffffffffu, bound, 4 * r + q);
+                    const int most = __shfl_sync(0xffffffffu, bound, 4 * r + q + 16);
+                    while (rank < most && sB_k[rank] < kk[r][q]) ++rank;
+                    pos[q] = li < na ? (unsigned int)(li + rank) : ~0u;  // ~0: no entry
                 }
-                update4<kU16, K>(kk[r], vv[r], pos, upd_end, fc, w2c, g, depth);
+                update4<kU16, K>(kk[r], vv[r], pos, upd, fc, w2c, g, depth);
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (pos[q] != ~0ull) {
-                        __stcs(outK + pos[q], kk[r][q]);
-                        __stcs(outV + pos[q], vv[r][q]);
+                    if (pos[q] != ~0u) {
+                        __stcs(outK + d0 + pos[q], kk[r][q]);
+                        __stcs(outV + d0 + pos[q], vv[r][q]);
                     }
             }
             if ((int)threadIdx.x < nb) {
@@ -799,10 +754,10 @@ __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, c
                     if (sA_k[mid] < key[0]) lo = mid + 1;
                     else hi = mid;
                 }
-                const unsigned long long pos[4] = {d0 + (unsigned long long)(j + lo), ~0ull, ~0ull, ~0ull};
-                update4<kU16, K>(key, val, pos, upd_end, fc, w2c, g, depth);
-                __stcs(outK + pos[0], key[0]);
-                __stcs(outV + pos[0], val[0]);
+                const unsigned int pos[4] = {(unsigned int)(j + lo), ~0u, ~0u, ~0u};
+                update4<kU16, K>(key, val, pos, upd, fc, w2c, g, depth);
+                __stcs(outK + d0 + pos[0], key[0]);
+                __stcs(outV + d0 + pos[0], val[0]);
             }
             __syncthreads();
             continue;
@@ -844,16 +799,16 @@ __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, c
         for (int j0 = threadIdx.x; j0 < len; j0 += 4 * kMergeThreads) {
             K key[4];
             float2 val[4];
-            unsigned long long pos[4];
+            unsigned int pos[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int j = j0 + q * kMergeThreads;
                 key[q] = (K)0;
                 val[q] = make_float2(0.0f, 0.0f);
-                pos[q] = ~0ull;  // no voxel: never updated
+                pos[q] = ~0u;  // no voxel: never updated
                 if (j < len) {
                     const uint16_t src = sSrc[j];
-                    pos[q] = d0 + j;
+                    pos[q] = (unsigned int)j;
                     if (!(src & kFromB)) {
                         key[q] = sA_k[koff + src];
                         val[q] = sA_v[voff + src];
@@ -864,7 +819,7 @@ __device__ __forceinline__ void merge_update_body(DeviceCtl* __restrict__ ctl, c
                     }
                 }
             }
-            update4<kU16, K>(key, val, pos, upd_end, fc, w2c, g, depth);
+            update4<kU16, K>(key, val, pos, upd, fc, w2c, g, depth);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int j = j0 + q * kMergeThreads;
