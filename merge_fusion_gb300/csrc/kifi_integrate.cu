@@ -1065,7 +1065,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_fuse_queue(const FuseJob* __r
                 K* keys = (K*)j.vb.new_keys;
                 K* alt = (K*)j.ss.alt_keys;
                 sort_detail::sort_pass_body<false, K, 8>(pass & 1 ? alt : keys, pass & 1 ? keys : alt, nullptr,
-                                                         nullptr, &j.ctl->n_new, j.ss, pass, c, sm.pass);
+                                                         nullptr, &j.ctl->n_new, j.ss, pass, c, nb, sm.pass);
             } else {
                 const MergeInputs<K> in{(const K*)j.vb.new_keys, nullptr, nullptr, &j.ctl->n_new, true};
                 if (pass == q.passes)
@@ -1157,7 +1157,7 @@ static cudaError_t integrate_enqueue_t(DeviceCtl* ctl, const Geom& g, VolumeBuff
     if (events) cudaEventRecord(events[1], st);
     const void* sorted = nullptr;
     if (!e)
-        e = sort_frame_keys(nk, (int)sizeof(K), kb, &ctl->n_new, ss, &ctl->status, ls.sort_ctas, chained, st, &sorted);
+        e = sort_frame_keys(nk, (int)sizeof(K), kb, &ctl->n_new, ss, &ctl->status, ls.sort_ctas, !ls.beside_tracking, chained, st, &sorted);
     if (e != cudaSuccess) return e;
     if (events) cudaEventRecord(events[2], st);
     MergeInputs<K> in{(const K*)sorted, nullptr, nullptr, &ctl->n_new, true};

@@ -67,7 +67,7 @@ struct SortScratch {
     unsigned int* hist = nullptr;           // [passes][radix] digit counts
     unsigned int* tile_counter = nullptr;   // [passes] dynamic tile ids per pass
     unsigned long long* epoch = nullptr;    // look-back generation tag
-    unsigned long long* lookback = nullptr; // [passes][max_tiles][radix]
+    unsigned long long* lookback = nullptr; // [passes][tiles, then groups of tiles][radix]
     void* alt_keys = nullptr;               // ping-pong buffers, max_n (+pad), 8 bytes per key
     uint32_t* alt_vals = nullptr;
     unsigned int* status = nullptr;         // where timeouts are reported
@@ -95,7 +95,7 @@ cudaError_t sort_keys(void* keys, int key_bytes, int key_bits, uint32_t* vals, c
 // pass counters are already set (see kFrameDigitBits); *sorted receives the
 // buffer holding the result
 cudaError_t sort_frame_keys(void* keys, int key_bytes, int kb, const unsigned int* n_dev, SortScratch& s,
-                            unsigned int* status, int grid_ctas, bool chained, cudaStream_t st, const void** sorted);
+                            unsigned int* status, int grid_ctas, bool alone, bool chained, cudaStream_t st, const void** sorted);
 
 // ------------------------------------------------------------- integrate
 struct VolumeBuffers {

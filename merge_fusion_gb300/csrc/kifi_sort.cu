@@ -16,14 +16,15 @@
 //    counters, bump the look-back generation tag.
 //  * k_sort_histogram: one read of the keys builds all four 256-bin digit
 //    histograms (shared-memory counters, then one global atomic per bin).
-//  * k_sort_pass: persistent CTAs take 2048-key tiles in increasing order
-//    from an atomic counter.  Each warp ranks its keys with
+//  * k_sort_pass: a CTA per tile of 2048 keys, or, where the grid is smaller,
+//    persistent CTAs that take tiles in increasing order from an atomic
+//    counter.  Each warp ranks its keys with
 //    __match_any_sync (a stable rank among lanes holding the same digit),
 //    per-warp digit counts are scanned across warps in shared memory, the
 //    tile's counts are published to a decoupled look-back array and the
-//    tile's global offsets are resolved by walking back over predecessor
-//    tiles.  Keys (and values) are scattered to their final position of the
-//    pass.
+//    tile's global offsets are resolved by walking back over the predecessors
+//    in its group of 16 tiles and then over the groups.  Keys (and values) are
+//    scattered to their final position of the pass.
 // The look-back words pack {generation:32 | status:2 | count:30}, so the
 // count and its flag are one atomic 64-bit store and stale words of an
 // earlier sort are ignored without clearing.  Every wait on a predecessor is
@@ -56,17 +57,25 @@ __global__ void __launch_bounds__(kThreads) k_sort_pass(const K* keys_in, K* __r
                                                         const unsigned int* n_ptr,
                                                         SortScratch s, int pass) {
     __shared__ SortPassSmem<8> sm;
-    sort_pass_body<kWithValues, K, 8>(keys_in, keys_out, vals_in, vals_out, n_ptr, s, pass, blockIdx.x, sm);
+    sort_pass_body<kWithValues, K, 8>(keys_in, keys_out, vals_in, vals_out, n_ptr, s, pass, blockIdx.x, gridDim.x, sm);
 }
 
-// a pass of a frame's new keys
-template <typename K>
-__global__ void __launch_bounds__(kThreads) k_sort_pass_frame(const K* keys_in, K* __restrict__ keys_out,
-                                                              const unsigned int* n_ptr,
-                                                              SortScratch s, int pass) {
-    __shared__ SortPassSmem<kFrameDigitBits<K>> sm;
+// A pass of a frame's new keys, in tiles of 8 kT keys.  A tile takes about 7 us
+// of latencies (keys and histogram 1.5, ranks 1.8, look-back 3, scatter 1.1) and
+// few tiles fill the GPU, so alone a CTA has 512 threads -- half the tiles to
+// look back over -- and all the registers it wants, except with 64-bit keys, where a
+// large frame has more tiles than SMs and two CTAs per SM pay (the three passes of
+// a 640x480 frame 48 -> 39 us, the five of a 512x424 frame with 64-bit keys 103 ->
+// 89; with one look-back level 39 and 103).  Beside tracking CTAs stay small, to
+// fit in where a step's CTAs leave (10 frames at 1024x848: 6141 us, with 512 threads
+// 6220).
+template <typename K, int kT>
+__global__ void __launch_bounds__(kT, sizeof(K) == 8 ? 2 + (kT == kThreads) : 1 + (kT == kThreads))
+    k_sort_pass_frame(const K* keys_in, K* __restrict__ keys_out, const unsigned int* n_ptr, SortScratch s, int pass) {
+    __shared__ SortPassSmem<kFrameDigitBits<K>, kT> sm;
     chain_begin();
-    sort_pass_body<false, K, kFrameDigitBits<K>>(keys_in, keys_out, nullptr, nullptr, n_ptr, s, pass, blockIdx.x, sm);
+    sort_pass_body<false, K, kFrameDigitBits<K>, kT>(keys_in, keys_out, nullptr, nullptr, n_ptr, s, pass, blockIdx.x,
+                                                     gridDim.x, sm);
 }
 
 // ---- batched: every volume of a batch sorts its frame's new keys, one
@@ -96,7 +105,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_pass_batch(const FuseJob* __r
     // passes alternate between the new-key buffer and the sort's spare one
     __shared__ SortPassSmem<8> sm;
     sort_pass_body<false, K, 8>(pass & 1 ? alt : keys, pass & 1 ? keys : alt, nullptr, nullptr, &j.ctl->n_new,
-                                j.ss, pass, blockIdx.x - m.first[v], sm);
+                                j.ss, pass, blockIdx.x - m.first[v], m.first[v + 1] - m.first[v], sm);
 }
 
 // process-wide look-back limits (kifi_sort_set_fault_injection)
@@ -116,7 +125,7 @@ cudaError_t sort_scratch_alloc(SortScratch* s, size_t max_n, cudaStream_t st) {
     if ((e = cudaMalloc(&s->tile_counter, 8 * sizeof(unsigned int)))) return e;
     if ((e = cudaMalloc(&s->epoch, sizeof(unsigned long long)))) return e;
     if ((e = cudaMemsetAsync(s->epoch, 0, sizeof(unsigned long long), st))) return e;
-    size_t lb = (size_t)kSortHistWords * s->max_tiles * sizeof(unsigned long long);
+    size_t lb = (size_t)kSortHistWords * lookback_rows(s->max_tiles) * sizeof(unsigned long long);
     if ((e = cudaMalloc(&s->lookback, lb))) return e;
     if ((e = cudaMemsetAsync(s->lookback, 0, lb, st))) return e;
     if ((e = cudaMalloc(&s->alt_keys, (max_n + 64) * sizeof(uint64_t)))) return e;
@@ -167,12 +176,13 @@ void sort_limits(SortScratch* s) {
 // keys -> alt -> keys ...: the sorted keys end in s.alt_keys after an odd number of passes
 template <typename K>
 static cudaError_t sort_frame_t(K* keys, int passes, const unsigned int* n_dev, SortScratch& s,
-                                unsigned int* status, int grid_ctas, bool chained, cudaStream_t st,
+                                unsigned int* status, int grid_ctas, bool alone, bool chained, cudaStream_t st,
                                 const void** sorted) {
     s.status = status;
     K* alt = (K*)s.alt_keys;
     for (int pass = 0; pass < passes; ++pass) {
-        const cudaError_t e = chain_launch(chained, dim3(grid_ctas), dim3(kThreads), st, k_sort_pass_frame<K>,
+        const cudaError_t e = chain_launch(chained, dim3(grid_ctas), dim3(alone ? 512 : kThreads), st,
+                                           alone ? k_sort_pass_frame<K, 512> : k_sort_pass_frame<K, kThreads>,
                                            (const K*)(pass & 1 ? alt : keys), pass & 1 ? keys : alt, n_dev, s, pass);
         if (e != cudaSuccess) return e;
     }
@@ -181,10 +191,10 @@ static cudaError_t sort_frame_t(K* keys, int passes, const unsigned int* n_dev, 
 }
 
 cudaError_t sort_frame_keys(void* keys, int key_bytes, int kb, const unsigned int* n_dev, SortScratch& s,
-                            unsigned int* status, int grid_ctas, bool chained, cudaStream_t st, const void** sorted) {
+                            unsigned int* status, int grid_ctas, bool alone, bool chained, cudaStream_t st, const void** sorted) {
     if (key_bytes == 8)
-        return sort_frame_t((uint64_t*)keys, frame_sort_passes<uint64_t>(kb), n_dev, s, status, grid_ctas, chained, st, sorted);
-    return sort_frame_t((uint32_t*)keys, frame_sort_passes<uint32_t>(kb), n_dev, s, status, grid_ctas, chained, st, sorted);
+        return sort_frame_t((uint64_t*)keys, frame_sort_passes<uint64_t>(kb), n_dev, s, status, grid_ctas, alone, chained, st, sorted);
+    return sort_frame_t((uint32_t*)keys, frame_sort_passes<uint32_t>(kb), n_dev, s, status, grid_ctas, alone, chained, st, sorted);
 }
 
 template <typename K>

@@ -16,6 +16,8 @@ constexpr int kTile = kThreads * kKeysPerThread;  // 2048
 constexpr int kRadix = 256;
 constexpr unsigned long long kSpinLimit = 1ull << 22;
 constexpr int kLookAhead = 8;  // predecessor look-back words fetched per round
+constexpr unsigned int kGroup = 16;  // tiles whose sum the look-back takes at once
+__host__ __device__ constexpr size_t lookback_rows(size_t max_tiles) { return max_tiles + max_tiles / kGroup + 1; }
 
 constexpr unsigned long long kFlagAggregate = 1ull << 30;
 constexpr unsigned long long kFlagInclusive = 2ull << 30;
@@ -74,23 +76,26 @@ __device__ __forceinline__ void st_volatile_u64(unsigned long long* p, unsigned 
 // One digit pass of kBits bits (radix R = 2^kBits, R / kThreads digits per
 // thread in the scans and the look-back: one for 8-bit digits, four for the
 // frame keys' 10-bit digits).
-template <int kBits>
+template <int kBits, int kT = kThreads>
 struct SortPassSmem {
-    unsigned int warp_hist[kWarps][(1 << kBits) + 1];  // last column: out-of-range keys
+    uint16_t warp_hist[kT / 32][(1 << kBits) + 2];  // last columns: out-of-range keys
     unsigned int digit_base[1 << kBits];
     unsigned int pass_offset[1 << kBits];
-    unsigned int wsum[kWarps];
+    unsigned int wsum[kT / 32];
     unsigned int tile_id;
 };
-template <bool kWithValues, typename K, int kBits>
+template <bool kWithValues, typename K, int kBits, int kT = kThreads>
 __device__ __forceinline__ void sort_pass_body(const K* keys_in, K* __restrict__ keys_out,
                                                const uint32_t* vals_in, uint32_t* __restrict__ vals_out,
                                                const unsigned int* n_ptr, const SortScratch& s,
-                                               int pass, unsigned int blk, SortPassSmem<kBits>& sm) {
+                                               int pass, unsigned int blk, unsigned int nblk,
+                                               SortPassSmem<kBits, kT>& sm) {
     constexpr int R = 1 << kBits;
-    constexpr int D = R / kThreads;
+    constexpr int D = R > kT ? R / kT : 1;         // digits per thread (of the first R threads)
     constexpr int kLA = D == 1 ? kLookAhead : kLookAhead / 2;  // look-back words per digit and round
-    static_assert(D >= 1 && D * kThreads == R, "whole digits per thread");
+    constexpr int kWarps = kT / 32, kTile = kT * kKeysPerThread;
+    static_assert(D * kT == R || kT > R, "whole digits per thread");
+    const bool digits = kT <= R || threadIdx.x < R;  // this thread has digits
     auto& warp_hist = sm.warp_hist;
     auto& digit_base = sm.digit_base;
     auto& pass_offset = sm.pass_offset;
@@ -106,43 +111,24 @@ __device__ __forceinline__ void sort_pass_body(const K* keys_in, K* __restrict__
     if (blk >= n_tiles) return;
     const int shift = pass * kBits;
     const unsigned long long gen = (*s.epoch & 0xffffffffull) << 32;
-    unsigned long long* lb = s.lookback + (size_t)pass * s.max_tiles * R;
+    unsigned long long* lb = s.lookback + (size_t)pass * lookback_rows(s.max_tiles) * R;  // tiles, then groups
 
+    // A CTA per tile where the grid has them, in the order the CTAs start;
+    // else the CTAs take tiles from the counter, so that every tile a CTA
+    // waits for has been taken by one that runs.
+    const bool one_each = n_tiles <= nblk;
     bool have_offsets = false;
     for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) tile_id = atomicAdd(&s.tile_counter[pass], 1u);
-        __syncthreads();
-        const unsigned int tile = tile_id;
-        if (tile >= n_tiles) break;  // (CTAs without a tile leave before any other work)
-        for (int i = threadIdx.x; i < kWarps * (R + 1); i += kThreads) (&warp_hist[0][0])[i] = 0u;
-        if (!have_offsets) {
-            // exclusive scan of this pass's global digit histogram: thread t
-            // holds digits t*D .. t*D + D - 1
-            unsigned int c[D], sum = 0;
-#pragma unroll
-            for (int q = 0; q < D; ++q) {
-                c[q] = __ldcg(s.hist + pass * R + threadIdx.x * D + q);
-                sum += c[q];
-            }
-            unsigned int x = sum;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            if (lane == 31) wsum[warp] = x;
+        if (one_each) {
+            if (have_offsets) break;
+        } else {
             __syncthreads();
-            unsigned int run = x - sum;
-            for (int w = 0; w < warp; ++w) run += wsum[w];
-#pragma unroll
-            for (int q = 0; q < D; ++q) {
-                pass_offset[threadIdx.x * D + q] = run;
-                run += c[q];
-            }
-            have_offsets = true;  // read after the next barrier, before the scatter
+            if (threadIdx.x == 0) tile_id = atomicAdd(&s.tile_counter[pass], 1u);
+            __syncthreads();
         }
-        __syncthreads();  // warp_hist cleared
-
+        const unsigned int tile = one_each ? s.first_tile + blk : tile_id;
+        if (tile >= n_tiles) break;  // (CTAs without a tile leave before any other work)
+        // the tile's keys and, once, the digit histogram: independent reads
         const unsigned int base = tile * kTile + warp * (32 * kKeysPerThread);
         K k[kKeysPerThread];
         uint32_t v[kKeysPerThread];
@@ -154,103 +140,147 @@ __device__ __forceinline__ void sort_pass_body(const K* keys_in, K* __restrict__
             bool ok = i < n;
             k[j] = ok ? ld_l2(keys_in + i) : (K)0;
             if (kWithValues) v[j] = ok ? __ldcg(vals_in + i) : 0u;
-            dig[j] = ok ? (int)((unsigned int)(k[j] >> shift) & (unsigned int)(R - 1)) : R;
         }
+        unsigned int c[D];
+        if (!have_offsets) {
+#pragma unroll
+            for (int q = 0; q < D; ++q) c[q] = digits ? __ldcg(s.hist + pass * R + threadIdx.x * D + q) : 0u;
+        }
+        for (int i = threadIdx.x; i < kWarps * (R + 2) / 2; i += kT)
+            reinterpret_cast<unsigned int*>(&warp_hist[0][0])[i] = 0u;
+        if (!have_offsets) {
+            // exclusive scan of this pass's global digit histogram: thread t
+            // holds digits t*D .. t*D + D - 1
+            unsigned int sum = 0;
+#pragma unroll
+            for (int q = 0; q < D; ++q) sum += c[q];
+            unsigned int x = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) wsum[warp] = x;
+            __syncthreads();
+            unsigned int run = x - sum;
+            for (int w = 0; w < warp; ++w) run += wsum[w];
+#pragma unroll
+            for (int q = 0; q < D; ++q) {
+                if (digits) pass_offset[threadIdx.x * D + q] = run;
+                run += c[q];
+            }
+            have_offsets = true;  // read after the next barrier, before the scatter
+        }
+        __syncthreads();  // warp_hist cleared
         // stable warp-local ranks: lanes with equal digits, in (j, lane) order
+        unsigned int peers[kKeysPerThread];
 #pragma unroll
         for (int j = 0; j < kKeysPerThread; ++j) {
-            unsigned int peers = __match_any_sync(0xffffffffu, dig[j]);
+            dig[j] = base + j * 32 + lane < n ? (int)((unsigned int)(k[j] >> shift) & (unsigned int)(R - 1)) : R;
+            peers[j] = __match_any_sync(0xffffffffu, dig[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < kKeysPerThread; ++j) {
             unsigned int before = warp_hist[warp][dig[j]];
-            rank[j] = before + __popc(peers & lanemask_lt());
+            rank[j] = before + __popc(peers[j] & lanemask_lt());
             __syncwarp();
-            if (lane == __ffs(peers) - 1) warp_hist[warp][dig[j]] = before + __popc(peers);
+            if (lane == __ffs(peers[j]) - 1) warp_hist[warp][dig[j]] = (uint16_t)(before + __popc(peers[j]));
             __syncwarp();
         }
         __syncthreads();
-        // per digit d = threadIdx.x + q * kThreads: counts across warps ->
+        // per digit d = threadIdx.x + q * kT: counts across warps ->
         // exclusive prefix over warps
         unsigned int tile_count[D];
 #pragma unroll
         for (int q = 0; q < D; ++q) {
-            const int d = threadIdx.x + q * kThreads;
+            const int d = threadIdx.x + q * kT;
             unsigned int tc = 0;
-            for (int w = 0; w < kWarps; ++w) {
-                unsigned int c = warp_hist[w][d];
-                warp_hist[w][d] = tc;
+            for (int w = 0; digits && w < kWarps; ++w) {
+                const unsigned int c = warp_hist[w][d];
+                warp_hist[w][d] = (uint16_t)tc;
                 tc += c;
             }
             tile_count[q] = tc;
         }
-        // decoupled look-back for the thread's digits
-        if (tile == 0) {
+        // Decoupled look-back for the thread's digits, in two levels, as a walk
+        // over all predecessors costs a memory latency per kLA of them (13 of
+        // 20 us at 250 tiles): a tile sums up its predecessors within its
+        // group of kGroup, whose last tile publishes the group's sum, and walks
+        // the groups before.
+        unsigned int excl[D];
 #pragma unroll
-            for (int q = 0; q < D; ++q) {
-                const int d = threadIdx.x + q * kThreads;
-                st_volatile_u64(lb + d, gen | kFlagInclusive | tile_count[q]);
-                digit_base[d] = pass_offset[d];
-            }
-        } else {
+        for (int q = 0; q < D; ++q) excl[q] = 0;
+        if (digits) {
 #pragma unroll
             for (int q = 0; q < D; ++q)
-                st_volatile_u64(lb + (size_t)tile * R + threadIdx.x + q * kThreads,
-                                gen | kFlagAggregate | tile_count[q]);
-            // Walk back kLA predecessor words per digit and round: the loads of
-            // a round are independent, so a chain of aggregate-only tiles
-            // costs one memory latency per kLA tiles, not one per tile.
-            unsigned int excl[D];
-            int t[D];
-            unsigned int pending = 0;
-#pragma unroll
-            for (int q = 0; q < D; ++q) {
-                excl[q] = 0;
-                t[q] = (int)tile - 1;
-                pending |= 1u << q;
-            }
+                st_volatile_u64(lb + (size_t)tile * R + threadIdx.x + q * kT, gen | kFlagAggregate | tile_count[q]);
+            const unsigned int group = tile / kGroup;
             unsigned long long spins = 0;
-            while (pending) {
-                unsigned long long w[D][kLA];
+            // words first - i, i in [0, count): waits for each (independent loads, kLA at a time) and adds
+            // them to excl; with `incl` up to the first inclusive one
+            auto look_back = [&](const unsigned long long* words, int first, int count, bool incl) {
+                int t[D];  // words left
+                unsigned int pending = 0;
 #pragma unroll
                 for (int q = 0; q < D; ++q) {
-                    const int d = threadIdx.x + q * kThreads;
-#pragma unroll
-                    for (int i = 0; i < kLA; ++i)
-                        w[q][i] = ((pending >> q) & 1u) && t[q] - i >= 0
-                                      ? ld_volatile_u64(lb + (size_t)(t[q] - i) * R + d)
-                                      : 0ull;
+                    t[q] = count;
+                    if (count > 0) pending |= 1u << q;
                 }
-                // consume each digit's words in order, up to the first inclusive
-                // one or the first one not yet published
-                bool stalled_any = false;
+                while (pending) {
+                    unsigned long long w[D][kLA];
 #pragma unroll
-                for (int q = 0; q < D; ++q) {
-                    if (!((pending >> q) & 1u)) continue;
-                    int used = 0;
-                    bool done = false, stalled = false;
+                    for (int q = 0; q < D; ++q) {
+                        const unsigned long long* at =
+                            words + (size_t)(first - (count - t[q])) * R + threadIdx.x + q * kT;
 #pragma unroll
-                    for (int i = 0; i < kLA; ++i) {
-                        if (done || stalled || t[q] - i < 0) continue;
-                        const unsigned long long x = w[q][i];
-                        if ((x & 0xffffffff00000000ull) != gen || (x & (3ull << 30)) == 0) {
-                            stalled = true;
-                            continue;
-                        }
-                        excl[q] += (unsigned int)(x & kCountMask);
-                        ++used;
-                        done = (x & kFlagInclusive) != 0;
+                        for (int i = 0; i < kLA; ++i)
+                            w[q][i] = ((pending >> q) & 1u) && i < t[q] ? ld_volatile_u64(at - (size_t)i * R) : 0ull;
                     }
-                    t[q] -= used;
-                    if (done || t[q] < 0) pending &= ~(1u << q);
-                    else if (stalled) stalled_any = true;
+                    // consume each digit's words in order, up to the first inclusive
+                    // one or the first one not yet published
+                    bool stalled_any = false;
+#pragma unroll
+                    for (int q = 0; q < D; ++q) {
+                        if (!((pending >> q) & 1u)) continue;
+                        int used = 0;
+                        bool done = false, stalled = false;
+#pragma unroll
+                        for (int i = 0; i < kLA; ++i) {
+                            if (done || stalled || i >= t[q]) continue;
+                            const unsigned long long x = w[q][i];
+                            if ((x & 0xffffffff00000000ull) != gen || (x & (3ull << 30)) == 0) {
+                                stalled = true;
+                                continue;
+                            }
+                            excl[q] += (unsigned int)(x & kCountMask);
+                            ++used;
+                            done = incl && (x & kFlagInclusive) != 0;
+                        }
+                        t[q] -= used;
+                        if (done || t[q] == 0) pending &= ~(1u << q);
+                        else if (stalled) stalled_any = true;
+                    }
+                    if (stalled_any && ++spins > s.spin_limit) {
+                        atomicOr(s.status, KIFI_DEV_ERR_TIMEOUT);
+                        break;
+                    }
                 }
-                if (stalled_any && ++spins > s.spin_limit) {
-                    atomicOr(s.status, KIFI_DEV_ERR_TIMEOUT);
-                    break;
-                }
-            }
+            };
+            unsigned long long* groups = lb + (size_t)s.max_tiles * R;
+            look_back(lb, (int)tile - 1, (int)(tile % kGroup), false);
+            const bool last = tile % kGroup == kGroup - 1;
 #pragma unroll
             for (int q = 0; q < D; ++q) {
-                const int d = threadIdx.x + q * kThreads;
-                st_volatile_u64(lb + (size_t)tile * R + d, gen | kFlagInclusive | ((excl[q] + tile_count[q]) & kCountMask));
+                if (last && group)
+                    st_volatile_u64(groups + (size_t)group * R + threadIdx.x + q * kT,
+                                    gen | kFlagAggregate | ((excl[q] + tile_count[q]) & kCountMask));
+            }
+            look_back(groups, (int)group - 1, (int)group, true);
+#pragma unroll
+            for (int q = 0; q < D; ++q) {
+                const int d = threadIdx.x + q * kT;
+                if (last)
+                    st_volatile_u64(groups + (size_t)group * R + d,
+                                    gen | kFlagInclusive | ((excl[q] + tile_count[q]) & kCountMask));
                 digit_base[d] = pass_offset[d] + excl[q];
             }
         }
