@@ -23,10 +23,10 @@ struct kifi_icp {
     IcpState* st = nullptr;
     void* depth_dev = nullptr;
     size_t depth_bytes = 0;
-    float4* synth = nullptr;  // target in the association's float4 layout
+    // target in the association's float4 layout, then its blocks' bounding boxes,
+    // then a word per source of a frame of its size (winner_of)
+    float4* synth = nullptr;
     size_t synth_cap = 0;     // bytes
-    float4* boxes = nullptr;  // its blocks' bounding boxes
-    size_t boxes_cap = 0;     // bytes
     void* staging = nullptr;  // host float3 targets on their way in
     size_t staging_cap = 0;
     int sw = 0, sh = 0;
@@ -41,7 +41,7 @@ struct kifi_icp {
     long long* pairs = nullptr;      // per source: target index, or -1
     float* pairs_len2 = nullptr;     // per source: len^2
     size_t pairs_cap = 0, pairs_n = 0;
-    unsigned int* winner = nullptr;  // per source: IcpArgs::winner
+    unsigned int* winner = nullptr;  // the same for larger frames: IcpArgs::winner
     size_t winner_cap = 0;           // bytes
     void* zbuf = nullptr;            // Bin's z-buffer (8 bytes per target pixel)
     size_t zbuf_cap = 0;
@@ -71,15 +71,23 @@ kifi_status reserve_bytes(void** p, size_t* cap, size_t bytes, cudaStream_t st) 
     return KIFI_OK;
 }
 
-kifi_status reserve_sources(kifi_icp* c, const kifi_camera* cam) {
-    return reserve_bytes((void**)&c->winner, &c->winner_cap,
-                         (size_t)((cam->width + 3) / 4) * cam->height * sizeof(unsigned int), c->stream);
-}
+size_t source_bytes(int w, int h) { return (size_t)((w + 3) / 4) * h * sizeof(unsigned int); }
 
 kifi_status reserve_target(kifi_icp* c, int w, int h) {
-    const kifi_status s = reserve_bytes((void**)&c->boxes, &c->boxes_cap, icp_box_count(w, h) * sizeof(float4),
-                                        c->stream);
-    return s ? s : reserve_bytes((void**)&c->synth, &c->synth_cap, (size_t)w * h * sizeof(float4), c->stream);
+    return reserve_bytes((void**)&c->synth, &c->synth_cap,
+                         ((size_t)w * h + icp_box_count(w, h)) * sizeof(float4) + source_bytes(w, h), c->stream);
+}
+float4* boxes_of(const kifi_icp* c, int w, int h) { return c->synth + (size_t)w * h; }
+// IcpArgs::winner of a frame: behind the target where it fits, as it does for frames of the target's size
+unsigned int* winner_of(const kifi_icp* c, const kifi_camera* cam) {
+    return source_bytes(cam->width, cam->height) <= source_bytes(c->sw, c->sh)
+               ? (unsigned int*)(boxes_of(c, c->sw, c->sh) + icp_box_count(c->sw, c->sh))
+               : c->winner;
+}
+kifi_status reserve_sources(kifi_icp* c, const kifi_camera* cam) {
+    const size_t bytes = source_bytes(cam->width, cam->height);
+    if (bytes <= source_bytes(c->sw, c->sh)) return KIFI_OK;
+    return reserve_bytes((void**)&c->winner, &c->winner_cap, bytes, c->stream);
 }
 
 // What is known about where the target's points project through `proj`, for
@@ -157,7 +165,7 @@ kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const ki
     kifi_status s = reserve_sources(c, cam);
     if (s) return s;
     IcpArgs a{};
-    a.winner = c->winner;
+    a.winner = winner_of(c, cam);
     a.depth = depth_dev;
     a.depth_u16 = u16 ? 1 : 0;
     a.width = cam->width;
@@ -172,7 +180,7 @@ kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const ki
     a.synth = c->synth;
     a.synth_w = c->sw;
     a.synth_h = c->sh;
-    a.boxes = c->boxes;
+    a.boxes = boxes_of(c, c->sw, c->sh);
     a.neg_zero = -0.0f;
     set_prune(*c, *cam, proj, &a);
     if (c->record) {
@@ -208,7 +216,7 @@ kifi_status kifi_icp_batch_args(kifi_icp* c, const void* depth_dev, const kifi_c
     kifi_status s = reserve_sources(c, cam);
     if (s) return s;
     *a = IcpArgs{};
-    a->winner = c->winner;
+    a->winner = winner_of(c, cam);
     a->depth = depth_dev;
     a->depth_u16 = 1;
     a->width = cam->width;
@@ -222,7 +230,7 @@ kifi_status kifi_icp_batch_args(kifi_icp* c, const void* depth_dev, const kifi_c
     a->synth = c->synth;
     a->synth_w = c->sw;
     a->synth_h = c->sh;
-    a->boxes = c->boxes;
+    a->boxes = boxes_of(c, c->sw, c->sh);
     a->neg_zero = -0.0f;
     set_prune(*c, *cam, proj, a);
     if (a->prune == kPruneMeasured) a->prune = kPruneOff;  // a batch measures no targets
@@ -245,7 +253,7 @@ kifi_status kifi_icp_batch_target(kifi_icp* c, const kifi_camera* cam, const flo
     c->target_cam = *cam;
     c->have_target = true;
     *out = c->synth;
-    *boxes = c->boxes;
+    *boxes = boxes_of(c, c->sw, c->sh);
     return KIFI_OK;
 }
 
@@ -316,7 +324,6 @@ kifi_status kifi_icp_destroy(kifi_icp* c) {
     cudaFreeHost(c->mail);
     cudaFree(c->depth_dev);
     cudaFree(c->synth);
-    cudaFree(c->boxes);
     cudaFree(c->pairs);
     cudaFree(c->pairs_len2);
     cudaFree(c->winner);
@@ -359,7 +366,7 @@ kifi_status kifi_icp_set_target(kifi_icp* c, const float* points, int width, int
     const size_t bytes = (size_t)width * height * 12;
     if ((s = reserve_bytes(&c->staging, &c->staging_cap, bytes, c->stream))) return s;
     KIFI_CUDA(cudaMemcpyAsync(c->staging, points, bytes, cudaMemcpyHostToDevice, c->stream));
-    KIFI_CUDA(expand_target_enqueue((const float*)c->staging, width, height, c->synth, c->boxes,
+    KIFI_CUDA(expand_target_enqueue((const float*)c->staging, width, height, c->synth, boxes_of(c, width, height),
                                     c->ls.sms * 4, c->stream));
     KIFI_CUDA(cudaStreamSynchronize(c->stream));
     c->sw = width;
@@ -386,8 +393,8 @@ kifi_status kifi_icp_set_target_from_depth(kifi_icp* c, const void* depth, int o
         src = c->depth_dev;
     }
     const Mat4 e2w = load_mat(eye_to_world);
-    KIFI_CUDA(backproject_enqueue(src, depth_is_u16 != 0, *cam, e2w, c->synth, c->boxes, c->ls.sms * 4,
-                                  c->stream));
+    KIFI_CUDA(backproject_enqueue(src, depth_is_u16 != 0, *cam, e2w, c->synth,
+                                  boxes_of(c, cam->width, cam->height), c->ls.sms * 4, c->stream));
     if (!on_device) KIFI_CUDA(cudaStreamSynchronize(c->stream));
     c->sw = cam->width;
     c->sh = cam->height;
@@ -409,7 +416,8 @@ kifi_status kifi_icp_set_target_bin_device(kifi_icp* c, const float* points_dev,
     if (s) return s;
     if ((s = reserve_bytes(&c->zbuf, &c->zbuf_cap, (size_t)width * height * 8, c->stream))) return s;
     KIFI_CUDA(bin_target_enqueue(points_dev, (unsigned int)n, load_mat(world_to_clip), width, height,
-                                 (unsigned long long*)c->zbuf, c->synth, c->boxes, c->ls.sms * 4, c->stream));
+                                 (unsigned long long*)c->zbuf, c->synth, boxes_of(c, width, height), c->ls.sms * 4,
+                                 c->stream));
     c->sw = width;
     c->sh = height;
     c->synth_e2w = load_mat(synth_eye_to_world);

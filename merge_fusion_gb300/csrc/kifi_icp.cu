@@ -34,6 +34,7 @@
 // out-of-range); the reference's 640x480 window clamp (:108-109) is kept,
 // with reads past the end of a smaller target buffer treated as invalid
 // points.
+#include <atomic>
 #include <type_traits>
 
 #include "kifi_internal.h"
@@ -173,7 +174,18 @@ constexpr int kBlockW = 8, kBlockH = 4;  // target pixels per bounding box, a wa
 constexpr int kTileThreads = kTileCols * kTileRows;  // one source per thread
 constexpr int kPredMargin = 4;  // pixels added around the rectangles that a tile searched in the last step,
 constexpr int kUseMargin = 4;   // and that the region so staged must leave around the projections to be used
-constexpr int kStagePixels = 5120;  // float4 target points staged per tile: 80 KB, two tiles per SM
+// Target points (float4) staged per tile, by the tiles that share an SM.  Two: 80
+// KB each and 128 registers a thread, for launches that fill no more than that
+// in one round, where a tile's own time counts.  Three: 52 KB and 80 registers (a
+// few spilled words), for more tiles than that: a tile takes longer, but 24
+// warps hide more of the waits (of an SM's issue slots 0.43 were used with 16).
+// Eight sequences, 15 steps: 11937 -> 10784 us; tracking at 1024x848 (864 tiles):
+// 6140 -> 5817; at 640x480 (300 tiles) 327 against 333.  52 KB hold a tile's windows
+// (32 pixels and 20 around) while the target's pixels are no finer than 1 / 1.15 of
+// the source's; for finer targets the two stay (a 1024x768 target for 640x480
+// frames: 2100 against 2365).
+template <int kPerSm>
+constexpr int kStagePixels = kPerSm == 2 ? 5120 : 3328;
 
 // Row pitch of a staged region `w` pixels wide: odd, so that the 16-byte
 // loads of eight lanes one row apart cover all banks.
@@ -565,6 +577,7 @@ __device__ __forceinline__ FF two_prod(float a, float b) {
 // One AlignStep of one frame pair; `blk` / `nblk`: this CTA's index among
 // the nblk CTAs that work on the pair (the launch's own grid, or a share of
 // a batched launch over several pairs).
+template <int kPerSm>
 __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __restrict__ st, bool first,
                                               unsigned int blk, unsigned int nblk) {
     static_assert(2 * kTileThreads / 32 == kMoments - 1, "two moments after the count per warp");
@@ -591,7 +604,8 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             if (b2 > b0 && b3 > b1 && b0 >= 0 && b1 >= 0) {
                 const int x0 = max(b0 - kPredMargin, 0), y0 = max(b1 - kPredMargin, 0);
                 const int w = b2 + kPredMargin - x0, h = b3 + kPredMargin - y0;
-                if (w <= kStagePixels && h <= kStagePixels && stage_pitch(w) * h <= kStagePixels) {
+                constexpr int most = kStagePixels<kPerSm>;
+                if (w <= most && h <= most && stage_pitch(w) * h <= most) {
                     p[0] = x0;
                     p[1] = y0;
                     p[2] = w;
@@ -724,7 +738,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             for (int m = 10; m >= 0; m -= m > 4 ? 3 : 1) {
                 const int x0 = max(ax0 - m, 0), y0 = max(ay0 - m, 0);
                 const int w0 = min(ax1 + m, 640) - x0, h0 = min(ay1 + m, 480) - y0;
-                if (stage_pitch(w0) * h0 > kStagePixels) continue;
+                if (stage_pitch(w0) * h0 > kStagePixels<kPerSm>) continue;
                 reg = Region{0, x0, y0, x0 + w0, y0 + h0, stage_pitch(w0)};
                 stage_region(stage_all, a.synth, n_synth, a.synth_w, x0, y0, w0, h0, reg.pitch);
                 stage_wait();
@@ -830,8 +844,9 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
     if (threadIdx.x < 32) finish_step(st, tot, a.mail, a.mail_seq);
 }
 
-__global__ void __launch_bounds__(kTileThreads, 2) k_icp_step(IcpArgs a, IcpState* __restrict__ st, bool first) {
-    icp_step_body(a, st, first, blockIdx.x, gridDim.x);
+template <int kPerSm>
+__global__ void __launch_bounds__(kTileThreads, kPerSm) k_icp_step(IcpArgs a, IcpState* __restrict__ st, bool first) {
+    icp_step_body<kPerSm>(a, st, first, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------- Horn solve
@@ -1410,11 +1425,12 @@ __global__ void k_icp_begin_batch(const IcpJob* __restrict__ jobs, int n) {
     if (v < n) icp_begin_body(jobs[v].st, jobs[v].guess);
 }
 
-__global__ void __launch_bounds__(kTileThreads, 2) k_icp_step_batch(const IcpJob* __restrict__ jobs, BlockMap m,
-                                                                   bool first) {
+template <int kPerSm>
+__global__ void __launch_bounds__(kTileThreads, kPerSm) k_icp_step_batch(const IcpJob* __restrict__ jobs, BlockMap m,
+                                                                        bool first) {
     const int v = block_owner(m, blockIdx.x);
     const unsigned int b0 = m.first[v];
-    icp_step_body(jobs[v].a, jobs[v].st, first, blockIdx.x - b0, m.first[v + 1] - b0);
+    icp_step_body<kPerSm>(jobs[v].a, jobs[v].st, first, blockIdx.x - b0, m.first[v + 1] - b0);
 }
 
 __global__ void k_backproject_batch(const BackprojectJob* __restrict__ jobs, BlockMap m) {
@@ -1452,6 +1468,13 @@ int icp_tiles(int width, int height) {
     return tiles < kIcpMaxCtas ? tiles : kIcpMaxCtas;
 }
 
+static int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess, int iterations,
                               int /*ctas*/, cudaStream_t stream, IcpPoseMail* mail, unsigned long long seq) {
     k_icp_begin<<<1, 32, 0, stream>>>(st, guess);
@@ -1459,7 +1482,10 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
         k_target_range<<<(a.synth_w * a.synth_h + kThreads * 4 - 1) / (kThreads * 4), kThreads, 0, stream>>>(
             a, a.w_min * 0.125f, st);
     const int ctas = icp_tiles(a.width, a.height);
-    const size_t smem = kStagePixels * sizeof(float4);
+    // three tiles per SM (kStagePixels) where two would take more than one round and the windows fit
+    const bool three = ctas > 2 * sm_count() && 20 * a.synth_w <= 23 * a.width && 20 * a.synth_h <= 23 * a.height;
+    const auto step = three ? k_icp_step<3> : k_icp_step<2>;
+    const size_t smem = (three ? kStagePixels<3> : kStagePixels<2>) * sizeof(float4);
     // programmatic dependent launch: each step's grid is scheduled as soon as
     // every CTA of the one before has finished its association, overlapping
     // its launch with the previous finisher (k_icp_step waits for it)
@@ -1479,7 +1505,7 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
     IcpArgs other = a;
     other.mail = nullptr;
     for (int it = 0; it < iterations; ++it) {
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_icp_step, it + 1 == iterations ? last : other, st, it == 0);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, step, it + 1 == iterations ? last : other, st, it == 0);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
@@ -1488,11 +1514,20 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
 // The association's dynamic shared memory above the default 48 KB limit; set
 // once per device, outside any stream capture.
 cudaError_t icp_init_device() {
-    cudaError_t e = cudaFuncSetAttribute(k_icp_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kStagePixels * sizeof(float4)));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_icp_step_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(kStagePixels * sizeof(float4)));
+    static std::atomic<unsigned long long> ready{0};  // a bit per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (ready.load() & bit) return cudaSuccess;
+    auto allow = [](auto kernel, int pixels) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pixels * (int)sizeof(float4));
+    };
+    e = allow(k_icp_step<2>, kStagePixels<2>);
+    if (!e) e = allow(k_icp_step<3>, kStagePixels<3>);
+    if (!e) e = allow(k_icp_step_batch<2>, kStagePixels<2>);
+    if (!e) e = allow(k_icp_step_batch<3>, kStagePixels<3>);
+    if (!e) ready.fetch_or(bit);
     return e;
 }
 
@@ -1500,7 +1535,9 @@ cudaError_t icp_align_batch_enqueue(const IcpJob* jobs, int n, const BlockMap& m
                                     cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     k_icp_begin_batch<<<(n + 63) / 64, 64, 0, stream>>>(jobs, n);
-    const size_t smem = kStagePixels * sizeof(float4);
+    const bool three = (int)map.grid > 2 * sm_count();  // (targets have their sources' sizes)
+    const auto step = three ? k_icp_step_batch<3> : k_icp_step_batch<2>;
+    const size_t smem = (three ? kStagePixels<3> : kStagePixels<2>) * sizeof(float4);
     // programmatic dependent launch, as for a single pair: each step's grid
     // is scheduled once every CTA of the step before has finished its association
     cudaLaunchAttribute attr[1];
@@ -1514,7 +1551,7 @@ cudaError_t icp_align_batch_enqueue(const IcpJob* jobs, int n, const BlockMap& m
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     for (int it = 0; it < iterations; ++it) {
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_icp_step_batch, jobs, map, it == 0);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, step, jobs, map, it == 0);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
