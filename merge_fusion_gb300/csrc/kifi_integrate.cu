@@ -953,8 +953,9 @@ __global__ void __launch_bounds__(256) k_merge_partition_batch(const FuseJob* __
                             sm);
 }
 
+// (64 registers and four CTAs per SM, as alone: 8 sequences, 4 steps 10788 -> 10580 us)
 template <typename K>
-__global__ void __launch_bounds__(kMergeThreads) k_merge_update_batch(const FuseJob* __restrict__ jobs, BlockMap m) {
+__global__ void __launch_bounds__(kMergeThreads, 4) k_merge_update_batch(const FuseJob* __restrict__ jobs, BlockMap m) {
     const int v = block_owner(m, blockIdx.x);
     const FuseJob& j = jobs[v];
     const unsigned int b0 = m.first[v];
@@ -1146,7 +1147,15 @@ static cudaError_t integrate_enqueue_t(DeviceCtl* ctl, const Geom& g, VolumeBuff
     // kernels; the sort is its digit passes.  The splat takes at most one CTA
     // per kEmitThreads pixels (a CTA without pixels would only launch and leave).
     const size_t pix_ctas = ((size_t)cam.width * cam.height + kEmitThreads - 1) / kEmitThreads;
-    const int splat_ctas = (int)std::min<size_t>((size_t)ls.splat_ctas, std::max<size_t>(pix_ctas, 1));
+    int splat_ctas = (int)std::min<size_t>((size_t)ls.splat_ctas, std::max<size_t>(pix_ctas, 1));
+    if (sizeof(K) == 8) {
+        // with 64-bit keys (41 registers) half as many again are resident; in rounds of equal length
+        // (512x424: 848 CTAs of one round instead of 608 of which 240 take two, 47 -> 44 us; with
+        // 32-bit keys 45 registers allow five per SM, which gained nothing)
+        const size_t cap = (size_t)ls.splat_ctas + ls.splat_ctas / 2;
+        const size_t rounds = std::max<size_t>((pix_ctas + cap - 1) / cap, 1);
+        splat_ctas = (int)std::max<size_t>((pix_ctas + rounds - 1) / rounds, 1);
+    }
     sort_limits(&ss);
     const int kb = sizeof(K) == 4 ? 10 : g.kb;
     cudaError_t e = chain_launch(chained, dim3(1), dim3(256), st, k_frame_setup_sort, ctl, ss, frame_sort_passes<K>(kb));
