@@ -125,7 +125,7 @@ __device__ __forceinline__ bool last_cta(unsigned long long* counter, const unsi
 
 // Totals of the per-CTA float-float partials, by the whole (last) CTA.  The
 // partials are stored component-major (hi row, then lo row, each
-// kIcpMaxCtas long), so warp w reduces components w + 1 and w + 9 (the count,
+// kIcpMaxCtas long), so warp w (of 8) reduces components w + 1 and w + 9 (the count,
 // component 0, comes with the last-CTA counter) with coalesced loads: lane l adds CTAs
 // l, l + 32, ... in float-float -- all of a lane's loads (up to 320 CTAs)
 // issued in one round -- then a shuffle tree.
@@ -145,9 +145,9 @@ __device__ __forceinline__ FF lane_partials(const float* ph, int b0, int n) {
     for (int k = 1; k < kTotalsPerLane; ++k) acc = ff_add(acc, FF{h[k], l[k]});
     return acc;
 }
-template <int NV>
+template <int NV, int kWarps>
 __device__ __forceinline__ void moments_total(const IcpState* st, unsigned int count, FF* out, int n) {
-    constexpr int kPer = 2;  // moments w + 1 and w + 9 side by side
+    constexpr int kPer = 16 / kWarps;  // moments w + 1 and, with 8 warps, w + 9 side by side
     const int lane = threadIdx.x & 31, c0 = (threadIdx.x >> 5) + 1;
     static_assert(NV == 17, "16 moments after the count");
     if (threadIdx.x == 0) out[0] = FF{(float)count, 0.0f};  // exact: at most 2^24 sources
@@ -157,7 +157,7 @@ __device__ __forceinline__ void moments_total(const IcpState* st, unsigned int c
     for (int b0 = lane; b0 < n; b0 += 32 * kTotalsPerLane)
 #pragma unroll
         for (int h = 0; h < kPer; ++h)
-            a[h] = ff_add(a[h], lane_partials(st->part + (size_t)(2 * (c0 + 8 * h)) * kIcpMaxCtas, b0, n));
+            a[h] = ff_add(a[h], lane_partials(st->part + (size_t)(2 * (c0 + kWarps * h)) * kIcpMaxCtas, b0, n));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -165,7 +165,7 @@ __device__ __forceinline__ void moments_total(const IcpState* st, unsigned int c
             const FF x{__shfl_xor_sync(0xffffffffu, a[h].hi, o), __shfl_xor_sync(0xffffffffu, a[h].lo, o)};
             a[h] = ff_add(a[h], x);
         }
-    if (lane < kPer) out[c0 + 8 * lane] = lane ? a[kPer - 1] : a[0];
+    if (lane < kPer) out[c0 + kWarps * lane] = lane ? a[kPer - 1] : a[0];
     __syncthreads();
 }
 
@@ -185,7 +185,15 @@ constexpr int kUseMargin = 4;   // and that the region so staged must leave arou
 // the source's; for finer targets the two stay (a 1024x768 target for 640x480
 // frames: 2100 against 2365).
 template <int kPerSm>
-constexpr int kStagePixels = kPerSm == 2 ? 5120 : 3328;
+constexpr int kStagePixels = kPerSm == 3 ? 3328 : 5120;
+// One: launches of no more tiles than SMs have two threads per source (two
+// halves of the CTA), which bound alike and search half of the rectangle's rows
+// each: with one thread a source, 8 warps have an SM to themselves, and fast
+// motion leaves rectangles of hundreds of candidates (a 410x307 pair three
+// frames apart, 10 steps 398 -> 333 us; a 348x288 pair, 9 steps 199 -> 183;
+// tracking at 384x315, 9 frames 2297 -> 2109).
+template <int kPerSm>
+constexpr int kHalves = kPerSm == 1 ? 2 : 1;
 
 // Row pitch of a staged region `w` pixels wide: odd, so that the 16-byte
 // loads of eight lanes one row apart cover all banks.
@@ -193,14 +201,15 @@ __host__ __device__ constexpr int stage_pitch(int w) { return w | 1; }
 
 // The target pixels [x0, x0 + w) x [y0, y0 + h) (linear index y * synth_w + x,
 // as the reference reads them) into `stage` with row pitch `pitch`, by the
-// tile's eight warps, as 16-byte asynchronous copies (stage_wait, then a
+// CTA's warps, as 16-byte asynchronous copies (stage_wait, then a
 // barrier, before they are read).  Points that are none (ICP.cpp:112) hold NaN in the
 // target buffer; indices past the buffer's end are none too.
+template <int kWarps>
 __device__ __forceinline__ void stage_region(float4* stage, const float4* __restrict__ synth, size_t n_synth,
                                              int synth_w, int x0, int y0, int w, int h, int pitch) {
     // warps take rows, lanes take columns
-    const int warp = threadIdx.x >> 5 & 7, lane = threadIdx.x & 31;
-    for (int ry = warp; ry < h; ry += 8) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int ry = warp; ry < h; ry += kWarps) {
         for (int rx = lane; rx < w; rx += 32) {
             const size_t at = (size_t)(y0 + ry) * synth_w + (x0 + rx);
             float4* dst = stage + ry * pitch + rx;
@@ -278,12 +287,13 @@ struct Rect {
     int number;       // the first candidate's number r * 32 + c << 8 | columns
 };
 constexpr int kItems = 21 * kTileThreads;  // every row of every window
+template <int kH>
 struct SearchSmem {
-    struct List {
-        Packed p[kTileThreads];                // per source: world point
-        Rect rect[kTileThreads];
-        unsigned long long key[kTileThreads];  // best so far: len^2 bits << 32 | candidate number
-        unsigned short item[kItems];           // rows to search: source << 5 | row
+    struct List {  // per thread: kH to a source
+        Packed p[kTileThreads * kH];                // world point
+        Rect rect[kTileThreads * kH];
+        unsigned long long key[kTileThreads * kH];  // best so far: len^2 bits << 32 | candidate number
+        unsigned short item[kItems];           // rows to search: thread << 5 | row
     };
     union {
         List list;
@@ -368,10 +378,11 @@ __device__ __forceinline__ void scan_row(const float4* __restrict__ synth, long 
 // the most candidates.
 constexpr int kOwnArea = 32;    // rectangles up to this, and up to 1.5 times the warp's average, are scanned by their thread
 constexpr int kBoxArea = 72;    // rectangles above this are cut down by the blocks' boxes
+template <int kH>
 __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const Region& reg, int nr, int nc, int cr,
                                                          int cc, int hr, int hc, bool first, int u, int v, float X,
                                                          float Y, float w, const Prune& pr, const float (&p)[4],
-                                                         SearchSmem& ss, bool& listed) {
+                                                         int half, SearchSmem<kH>& ss, bool& listed) {
     const int W = a.synth_w, H = a.synth_h;
     const Packed pp{f2_pack(p[0], p[1]), f2_pack(p[2], p[3])};
     const unsigned long long nz = f2_pack(a.neg_zero, a.neg_zero);
@@ -437,6 +448,11 @@ __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const
         }
     }
     rows = min(rows, H - v - r0);  // past the target's last row there is nothing
+    if (kH == 2 && rows > 0) {     // this half's rows
+        const int mid = (rows + 1) >> 1;
+        r0 += half ? mid : 0;
+        rows = half ? rows - mid : mid;
+    }
     if (rows <= 0 || cols <= 0) rows = cols = 0;
     const bool wraps = u + c0 + cols > W;
     if (rows * cols > kBoxArea && !wraps) {  // (blocks do not follow a window into the next row)
@@ -487,6 +503,7 @@ __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const
     const bool in = reg.holds(x0, y0, cols, rows);
     const int number = r0 * 32 + c0;
     if (n > most && !wraps) {
+        listed = true;
         const int me = threadIdx.x;
         ss.list.p[me] = pp;
         ss.list.rect[me] = in ? Rect{reg.at(x0, y0), reg.pitch, number << 8 | cols}
@@ -494,7 +511,6 @@ __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const
         ss.list.key[me] = kNoPair;
         const unsigned int i0 = atomicAdd(&ss.n_items, (unsigned int)rows);
         for (int r = 0; r < rows; ++r) ss.list.item[i0 + r] = (unsigned short)(me << 5 | r);
-        listed = true;
         return kNoPair;
     }
     float best = 0.01f;
@@ -514,10 +530,11 @@ __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const
 // The listed rows, dealt out to the CTA's threads; a source's key takes the
 // lexicographic (len^2, candidate number) minimum, the first strict minimum
 // in row-major order.
+template <int kH>
 __device__ __forceinline__ void search_items(const float4* __restrict__ synth, unsigned int n_items, float neg_zero,
-                                             SearchSmem& ss) {
+                                             SearchSmem<kH>& ss) {
     const unsigned long long nz = f2_pack(neg_zero, neg_zero);
-    for (unsigned int i = threadIdx.x; i < n_items; i += kTileThreads) {
+    for (unsigned int i = threadIdx.x; i < n_items; i += kTileThreads * kH) {
         const int it = ss.list.item[i], s = it >> 5, row = it & 31;
         const Packed p = ss.list.p[s];
         const Rect rect = ss.list.rect[s];
@@ -538,7 +555,7 @@ __device__ __noinline__ void finish_step(IcpState* __restrict__ st, const FF* __
 // One ICP::AlignStep (ICP.cpp:35-265) as one kernel.
 //
 // Association (:66-131): a CTA owns a tile of 8 source columns x 32 source
-// rows, a thread one source, a warp 32 vertically adjacent ones.  Each thread
+// rows, a thread one source (two threads where kHalves is 2), a warp 32 vertically adjacent ones.  Each thread
 // back-projects and projects its source, the CTA stages the part of the
 // target that the tile's searches will mostly read in shared memory, and
 // search_own and search_items find each source's nearest candidate, the
@@ -580,9 +597,13 @@ __device__ __forceinline__ FF two_prod(float a, float b) {
 template <int kPerSm>
 __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __restrict__ st, bool first,
                                               unsigned int blk, unsigned int nblk) {
-    static_assert(2 * kTileThreads / 32 == kMoments - 1, "two moments after the count per warp");
-    __shared__ SearchSmem ss;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kH = kHalves<kPerSm>, kWarps = kH * kTileThreads / 32;
+    static_assert(16 % kWarps == 0 && kMoments == 17, "one or two moments after the count per warp");
+    static_assert(offsetof(typename SearchSmem<kH>::List, key) >= sizeof(SearchSmem<kH>::rec), "keys outlive the records' start");
+    __shared__ SearchSmem<kH> ss;
+    __shared__ unsigned int s_hint[kH == 2 ? kTileThreads : 1];  // the halves' common hints
+    const int lane = threadIdx.x & 31, half = kH == 2 ? threadIdx.x / kTileThreads : 0;
+    const int source = threadIdx.x % kTileThreads, warp = source >> 5;  // the tile's source, its column
     // Steps are launched programmatically behind one another: this grid may
     // start while the previous step's last CTA still updates the pose.  Wait
     // for that grid (and its memory) before touching the ICP state.
@@ -623,7 +644,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
     if (threadIdx.x < kMoments) ss.acc[threadIdx.x] = FF{0.0f, 0.0f};
     __syncthreads();
     const int px0 = ss.pred[0], py0 = ss.pred[1], pw = ss.pred[2], ph = ss.pred[3];
-    if (pw > 0) stage_region(stage_all, a.synth, n_synth, a.synth_w, px0, py0, pw, ph, stage_pitch(pw));
+    if (pw > 0) stage_region<kWarps>(stage_all, a.synth, n_synth, a.synth_w, px0, py0, pw, ph, stage_pitch(pw));
     // this thread's depth and last winner (a hint: it may be older, any pixel will do)
     float pre_d = 0.0f;
     unsigned int pre_hint = ~0u;
@@ -674,6 +695,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         unsigned int hint = ~0u;
         if (ahead) hint = pre_hint;
         else if (mine && !first) hint = a.winner[(size_t)y * n_cols + col];
+        if (kH == 2 && half == 0) s_hint[source] = hint;  // (two reads of it may differ)
         int u = 0, v = 0, nr = 0, nc = 0, cc = 0, cr = 0;
         if (mine) {
             const int x = col * 4;
@@ -708,7 +730,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             const int mv0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)py : 0x7fffffffu);
             const int mu1 = __reduce_max_sync(0xffffffffu, has ? px + 1 : -1);
             const int mv1 = __reduce_max_sync(0xffffffffu, has ? py + 1 : -1);
-            if (lane == 0 && mu1 >= 0) {
+            if (lane == 0 && mu1 >= 0 && half == 0) {
                 atomicMin(&ss.cbox[0], mu0);
                 atomicMin(&ss.cbox[1], mv0);
                 atomicMax(&ss.cbox[2], mu1);
@@ -740,16 +762,19 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
                 const int w0 = min(ax1 + m, 640) - x0, h0 = min(ay1 + m, 480) - y0;
                 if (stage_pitch(w0) * h0 > kStagePixels<kPerSm>) continue;
                 reg = Region{0, x0, y0, x0 + w0, y0 + h0, stage_pitch(w0)};
-                stage_region(stage_all, a.synth, n_synth, a.synth_w, x0, y0, w0, h0, reg.pitch);
+                stage_region<kWarps>(stage_all, a.synth, n_synth, a.synth_w, x0, y0, w0, h0, reg.pitch);
                 stage_wait();
                 __syncthreads();
                 break;
             }
         }
+        if (kH == 2) hint = s_hint[source];
         int hr = (int)(hint >> 16) - v, hc = (int)(hint & 0xffffu) - u;
         if ((unsigned)hr >= (unsigned)nr || (unsigned)hc >= (unsigned)nc) hr = hc = -1;
         bool listed = false;
-        unsigned long long key = search_own(a, reg, nr, nc, cr, cc, hr, hc, first, u, v, X, Y, w, pr, wp, ss, listed);
+        unsigned long long key =
+            search_own<kH>(a, reg, nr, nc, cr, cc, hr, hc, first, u, v, X, Y, w, pr, wp, half, ss, listed);
+        if (half && !listed) ss.list.key[threadIdx.x] = key;  // for the source's first thread
         __syncthreads();
         const unsigned int n_items = ss.n_items;
         if (threadIdx.x == 0 && tile < kIcpMaxCtas && ss.box[2] >= 0) {
@@ -758,12 +783,14 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             for (int k = 0; k < 4; ++k) tb[k] = ss.box[k];
         }
         if (n_items) {
-            search_items(a.synth, n_items, a.neg_zero, ss);
+            search_items<kH>(a.synth, n_items, a.neg_zero, ss);
             __syncthreads();
             if (listed) key = ss.list.key[threadIdx.x];
             __syncthreads();  // the records take the list's place
         }
-        const bool hit = mine && key < kNoPair;
+        if (kH == 2 && !half) key = min(key, ss.list.key[threadIdx.x + kTileThreads]);
+        const bool out = mine && half == 0;  // the source's pair is its first thread's
+        const bool hit = out && key < kNoPair;
         const float best = __uint_as_float((unsigned int)(key >> 32));
         const int rc = (int)(unsigned int)key;
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -771,15 +798,15 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             const int x = u + (rc & 31), yy = v + (rc >> 5);
             q = reg.holds(x, yy, 1, 1) ? stage_all[reg.at(x, yy)] : __ldg(a.synth + (size_t)yy * a.synth_w + x);
         }
-        if (mine) a.winner[(size_t)y * n_cols + col] = hit ? (unsigned int)(v + (rc >> 5)) << 16 | (u + (rc & 31)) : ~0u;
-        if (a.pairs && mine) {
+        if (out) a.winner[(size_t)y * n_cols + col] = hit ? (unsigned int)(v + (rc >> 5)) << 16 | (u + (rc & 31)) : ~0u;
+        if (a.pairs && out) {
             const size_t k = (size_t)y * n_cols + col;
             a.pairs[k] = hit ? (long long)(v + (rc >> 5)) * a.synth_w + (u + (rc & 31)) : -1ll;
             a.pairs_len2[k] = hit ? best : 0.01f;
         }
         // this source's pair for the tile's moments (zeros when none)
-        {
-            const int sidx = threadIdx.x;
+        if (half == 0) {
+            const int sidx = source;
             ss.rec[0][sidx] = hit ? wp[0] : 0.f;
             ss.rec[1][sidx] = hit ? wp[1] : 0.f;
             ss.rec[2][sidx] = hit ? wp[2] : 0.f;
@@ -799,11 +826,12 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         // the tile's raw moments: each warp reduces two of the 16 over all
         // sources (lane l takes sources l, l + 32, ...), in float-float
         {
-            constexpr int kPer = 2;
+            constexpr int kPer = 16 / kWarps;
+            const int w0 = threadIdx.x >> 5;
             FF acc[kPer];
 #pragma unroll
             for (int h = 0; h < kPer; ++h) {
-                const int c = warp + 1 + 8 * h;
+                const int c = w0 + 1 + kWarps * h;
                 acc[h] = FF{0.0f, 0.0f};
 #pragma unroll
                 for (int k = 0; k < kTileCols; ++k) {
@@ -823,7 +851,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
                     acc[h] = ff_add(acc[h], x);
                 }
             if (lane < kPer) {
-                const int c = warp + 1 + 8 * lane;
+                const int c = w0 + 1 + kWarps * lane;
                 ss.acc[c] = ff_add(ss.acc[c], lane ? acc[kPer - 1] : acc[0]);
             }
         }
@@ -840,12 +868,12 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
     unsigned int n_total;
     if (!last_cta(&st->done, ss.count, &n_total, nblk)) return;
     __shared__ FF tot[kMoments];
-    moments_total<kMoments>(st, n_total, tot, (int)nblk);
+    moments_total<kMoments, kWarps>(st, n_total, tot, (int)nblk);
     if (threadIdx.x < 32) finish_step(st, tot, a.mail, a.mail_seq);
 }
 
 template <int kPerSm>
-__global__ void __launch_bounds__(kTileThreads, kPerSm) k_icp_step(IcpArgs a, IcpState* __restrict__ st, bool first) {
+__global__ void __launch_bounds__(kTileThreads * kHalves<kPerSm>, kPerSm) k_icp_step(IcpArgs a, IcpState* __restrict__ st, bool first) {
     icp_step_body<kPerSm>(a, st, first, blockIdx.x, gridDim.x);
 }
 
@@ -1426,7 +1454,7 @@ __global__ void k_icp_begin_batch(const IcpJob* __restrict__ jobs, int n) {
 }
 
 template <int kPerSm>
-__global__ void __launch_bounds__(kTileThreads, kPerSm) k_icp_step_batch(const IcpJob* __restrict__ jobs, BlockMap m,
+__global__ void __launch_bounds__(kTileThreads * kHalves<kPerSm>, kPerSm) k_icp_step_batch(const IcpJob* __restrict__ jobs, BlockMap m,
                                                                         bool first) {
     const int v = block_owner(m, blockIdx.x);
     const unsigned int b0 = m.first[v];
@@ -1484,8 +1512,9 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
     const int ctas = icp_tiles(a.width, a.height);
     // three tiles per SM (kStagePixels) where two would take more than one round and the windows fit
     const bool three = ctas > 2 * sm_count() && 20 * a.synth_w <= 23 * a.width && 20 * a.synth_h <= 23 * a.height;
-    const auto step = three ? k_icp_step<3> : k_icp_step<2>;
-    const size_t smem = (three ? kStagePixels<3> : kStagePixels<2>) * sizeof(float4);
+    const bool one = ctas <= sm_count();
+    const auto step = three ? k_icp_step<3> : one ? k_icp_step<1> : k_icp_step<2>;
+    const size_t smem = (three ? kStagePixels<3> : one ? kStagePixels<1> : kStagePixels<2>) * sizeof(float4);
     // programmatic dependent launch: each step's grid is scheduled as soon as
     // every CTA of the one before has finished its association, overlapping
     // its launch with the previous finisher (k_icp_step waits for it)
@@ -1494,7 +1523,7 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(kTileThreads);
+    cfg.blockDim = dim3(one ? 2 * kTileThreads : kTileThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;
@@ -1523,7 +1552,8 @@ cudaError_t icp_init_device() {
     auto allow = [](auto kernel, int pixels) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pixels * (int)sizeof(float4));
     };
-    e = allow(k_icp_step<2>, kStagePixels<2>);
+    e = allow(k_icp_step<1>, kStagePixels<1>);
+    if (!e) e = allow(k_icp_step<2>, kStagePixels<2>);
     if (!e) e = allow(k_icp_step<3>, kStagePixels<3>);
     if (!e) e = allow(k_icp_step_batch<2>, kStagePixels<2>);
     if (!e) e = allow(k_icp_step_batch<3>, kStagePixels<3>);
