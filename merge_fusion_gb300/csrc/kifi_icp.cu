@@ -34,7 +34,6 @@
 // out-of-range); the reference's 640x480 window clamp (:108-109) is kept,
 // with reads past the end of a smaller target buffer treated as invalid
 // points.
-#include <atomic>
 #include <type_traits>
 
 #include "kifi_internal.h"
@@ -1541,23 +1540,16 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
 }
 
 // The association's dynamic shared memory above the default 48 KB limit; set
-// once per device, outside any stream capture.
+// with every context, outside any stream capture.
 cudaError_t icp_init_device() {
-    static std::atomic<unsigned long long> ready{0};  // a bit per device
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e) return e;
-    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-    if (ready.load() & bit) return cudaSuccess;
     auto allow = [](auto kernel, int pixels) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pixels * (int)sizeof(float4));
     };
-    e = allow(k_icp_step<1>, kStagePixels<1>);
+    cudaError_t e = allow(k_icp_step<1>, kStagePixels<1>);
     if (!e) e = allow(k_icp_step<2>, kStagePixels<2>);
     if (!e) e = allow(k_icp_step<3>, kStagePixels<3>);
     if (!e) e = allow(k_icp_step_batch<2>, kStagePixels<2>);
     if (!e) e = allow(k_icp_step_batch<3>, kStagePixels<3>);
-    if (!e) ready.fetch_or(bit);
     return e;
 }
 
