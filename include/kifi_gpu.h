@@ -257,7 +257,7 @@ KIFI_API kifi_status kifi_sort_set_fault_injection(unsigned int skip_tiles, unsi
  * values_dev is not NULL -- in place, in device memory, on `stream` (a
  * cudaStream_t; NULL for the default stream), with results identical to
  * kifi_radix_sort_pairs_u32.  Its scratch is a fixed area of static device
- * memory built into the library (12.0 MiB, present once the library's
+ * memory built into the library (12.3 MiB, present once the library's
  * module is loaded); it calls no cudaMalloc, cudaFree or other allocating
  * routine.  It is meant for processes whose device memory is handed out by
  * their own pool, and for frame loops that cannot pay for cudaMalloc /

@@ -114,7 +114,7 @@ std::atomic<unsigned int> g_first_tile{0u};
 
 }  // namespace
 
-size_t sort_max_tiles(size_t max_n) { return (max_n + kTile - 1) / kTile + 1; }
+size_t sort_max_tiles(size_t max_n) { return tiles_of(max_n); }
 
 cudaError_t sort_scratch_alloc(SortScratch* s, size_t max_n, cudaStream_t st) {
     *s = SortScratch{};
@@ -125,7 +125,7 @@ cudaError_t sort_scratch_alloc(SortScratch* s, size_t max_n, cudaStream_t st) {
     if ((e = cudaMalloc(&s->tile_counter, 8 * sizeof(unsigned int)))) return e;
     if ((e = cudaMalloc(&s->epoch, sizeof(unsigned long long)))) return e;
     if ((e = cudaMemsetAsync(s->epoch, 0, sizeof(unsigned long long), st))) return e;
-    size_t lb = (size_t)kSortHistWords * lookback_rows(s->max_tiles) * sizeof(unsigned long long);
+    const size_t lb = lookback_bytes(s->max_tiles, kSortHistWords);
     if ((e = cudaMalloc(&s->lookback, lb))) return e;
     if ((e = cudaMemsetAsync(s->lookback, 0, lb, st))) return e;
     if ((e = cudaMalloc(&s->alt_keys, (max_n + 64) * sizeof(uint64_t)))) return e;

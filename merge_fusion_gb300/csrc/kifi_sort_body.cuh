@@ -18,6 +18,11 @@ constexpr unsigned long long kSpinLimit = 1ull << 22;
 constexpr int kLookAhead = 8;  // predecessor look-back words fetched per round
 constexpr unsigned int kGroup = 16;  // tiles whose sum the look-back takes at once
 __host__ __device__ constexpr size_t lookback_rows(size_t max_tiles) { return max_tiles + max_tiles / kGroup + 1; }
+// Every scratch's sizes: tiles of up to max_n keys, and the look-back words of `digits` counters (passes x radix).
+constexpr size_t tiles_of(size_t max_n) { return (max_n + kTile - 1) / kTile + 1; }
+constexpr size_t lookback_bytes(size_t max_tiles, size_t digits) {
+    return digits * lookback_rows(max_tiles) * sizeof(unsigned long long);
+}
 
 constexpr unsigned long long kFlagAggregate = 1ull << 30;
 constexpr unsigned long long kFlagInclusive = 2ull << 30;

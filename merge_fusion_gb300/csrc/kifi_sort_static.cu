@@ -10,15 +10,18 @@
 //   12         key count (u32)                                   written per call
 //   256        dynamic tile counters, 8 x u32                    cleared per call
 //   512        digit histograms, 4 x 256 x u32 (+64 B)           cleared per call
-//   kLookback  look-back words, 4 x kTiles x 256 x u64           zero at load
+//   kLookback  look-back words, 4 x 256 x lookback_rows(kTiles)  zero at load
+//              u64: per pass a row for every tile, then for every group of tiles
 //   kAltKeys   ping-pong keys,   (kMaxKeys + 64) x u32
 //   kAltVals   ping-pong values, (kMaxKeys + 64) x u32
 //
 // What must start at zero: the generation counter and the look-back words.
 // Each sort bumps the counter and tags its look-back words with it, so words
 // left by an earlier sort are ignored without clearing -- provided no word
-// ever carries a tag the counter has not reached yet.  Static device memory
-// is zero-initialised when the module is loaded, which gives exactly that.
+// ever carries a tag the counter has not reached yet, so the look-back words
+// share their memory with nothing else (keys could look like such words).
+// Static device memory is zero-initialised when the module is loaded, which
+// gives exactly that.
 // Everything else is (re)initialised by every call before it is read.
 //
 // Set-up: the first call on a device (with that device current) looks up the
@@ -30,18 +33,19 @@
 #include <mutex>
 
 #include "kifi_api_util.h"
+#include "kifi_sort_body.cuh"
 
 namespace kifi {
 namespace {
 
 constexpr size_t kMaxKeys = (size_t)KIFI_RADIX_SORT_STATIC_MAX;
-constexpr size_t kSortTile = 2048;  // keys per tile of k_sort_pass
-constexpr size_t kTiles = (kMaxKeys + kSortTile - 1) / kSortTile + 1;
+constexpr size_t kDigits = 4 * sort_detail::kRadix;  // four 8-bit passes
+constexpr size_t kTiles = sort_detail::tiles_of(kMaxKeys);
 constexpr size_t kLookback = 5120;
-constexpr size_t kAltKeys = kLookback + 4 * kTiles * 256 * sizeof(unsigned long long);
+constexpr size_t kAltKeys = kLookback + (sort_detail::lookback_bytes(kTiles, kDigits) + 255) / 256 * 256;
 constexpr size_t kAltVals = kAltKeys + ((kMaxKeys + 64) * sizeof(uint32_t) + 255) / 256 * 256;
 constexpr size_t kScratchBytes = kAltVals + ((kMaxKeys + 64) * sizeof(uint32_t) + 255) / 256 * 256;
-static_assert(512 + 4 * 256 * sizeof(unsigned int) + 64 <= kLookback, "histograms overlap the look-back words");
+static_assert(512 + kDigits * sizeof(unsigned int) + 64 <= kLookback, "histograms overlap the look-back words");
 
 static __device__ __align__(256) unsigned char g_sort_scratch[kScratchBytes];
 
