@@ -16,9 +16,9 @@
 //    counters, bump the look-back generation tag.
 //  * k_sort_histogram: one read of the keys builds all four 256-bin digit
 //    histograms (shared-memory counters, then one global atomic per bin).
-//  * k_sort_pass: a CTA per tile of 2048 keys, or, where the grid is smaller,
-//    persistent CTAs that take tiles in increasing order from an atomic
-//    counter.  Each warp ranks its keys with
+//  * k_sort_pass: CTAs take tiles of 2048 keys in increasing order from an
+//    atomic counter (one each where the grid has a CTA per tile).  Each warp
+//    ranks its keys with
 //    __match_any_sync (a stable rank among lanes holding the same digit),
 //    per-warp digit counts are scanned across warps in shared memory, the
 //    tile's counts are published to a decoupled look-back array and the
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_pass(const K* keys_in, K* __r
 }
 
 // A pass of a frame's new keys, in tiles of 8 kT keys.  A tile takes about 7 us
-// of latencies (keys and histogram 1.5, ranks 1.8, look-back 3, scatter 1.1) and
+// of latencies (ticket, keys and histogram 1.5, ranks 1.8, look-back 3, scatter 1.1) and
 // few tiles fill the GPU, so alone a CTA has 512 threads -- half the tiles to
 // look back over -- and all the registers it wants, except with 64-bit keys, where a
 // large frame has more tiles than SMs and two CTAs per SM pay (the three passes of

@@ -108,32 +108,38 @@ __device__ __forceinline__ void sort_pass_body(const K* keys_in, K* __restrict__
     auto& tile_id = sm.tile_id;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // Tiles come from a counter, so that every tile a CTA waits for has been
+    // taken by a CTA that runs, in whatever order the CTAs start (their order
+    // is not promised, and beside other work not all are resident).
+    auto take_tile = [&] {
+        if (threadIdx.x == 0) tile_id = atomicAdd(&s.tile_counter[pass], 1u);
+        for (int i = threadIdx.x; i < kWarps * (R + 2) / 2; i += kT)
+            reinterpret_cast<unsigned int*>(&warp_hist[0][0])[i] = 0u;
+    };
+    // Grids are sized before the key count exists.  CTAs beyond the tile count
+    // leave before the counter, at which they would queue; of a frame's alone
+    // (kT > kThreads: four CTAs per SM) the first quarter take a ticket while the
+    // count is read.  Ten 320x240 frames at 8 mm, 640x480 at 4 mm and 512x424 with
+    // 64-bit keys, us: tiles by block index 512, 2732, 2214; every ticket behind
+    // the count 520, 2733, 2272; the first quarter ahead of it 506, 2707, 2244; the
+    // first half 509, 2712, 2310.
+    const bool early = kT > kThreads && blk < nblk / 4;
+    if (early) take_tile();
     const unsigned int n = (unsigned int)min((size_t)*n_ptr, s.max_n);
     const unsigned int n_tiles = (n + kTile - 1) / kTile;
-    // Grids are sized before the key count exists.  CTAs beyond the tile
-    // count leave before the tile counter: n_tiles CTAs (or the whole grid,
-    // when smaller) take every tile, and the counter sees only them.
-    if (blk >= n_tiles) return;
+    if (!early) {
+        if (blk >= n_tiles) return;
+        take_tile();
+    }
     const int shift = pass * kBits;
     const unsigned long long gen = (*s.epoch & 0xffffffffull) << 32;
     unsigned long long* lb = s.lookback + (size_t)pass * lookback_rows(s.max_tiles) * R;  // tiles, then groups
-
-    // A CTA per tile where the grid has them, in the order the CTAs start;
-    // else the CTAs take tiles from the counter, so that every tile a CTA
-    // waits for has been taken by one that runs.
-    const bool one_each = n_tiles <= nblk;
-    bool have_offsets = false;
-    for (;;) {
-        if (one_each) {
-            if (have_offsets) break;
-        } else {
-            __syncthreads();
-            if (threadIdx.x == 0) tile_id = atomicAdd(&s.tile_counter[pass], 1u);
-            __syncthreads();
-        }
-        const unsigned int tile = one_each ? s.first_tile + blk : tile_id;
-        if (tile >= n_tiles) break;  // (CTAs without a tile leave before any other work)
-        // the tile's keys and, once, the digit histogram: independent reads
+    unsigned int c[D];
+#pragma unroll
+    for (int q = 0; q < D; ++q) c[q] = digits ? __ldcg(s.hist + pass * R + threadIdx.x * D + q) : 0u;
+    __syncthreads();
+    unsigned int tile = tile_id;
+    for (bool first = true; tile < n_tiles; first = false) {
         const unsigned int base = tile * kTile + warp * (32 * kKeysPerThread);
         K k[kKeysPerThread];
         uint32_t v[kKeysPerThread];
@@ -146,14 +152,7 @@ __device__ __forceinline__ void sort_pass_body(const K* keys_in, K* __restrict__
             k[j] = ok ? ld_l2(keys_in + i) : (K)0;
             if (kWithValues) v[j] = ok ? __ldcg(vals_in + i) : 0u;
         }
-        unsigned int c[D];
-        if (!have_offsets) {
-#pragma unroll
-            for (int q = 0; q < D; ++q) c[q] = digits ? __ldcg(s.hist + pass * R + threadIdx.x * D + q) : 0u;
-        }
-        for (int i = threadIdx.x; i < kWarps * (R + 2) / 2; i += kT)
-            reinterpret_cast<unsigned int*>(&warp_hist[0][0])[i] = 0u;
-        if (!have_offsets) {
+        if (first) {
             // exclusive scan of this pass's global digit histogram: thread t
             // holds digits t*D .. t*D + D - 1
             unsigned int sum = 0;
@@ -170,12 +169,10 @@ __device__ __forceinline__ void sort_pass_body(const K* keys_in, K* __restrict__
             for (int w = 0; w < warp; ++w) run += wsum[w];
 #pragma unroll
             for (int q = 0; q < D; ++q) {
-                if (digits) pass_offset[threadIdx.x * D + q] = run;
+                if (digits) pass_offset[threadIdx.x * D + q] = run;  // read behind later barriers
                 run += c[q];
             }
-            have_offsets = true;  // read after the next barrier, before the scatter
         }
-        __syncthreads();  // warp_hist cleared
         // stable warp-local ranks: lanes with equal digits, in (j, lane) order
         unsigned int peers[kKeysPerThread];
 #pragma unroll
@@ -301,6 +298,11 @@ __device__ __forceinline__ void sort_pass_body(const K* keys_in, K* __restrict__
             keys_out[pos] = k[j];
             if (kWithValues) vals_out[pos] = v[j];
         }
+        if (n_tiles <= nblk) break;  // a CTA per tile: this was its only one
+        __syncthreads();
+        take_tile();
+        __syncthreads();
+        tile = tile_id;
     }
 }
 
