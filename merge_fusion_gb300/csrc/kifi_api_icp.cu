@@ -23,8 +23,7 @@ struct kifi_icp {
     IcpState* st = nullptr;
     void* depth_dev = nullptr;
     size_t depth_bytes = 0;
-    // target in the association's float4 layout, then its blocks' bounding boxes,
-    // then a word per source of a frame of its size (winner_of)
+    // target in the association's float4 layout, then its blocks' bounding boxes
     float4* synth = nullptr;
     size_t synth_cap = 0;     // bytes
     void* staging = nullptr;  // host float3 targets on their way in
@@ -41,8 +40,6 @@ struct kifi_icp {
     long long* pairs = nullptr;      // per source: target index, or -1
     float* pairs_len2 = nullptr;     // per source: len^2
     size_t pairs_cap = 0, pairs_n = 0;
-    unsigned int* winner = nullptr;  // the same for larger frames: IcpArgs::winner
-    size_t winner_cap = 0;           // bytes
     void* zbuf = nullptr;            // Bin's z-buffer (8 bytes per target pixel)
     size_t zbuf_cap = 0;
     IcpPoseMail* mail = nullptr;     // page-locked, mapped: the last step's pose ...
@@ -71,24 +68,11 @@ kifi_status reserve_bytes(void** p, size_t* cap, size_t bytes, cudaStream_t st) 
     return KIFI_OK;
 }
 
-size_t source_bytes(int w, int h) { return (size_t)((w + 3) / 4) * h * sizeof(unsigned int); }
-
 kifi_status reserve_target(kifi_icp* c, int w, int h) {
-    return reserve_bytes((void**)&c->synth, &c->synth_cap,
-                         ((size_t)w * h + icp_box_count(w, h)) * sizeof(float4) + source_bytes(w, h), c->stream);
+    return reserve_bytes((void**)&c->synth, &c->synth_cap, ((size_t)w * h + icp_box_count(w, h)) * sizeof(float4),
+                         c->stream);
 }
 float4* boxes_of(const kifi_icp* c, int w, int h) { return c->synth + (size_t)w * h; }
-// IcpArgs::winner of a frame: behind the target where it fits, as it does for frames of the target's size
-unsigned int* winner_of(const kifi_icp* c, const kifi_camera* cam) {
-    return source_bytes(cam->width, cam->height) <= source_bytes(c->sw, c->sh)
-               ? (unsigned int*)(boxes_of(c, c->sw, c->sh) + icp_box_count(c->sw, c->sh))
-               : c->winner;
-}
-kifi_status reserve_sources(kifi_icp* c, const kifi_camera* cam) {
-    const size_t bytes = source_bytes(cam->width, cam->height);
-    if (bytes <= source_bytes(c->sw, c->sh)) return KIFI_OK;
-    return reserve_bytes((void**)&c->winner, &c->winner_cap, bytes, c->stream);
-}
 
 // What is known about where the target's points project through `proj`, for
 // the window search (kifi_icp.cu, Prune).  A back-projected frame aligned
@@ -162,10 +146,7 @@ kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const ki
     if (iterations < 0 || iterations > kIcpMaxStats)
         return fail(KIFI_ERR_INVALID_ARGUMENT, "iterations must be in [0, 64]");
     const size_t n_src = (size_t)((cam->width + 3) / 4) * cam->height;
-    kifi_status s = reserve_sources(c, cam);
-    if (s) return s;
     IcpArgs a{};
-    a.winner = winner_of(c, cam);
     a.depth = depth_dev;
     a.depth_u16 = u16 ? 1 : 0;
     a.width = cam->width;
@@ -213,10 +194,7 @@ kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const ki
 kifi_status kifi_icp_batch_args(kifi_icp* c, const void* depth_dev, const kifi_camera* cam, IcpArgs* a,
                                 IcpState** st, int iterations) {
     if (!c->have_target) return fail(KIFI_ERR_INVALID_ARGUMENT, "ICP target not set");
-    kifi_status s = reserve_sources(c, cam);
-    if (s) return s;
     *a = IcpArgs{};
-    a->winner = winner_of(c, cam);
     a->depth = depth_dev;
     a->depth_u16 = 1;
     a->width = cam->width;
@@ -260,8 +238,7 @@ kifi_status kifi_icp_batch_target(kifi_icp* c, const kifi_camera* cam, const flo
 // Everything an alignment against a target of the camera's size may need to
 // allocate, done ahead (outside any stream capture).
 kifi_status kifi_icp_prepare_frame(kifi_icp* c, const kifi_camera* cam) {
-    kifi_status s = reserve_sources(c, cam);
-    return s ? s : reserve_target(c, cam->width, cam->height);
+    return reserve_target(c, cam->width, cam->height);
 }
 
 extern "C" {
@@ -326,7 +303,6 @@ kifi_status kifi_icp_destroy(kifi_icp* c) {
     cudaFree(c->synth);
     cudaFree(c->pairs);
     cudaFree(c->pairs_len2);
-    cudaFree(c->winner);
     cudaFree(c->staging);
     cudaFree(c->zbuf);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);

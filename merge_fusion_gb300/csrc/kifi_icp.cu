@@ -171,6 +171,7 @@ __device__ __forceinline__ void moments_total(const IcpState* st, unsigned int c
 constexpr int kTileCols = 8, kTileRows = 32;
 constexpr int kBlockW = 8, kBlockH = 4;  // target pixels per bounding box, a warp's worth
 constexpr int kTileThreads = kTileCols * kTileRows;  // one source per thread
+static_assert(kTileThreads == kIcpTileSources, "a winner per source");
 constexpr int kPredMargin = 4;  // pixels added around the rectangles that a tile searched in the last step,
 constexpr int kUseMargin = 4;   // and that the region so staged must leave around the projections to be used
 // Target points (float4) staged per tile, by the tiles that share an SM.  Two: 80
@@ -651,7 +652,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         const int col = (tile0 % tiles_x) * kTileCols + warp, y = (tile0 / tiles_x) * kTileRows + lane;
         if (col < n_cols && y < a.height) {
             pre_d = load_depth(a.depth, (size_t)y * a.width + col * 4, a.depth_u16);
-            if (!first) pre_hint = __ldcg(a.winner + (size_t)y * n_cols + col);
+            if (!first && tile0 < kIcpMaxCtas) pre_hint = __ldcg(st->winner + tile0 * kTileThreads + source);
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -693,7 +694,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         float X = 0.f, Y = 0.f, w = 0.f;
         unsigned int hint = ~0u;
         if (ahead) hint = pre_hint;
-        else if (mine && !first) hint = a.winner[(size_t)y * n_cols + col];
+        else if (mine && !first && tile < kIcpMaxCtas) hint = st->winner[tile * kTileThreads + source];
         if (kH == 2 && half == 0) s_hint[source] = hint;  // (two reads of it may differ)
         int u = 0, v = 0, nr = 0, nc = 0, cc = 0, cr = 0;
         if (mine) {
@@ -772,7 +773,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         if ((unsigned)hr >= (unsigned)nr || (unsigned)hc >= (unsigned)nc) hr = hc = -1;
         bool listed = false;
         unsigned long long key =
-            search_own<kH>(a, reg, nr, nc, cr, cc, hr, hc, first, u, v, X, Y, w, pr, wp, half, ss, listed);
+            search_own<kH>(a, reg, nr, nc, cr, cc, hr, hc, first || tile >= kIcpMaxCtas, u, v, X, Y, w, pr, wp, half, ss, listed);
         if (half && !listed) ss.list.key[threadIdx.x] = key;  // for the source's first thread
         __syncthreads();
         const unsigned int n_items = ss.n_items;
@@ -797,7 +798,8 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             const int x = u + (rc & 31), yy = v + (rc >> 5);
             q = reg.holds(x, yy, 1, 1) ? stage_all[reg.at(x, yy)] : __ldg(a.synth + (size_t)yy * a.synth_w + x);
         }
-        if (out) a.winner[(size_t)y * n_cols + col] = hit ? (unsigned int)(v + (rc >> 5)) << 16 | (u + (rc & 31)) : ~0u;
+        if (out && tile < kIcpMaxCtas)
+            st->winner[tile * kTileThreads + source] = hit ? (unsigned int)(v + (rc >> 5)) << 16 | (u + (rc & 31)) : ~0u;
         if (a.pairs && out) {
             const size_t k = (size_t)y * n_cols + col;
             a.pairs[k] = hit ? (long long)(v + (rc >> 5)) * a.synth_w + (u + (rc & 31)) : -1ll;

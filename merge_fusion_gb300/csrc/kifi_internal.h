@@ -274,6 +274,7 @@ cudaError_t mesh_snapshot_enqueue(const DeviceCtl* ctl, const VolumeBuffers& vb,
 // ------------------------------------------------------------------ ICP
 constexpr int kIcpMaxStats = 64;
 constexpr int kIcpMaxCtas = 2048;
+constexpr int kIcpTileSources = 256;  // sources per association tile
 
 // Where the last step of an alignment publishes its pose for a host that
 // polls instead of synchronising (page-locked, mapped host memory): the pose
@@ -298,7 +299,6 @@ struct IcpArgs {
     int prune;              // kPruneOff, kPruneKnown (lo, hi below) or kPruneMeasured (IcpState::range)
     float kx, ky, eps, eps0, w_min;
     float lo[2], hi[2];
-    unsigned int* winner;   // per source: the pixel that won the last step (row << 16 | column), or ~0
     long long* pairs;       // optional: per source the winner's target index (-1: none) ...
     float* pairs_len2;      // ... and its len^2, overwritten by every iteration
     float neg_zero;         // -0.0f, a value the device code cannot see at compile time
@@ -326,6 +326,9 @@ struct IcpState {
     IcpIterStats stats[kIcpMaxStats];
     float part[34 * kIcpMaxCtas];   // per-CTA float-float partials: hi, lo rows of 17 components
     int tile_box[4 * kIcpMaxCtas];  // each tile's window box in the last step: x0, y0, x1, y1
+    // per tile and source: the pixel that won the last step (row << 16 | column), or ~0; here, so that
+    // an alignment allocates nothing, whatever its frame's size (tiles from kIcpMaxCtas on keep none)
+    unsigned int winner[kIcpTileSources * kIcpMaxCtas];
 };
 
 cudaError_t icp_init_device();
