@@ -46,6 +46,7 @@ struct kifi_icp {
     IcpPoseMail* mail_dev = nullptr; // ... its device address
     unsigned long long mail_seq = 0; // ... and the number of the latest alignment
     bool publish = false;            // alignments publish their pose (icp_publish_pose)
+    bool graph_keeps_target = false; // the next alignment's graph is updated to its target (kifi_icp_prepare_frame)
 };
 
 namespace {
@@ -164,6 +165,14 @@ kifi_status enqueue_align(kifi_icp* c, const void* depth_dev, bool u16, const ki
     a.boxes = boxes_of(c, c->sw, c->sh);
     a.neg_zero = -0.0f;
     set_prune(*c, *cam, proj, &a);
+    const bool keeps_target = c->graph_keeps_target;
+    c->graph_keeps_target = false;
+    if (a.prune == kPruneKnown && !keeps_target) {
+        // a graph may be replayed after its caller has put other points in the target's place: measured then
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone)
+            a.prune = kPruneMeasured;
+    }
     if (c->record) {
         if (n_src > c->pairs_cap) {
             KIFI_CUDA(cudaStreamSynchronize(c->stream));
@@ -236,8 +245,10 @@ kifi_status kifi_icp_batch_target(kifi_icp* c, const kifi_camera* cam, const flo
 }
 
 // Everything an alignment against a target of the camera's size may need to
-// allocate, done ahead (outside any stream capture).
+// allocate, done ahead (outside any stream capture) of a pipeline's frame graph,
+// which is updated to every frame's target.
 kifi_status kifi_icp_prepare_frame(kifi_icp* c, const kifi_camera* cam) {
+    c->graph_keeps_target = true;
     return reserve_target(c, cam->width, cam->height);
 }
 

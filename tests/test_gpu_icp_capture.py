@@ -62,3 +62,30 @@ def test_a_frame_larger_than_its_target_needs_no_allocation(gpu):
         g.replay()
     a, b = plain.Result(), captured.Result()
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[2], b[2]) and a[2].size == 3
+
+
+def test_a_graph_searches_the_target_it_finds(gpu, oracle_cpu):
+    # captured against a back-projected frame, replayed after the caller put other points there
+    import torch
+    from merge_fusion_gb300 import kifi
+    seq = _rooms(320, 240)
+    cam, pose = seq.camera, seq.eye_to_world_f32(0)
+    t, d = _device(seq.frames[0]), _device(seq.frames[1])
+    s = torch.cuda.Stream()
+    icp = kifi.ICP(stream=s.cuda_stream)
+    icp.RecordAssociations(True)
+    torch.cuda.synchronize()
+    _target(icp, t, cam, pose)
+    _align(icp, d, cam, pose, 1)  # reserves the records
+    torch.cuda.synchronize()
+    g = _capture(s, lambda: _align(icp, d, cam, pose, 1))
+    target = oracle_cpu.backproject(seq.depth_m(0), cam, pose)
+    flat = target.reshape(-1, 3)
+    flat[::3] = np.roll(flat[::3], 5, axis=0)  # points that project five pixels' rows from their own
+    icp.SetTarget(target, pose)
+    with torch.cuda.stream(s):
+        g.replay()
+    torch.cuda.synchronize()
+    gi, gl = icp.Associations()
+    oi, ol = oracle_cpu.icp_associate(seq.depth_m(1), cam, pose, target, pose)
+    assert np.array_equal(gi, oi) and np.array_equal(gl.view(np.uint32), ol.view(np.uint32))
