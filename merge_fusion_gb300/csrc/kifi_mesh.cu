@@ -128,11 +128,14 @@ __device__ __forceinline__ unsigned int run_length(unsigned int n, unsigned int 
     return ((n + runs - 1) / runs + whole - 1u) / whole * whole;
 }
 
-// words that start in each run of voxels; and the row table cleared
+// words that start in each run of voxels; and the row table cleared, for which
+// there are more CTAs than runs where the volume is small (a table is 4 MB at 10
+// bits per axis and 268 MB at 13, which one CTA took 35 and 4000 us to clear: a mesh
+// of 30 voxels at 1024 and 8192 voxels per axis 115 -> 54, 4107 -> 93 us)
 template <typename K>
 __global__ void __launch_bounds__(kThreads) k_word_count(const K* __restrict__ keys,
                                                          const unsigned int* __restrict__ n_dev,
-                                                         unsigned int* __restrict__ run_words,
+                                                         unsigned int* __restrict__ run_words, unsigned int runs,
                                                          uint4* __restrict__ rows, unsigned int row_vecs,
                                                          MeshCounts* __restrict__ mc) {
     const unsigned int n = *n_dev;
@@ -142,7 +145,8 @@ __global__ void __launch_bounds__(kThreads) k_word_count(const K* __restrict__ k
         mc->missing_min = ~0ull;
         mc->runs_done = 0u;
     }
-    const unsigned int len = run_length(n, gridDim.x, kBuildTile);
+    if (blockIdx.x >= runs) return;
+    const unsigned int len = run_length(n, runs, kBuildTile);
     const unsigned int lo = min(blockIdx.x * len, n), hi = min(lo + len, n);
     const unsigned int lane = threadIdx.x & 31u;
     unsigned int cnt = 0;
@@ -1009,7 +1013,10 @@ static void mesh_count_t(const K* keys, const float2* vals, size_t n_cap, int kb
                          cudaStream_t st, cudaEvent_t* stage_events) {
     const unsigned int vruns = mesh_runs(n_cap, kVoxelRuns), wruns = mesh_runs(n_cap, kWordRuns);
     const unsigned int row_vecs = (unsigned int)(((size_t)1 << (2 * kb)) / 4);
-    k_word_count<K><<<vruns, kThreads, 0, st>>>(keys, ms.n_dev, ms.run_words, (uint4*)ms.rows, row_vecs, ms.counts);
+    // four vectors of the row table per thread, eight CTAs per SM of the 152 at most
+    const unsigned int clear = row_vecs / (4 * kThreads) < kVoxelRuns / 2 ? row_vecs / (4 * kThreads) : kVoxelRuns / 2;
+    k_word_count<K><<<vruns > clear ? vruns : clear, kThreads, 0, st>>>(keys, ms.n_dev, ms.run_words, vruns,
+                                                                        (uint4*)ms.rows, row_vecs, ms.counts);
     k_word_build<K><<<vruns, kThreads, 0, st>>>(keys, kb, vals, ms.n_dev, ms.run_words, ms.rows, ms.words);
     if (stage_events) cudaEventRecord(stage_events[0], st);
     if (with_indices)
