@@ -244,8 +244,9 @@ __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ 
 // The gradient of a layer's pre-activation, in one pass: its value from the
 // layer above, through the ReLU (act > 0, where there is one), as BF16 [M][C]
 // and its transpose [C][M] for the two products that read it, and its column
-// sums (the bias gradient, added to db).  A thread keeps one column; a tile
-// of 64 rows is transposed in shared memory.  Values:
+// sums per CTA (part[c][CTA], which k_bias_sum turns into the bias gradient in a
+// fixed order: it repeats bit for bit).  A thread keeps one column; a tile of 64
+// rows is transposed in shared memory.  Values:
 //   kPlain   src[m][c]
 //   kPool    src[b][c] / P: the global average pool's gradient
 //   kConv    the gather form of col2im over src = dcol [M'][Kp] of the
@@ -255,13 +256,13 @@ __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ 
 // Bound by its bytes and the gathers' latency: the lowest layer's pass moves
 // 150 MB in 61 us.  Before, col2im, the ReLU, the column sums (one strided
 // column per CTA, 830 of 2080 us at batch 256) and the transpose were passes of
-// their own; a gradient step 1750 -> 677 us.
+// their own; a gradient step 1750 -> 678 us.
 // L is the convolution above for kConv.
 enum class GradSrc { kPlain, kPool, kConv };
 template <int C, GradSrc kSrc, int L = 0>
 __global__ void __launch_bounds__(kThreads) k_grad(const float* __restrict__ src, const bf16* __restrict__ act, int M,
                                                    bf16* __restrict__ gb, bf16* __restrict__ gbT,
-                                                   float* __restrict__ db) {
+                                                   float* __restrict__ part) {
     constexpr int H = kHin[L], W = kWin[L], Ho = kHout[L], Wo = kWout[L], Kp = kKp[L], P = kHout[3] * kWout[3];
     constexpr int kGroups = kThreads / C;  // rows taken side by side
     __shared__ __align__(16) bf16 t[C][kTileP];
@@ -312,7 +313,41 @@ __global__ void __launch_bounds__(kThreads) k_grad(const float* __restrict__ src
         float s = 0.0f;
 #pragma unroll
         for (int k = 0; k < kGroups; ++k) s += red[k][c];
-        atomicAdd(db + c, s);
+        part[(size_t)c * gridDim.x + blockIdx.x] = s;
+    }
+}
+
+// The bias gradients of all layers from k_grad's sums per CTA: a CTA per
+// column, whose threads take every 256th sum and join in a tree.  Latency-bound,
+// 4.7 us: a gradient step at batch 256 takes 678 us, and 672 with one atomic per
+// CTA and column, whose order changes from run to run.
+struct BiasJob {
+    const float* part;
+    float* db;
+    int ctas, cols;
+};
+constexpr int kBiases = kConvs + 2;
+struct BiasJobs {
+    BiasJob j[kBiases];
+    int n, cols;  // cols: of all of them, a CTA each
+};
+__global__ void __launch_bounds__(kThreads) k_bias_sum(BiasJobs jobs) {
+    chain_begin();
+    int c = (int)blockIdx.x, k = 0;
+    while (c >= jobs.j[k].cols) c -= jobs.j[k++].cols;
+    const BiasJob& q = jobs.j[k];
+    float s = 0.0f;
+#pragma unroll 5
+    for (int b = threadIdx.x; b < q.ctas; b += kThreads) s += q.part[(size_t)c * q.ctas + b];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    __shared__ float red[kThreads / 32];
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) s += red[w];
+        q.db[c] = s;
     }
 }
 
@@ -364,6 +399,7 @@ struct kifi_proposer {
     bf16 *h1 = nullptr, *h1T = nullptr;     // [B][64], [64][B]
     float* out = nullptr;                   // [B][16]
     bf16 *dbf = nullptr, *dbfT = nullptr;   // BF16 gradient [M][C] and transpose
+    float* bias_part = nullptr;             // column sums per CTA of the gradient passes
     bf16* wT[12] = {};                      // transposed weights (those whose layer passes a gradient on)
 };
 
@@ -376,8 +412,14 @@ kifi_status gemm(kifi_proposer* pr, const void* A, const void* B, float* C, int 
     KIFI_CUDA(gemm_bf16_enqueue(A, B, C, M, N, K, lda, ldb, ldc, k_split, acc, pr->status, pr->stream, epi));
     return KIFI_OK;
 }
-// CTAs of a gradient pass, 64 rows a tile, at most eight per SM
+// CTAs of a gradient pass, 64 rows a tile, at most eight on each of the GPU's 152 SMs
 int tile_grid(int M) { return std::min((M + kTileM - 1) / kTileM, 8 * 152); }
+// floats of the gradient passes' column sums
+size_t bias_part_size(int batch) {
+    size_t n = (size_t)tile_grid(batch) * (kOutPad + kFc1);
+    for (int l = 0; l < kConvs; ++l) n += (size_t)tile_grid((int)conv_m(l, batch)) * kCout[l];
+    return n;
+}
 
 const bf16* wb(const kifi_proposer* pr, int t) { return pr->pb + kLayout.off[t]; }
 const float* pf(const kifi_proposer* pr, int t) { return pr->p + kLayout.off[t]; }
@@ -448,15 +490,25 @@ kifi_status backward(kifi_proposer* pr, int batch) {
         for (int l = 1; l < kConvs; ++l) add(wb(pr, 2 * l), kCout[l], kKp[l], pr->wT[2 * l]);
         k_transpose<<<tiles, dim3(32, 8), 0, st>>>(tj);
     }
+    BiasJobs bj{};
+    float* next = pr->bias_part;
+    // the place of a pass's column sums, whose total goes to parameter t's gradient
+    auto sums = [&](int t, int ctas, int cols) {
+        bj.j[bj.n++] = BiasJob{next, gf(pr, t), ctas, cols};
+        bj.cols += cols;
+        float* const at = next;
+        next += (size_t)ctas * cols;
+        return at;
+    };
     // fc2: db2 = colsum(dout), dW2 [16 x 64] = dout^T h1, dh1 = dout W2
     k_grad<kOutPad, GradSrc::kPlain><<<tile_grid(batch), kThreads, 0, st>>>(pr->y2, nullptr, batch, nullptr,
-                                                                          pr->dbfT, gf(pr, 11));
+                                                                          pr->dbfT, sums(11, tile_grid(batch), kOutPad));
     if ((s = gemm(pr, pr->dbfT, pr->h1T, gf(pr, 10), kOutPad, kFc1, batch, batch, batch, kFc1, batch, true)))
         return s;
     if ((s = gemm(pr, pr->dbf, pr->wT[10], pr->y, batch, kFc1, kOutPad, kOutPad, kOutPad, kFc1, 0, false))) return s;
     // fc1: through its ReLU; db1, dW1 [64 x 128] = dh^T gap, dgap = dh W1
     k_grad<kFc1, GradSrc::kPlain><<<tile_grid(batch), kThreads, 0, st>>>(pr->y, pr->h1, batch, pr->dbf,
-                                                                       pr->dbfT, gf(pr, 9));
+                                                                       pr->dbfT, sums(9, tile_grid(batch), kFc1));
     if ((s = gemm(pr, pr->dbfT, pr->gapT, gf(pr, 8), kFc1, 128, batch, batch, batch, 128, batch, true))) return s;
     if ((s = gemm(pr, pr->dbf, pr->wT[8], pr->y2, batch, 128, kFc1, kFc1, kFc1, 128, 0, false))) return s;
     for (int l = kConvs - 1; l >= 0; --l) {
@@ -465,7 +517,7 @@ kifi_status backward(kifi_proposer* pr, int batch) {
         // the convolution above (y2 = its dcol)
         bf16* const db = pr->dbf;
         bf16* const dt = pr->dbfT;
-        float* const bias = gf(pr, 2 * l + 1);
+        float* const bias = sums(2 * l + 1, grid, kCout[l]);
         if (l == 3) k_grad<128, GradSrc::kPool><<<grid, kThreads, 0, st>>>(pr->y2, pr->act[3], M, db, dt, bias);
         else if (l == 2) k_grad<64, GradSrc::kConv, 3><<<grid, kThreads, 0, st>>>(pr->y2, pr->act[2], M, db, dt, bias);
         else if (l == 1) k_grad<64, GradSrc::kConv, 2><<<grid, kThreads, 0, st>>>(pr->y2, pr->act[1], M, db, dt, bias);
@@ -476,6 +528,7 @@ kifi_status backward(kifi_proposer* pr, int batch) {
         // dcol = dY W for the layer below
         if ((s = gemm(pr, pr->dbf, pr->wT[2 * l], pr->y2, M, Kp, Co, Co, Co, Kp, 0, false))) return s;
     }
+    KIFI_CUDA(chain_launch(true, dim3(bj.cols), dim3(kThreads), st, k_bias_sum, bj));
     KIFI_CUDA(cudaGetLastError());
     return KIFI_OK;
 }
@@ -505,7 +558,7 @@ kifi_status kifi_proposer_destroy(kifi_proposer* pr) {
     if (!pr) return KIFI_OK;
     if (pr->stream) cudaStreamSynchronize(pr->stream);
     void* bufs[] = {pr->status, pr->loss, pr->p, pr->g, pr->m1, pr->m2, pr->pb, pr->mask, pr->x, pr->y, pr->y2,
-                    pr->gap, pr->gapT, pr->h1, pr->h1T, pr->out, pr->dbf, pr->dbfT, pr->col};
+                    pr->gap, pr->gapT, pr->h1, pr->h1T, pr->out, pr->dbf, pr->dbfT, pr->col, pr->bias_part};
     for (void* b : bufs) cudaFree(b);
     for (int l = 0; l < kConvs; ++l) {
         cudaFree(pr->colT[l]);
@@ -557,6 +610,7 @@ kifi_status kifi_proposer_create(int device, int max_batch, kifi_proposer** out)
     alloc(&pr->out, B * kOutPad * 4);
     alloc(&pr->dbf, dmax * 2);
     alloc(&pr->dbfT, dmax * 2);
+    alloc(&pr->bias_part, bias_part_size(max_batch) * 4);
     for (int t = 2; t <= 10; t += 2) alloc(&pr->wT[t], kLayout.size[t] * 2);
     if (!e) e = cudaMemsetAsync(pr->status, 0, 16, pr->stream);
     if (!e) e = cudaMemsetAsync(pr->p, 0, P * 4, pr->stream);
