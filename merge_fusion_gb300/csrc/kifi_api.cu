@@ -633,9 +633,8 @@ static kifi_status mesh_to_device(kifi_volume* v, int with_indices, size_t* n_ve
     if (n >= ((size_t)1 << 28)) return fail(KIFI_ERR_UNSUPPORTED, "mesh of more than 2^28 voxels");
     const unsigned int cur = v->ctl_host->cur;
     // with headroom: a growing volume's next meshes still fit
-    if (v->ms.cap < n) KIFI_CUDA(mesh_scratch_reserve(&v->ms, n + n / 4, v->g.kb));
+    KIFI_CUDA(mesh_scratch_reserve(&v->ms, n, n + n / 4, 0, v->g.kb));
     const unsigned int n32 = (unsigned int)n;
-    KIFI_CUDA(cudaMemcpyAsync(v->ms.n_dev, &n32, sizeof n32, cudaMemcpyHostToDevice, v->stream));
     std::array<cudaEvent_t, 5> ev{};
     if (v->profiling) {
         for (int k = 0; k < 5; ++k) {
@@ -647,24 +646,35 @@ static kifi_status mesh_to_device(kifi_volume* v, int with_indices, size_t* n_ve
             ev[k] = v->event_pool.back();
             v->event_pool.pop_back();
         }
-        KIFI_CUDA(cudaEventRecord(ev[0], v->stream));
     }
-    KIFI_CUDA(mesh_count_enqueue(v->vb.keys[cur], v->vb.key_bytes, v->vb.vals[cur], n, v->g.kb,
-                                 with_indices ? 1 : 0, v->ms, v->stream, ev[0] ? &ev[1] : nullptr));
-    if (ev[0]) KIFI_CUDA(cudaEventRecord(ev[3], v->stream));
     MeshCounts* mc = &v->ctl_host_mesh;
-    for (int attempt = 0; attempt < 2; ++attempt) {
+    bool counted = false, timed = ev[0] != nullptr;
+    for (int attempt = 0;; ++attempt) {
+        if (!counted) {
+            KIFI_CUDA(cudaMemcpyAsync(v->ms.n_dev, &n32, sizeof n32, cudaMemcpyHostToDevice, v->stream));
+            if (timed) KIFI_CUDA(cudaEventRecord(ev[0], v->stream));
+            KIFI_CUDA(mesh_count_enqueue(v->vb.keys[cur], v->vb.key_bytes, v->vb.vals[cur], n, v->g.kb,
+                                         with_indices ? 1 : 0, v->ms, v->stream, timed ? &ev[1] : nullptr));
+            if (timed) KIFI_CUDA(cudaEventRecord(ev[3], v->stream));
+            counted = true;
+        }
         KIFI_CUDA(mesh_emit_enqueue(v->g, v->vb.key_bytes, v->vb.vals[cur], n,
                                     with_indices ? 1 : 0, v->ms, v->mesh_verts_cap, v->mesh_idx_cap, v->mesh_verts,
                                     v->mesh_idx, v->ls.sms, v->stream));
-        if (attempt == 0 && ev[0]) {
-            KIFI_CUDA(cudaEventRecord(ev[4], v->stream));
-            v->mesh_pending.push_back(ev);
-        }
+        if (timed) KIFI_CUDA(cudaEventRecord(ev[4], v->stream));
         KIFI_CUDA(cudaMemcpyAsync(mc, v->ms.counts, sizeof(MeshCounts), cudaMemcpyDeviceToHost, v->stream));
         KIFI_CUDA(cudaStreamSynchronize(v->stream));
+        if (timed && mc->overflow != kMeshWords) {
+            v->mesh_pending.push_back(ev);
+            timed = false;
+        }
         if (!mc->overflow) break;
-        if (attempt == 1) return fail(KIFI_ERR_CUDA, "mesh emission overflowed buffers sized to its counts");
+        if (attempt == 2) return fail(KIFI_ERR_CUDA, "mesh emission overflowed buffers sized to its counts");
+        if (mc->overflow == kMeshWords) {
+            KIFI_CUDA(mesh_scratch_reserve(&v->ms, n, n + n / 4, mc->n_words, v->g.kb));
+            counted = false;
+            continue;
+        }
         const size_t nv = (size_t)mc->n_verts, ni = with_indices ? (size_t)mc->n_idx : 0;
         if (nv > v->mesh_verts_cap) {
             cudaFree(v->mesh_verts);

@@ -172,8 +172,8 @@ kifi_status mesh_emit(kifi_pipeline* p, std::array<cudaEvent_t, 2>* ev) {
 // were too small -- grow them and emit again.  With `wait`, until it is done.
 kifi_status mesh_poll(kifi_pipeline* p, bool wait) {
     for (int emitted = 0; p->counting; ++emitted) {
-        // buffers grown to the counts hold the mesh: a second overflow is an internal error
-        if (emitted > 1) return fail(KIFI_ERR_CUDA, "mesh emission overflowed buffers sized to its counts");
+        // scratch and buffers grown to the counts hold the mesh: a third overflow is an internal error
+        if (emitted > 2) return fail(KIFI_ERR_CUDA, "mesh emission overflowed buffers sized to its counts");
         if (wait) {
             KIFI_CUDA(cudaEventSynchronize(p->counts_ready));
         } else {
@@ -189,6 +189,16 @@ kifi_status mesh_poll(kifi_pipeline* p, bool wait) {
             p->counting = false;
             ++p->meshes;
             return KIFI_OK;
+        }
+        if (c.overflow == kMeshWords) {  // more words than the scratch holds: counted again in a larger one
+            kifi_volume* v = p->vol;
+            KIFI_CUDA(mesh_scratch_reserve(&p->mscr, p->snap_n, std::min(p->snap_n + p->snap_n / 4, p->snap_cap),
+                                           c.n_words, v->g.kb));
+            KIFI_CUDA(mesh_count_enqueue(p->snap_keys, v->vb.key_bytes, p->snap_vals, p->snap_n, v->g.kb,
+                                         p->desc.mesh_with_indices, p->mscr, p->ms));
+            kifi_status s = mesh_emit(p, nullptr);
+            if (s) return s;
+            continue;
         }
         // half again as much: a growing volume's next meshes still fit
         if (nv > p->mverts_cap) {
@@ -228,10 +238,8 @@ kifi_status mesh_begin(kifi_pipeline* p) {
     }
     // the passes' grids cover the host's upper bound of the voxel count
     p->snap_n = v->n_upper < p->snap_cap ? v->n_upper : p->snap_cap;
-    if (p->mscr.cap < p->snap_n) {  // with headroom: freeing scratch waits for the device
-        const size_t want = p->snap_n + p->snap_n / 4;
-        KIFI_CUDA(mesh_scratch_reserve(&p->mscr, want < p->snap_cap ? want : p->snap_cap, v->g.kb));
-    }
+    // with headroom: freeing scratch waits for the device
+    KIFI_CUDA(mesh_scratch_reserve(&p->mscr, p->snap_n, std::min(p->snap_n + p->snap_n / 4, p->snap_cap), 0, v->g.kb));
     KIFI_CUDA(cudaEventRecord(p->frame_done, p->vs));
     KIFI_CUDA(cudaStreamWaitEvent(p->ms, p->frame_done, 0));
     KIFI_CUDA(mesh_snapshot_enqueue(v->ctl, v->vb, p->snap_keys, p->snap_vals, p->snap_n, p->mscr.n_dev, v->ls.sms,

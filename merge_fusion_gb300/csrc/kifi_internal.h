@@ -227,9 +227,11 @@ struct MeshCounts {
     unsigned long long n_verts;
     unsigned long long n_idx;
     unsigned long long missing_min;  // smallest triangle edge id without a vertex (or ~0)
-    unsigned long long overflow;     // emission skipped: the output buffers were too small
+    unsigned long long overflow;     // emission skipped: kMeshBuffers or kMeshWords were too small
     unsigned int runs_done;          // classification CTAs that have finished
+    unsigned int n_words;
 };
+constexpr unsigned long long kMeshBuffers = 1, kMeshWords = 2;  // the output buffers, the scratch's words
 
 // The volume as words: runs of 32 consecutive keys (key >> 5) with at least
 // one resident voxel, ascending; at most one per voxel.
@@ -243,7 +245,8 @@ struct MeshWords {
 };
 
 struct MeshScratch {
-    void* block = nullptr;  // the allocation that holds the arrays below
+    void* tables = nullptr;  // the allocation that holds the arrays whose sizes the volume does not change
+    void* block = nullptr;   // and the one for the words and the list
     MeshWords words;
     uint2* flagged = nullptr;            // a slot per voxel: those with output, run by run, ascending --
                                          // word within the run << 13 | bit << 8 | case; first index, from the word's link
@@ -252,10 +255,14 @@ struct MeshScratch {
     unsigned int* rows = nullptr;         // first word of each (z, y) key row
     MeshCounts* counts = nullptr;
     unsigned int* n_dev = nullptr;        // the voxel count the passes read
-    size_t cap = 0, rows_cap = 0;
+    size_t cap = 0, words_cap = 0, rows_cap = 0;
 };
 
-cudaError_t mesh_scratch_reserve(MeshScratch* m, size_t n, int kb);
+// Scratch for a mesh of up to n voxels: room for `want` (>= n) where it can be
+// had.  Its words are an estimate until a mesh has asked for more: a mesh with
+// more words than they hold is not emitted (MeshCounts::overflow kMeshWords), and
+// is to be counted again after a call with its n_words.
+cudaError_t mesh_scratch_reserve(MeshScratch* m, size_t n, size_t want, size_t n_words, int kb);
 void mesh_scratch_free(MeshScratch* m);
 // stage_events (optional, 2 entries): recorded after the words are built and
 // after the classification

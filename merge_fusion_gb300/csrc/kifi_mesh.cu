@@ -190,7 +190,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_word_build(const K* __restrict_
                                                             const float2* __restrict__ vals,
                                                             const unsigned int* __restrict__ n_dev,
                                                             const unsigned int* __restrict__ run_words,
-                                                            unsigned int* __restrict__ rows, MeshWords words) {
+                                                            unsigned int* __restrict__ rows, MeshWords words,
+                                                            unsigned int words_cap, MeshCounts* __restrict__ mc) {
     constexpr unsigned int kWarps = kThreads / 32, kSteps = kBuildTile / (4 * kThreads);  // 128 voxels per warp step
     __shared__ __align__(16) K s_key[kBuildTile + 32];
     __shared__ unsigned short s_list[kBuildTile + 1];  // positions where words start, then the last one's end
@@ -215,7 +216,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_word_build(const K* __restrict_
         unsigned long long total;
         block_exclusive_scan<kThreads>((unsigned long long)all << 32 | before, &total);
         base = (unsigned int)total;
-        if (blockIdx.x == 0 && threadIdx.x == 0) *words.count = (unsigned int)(total >> 32);
+        const unsigned int n_words = (unsigned int)(total >> 32);
+        const bool fit = n_words <= words_cap;  // else none is written (every CTA alike), and the emission says so
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            *words.count = fit ? n_words : 0u;
+            mc->n_words = n_words;
+        }
+        if (!fit) return;
     }
     K* wkey = (K*)words.key;
     // four bits per lane, eight lanes to a group's 32: to every lane of the group
@@ -760,7 +767,8 @@ __global__ void __launch_bounds__(kThreads) k_mesh_emit(int kb, const float2* __
                                                         MeshWords words, const uint4* __restrict__ run_out,
                                                         unsigned int runs,
                                                         const uint2* __restrict__ flagged,
-                                                        MeshCounts* __restrict__ mc, unsigned long long vert_cap,
+                                                        MeshCounts* __restrict__ mc, unsigned int words_cap,
+                                                        unsigned long long vert_cap,
                                                         unsigned long long idx_cap, float* __restrict__ verts,
                                                         uint32_t* __restrict__ idx) {
     __shared__ uint64_t s_mc[256];
@@ -770,11 +778,12 @@ __global__ void __launch_bounds__(kThreads) k_mesh_emit(int kb, const float2* __
     __syncthreads();
     const unsigned int n_verts = run_out[runs].x, n_idx = run_out[runs].y, n_out = s_cf[runs];
     // outputs that do not fit are not written (every CTA returns alike; the host grows and re-emits)
-    const bool overflow = n_verts > vert_cap || (kTris && n_idx > idx_cap);
+    const bool too_many = mc->n_words > words_cap;
+    const bool overflow = too_many || n_verts > vert_cap || (kTris && n_idx > idx_cap);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         mc->n_verts = n_verts;
         mc->n_idx = n_idx;
-        mc->overflow = overflow ? 1ull : 0ull;
+        mc->overflow = too_many ? kMeshWords : overflow ? kMeshBuffers : 0ull;
     }
     if (overflow) return;
     const unsigned long long bound = kTris ? mc->missing_min : ~0ull;  // ids from here on stay ids
@@ -956,68 +965,125 @@ __global__ void __launch_bounds__(kThreads) k_mesh_emit(int kb, const float2* __
 
 }  // namespace
 
-cudaError_t mesh_scratch_reserve(MeshScratch* m, size_t n, int kb) {
-    const size_t rows = (size_t)1 << (2 * kb);
-    if (m->cap >= n && m->block && m->rows_cap >= rows) return cudaSuccess;
-    if (n < m->cap) n = m->cap;
-    mesh_scratch_free(m);
-    const size_t cap = n < 1024 ? 1024 : n;
-    const size_t key_words = (size_t)1 << (3 * kb - 5);
-    const size_t words = (cap < key_words ? cap : key_words) + 1;
-    // one allocation, cut into 256-byte aligned arrays
+namespace {
+
+// one allocation, cut into 256-byte aligned arrays
+struct Cut {
     size_t size = 0;
-    auto take = [&](size_t bytes) {
+    size_t take(size_t bytes) {
         const size_t at = size;
         size += (bytes + 255) / 256 * 256;
         return at;
-    };
-    const size_t key = take(words * sizeof(uint64_t)), a = take(words * sizeof(uint4)), b = take(words * sizeof(uint2)),
-                 v = take(words * sizeof(uint4)), link = take(words * sizeof(uint4)), flagged = take(cap * sizeof(uint2)),
-                 run_words = take(kVoxelRuns * sizeof(unsigned int)), run_out = take((kWordRuns + 1) * sizeof(uint4)),
-                 row = take(rows * sizeof(unsigned int)), counts = take(sizeof(MeshCounts)),
-                 single = take(2 * sizeof(unsigned int));
-    const cudaError_t e = cudaMalloc(&m->block, size);
-    if (e) return e;
+    }
+};
+
+// The words to expect of `cap` voxels: scans have 10 to 20 voxels to a word.  A
+// word takes 64 B, so one per voxel (any volume fits then) is for small ones only;
+// 16 B per voxel in all for the others, unless their words turn out to be more (of
+// 14.6 M voxels in 1.36 M words 292 MB with headroom, where one per voxel took 1.3 GB).
+size_t likely_words(size_t cap) {
+    const size_t small = cap < 65536 ? cap : 65536;
+    return cap / 8 > small ? cap / 8 : small;
+}
+
+cudaError_t alloc_block(MeshScratch* m, size_t cap, size_t words) {
+    cudaFree(m->block);
+    m->block = nullptr;
+    m->cap = m->words_cap = 0;
+    Cut c;
+    ++words;  // reads go to the word behind the last
+    const size_t key = c.take(words * sizeof(uint64_t)), a = c.take(words * sizeof(uint4)),
+                 b = c.take(words * sizeof(uint2)), v = c.take(words * sizeof(uint4)),
+                 link = c.take(words * sizeof(uint4)), flagged = c.take(cap * sizeof(uint2));
+    const cudaError_t e = cudaMalloc(&m->block, c.size);
+    if (e) {
+        cudaGetLastError();
+        return e;
+    }
     unsigned char* p = (unsigned char*)m->block;
     m->words.key = p + key;
     m->words.a = (uint4*)(p + a);
     m->words.b = (uint2*)(p + b);
     m->words.v = (uint4*)(p + v);
     m->words.link = (uint4*)(p + link);
-    m->words.count = (unsigned int*)(p + single) + 1;
     m->flagged = (uint2*)(p + flagged);
+    m->cap = cap;
+    m->words_cap = words - 1;
+    return cudaSuccess;
+}
+
+// The voxel count is read on the device from ms.n_dev (<= n_cap, which sizes
+// the grids), so the passes can be enqueued before the count is known.
+unsigned int mesh_runs(size_t n_cap, unsigned int most) {
+    const size_t r = (n_cap + kBuildTile - 1) / kBuildTile;
+    return (unsigned int)(r < 1 ? 1 : (r < most ? r : most));
+}
+
+template <typename K>
+void count_words(const K* keys, size_t n_cap, int kb, const MeshScratch& ms, cudaStream_t st) {
+    const unsigned int vruns = mesh_runs(n_cap, kVoxelRuns);
+    const unsigned int row_vecs = (unsigned int)(((size_t)1 << (2 * kb)) / 4);
+    // four vectors of the row table per thread, eight CTAs per SM of the 152 at most
+    const unsigned int clear = row_vecs / (4 * kThreads) < kVoxelRuns / 2 ? row_vecs / (4 * kThreads) : kVoxelRuns / 2;
+    k_word_count<K><<<vruns > clear ? vruns : clear, kThreads, 0, st>>>(keys, ms.n_dev, ms.run_words, vruns,
+                                                                        (uint4*)ms.rows, row_vecs, ms.counts);
+}
+
+cudaError_t alloc_tables(MeshScratch* m, int kb) {
+    const size_t rows = (size_t)1 << (2 * kb);
+    if (m->tables && m->rows_cap >= rows) return cudaSuccess;
+    cudaFree(m->tables);
+    m->tables = nullptr;
+    m->rows_cap = 0;
+    Cut c;
+    const size_t run_words = c.take(kVoxelRuns * sizeof(unsigned int)), run_out = c.take((kWordRuns + 1) * sizeof(uint4)),
+                 row = c.take(rows * sizeof(unsigned int)), counts = c.take(sizeof(MeshCounts)),
+                 single = c.take(2 * sizeof(unsigned int));
+    const cudaError_t e = cudaMalloc(&m->tables, c.size);
+    if (e) {
+        cudaGetLastError();
+        return e;
+    }
+    unsigned char* p = (unsigned char*)m->tables;
+    m->words.count = (unsigned int*)(p + single) + 1;
     m->run_words = (unsigned int*)(p + run_words);
     m->run_out = (uint4*)(p + run_out);
     m->rows = (unsigned int*)(p + row);
     m->counts = (MeshCounts*)(p + counts);
     m->n_dev = (unsigned int*)(p + single);
     m->rows_cap = rows;
-    m->cap = cap;
     return cudaSuccess;
 }
 
-void mesh_scratch_free(MeshScratch* m) {
-    cudaFree(m->block);
-    *m = MeshScratch{};
+}  // namespace
+
+cudaError_t mesh_scratch_reserve(MeshScratch* m, size_t n, size_t want, size_t n_words, int kb) {
+    cudaError_t e = alloc_tables(m, kb);
+    if (e || (m->block && m->cap >= n && m->words_cap >= n_words)) return e;
+    if (want < m->cap) want = m->cap;
+    if (want < 1024) want = 1024;
+    const size_t likely = likely_words(want), ahead = n_words + n_words / 4;
+    e = alloc_block(m, want, likely > ahead ? likely : ahead);
+    if (e == cudaErrorMemoryAllocation) {
+        const size_t words = likely_words(n);
+        e = alloc_block(m, n, words > n_words ? words : n_words);
+    }
+    return e;
 }
 
-// The voxel count is read on the device from ms.n_dev (<= n_cap, which sizes
-// the grids), so the passes can be enqueued before the count is known.
-static unsigned int mesh_runs(size_t n_cap, unsigned int most) {
-    const size_t r = (n_cap + kBuildTile - 1) / kBuildTile;
-    return (unsigned int)(r < 1 ? 1 : (r < most ? r : most));
+void mesh_scratch_free(MeshScratch* m) {
+    cudaFree(m->tables);
+    cudaFree(m->block);
+    *m = MeshScratch{};
 }
 
 template <typename K>
 static void mesh_count_t(const K* keys, const float2* vals, size_t n_cap, int kb, int with_indices, MeshScratch& ms,
                          cudaStream_t st, cudaEvent_t* stage_events) {
     const unsigned int vruns = mesh_runs(n_cap, kVoxelRuns), wruns = mesh_runs(n_cap, kWordRuns);
-    const unsigned int row_vecs = (unsigned int)(((size_t)1 << (2 * kb)) / 4);
-    // four vectors of the row table per thread, eight CTAs per SM of the 152 at most
-    const unsigned int clear = row_vecs / (4 * kThreads) < kVoxelRuns / 2 ? row_vecs / (4 * kThreads) : kVoxelRuns / 2;
-    k_word_count<K><<<vruns > clear ? vruns : clear, kThreads, 0, st>>>(keys, ms.n_dev, ms.run_words, vruns,
-                                                                        (uint4*)ms.rows, row_vecs, ms.counts);
-    k_word_build<K><<<vruns, kThreads, 0, st>>>(keys, kb, vals, ms.n_dev, ms.run_words, ms.rows, ms.words);
+    count_words<K>(keys, n_cap, kb, ms, st);
+    k_word_build<K><<<vruns, kThreads, 0, st>>>(keys, kb, vals, ms.n_dev, ms.run_words, ms.rows, ms.words,
+                                                  (unsigned int)ms.words_cap, ms.counts);
     if (stage_events) cudaEventRecord(stage_events[0], st);
     if (with_indices)
         k_word_classify<true, K><<<wruns, kClassThreads, 0, st>>>(kb, vals, ms.n_dev, ms.rows, ms.words, ms.run_out,
@@ -1047,10 +1113,10 @@ static void mesh_emit_t(const Geom& g, const float2* vals, size_t n_cap, int wit
     const int grid = (int)(want < 1 ? 1 : (want > (size_t)sms * 4 ? (size_t)sms * 4 : want));
     if (with_indices)
         k_mesh_emit<true, K><<<grid, kThreads, 0, st>>>(kb, vals, g, ms.words, ms.run_out, runs, ms.flagged, ms.counts,
-                                                       vert_cap, idx_cap, verts_dev, idx_dev);
+                                                       (unsigned int)ms.words_cap, vert_cap, idx_cap, verts_dev, idx_dev);
     else
         k_mesh_emit<false, K><<<grid, kThreads, 0, st>>>(kb, vals, g, ms.words, ms.run_out, runs, ms.flagged, ms.counts,
-                                                        vert_cap, idx_cap, verts_dev, idx_dev);
+                                                        (unsigned int)ms.words_cap, vert_cap, idx_cap, verts_dev, idx_dev);
 }
 
 cudaError_t mesh_emit_enqueue(const Geom& g, int key_bytes, const float2* vals, size_t n_cap, int with_indices,
