@@ -336,7 +336,10 @@ kifi_status kifi_batch_step_device(kifi_batch* b, const void* const* depth_dev, 
     // tracking first: the step's critical path, on the higher-priority stream
     if (!ijobs.empty()) {
         BlockMap im{(const unsigned int*)(dv + o_im), (int)ijobs.size(), imap.back()};
-        KIFI_CUDA(icp_align_batch_enqueue((const IcpJob*)(dv + o_ij), (int)ijobs.size(), im, iters, b->ts));
+        KIFI_CUDA(icp_align_batch_enqueue((const IcpJob*)(dv + o_ij), (int)ijobs.size(), im, iters,
+                                          std::all_of(ijobs.begin(), ijobs.end(),
+                                                      [](const IcpJob& j) { return j.a.prune != kPruneOff; }),
+                                          b->ts));
     }
     if (!bjobs.empty()) {
         BlockMap bm{(const unsigned int*)(dv + o_bm), (int)bjobs.size(), bmap.back()};

@@ -13,8 +13,11 @@
 //                (:100-131; the first minimum in scan order wins).  Only the
 //                candidates that can win are read: a bound on the distance
 //                (the last step's winner, or a few probes) cuts the window to
-//                a rectangle, see Prune.  CTAs own tiles of sources and stage
-//                the part of the target they will read in shared memory.
+//                a rectangle, see Prune.  Where that is much of the window
+//                (the first step, fast motion, targets of which nothing is
+//                known) a tile scans its windows whole, two candidates at a
+//                time.  CTAs own tiles of sources and stage the part of the
+//                target they will read in shared memory.
 //  moments       the associated pairs are not stored: count, sum p, sum q,
 //                sum p q^T and the squared distances are accumulated per
 //                CTA in float-float, each product split exactly by an FMA.
@@ -174,26 +177,29 @@ constexpr int kTileThreads = kTileCols * kTileRows;  // one source per thread
 static_assert(kTileThreads == kIcpTileSources, "a winner per source");
 constexpr int kPredMargin = 4;  // pixels added around the rectangles that a tile searched in the last step,
 constexpr int kUseMargin = 4;   // and that the region so staged must leave around the projections to be used
-// Target points (float4) staged per tile, by the tiles that share an SM.  Two: 80
-// KB each and 128 registers a thread, for launches that fill no more than that
-// in one round, where a tile's own time counts.  Three: 52 KB and 80 registers (a
-// few spilled words), for more tiles than that: a tile takes longer, but 24
-// warps hide more of the waits (of an SM's issue slots 0.43 were used with 16).
-// Eight sequences, 15 steps: 11937 -> 10784 us; tracking at 1024x848 (864 tiles):
-// 6140 -> 5817; at 640x480 (300 tiles) 327 against 333.  52 KB hold a tile's windows
-// (32 pixels and 20 around) while the target's pixels are no finer than 1 / 1.15 of
-// the source's; for finer targets the two stay (a 1024x768 target for 640x480
-// frames: 2100 against 2365).
-template <int kPerSm>
-constexpr int kStagePixels = kPerSm == 3 ? 3328 : 5120;
-// One: launches of no more tiles than SMs have two threads per source (two
-// halves of the CTA), which bound alike and search half of the rectangle's rows
-// each: with one thread a source, 8 warps have an SM to themselves, and fast
-// motion leaves rectangles of hundreds of candidates (a 410x307 pair three
-// frames apart, 10 steps 398 -> 333 us; a 348x288 pair, 9 steps 199 -> 183;
-// tracking at 384x315, 9 frames 2297 -> 2109).
-template <int kPerSm>
-constexpr int kHalves = kPerSm == 1 ? 2 : 1;
+// The step's builds.  Build kWhole scans whole windows only; the others scan
+// windows or search rectangles, tile by tile (whole_next), and differ in how
+// many tiles share an SM.  One: launches of no more tiles than SMs, with two
+// threads per source.  Two: 80 KB of target and 128 registers a thread, for
+// launches that fill no more than that in one round, where a tile's own time
+// counts.  Three: 52 KB and 80 registers (a few spilled words) for more tiles: a
+// tile takes longer, but 24 warps hide more of the waits (tracking at 1024x848,
+// 864 tiles, ten frames 6140 -> 5817 us; at 640x480, 300 tiles, 327 against 333).
+// 52 KB hold a tile's rectangles (32 pixels and up to 20 around) while the target's
+// pixels are no finer than 1 / 1.15 of the source's; for finer ones the 80 KB stay
+// (a 1024x768 target for 640x480 frames, the closed loop: 2100 us against 2365).
+constexpr int kWhole = 0;
+// Two halves of the CTA per source search half of the rows each: whole windows
+// in 19 us a step at 640x480 (with one thread per source 21 to 26), and in small
+// launches, where 8 warps would have an SM to themselves.
+template <int kS>
+constexpr int kHalves = kS <= 1 ? 2 : 1;
+template <int kS>
+constexpr int kResident = kS == kWhole ? 2 : kS;  // CTAs per SM
+// Target points (float4) staged per tile.
+template <int kS>
+constexpr int kStagePixels = kS == kWhole ? 0 : kS == 3 ? 3328 : 5120;
+constexpr int kWindowMargin = 5;  // pixels added around the windows that a tile scanned
 
 // Row pitch of a staged region `w` pixels wide: odd, so that the 16-byte
 // loads of eight lanes one row apart cover all banks.
@@ -223,6 +229,41 @@ __device__ __forceinline__ void stage_region(float4* stage, const float4* __rest
     }
 }
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The same region as three float planes (x, y, z), for the whole-window scan:
+// two adjacent candidates are one 64-bit load per plane.  The pitch is even, so
+// that such pairs are aligned, with pitch / 2 odd, so that the 64-bit loads of
+// lanes whose windows lie one row apart hit distinct banks.  Asynchronous copies
+// (stage_wait) of 4 bytes: they take no registers, and the planes of a region
+// staged ahead arrive while the step before finishes.
+__host__ __device__ constexpr int plane_pitch(int w) {
+    return ((w + 1) & ~1) + ((((w + 1) & ~1) >> 1) & 1 ? 0 : 2);
+}
+struct Planes {
+    float *x, *y, *z;
+};
+template <int kWarps>
+__device__ __forceinline__ void stage_planes(const Planes& stage, const float4* __restrict__ synth, size_t n_synth,
+                                             int synth_w, int x0, int y0, int w, int h, int pitch) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned int dx = (unsigned int)__cvta_generic_to_shared(stage.x), dy = (unsigned int)__cvta_generic_to_shared(stage.y),
+                       dz = (unsigned int)__cvta_generic_to_shared(stage.z);
+    for (int ry = warp; ry < h; ry += kWarps) {
+        for (int rx = lane; rx < w; rx += 32) {
+            const size_t at = (size_t)(y0 + ry) * synth_w + (x0 + rx);
+            const int to = ry * pitch + rx;
+            if (at < n_synth && x0 + rx < 640) {  // (the reference's windows end at column 640)
+                const float* q = reinterpret_cast<const float*>(synth + at);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dx + 4u * to), "l"(q) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dy + 4u * to), "l"(q + 1) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dz + 4u * to), "l"(q + 2) : "memory");
+            } else {
+                stage.x[to] = __int_as_float(0x7fffffff);
+                stage.y[to] = stage.z[to] = 0.0f;
+            }
+        }
+    }
+}
 
 // Which candidates of a source's window can win.
 //
@@ -287,25 +328,52 @@ struct Rect {
     int number;       // the first candidate's number r * 32 + c << 8 | columns
 };
 constexpr int kItems = 21 * kTileThreads;  // every row of every window
-template <int kH>
+template <int kS>
+struct TileList {  // per thread: kHalves to a source
+    static constexpr int kThreads = kTileThreads * kHalves<kS>;
+    Packed p[kThreads];               // world point
+    Rect rect[kThreads];
+    unsigned short item[kItems];      // rows to search: thread << 5 | row
+    unsigned long long key[kThreads]; // best so far: len^2 bits << 32 | candidate number
+};
+template <>
+struct TileList<kWhole> {
+    float rec[7][kTileThreads];
+    unsigned long long key[2 * kTileThreads];
+};
+// The tile's dynamic shared memory: the staged float4s and the list, whose start
+// the sources' records take after the search -- per source p xyz, q xyz, len^2
+// (zeros when no pair).  Planes of a whole-window scan reach over both, up to
+// the keys.
+template <int kS>
+constexpr size_t kStageBytes = kS == kWhole ? 5120 * 12 : kStagePixels<kS> * sizeof(float4);
+template <int kS>
+constexpr size_t kTileBytes = kStageBytes<kS> + sizeof(TileList<kS>);
+template <int kS>
+constexpr int kPlanePixels =
+    (int)((kStageBytes<kS> + (kS == kWhole ? 0 : offsetof(TileList<kS>, key))) / 12) & ~1;
 struct SearchSmem {
-    struct List {  // per thread: kH to a source
-        Packed p[kTileThreads * kH];                // world point
-        Rect rect[kTileThreads * kH];
-        unsigned long long key[kTileThreads * kH];  // best so far: len^2 bits << 32 | candidate number
-        unsigned short item[kItems];           // rows to search: thread << 5 | row
-    };
-    union {
-        List list;
-        float rec[7][kTileThreads];  // per source: p xyz, q xyz, len^2 (0 when no pair)
-    };
     unsigned int n_items;
     int box[4];      // the tile's rectangles: x0, y0, x1, y1
-    int cbox[4];     // and projections
+    int cbox[4];     // and projections (or windows)
     int pred[4];     // the region staged ahead: x0, y0, w, h
+    int ahead_whole; // as planes, for a whole-window scan
+    unsigned int area, windows;  // candidates in the rectangles and in the windows
     FF acc[17];      // the CTA's moments (index 0 unused: count)
     unsigned int count;
 };
+// Whether the tile's next step scans whole windows: where its rectangles hold
+// more than a quarter of the windows' candidates.  The whole-window scan reads two
+// candidates at a time with no bounds or boxes before it, and all of a warp's
+// lanes alike; with fast motion a tile of large rectangles holds up its whole step.
+// The share is the step's own after a search, and after a scan what the distances
+// to the winners would leave.  Times, us, searching rectangles only / whole windows
+// only / by tile: 640x480, 15 steps, frames one apart 375 / 423 / 372, three apart
+// 498 / 461 / 456; 410x307, 10 steps, three apart 263 / 232 / 213; tracking at 640x480,
+// ten frames 5267 / - / 5069.  An eighth instead of a quarter: 358 and 440, but
+// the closed loop 2117 -> 2175 us; a half: 376 and 501.
+constexpr unsigned int kWholeShare = 4;  // sixteenths
+__device__ __forceinline__ int whole_next(const SearchSmem& ss) { return ss.area * 16u > ss.windows * kWholeShare; }
 // What part of the target a tile has staged: pixels [x0, x1) x [y0, y1).
 struct Region {
     int buf;  // its first pixel's index in the CTA's staging buffer
@@ -360,6 +428,129 @@ __device__ __forceinline__ void scan_row(const float4* __restrict__ synth, long 
     }
 }
 
+__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long f2_sq(unsigned long long a, unsigned long long neg_zero) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(a), "l"(neg_zero));
+    return d;
+}
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// The whole-window scan of a thread's rows (`base`: its first candidate's plane
+// index).  A row is 21 wide (past the window's clamp at 640 columns the planes
+// hold no points): ten aligned pairs of adjacent candidates, whose
+// squared distances are formed two at a time (each half with the reference's
+// operations and rounding), plus the one left over: the first when the window
+// starts on an odd plane index, else the last.  Three chains -- the pairs' first
+// halves, their second halves and the left-over ones -- keep their own first
+// strict minimum; the lexicographic (len^2, candidate) minimum of the chains is
+// the first strict minimum of the row-major scan.  Returns the best squared
+// distance (0.01 when none) and its candidate number r * 32 + c (-1 when none).
+// For sources with w = 1 (dz^2 + dw^2 == dz^2 exactly when dw == 0, as dz^2 >= 0).
+__device__ __forceinline__ float scan_planes(const Planes& sp, int base, int pitch, int nr, float px, float py, float pz,
+                                             float neg_zero, int* best_rc) {
+    float b0 = 0.01f, b1 = 0.01f, b2 = 0.01f;
+    int i0 = 0x7fffffff, i1 = 0x7fffffff, i2 = 0x7fffffff;
+    const int o = base & 1;     // the pairs start at an even plane index
+    const int cs = o ? 0 : 20;  // the left-over candidate's column
+    const unsigned long long PX = f2_pack(px, px), PY = f2_pack(py, py), PZ = f2_pack(pz, pz);
+    const unsigned long long NZ = f2_pack(neg_zero, neg_zero);
+    for (int r = 0; r < nr; ++r, base += pitch) {
+        // a candidate records only its pair number (a constant of the
+        // unrolled row); the row and the parity are folded in once per row
+        int c0 = -1, c1 = -1;
+        const int pb = base + o;
+#pragma unroll
+        for (int k = 0; k < 10; ++k) {
+            const int at = pb + 2 * k;
+            const unsigned long long X = *(const unsigned long long*)(sp.x + at);
+            const unsigned long long Y = *(const unsigned long long*)(sp.y + at);
+            const unsigned long long Z = *(const unsigned long long*)(sp.z + at);
+            const unsigned long long dx = f2_sub(X, PX), dy = f2_sub(Y, PY), dz = f2_sub(Z, PZ);
+            const unsigned long long l2 = f2_add(f2_add(f2_sq(dx, NZ), f2_sq(dy, NZ)), f2_sq(dz, NZ));
+            float lo, hi;
+            f2_unpack(l2, lo, hi);
+            if (lo < b0) {
+                b0 = lo;
+                c0 = 2 * k;
+            }
+            if (hi < b1) {
+                b1 = hi;
+                c1 = 2 * k;
+            }
+        }
+        const int r32 = r * 32;
+        {  // one candidate in scalar float, the reference's order: (dx^2 + dy^2) + dz^2
+            const int at = base + cs;
+            const float dx = fsub(sp.x[at], px), dy = fsub(sp.y[at], py), dz = fsub(sp.z[at], pz);
+            const float l2 = fadd(fadd(fmul(dx, dx), fmul(dy, dy)), fmul(dz, dz));
+            if (l2 < b2) {
+                b2 = l2;
+                i2 = r32 + cs;
+            }
+        }
+        if (c0 >= 0) i0 = r32 + o + c0;
+        if (c1 >= 0) i1 = r32 + o + c1 + 1;
+    }
+    if (b1 < b0 || (b1 == b0 && i1 < i0)) {
+        b0 = b1;
+        i0 = i1;
+    }
+    if (b2 < b0 || (b2 == b0 && i2 < i0)) {
+        b0 = b2;
+        i0 = i2;
+    }
+    *best_rc = i0 == 0x7fffffff ? -1 : i0;
+    return b0;
+}
+
+// Any rows of a window in the target itself, one candidate at a time: where the
+// windows are not staged (they span too much), and for sources with w != 1.
+__device__ __noinline__ unsigned long long scan_target(const float4* __restrict__ synth, long long n_synth, int synth_w,
+                                                       int u, int v, int r0, int r1, int nc, float px, float py, float pz,
+                                                       float pw) {
+    const float dw = fsub(1.0f, pw), dw2 = fmul(dw, dw);
+    float best = 0.01f;
+    int rc = -1;
+    for (int r = r0; r < r1; ++r)
+#pragma unroll 3
+        for (int c = 0; c < nc; ++c) {
+            const long long at = (long long)(v + r) * synth_w + (u + c);
+            if (at >= n_synth) break;
+            const float4 q = __ldg(synth + at);
+            const float dx = fsub(q.x, px), dy = fsub(q.y, py), dz = fsub(q.z, pz);
+            const float l2 = fadd(fadd(fmul(dx, dx), fmul(dy, dy)), fadd(fmul(dz, dz), dw2));
+            if (l2 < best) {
+                best = l2;
+                rc = r * 32 + c;
+            }
+        }
+    return rc < 0 ? kNoPair : (unsigned long long)__float_as_uint(best) << 32 | (unsigned int)rc;
+}
+
+// A thread's rows of its window, all candidates, in the staged planes (whose pitch
+// is 0 where they are not staged; `base`: its first candidate's plane index).
+constexpr int kSplitRow = 10;  // of two threads, the first takes window rows [0, 10)
+template <int kH>
+__device__ __forceinline__ unsigned long long search_whole(const IcpArgs& a, const Planes& planes, int pitch, int base,
+                                                           int nr, int nc, int u, int v, const float (&p)[4], int half) {
+    const int r0 = kH == 2 && half ? kSplitRow : 0, r1 = kH == 2 && !half ? min(nr, kSplitRow) : nr;
+    if (r1 <= r0) return kNoPair;
+    if (!pitch || p[3] != 1.0f)
+        return scan_target(a.synth, (long long)a.synth_w * a.synth_h, a.synth_w, u, v, r0, r1, nc, p[0], p[1], p[2], p[3]);
+    int rc = -1;
+    const float best = scan_planes(planes, base + r0 * pitch, pitch, r1 - r0, p[0], p[1], p[2], a.neg_zero, &rc);
+    return rc < 0 ? kNoPair : (unsigned long long)__float_as_uint(best) << 32 | (unsigned int)(rc + r0 * 32);
+}
+
 // The search of a source's window [nr x nc] (first candidate: target pixel
 // (u, v)) by its own thread.  It bounds the distance to the nearest candidate,
 // cuts the window down to the rectangle that can win and, where that is still
@@ -372,17 +563,18 @@ __device__ __forceinline__ void scan_row(const float4* __restrict__ synth, long 
 // coordinate (upwards) and clip w; (hr, hc): a candidate likely to be near
 // (-1: none).  Returns the best key so far; by whole warps.  Measured at
 // 640x480: 10-40 candidates per source instead of 441 after the first two
-// steps, an alignment of 15 steps 335 us (433 us with the whole windows); the
+// steps, an alignment of 15 steps 329 us (433 us with the whole windows); the
 // step is then held by its serial parts -- the projection, the moments, the
 // last CTA's totals and Horn solve, about 11 of 16 us -- and by the tile with
 // the most candidates.
 constexpr int kOwnArea = 32;    // rectangles up to this, and up to 1.5 times the warp's average, are scanned by their thread
 constexpr int kBoxArea = 72;    // rectangles above this are cut down by the blocks' boxes
-template <int kH>
+template <int kS>
 __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const Region& reg, int nr, int nc, int cr,
                                                          int cc, int hr, int hc, bool first, int u, int v, float X,
                                                          float Y, float w, const Prune& pr, const float (&p)[4],
-                                                         int half, SearchSmem<kH>& ss, bool& listed) {
+                                                         int half, SearchSmem& ss, TileList<kS>& list, bool& listed) {
+    constexpr int kH = kHalves<kS>;
     const int W = a.synth_w, H = a.synth_h;
     const Packed pp{f2_pack(p[0], p[1]), f2_pack(p[2], p[3])};
     const unsigned long long nz = f2_pack(a.neg_zero, a.neg_zero);
@@ -499,18 +691,19 @@ __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const
     // (a warp's own rectangles, of vertical neighbours, read shared memory
     // without conflicts; the list's rows do not)
     const int total = (int)__reduce_add_sync(0xffffffffu, (unsigned int)n);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&ss.area, (unsigned int)total);
     const int most = max(kOwnArea, total * 3 >> 6);
     const bool in = reg.holds(x0, y0, cols, rows);
     const int number = r0 * 32 + c0;
     if (n > most && !wraps) {
         listed = true;
         const int me = threadIdx.x;
-        ss.list.p[me] = pp;
-        ss.list.rect[me] = in ? Rect{reg.at(x0, y0), reg.pitch, number << 8 | cols}
+        list.p[me] = pp;
+        list.rect[me] = in ? Rect{reg.at(x0, y0), reg.pitch, number << 8 | cols}
                               : Rect{(long long)y0 * W + x0, -W, number << 8 | cols};
-        ss.list.key[me] = kNoPair;
+        list.key[me] = kNoPair;
         const unsigned int i0 = atomicAdd(&ss.n_items, (unsigned int)rows);
-        for (int r = 0; r < rows; ++r) ss.list.item[i0 + r] = (unsigned short)(me << 5 | r);
+        for (int r = 0; r < rows; ++r) list.item[i0 + r] = (unsigned short)(me << 5 | r);
         return kNoPair;
     }
     float best = 0.01f;
@@ -530,14 +723,14 @@ __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const
 // The listed rows, dealt out to the CTA's threads; a source's key takes the
 // lexicographic (len^2, candidate number) minimum, the first strict minimum
 // in row-major order.
-template <int kH>
+template <int kS>
 __device__ __forceinline__ void search_items(const float4* __restrict__ synth, unsigned int n_items, float neg_zero,
-                                             SearchSmem<kH>& ss) {
+                                             TileList<kS>& list) {
     const unsigned long long nz = f2_pack(neg_zero, neg_zero);
-    for (unsigned int i = threadIdx.x; i < n_items; i += kTileThreads * kH) {
-        const int it = ss.list.item[i], s = it >> 5, row = it & 31;
-        const Packed p = ss.list.p[s];
-        const Rect rect = ss.list.rect[s];
+    for (unsigned int i = threadIdx.x; i < n_items; i += TileList<kS>::kThreads) {
+        const int it = list.item[i], s = it >> 5, row = it & 31;
+        const Packed p = list.p[s];
+        const Rect rect = list.rect[s];
         float best = 0.01f;
         int at = -1;
         const int cols = rect.number & 0xff, number = (rect.number >> 8) + row * 32;
@@ -545,7 +738,7 @@ __device__ __forceinline__ void search_items(const float4* __restrict__ synth, u
             scan_row<true>(nullptr, (int)rect.first + row * rect.stride, cols, p, nz, best, at, number);
         else
             scan_row<false>(synth, rect.first - (long long)row * rect.stride, cols, p, nz, best, at, number);
-        if (at >= 0) atomicMin(&ss.list.key[s], (unsigned long long)__float_as_uint(best) << 32 | (unsigned int)at);
+        if (at >= 0) atomicMin(&list.key[s], (unsigned long long)__float_as_uint(best) << 32 | (unsigned int)at);
     }
 }
 
@@ -594,13 +787,16 @@ __device__ __forceinline__ FF two_prod(float a, float b) {
 // One AlignStep of one frame pair; `blk` / `nblk`: this CTA's index among
 // the nblk CTAs that work on the pair (the launch's own grid, or a share of
 // a batched launch over several pairs).
-template <int kPerSm>
+// kRects: rectangles only
+template <int kS, bool kRects = false>
 __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __restrict__ st, bool first,
                                               unsigned int blk, unsigned int nblk) {
-    constexpr int kH = kHalves<kPerSm>, kWarps = kH * kTileThreads / 32;
+    constexpr int kH = kHalves<kS>, kWarps = kH * kTileThreads / 32;
     static_assert(16 % kWarps == 0 && kMoments == 17, "one or two moments after the count per warp");
-    static_assert(offsetof(typename SearchSmem<kH>::List, key) >= sizeof(SearchSmem<kH>::rec), "keys outlive the records' start");
-    __shared__ SearchSmem<kH> ss;
+    static_assert(offsetof(TileList<kS>, key) >= 7 * kTileThreads * sizeof(float), "keys outlive the records' start");
+    __shared__ SearchSmem ss;
+    TileList<kS>& list = *reinterpret_cast<TileList<kS>*>(reinterpret_cast<unsigned char*>(stage_all) + kStageBytes<kS>);
+    float(*const rec)[kTileThreads] = reinterpret_cast<float(*)[kTileThreads]>(&list);
     __shared__ unsigned int s_hint[kH == 2 ? kTileThreads : 1];  // the halves' common hints
     const int lane = threadIdx.x & 31, half = kH == 2 ? threadIdx.x / kTileThreads : 0;
     const int source = threadIdx.x % kTileThreads, warp = source >> 5;  // the tile's source, its column
@@ -617,16 +813,35 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
     // only a guess) and shared, so every thread stages the same region; after
     // the wait the guess is used if it holds every projection with a margin.
     const int tile0 = (int)blk;
+    // this thread's depth and last winner (a hint: it may be older, any pixel will do)
+    float pre_d = 0.0f;
+    unsigned int pre_hint = ~0u;
+    if (tile0 < tiles) {
+        const int col = (tile0 % tiles_x) * kTileCols + warp, y = (tile0 / tiles_x) * kTileRows + lane;
+        if (col < n_cols && y < a.height) {
+            pre_d = load_depth(a.depth, (size_t)y * a.width + col * 4, a.depth_u16);
+            if (!first && tile0 < kIcpMaxCtas) pre_hint = __ldcg(st->winner + tile0 * kTileThreads + source);
+        }
+    }
+    const Planes planes{(float*)stage_all, (float*)stage_all + kPlanePixels<kS>,
+                        (float*)stage_all + 2 * kPlanePixels<kS>};
     if (threadIdx.x == 0) {
         int p[4] = {0, 0, 0, 0};
-        if (!first && tile0 < tiles && tile0 < kIcpMaxCtas) {  // (the first step's windows are searched widely)
-            const volatile int* tb = st->tile_box + 4 * tile0;
-            const int b0 = tb[0], b1 = tb[1], b2 = tb[2], b3 = tb[3];
+        bool guess = !kRects;
+        if (tile0 < tiles && tile0 < kIcpMaxCtas && (!kRects || !first)) {
+            // (independent reads: one memory latency)
+            const volatile IcpTile* t = st->tile + tile0;
+            const int next_whole = t->whole;
+            const int c0 = t->near[0], c1 = t->near[1], c2 = t->near[2], c3 = t->near[3];
+            const int r0 = t->rect[0], r1 = t->rect[1], r2 = t->rect[2], r3 = t->rect[3];
+            guess = kRects ? false : kS == kWhole || first || next_whole != 0;
+            const int b0 = guess ? c0 : r0, b1 = guess ? c1 : r1, b2 = guess ? c2 : r2, b3 = guess ? c3 : r3;
             if (b2 > b0 && b3 > b1 && b0 >= 0 && b1 >= 0) {
-                const int x0 = max(b0 - kPredMargin, 0), y0 = max(b1 - kPredMargin, 0);
-                const int w = b2 + kPredMargin - x0, h = b3 + kPredMargin - y0;
-                constexpr int most = kStagePixels<kPerSm>;
-                if (w <= most && h <= most && stage_pitch(w) * h <= most) {
+                const int m = guess ? 10 + kWindowMargin : kPredMargin;
+                const int x0 = max(b0 - m, 0), y0 = max(b1 - m, 0);
+                const int w = b2 + m - x0, h = b3 + m - y0;
+                const int most = guess ? kPlanePixels<kS> : kStagePixels<kS>;
+                if (w <= most && h <= most && (guess ? plane_pitch(w) : stage_pitch(w)) * h <= most) {
                     p[0] = x0;
                     p[1] = y0;
                     p[2] = w;
@@ -639,21 +854,17 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             ss.pred[k] = p[k];
             ss.box[k] = ss.cbox[k] = k < 2 ? 0x7fffffff : -1;
         }
-        ss.n_items = ss.count = 0u;
+        ss.ahead_whole = guess;
+        ss.n_items = ss.count = ss.area = ss.windows = 0u;
     }
     if (threadIdx.x < kMoments) ss.acc[threadIdx.x] = FF{0.0f, 0.0f};
     __syncthreads();
     const int px0 = ss.pred[0], py0 = ss.pred[1], pw = ss.pred[2], ph = ss.pred[3];
-    if (pw > 0) stage_region<kWarps>(stage_all, a.synth, n_synth, a.synth_w, px0, py0, pw, ph, stage_pitch(pw));
-    // this thread's depth and last winner (a hint: it may be older, any pixel will do)
-    float pre_d = 0.0f;
-    unsigned int pre_hint = ~0u;
-    if (tile0 < tiles) {
-        const int col = (tile0 % tiles_x) * kTileCols + warp, y = (tile0 / tiles_x) * kTileRows + lane;
-        if (col < n_cols && y < a.height) {
-            pre_d = load_depth(a.depth, (size_t)y * a.width + col * 4, a.depth_u16);
-            if (!first && tile0 < kIcpMaxCtas) pre_hint = __ldcg(st->winner + tile0 * kTileThreads + source);
-        }
+    const bool ahead_whole = ss.ahead_whole != 0;
+    if (pw > 0) {
+        if (!kRects && (kS == kWhole || ahead_whole))
+            stage_planes<kWarps>(planes, a.synth, n_synth, a.synth_w, px0, py0, pw, ph, plane_pitch(pw));
+        else stage_region<kWarps>(stage_all, a.synth, n_synth, a.synth_w, px0, py0, pw, ph, stage_pitch(pw));
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const float half_w = fmul((float)a.synth_w, 0.5f), half_h = fmul((float)a.synth_h, 0.5f);
@@ -688,6 +899,8 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
     }
     for (int tile = (int)blk; tile < tiles; tile += (int)nblk) {
         const bool ahead = tile == tile0;  // its region, depths and hints were loaded above
+        // the tile's scan, as it found it best in the last step
+        const bool whole = kRects ? false : kS == kWhole || first || !pr.on || tile >= kIcpMaxCtas || (ahead ? ahead_whole : st->tile[tile].whole != 0);
         const int col = (tile % tiles_x) * kTileCols + warp, y = (tile / tiles_x) * kTileRows + lane;
         const bool mine = col < n_cols && y < a.height;
         float wp[4] = {0.f, 0.f, 0.f, 0.f};
@@ -723,18 +936,20 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             }
         }
         stage_wait();  // the region staged ahead
-        {  // the projections inside their windows; one shared atomic per warp and bound
+        {  // the windows, or the projections inside them; one shared atomic per warp and bound
             const bool has = nr > 0;
             const int px = min(max(cc, 0), nc - 1) + u, py = min(max(cr, 0), nr - 1) + v;
-            const int mu0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)px : 0x7fffffffu);
-            const int mv0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)py : 0x7fffffffu);
-            const int mu1 = __reduce_max_sync(0xffffffffu, has ? px + 1 : -1);
-            const int mv1 = __reduce_max_sync(0xffffffffu, has ? py + 1 : -1);
+            const int mu0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)(whole ? u : px) : 0x7fffffffu);
+            const int mv0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)(whole ? v : py) : 0x7fffffffu);
+            const int mu1 = __reduce_max_sync(0xffffffffu, has ? (whole ? u + 21 : px + 1) : -1);
+            const int mv1 = __reduce_max_sync(0xffffffffu, has ? (whole ? v + nr : py + 1) : -1);
+            const unsigned int mw = 441u * (unsigned int)__popc(__ballot_sync(0xffffffffu, has));  // (as if none were cut)
             if (lane == 0 && mu1 >= 0 && half == 0) {
                 atomicMin(&ss.cbox[0], mu0);
                 atomicMin(&ss.cbox[1], mv0);
                 atomicMax(&ss.cbox[2], mu1);
                 atomicMax(&ss.cbox[3], mv1);
+                atomicAdd(&ss.windows, mw);
             }
         }
         __syncthreads();
@@ -750,45 +965,77 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             __syncthreads();  // every thread has read the box before the next tile writes it
             continue;
         }
-        // the region staged ahead if it holds every projection of the tile with a
-        // margin, else the projections with as much of the windows around them as fits
-        Region reg{0, 0, 0, 0, 0, 1};
-        if (ahead && pw > 0 && max(ax0 - kUseMargin, 0) >= px0 && max(ay0 - kUseMargin, 0) >= py0 &&
-            min(ax1 + kUseMargin, 640) <= px0 + pw && min(ay1 + kUseMargin, 480) <= py0 + ph) {
-            reg = Region{0, px0, py0, px0 + pw, py0 + ph, stage_pitch(pw)};
-        } else {
-            for (int m = 10; m >= 0; m -= m > 4 ? 3 : 1) {
-                const int x0 = max(ax0 - m, 0), y0 = max(ay0 - m, 0);
-                const int w0 = min(ax1 + m, 640) - x0, h0 = min(ay1 + m, 480) - y0;
-                if (stage_pitch(w0) * h0 > kStagePixels<kPerSm>) continue;
-                reg = Region{0, x0, y0, x0 + w0, y0 + h0, stage_pitch(w0)};
-                stage_region<kWarps>(stage_all, a.synth, n_synth, a.synth_w, x0, y0, w0, h0, reg.pitch);
+        Region reg{0, 0, 0, 0, 0, 1};  // the staged part of the target, for the search by rectangles
+        unsigned long long key;
+        int wx0 = ax0, wy0 = ay0, wpitch = 0;  // and for the scan of whole windows: its corner, its pitch (0: not staged)
+        if (whole) {
+            if (ahead && ahead_whole && pw > 0 && ax0 >= px0 && ay0 >= py0 && ax1 <= px0 + pw && ay1 <= py0 + ph) {
+                wx0 = px0;
+                wy0 = py0;
+                wpitch = plane_pitch(pw);
+            } else if (plane_pitch(ax1 - ax0) * (ay1 - ay0) <= kPlanePixels<kS>) {
+                wpitch = plane_pitch(ax1 - ax0);
+                stage_planes<kWarps>(planes, a.synth, n_synth, a.synth_w, ax0, ay0, ax1 - ax0, ay1 - ay0, wpitch);
                 stage_wait();
                 __syncthreads();
-                break;
+            }
+            key = search_whole<kH>(a, planes, wpitch, (v - wy0) * wpitch + (u - wx0), nr, nc, u, v, wp, half);
+            if (half) list.key[threadIdx.x] = key;
+            if (threadIdx.x == 0 && tile < kIcpMaxCtas) {
+                // where the projections lie in windows of 21, and a little more for the next step's rectangles
+                IcpTile& t = st->tile[tile];
+                const int b[4] = {ax0 + 10, ay0 + 10, max(ax1 - 10, ax0 + 11), max(ay1 - 10, ay0 + 11)};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    t.near[k] = b[k];
+                    t.rect[k] = b[k] + (k < 2 ? -kUseMargin : kUseMargin);
+                }
+            }
+            __syncthreads();
+        } else if constexpr (kS != kWhole) {
+            // the region staged ahead if it holds every projection of the tile with a
+            // margin, else the projections with as much of the windows around them as fits
+            if (ahead && !ahead_whole && pw > 0 && max(ax0 - kUseMargin, 0) >= px0 && max(ay0 - kUseMargin, 0) >= py0 &&
+                min(ax1 + kUseMargin, 640) <= px0 + pw && min(ay1 + kUseMargin, 480) <= py0 + ph) {
+                reg = Region{0, px0, py0, px0 + pw, py0 + ph, stage_pitch(pw)};
+            } else {
+                for (int m = 10; m >= 0; m -= m > 4 ? 3 : 1) {
+                    const int x0 = max(ax0 - m, 0), y0 = max(ay0 - m, 0);
+                    const int w0 = min(ax1 + m, 640) - x0, h0 = min(ay1 + m, 480) - y0;
+                    if (stage_pitch(w0) * h0 > kStagePixels<kS>) continue;
+                    reg = Region{0, x0, y0, x0 + w0, y0 + h0, stage_pitch(w0)};
+                    stage_region<kWarps>(stage_all, a.synth, n_synth, a.synth_w, x0, y0, w0, h0, reg.pitch);
+                    stage_wait();
+                    __syncthreads();
+                    break;
+                }
+            }
+            if (kH == 2) hint = s_hint[source];
+            int hr = (int)(hint >> 16) - v, hc = (int)(hint & 0xffffu) - u;
+            if ((unsigned)hr >= (unsigned)nr || (unsigned)hc >= (unsigned)nc) hr = hc = -1;
+            bool listed = false;
+            key =
+                search_own<kS>(a, reg, nr, nc, cr, cc, hr, hc, first || tile >= kIcpMaxCtas, u, v, X, Y, w, pr, wp, half, ss, list, listed);
+            if (half && !listed) list.key[threadIdx.x] = key;  // for the source's first thread
+            __syncthreads();
+            const unsigned int n_items = ss.n_items;
+            if (threadIdx.x == 0 && tile < kIcpMaxCtas && ss.box[2] >= 0) {
+                IcpTile& t = st->tile[tile];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    t.near[k] = k == 0 ? ax0 : k == 1 ? ay0 : k == 2 ? ax1 : ay1;
+                    t.rect[k] = ss.box[k];
+                }
+                t.whole = whole_next(ss);
+            }
+            if (n_items) {
+                search_items<kS>(a.synth, n_items, a.neg_zero, list);
+                __syncthreads();
+                if (listed) key = list.key[threadIdx.x];
+                __syncthreads();  // the records take the list's place
             }
         }
-        if (kH == 2) hint = s_hint[source];
-        int hr = (int)(hint >> 16) - v, hc = (int)(hint & 0xffffu) - u;
-        if ((unsigned)hr >= (unsigned)nr || (unsigned)hc >= (unsigned)nc) hr = hc = -1;
-        bool listed = false;
-        unsigned long long key =
-            search_own<kH>(a, reg, nr, nc, cr, cc, hr, hc, first || tile >= kIcpMaxCtas, u, v, X, Y, w, pr, wp, half, ss, listed);
-        if (half && !listed) ss.list.key[threadIdx.x] = key;  // for the source's first thread
-        __syncthreads();
-        const unsigned int n_items = ss.n_items;
-        if (threadIdx.x == 0 && tile < kIcpMaxCtas && ss.box[2] >= 0) {
-            int* tb = st->tile_box + 4 * tile;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) tb[k] = ss.box[k];
-        }
-        if (n_items) {
-            search_items<kH>(a.synth, n_items, a.neg_zero, ss);
-            __syncthreads();
-            if (listed) key = ss.list.key[threadIdx.x];
-            __syncthreads();  // the records take the list's place
-        }
-        if (kH == 2 && !half) key = min(key, ss.list.key[threadIdx.x + kTileThreads]);
+        if (kH == 2 && !half) key = min(key, list.key[threadIdx.x + kTileThreads]);
         const bool out = mine && half == 0;  // the source's pair is its first thread's
         const bool hit = out && key < kNoPair;
         const float best = __uint_as_float((unsigned int)(key >> 32));
@@ -796,25 +1043,41 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
         if (hit) {
             const int x = u + (rc & 31), yy = v + (rc >> 5);
-            q = reg.holds(x, yy, 1, 1) ? stage_all[reg.at(x, yy)] : __ldg(a.synth + (size_t)yy * a.synth_w + x);
+            if (wpitch) {
+                const int at = (yy - wy0) * wpitch + (x - wx0);
+                q = make_float4(planes.x[at], planes.y[at], planes.z[at], 1.0f);
+            } else q = reg.holds(x, yy, 1, 1) ? stage_all[reg.at(x, yy)] : __ldg(a.synth + (size_t)yy * a.synth_w + x);
         }
         if (out && tile < kIcpMaxCtas)
             st->winner[tile * kTileThreads + source] = hit ? (unsigned int)(v + (rc >> 5)) << 16 | (u + (rc & 31)) : ~0u;
+        if (kS != kWhole && whole && pr.on) {  // what the next step's rectangles may hold, from the distance now
+            unsigned int n = nr * nc;
+            if (hit && w > pr.w_min) {
+                const float r = __fdividef(sqrtf(best), w);
+                n = (unsigned int)(fminf(fmaf(2.0f * pr.kx, r, 1.5f), (float)nc) * fminf(fmaf(2.0f * pr.ky, r, 1.5f), (float)nr));
+            }
+            const unsigned int total = __reduce_add_sync(0xffffffffu, n);
+            if (lane == 0 && half == 0) atomicAdd(&ss.area, total);
+        }
         if (a.pairs && out) {
             const size_t k = (size_t)y * n_cols + col;
             a.pairs[k] = hit ? (long long)(v + (rc >> 5)) * a.synth_w + (u + (rc & 31)) : -1ll;
             a.pairs_len2[k] = hit ? best : 0.01f;
         }
+        if (kS != kWhole && whole) {
+            __syncthreads();  // the records take the planes' end
+            if (threadIdx.x == 0 && tile < kIcpMaxCtas) st->tile[tile].whole = !pr.on || whole_next(ss);
+        }
         // this source's pair for the tile's moments (zeros when none)
         if (half == 0) {
             const int sidx = source;
-            ss.rec[0][sidx] = hit ? wp[0] : 0.f;
-            ss.rec[1][sidx] = hit ? wp[1] : 0.f;
-            ss.rec[2][sidx] = hit ? wp[2] : 0.f;
-            ss.rec[3][sidx] = q.x;
-            ss.rec[4][sidx] = q.y;
-            ss.rec[5][sidx] = q.z;
-            ss.rec[6][sidx] = hit ? best : 0.f;
+            rec[0][sidx] = hit ? wp[0] : 0.f;
+            rec[1][sidx] = hit ? wp[1] : 0.f;
+            rec[2][sidx] = hit ? wp[2] : 0.f;
+            rec[3][sidx] = q.x;
+            rec[4][sidx] = q.y;
+            rec[5][sidx] = q.z;
+            rec[6][sidx] = hit ? best : 0.f;
             const unsigned int nh = __popc(__ballot_sync(0xffffffffu, hit));
             if (lane == 0 && nh) atomicAdd(&ss.count, nh);
         }
@@ -822,7 +1085,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         if (threadIdx.x == 0) {  // for the next tile
 #pragma unroll
             for (int k = 0; k < 4; ++k) ss.box[k] = ss.cbox[k] = k < 2 ? 0x7fffffff : -1;
-            ss.n_items = 0u;
+            ss.n_items = ss.area = ss.windows = 0u;
         }
         // the tile's raw moments: each warp reduces two of the 16 over all
         // sources (lane l takes sources l, l + 32, ...), in float-float
@@ -838,9 +1101,9 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
                 for (int k = 0; k < kTileCols; ++k) {
                     const int sidx = lane + 32 * k;
                     FF m;
-                    if (c < 7) m = FF{ss.rec[c - 1][sidx], 0.0f};
-                    else if (c < 16) m = two_prod(ss.rec[(c - 7) / 3][sidx], ss.rec[3 + (c - 7) % 3][sidx]);
-                    else m = FF{ss.rec[6][sidx], 0.0f};
+                    if (c < 7) m = FF{rec[c - 1][sidx], 0.0f};
+                    else if (c < 16) m = two_prod(rec[(c - 7) / 3][sidx], rec[3 + (c - 7) % 3][sidx]);
+                    else m = FF{rec[6][sidx], 0.0f};
                     acc[h] = ff_add(acc[h], m);
                 }
             }
@@ -873,9 +1136,9 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
     if (threadIdx.x < 32) finish_step(st, tot, a.mail, a.mail_seq);
 }
 
-template <int kPerSm>
-__global__ void __launch_bounds__(kTileThreads * kHalves<kPerSm>, kPerSm) k_icp_step(IcpArgs a, IcpState* __restrict__ st, bool first) {
-    icp_step_body<kPerSm>(a, st, first, blockIdx.x, gridDim.x);
+template <int kS>
+__global__ void __launch_bounds__(kTileThreads * kHalves<kS>, kResident<kS>) k_icp_step(IcpArgs a, IcpState* __restrict__ st, bool first) {
+    icp_step_body<kS>(a, st, first, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------- Horn solve
@@ -1289,18 +1552,24 @@ __global__ void k_icp_begin(IcpState* st, Mat4 guess) {
 // Where the points of a caller's target project within their pixels: the
 // smallest and largest X(q) - x and Y(q) - (H - 1 - y) over the points in
 // front of the eye (a point nearer than w_far to the eye plane, or behind
-// it, is further than 0.1 m from every source that prunes).
-__global__ void __launch_bounds__(kThreads) k_target_range(IcpArgs a, float w_far, IcpState* __restrict__ st) {
+// it, is further than 0.1 m from every source that prunes).  A CTA joins its
+// threads' bounds first: one atomic per warp and bound queued at four words (18
+// us of a 1024x848 target, now 5, and 4 at 320x240).
+constexpr int kRangeThreads = 512;
+__global__ void __launch_bounds__(kRangeThreads) k_target_range(IcpArgs a, float w_far, IcpState* __restrict__ st) {
+    __shared__ int s_range[4];
+    if (threadIdx.x < 4) s_range[threadIdx.x] = threadIdx.x & 1 ? to_ordered(-INFINITY) : to_ordered(INFINITY);
+    __syncthreads();
     const int n = a.synth_w * a.synth_h;
     const float hw = fmul((float)a.synth_w, 0.5f), hh = fmul((float)a.synth_h, 0.5f);
     float lx = INFINITY, hx = -INFINITY, ly = INFINITY, hy = -INFINITY;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float4 q = __ldg(a.synth + i);
         const float p[4] = {q.x, q.y, q.z, 1.0f};
         float c[4];
         mat_vec(a.proj, p, c);
         if (!(isfinite(q.x) && isfinite(q.y) && isfinite(q.z)) || !(c[3] > w_far)) continue;
-        const int y = i / a.synth_w, x = i - y * a.synth_w;
+        const int y = (int)i / a.synth_w, x = (int)i - y * a.synth_w;
         const float dx = c[0] / c[3] * hw + hw - (float)x;
         const float dy = c[1] / c[3] * hh + hh - (float)(a.synth_h - 1 - y);
         lx = fminf(lx, dx);
@@ -1308,16 +1577,18 @@ __global__ void __launch_bounds__(kThreads) k_target_range(IcpArgs a, float w_fa
         ly = fminf(ly, dy);
         hy = fmaxf(hy, dy);
     }
-    int r[4] = {to_ordered(lx), to_ordered(hx), to_ordered(ly), to_ordered(hy)};
-    r[0] = __reduce_min_sync(0xffffffffu, r[0]);
-    r[1] = __reduce_max_sync(0xffffffffu, r[1]);
-    r[2] = __reduce_min_sync(0xffffffffu, r[2]);
-    r[3] = __reduce_max_sync(0xffffffffu, r[3]);
+    const int r0 = __reduce_min_sync(0xffffffffu, to_ordered(lx)), r1 = __reduce_max_sync(0xffffffffu, to_ordered(hx));
+    const int r2 = __reduce_min_sync(0xffffffffu, to_ordered(ly)), r3 = __reduce_max_sync(0xffffffffu, to_ordered(hy));
     if ((threadIdx.x & 31) == 0) {
-        atomicMin(&st->range[0], r[0]);
-        atomicMax(&st->range[1], r[1]);
-        atomicMin(&st->range[2], r[2]);
-        atomicMax(&st->range[3], r[3]);
+        atomicMin(&s_range[0], r0);
+        atomicMax(&s_range[1], r1);
+        atomicMin(&s_range[2], r2);
+        atomicMax(&s_range[3], r3);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        if (threadIdx.x & 1) atomicMax(&st->range[threadIdx.x], s_range[threadIdx.x]);
+        else atomicMin(&st->range[threadIdx.x], s_range[threadIdx.x]);
     }
 }
 
@@ -1454,12 +1725,16 @@ __global__ void k_icp_begin_batch(const IcpJob* __restrict__ jobs, int n) {
     if (v < n) icp_begin_body(jobs[v].st, jobs[v].guess);
 }
 
-template <int kPerSm>
-__global__ void __launch_bounds__(kTileThreads * kHalves<kPerSm>, kPerSm) k_icp_step_batch(const IcpJob* __restrict__ jobs, BlockMap m,
+// A batch's tiles search rectangles throughout (unless a target of the batch
+// allows none): they are many rounds of CTAs, so that their work counts and not the
+// slowest tile (8 sequences, 4 steps of 15: 10314 us, with windows by tile 10899,
+// with windows only 17463; frames three apart 11729, 12421, 18189).
+template <int kS>
+__global__ void __launch_bounds__(kTileThreads * kHalves<kS>, kResident<kS>) k_icp_step_batch(const IcpJob* __restrict__ jobs, BlockMap m,
                                                                         bool first) {
     const int v = block_owner(m, blockIdx.x);
     const unsigned int b0 = m.first[v];
-    icp_step_body<kPerSm>(jobs[v].a, jobs[v].st, first, blockIdx.x - b0, m.first[v + 1] - b0);
+    icp_step_body<kS, kS != kWhole>(jobs[v].a, jobs[v].st, first, blockIdx.x - b0, m.first[v + 1] - b0);
 }
 
 __global__ void k_backproject_batch(const BackprojectJob* __restrict__ jobs, BlockMap m) {
@@ -1504,38 +1779,72 @@ static int sm_count() {
     return sms;
 }
 
-cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess, int iterations,
-                              int /*ctas*/, cudaStream_t stream, IcpPoseMail* mail, unsigned long long seq) {
-    k_icp_begin<<<1, 32, 0, stream>>>(st, guess);
-    if (a.prune == kPruneMeasured && iterations > 0)
-        k_target_range<<<(a.synth_w * a.synth_h + kThreads * 4 - 1) / (kThreads * 4), kThreads, 0, stream>>>(
-            a, a.w_min * 0.125f, st);
-    const int ctas = icp_tiles(a.width, a.height);
-    // three tiles per SM (kStagePixels) where two would take more than one round and the windows fit
-    const bool three = ctas > 2 * sm_count() && 20 * a.synth_w <= 23 * a.width && 20 * a.synth_h <= 23 * a.height;
-    const bool one = ctas <= sm_count();
-    const auto step = three ? k_icp_step<3> : one ? k_icp_step<1> : k_icp_step<2>;
-    const size_t smem = (three ? kStagePixels<3> : one ? kStagePixels<1> : kStagePixels<2>) * sizeof(float4);
-    // programmatic dependent launch: each step's grid is scheduled as soon as
-    // every CTA of the one before has finished its association, overlapping
-    // its launch with the previous finisher (k_icp_step waits for it)
+// Which build an alignment's steps take, all of them the same: the first steps
+// after a change of kernels wait for the finisher's instructions, 2 us each.
+// Whole windows only where nothing is known of the target, and where there are too
+// few steps to win by rectangles: a 640x480 pair wins from the fifth step on and
+// loses a little before (4 steps 133 us against 127), one of 320x240 wins at once (4
+// steps 84 against 91).  A finer target's windows take more than that build stages.
+struct StepShape {
+    int shape;
+    template <typename F>
+    auto with(F f) const {
+        switch (shape) {
+            case kWhole: return f(std::integral_constant<int, kWhole>{});
+            case 1: return f(std::integral_constant<int, 1>{});
+            case 2: return f(std::integral_constant<int, 2>{});
+            default: return f(std::integral_constant<int, 3>{});
+        }
+    }
+};
+// fine: the target's pixels are finer than 1 / 1.15 of the source's
+static StepShape tile_shape(int ctas, bool fine) {
+    const int sms = sm_count();
+    return {ctas <= sms ? 1 : ctas > 2 * sms && !fine ? 3 : 2};
+}
+static StepShape step_shape(int ctas, int iterations, int prune, bool fine) {
+    const StepShape s = tile_shape(ctas, fine);
+    return prune == kPruneOff || (iterations < (s.shape == 2 ? 8 : 4) && !fine) ? StepShape{kWhole} : s;
+}
+
+// programmatic dependent launch: each step's grid is scheduled as soon as
+// every CTA of the one before has finished its association, overlapping
+// its launch with the previous finisher (k_icp_step waits for it)
+template <int kS, typename Kernel, typename... Args>
+static cudaError_t launch_step(Kernel kernel, int ctas, cudaStream_t stream, Args... args) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(one ? 2 * kTileThreads : kTileThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.blockDim = dim3(kTileThreads * kHalves<kS>);
+    cfg.dynamicSmemBytes = kTileBytes<kS>;
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    IcpArgs last = a;  // the last step publishes the pose
-    last.mail = mail;
-    last.mail_seq = seq;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess, int iterations,
+                              int /*ctas*/, cudaStream_t stream, IcpPoseMail* mail, unsigned long long seq) {
+    k_icp_begin<<<1, 32, 0, stream>>>(st, guess);
+    const int ctas = icp_tiles(a.width, a.height);
+    const bool fine = 20 * a.synth_w > 23 * a.width || 20 * a.synth_h > 23 * a.height;
     IcpArgs other = a;
     other.mail = nullptr;
+    const StepShape shape = step_shape(ctas, iterations, a.prune, fine);
+    if (shape.shape == kWhole) other.prune = kPruneOff;
+    if (other.prune == kPruneMeasured)
+        k_target_range<<<sm_count(), kRangeThreads, 0, stream>>>(a, a.w_min * 0.125f, st);
+    IcpArgs last = other;  // the last step publishes the pose
+    last.mail = mail;
+    last.mail_seq = seq;
     for (int it = 0; it < iterations; ++it) {
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, step, it + 1 == iterations ? last : other, st, it == 0);
+        const cudaError_t e =
+            shape.with([&](auto s) {
+                return launch_step<s.value>(k_icp_step<s.value>, ctas, stream, it + 1 == iterations ? last : other, st,
+                                            it == 0);
+            });
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
@@ -1544,38 +1853,27 @@ cudaError_t icp_align_enqueue(const IcpArgs& a, IcpState* st, const Mat4& guess,
 // The association's dynamic shared memory above the default 48 KB limit; set
 // with every context, outside any stream capture.
 cudaError_t icp_init_device() {
-    auto allow = [](auto kernel, int pixels) {
-        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pixels * (int)sizeof(float4));
-    };
-    cudaError_t e = allow(k_icp_step<1>, kStagePixels<1>);
-    if (!e) e = allow(k_icp_step<2>, kStagePixels<2>);
-    if (!e) e = allow(k_icp_step<3>, kStagePixels<3>);
-    if (!e) e = allow(k_icp_step_batch<2>, kStagePixels<2>);
-    if (!e) e = allow(k_icp_step_batch<3>, kStagePixels<3>);
+    cudaError_t e = cudaSuccess;
+    for (int shape = 0; shape < 4 && !e; ++shape)
+        e = StepShape{shape}.with([](auto s) {
+            const cudaError_t x = cudaFuncSetAttribute(k_icp_step<s.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)kTileBytes<s.value>);
+            return x ? x
+                     : cudaFuncSetAttribute(k_icp_step_batch<s.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)kTileBytes<s.value>);
+        });
     return e;
 }
 
-cudaError_t icp_align_batch_enqueue(const IcpJob* jobs, int n, const BlockMap& map, int iterations,
+cudaError_t icp_align_batch_enqueue(const IcpJob* jobs, int n, const BlockMap& map, int iterations, bool prune,
                                     cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     k_icp_begin_batch<<<(n + 63) / 64, 64, 0, stream>>>(jobs, n);
-    const bool three = (int)map.grid > 2 * sm_count();  // (targets have their sources' sizes)
-    const auto step = three ? k_icp_step_batch<3> : k_icp_step_batch<2>;
-    const size_t smem = (three ? kStagePixels<3> : kStagePixels<2>) * sizeof(float4);
-    // programmatic dependent launch, as for a single pair: each step's grid
-    // is scheduled once every CTA of the step before has finished its association
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(map.grid);
-    cfg.blockDim = dim3(kTileThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    const StepShape shape = prune ? tile_shape((int)map.grid, false) : StepShape{kWhole};  // (targets have their sources' sizes)
     for (int it = 0; it < iterations; ++it) {
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, step, jobs, map, it == 0);
+        const cudaError_t e = shape.with([&](auto s) {
+            return launch_step<s.value>(k_icp_step_batch<s.value>, (int)map.grid, stream, jobs, map, it == 0);
+        });
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();

@@ -321,6 +321,14 @@ struct IcpIterStats {
     float tail_us;    // last CTA end to the updated pose
 };
 
+// What an association tile leaves for its next step.
+struct IcpTile {
+    int near[4];  // where its sources project: x0, y0, x1, y1
+    int rect[4];  // the part of the target that it searched, likewise
+    int whole;    // scan whole windows (else the rectangles that can win)
+    int pad[3];
+};
+
 struct IcpState {
     alignas(16) float pose_f[16];   // eye-to-world estimate, kifi order (float-float high part)
     float pose_lo[16];  // and its low part
@@ -332,7 +340,7 @@ struct IcpState {
     unsigned long long t_start, t_body;  // globaltimer stamps of the running step
     IcpIterStats stats[kIcpMaxStats];
     float part[34 * kIcpMaxCtas];   // per-CTA float-float partials: hi, lo rows of 17 components
-    int tile_box[4 * kIcpMaxCtas];  // each tile's window box in the last step: x0, y0, x1, y1
+    IcpTile tile[kIcpMaxCtas];
     // per tile and source: the pixel that won the last step (row << 16 | column), or ~0; here, so that
     // an alignment allocates nothing, whatever its frame's size (tiles from kIcpMaxCtas on keep none)
     unsigned int winner[kIcpTileSources * kIcpMaxCtas];
@@ -349,7 +357,8 @@ struct IcpJob {
 // `iterations` AlignSteps of the n pairs of `jobs` (a device table), one
 // launch per step for all of them; pair v's CTAs are map.first[v] ..
 // map.first[v+1] - 1, one per association tile.
-cudaError_t icp_align_batch_enqueue(const IcpJob* jobs, int n, const BlockMap& map, int iterations,
+// prune: every pair's (IcpArgs::prune is not kPruneOff)
+cudaError_t icp_align_batch_enqueue(const IcpJob* jobs, int n, const BlockMap& map, int iterations, bool prune,
                                     cudaStream_t stream);
 // Back-projection of one frame per pair into its target (the next frame's
 // ICP target), for the n entries of `jobs` (device table).
