@@ -22,6 +22,7 @@ kifi_status fail(kifi_status s, const char* what) {
 }
 
 kifi_status cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();  // reported here: the next call's launches are checked anew
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
     if (e == cudaErrorMemoryAllocation) return KIFI_ERR_OUT_OF_MEMORY;
     if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return KIFI_ERR_NO_DEVICE;
