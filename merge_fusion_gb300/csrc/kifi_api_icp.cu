@@ -69,9 +69,11 @@ kifi_status reserve_bytes(void** p, size_t* cap, size_t bytes, cudaStream_t st) 
     return KIFI_OK;
 }
 
+// (the target that was there goes with its buffer, also where a larger one cannot be had)
 kifi_status reserve_target(kifi_icp* c, int w, int h) {
-    return reserve_bytes((void**)&c->synth, &c->synth_cap, ((size_t)w * h + icp_box_count(w, h)) * sizeof(float4),
-                         c->stream);
+    const size_t bytes = ((size_t)w * h + icp_box_count(w, h)) * sizeof(float4);
+    if (bytes > c->synth_cap) c->have_target = false;
+    return reserve_bytes((void**)&c->synth, &c->synth_cap, bytes, c->stream);
 }
 float4* boxes_of(const kifi_icp* c, int w, int h) { return c->synth + (size_t)w * h; }
 

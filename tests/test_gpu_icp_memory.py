@@ -1,5 +1,5 @@
 """A target that does not fit the device's memory is refused; the context's next
-target is used."""
+target is used.  Until then it has none, and aligning says so."""
 import numpy as np
 import pytest
 
@@ -34,3 +34,14 @@ def test_the_next_target_is_used(gpu, oracle_cpu):
     _refuse(icp, pose)
     icp.SetTarget(target, pose)
     assert np.array_equal(icp.AlignToTarget(seq.depth_m(1), pose, cam_params(seq.camera), 2), want)
+
+
+def test_a_refused_target_leaves_none(gpu, oracle_cpu):
+    from merge_fusion_gb300 import _lib, kifi
+    seq, pose, target = _room(oracle_cpu)
+    icp = kifi.ICP()
+    icp.SetTarget(target, pose)
+    _refuse(icp, pose)
+    with pytest.raises(_lib.KifiError) as err:
+        icp.AlignToTarget(seq.depth_m(1), pose, cam_params(seq.camera), 2)
+    assert err.value.status == _lib.KIFI_ERR_INVALID_ARGUMENT
