@@ -70,7 +70,7 @@ LAUNCHES_FUSION, LAUNCHES_TRACKING, LAUNCHES_MESH = 7, ICP_ITERS + 2, 8
 KERNELS_PER_MESH = 5
 # bytes the host reads back per tracked frame: the head of the ICP state
 # (float and float-float pose, counters, 64 iteration records of 20 bytes)
-ICP_HEAD_BYTES = 192 + 64 * 20
+ICP_HEAD_BYTES = 208 + 64 * 20
 MESH_COUNTS_BYTES = 40
 FP32_LANES_PER_SM = 128  # FP32 FMA lanes of a Blackwell SM: 2 flop per lane per clock
 

@@ -91,9 +91,9 @@ cudaError_t sort_u32(uint32_t* keys, uint32_t* vals, const unsigned int* n_dev, 
 // even count so the result lands back in `keys`
 cudaError_t sort_keys(void* keys, int key_bytes, int key_bits, uint32_t* vals, const unsigned int* n_dev,
                       SortScratch& s, unsigned int* status, int grid_ctas, cudaStream_t st);
-// the frame path's three 10-bit passes over 30-bit keys whose histograms and
-// pass counters are already set (see kFrameDigitBits); *sorted receives the
-// buffer holding the result
+// the frame path's passes (three of 10 bits over 30-bit keys, up to five of 8 bits
+// over 64-bit ones) over keys whose histograms and pass counters are already set
+// (see kFrameDigitBits); *sorted receives the buffer holding the result
 cudaError_t sort_frame_keys(void* keys, int key_bytes, int kb, const unsigned int* n_dev, SortScratch& s,
                             unsigned int* status, int grid_ctas, bool alone, bool chained, cudaStream_t st, const void** sorted);
 
@@ -387,7 +387,7 @@ cudaError_t expand_target_enqueue(const float* in, int width, int height, float4
 
 cudaError_t bin_enqueue(const float* pts, unsigned int n, const Mat4& w2c, int width, int height,
                         unsigned long long* zbuf, float* out, int ctas, cudaStream_t st);
-// Bin straight into an ICP target (float4 per pixel, w unused)
+// Bin straight into an ICP target (a float4 per pixel: w = 1, which the distances take in; x = NaN: no point)
 cudaError_t bin_target_enqueue(const float* pts, unsigned int n, const Mat4& w2c, int width, int height,
                                unsigned long long* zbuf, float4* out, float4* boxes, int ctas, cudaStream_t st);
 

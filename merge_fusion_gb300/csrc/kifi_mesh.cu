@@ -119,7 +119,8 @@ __device__ __noinline__ bool cross_exact(const float2* vals, unsigned int a, uns
 // CTA of the next kernel for itself; of words, the last CTA to finish turns the
 // runs' totals into offsets.  Up to 4 and 3 rounds of resident CTAs: runs differ
 // in what they hold, and in one round the longest sets the time (at the size
-// above, build 98 us in one round, 82 in four; classification 130 and 107).
+// above, build 98 us in one round, 82 in four; classification 130 and 107): 16 and
+// 24 runs for each of the GPU's 152 SMs.
 constexpr unsigned int kVoxelRuns = 2432, kWordRuns = 3648;
 constexpr int kClassThreads = 128;
 constexpr unsigned int kNoWord = 0xffffffffu;
