@@ -358,22 +358,23 @@ struct SearchSmem {
     int cbox[4];     // and projections (or windows)
     int pred[4];     // the region staged ahead: x0, y0, w, h
     int ahead_whole; // as planes, for a whole-window scan
-    unsigned int area, windows;  // candidates in the rectangles and in the windows
+    unsigned int area;  // the cost of the rectangles, in candidates, of the warp that has the most
     FF acc[17];      // the CTA's moments (index 0 unused: count)
     unsigned int count;
 };
-// Whether the tile's next step scans whole windows: where its rectangles hold
-// more than a quarter of the windows' candidates.  The whole-window scan reads two
+// Whether the tile's next step scans whole windows: where the rectangles of one of
+// its warps hold more than 5/16 of the windows' candidates (a step is as long as
+// the slowest warp, not as the average).  The whole-window scan reads two
 // candidates at a time with no bounds or boxes before it, and all of a warp's
 // lanes alike; with fast motion a tile of large rectangles holds up its whole step.
 // The share is the step's own after a search, and after a scan what the distances
-// to the winners would leave.  Times, us, searching rectangles only / whole windows
-// only / by tile: 640x480, 15 steps, frames one apart 375 / 423 / 372, three apart
-// 498 / 461 / 456; 410x307, 10 steps, three apart 263 / 232 / 213; tracking at 640x480,
-// ten frames 5267 / - / 5069.  An eighth instead of a quarter: 358 and 440, but
-// the closed loop 2117 -> 2175 us; a half: 376 and 501.
-constexpr unsigned int kWholeShare = 4;  // sixteenths
-__device__ __forceinline__ int whole_next(const SearchSmem& ss) { return ss.area * 16u > ss.windows * kWholeShare; }
+// to the winners would leave.  Times, us, of 15 steps, windows only where a
+// launch's shape says so / by tile: 640x480, frames one apart 423 / 345, three
+// apart 461 / 422; 512x424 411 / 315, 452 / 395; 1024x848 626 / 459, 724 / 576;
+// tracking at 640x480, ten frames 5290 / 4990.  4/16: the closed loop 2130 ->
+// 2170 us; 6/16 and 8/16: three apart 459 and more.
+constexpr unsigned int kWholeShare = 5;  // sixteenths
+__device__ __forceinline__ int whole_next(const SearchSmem& ss) { return ss.area > 441u * 32u * kWholeShare / 16u; }
 // What part of the target a tile has staged: pixels [x0, x1) x [y0, y1).
 struct Region {
     int buf;  // its first pixel's index in the CTA's staging buffer
@@ -555,25 +556,33 @@ __device__ __forceinline__ unsigned long long search_whole(const IcpArgs& a, con
 // (u, v)) by its own thread.  It bounds the distance to the nearest candidate,
 // cuts the window down to the rectangle that can win and, where that is still
 // large (fast motion, a depth edge), to the blocks of 8 x 4 target pixels
-// whose bounding boxes are near enough; it scans the rectangle in the
+// whose bounding boxes are near enough (bound_own); it scans the rectangle in the
 // reference's row-major order, in the staged region where that holds it, else
-// in the target itself.  A rectangle far above its warp's average goes onto
+// in the target itself (scan_own).  A rectangle far above its warp's average goes onto
 // the tile's list row by row, for all threads (search_items).  (cr, cc): the
 // candidate the source projects to; X, Y, w: its projected column and row
 // coordinate (upwards) and clip w; (hr, hc): a candidate likely to be near
-// (-1: none).  Returns the best key so far; by whole warps.  Measured at
+// (-1: none), the last winner or the pixel nearest to it in a window that has
+// moved past it.  Where the rectangles leave the staged region, all of a tile's
+// are staged instead, if they fit (from global memory a few dozen of them take
+// longer than the step: 15 steps at 640x480 with frames three apart 446 -> 422 us).
+// Returns the best key so far; by whole warps.  Measured at
 // 640x480: 10-40 candidates per source instead of 441 after the first two
-// steps, an alignment of 15 steps 329 us (433 us with the whole windows); the
+// steps, an alignment of 15 steps 334 us (433 us with the whole windows); the
 // step is then held by its serial parts -- the projection, the moments, the
 // last CTA's totals and Horn solve, about 11 of 16 us -- and by the tile with
 // the most candidates.
 constexpr int kOwnArea = 32;    // rectangles up to this, and up to 1.5 times the warp's average, are scanned by their thread
-constexpr int kBoxArea = 72;    // rectangles above this are cut down by the blocks' boxes
+constexpr int kBoxArea = 72;    // rectangles above this are cut down by the blocks' boxes,
+constexpr int kBoxCost = 4;     // of which one takes about as long as this many candidates
+struct OwnRect {
+    int r0, rows, c0, cols;
+    bool wraps;  // reads on in the next row of the target
+};
 template <int kS>
-__device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const Region& reg, int nr, int nc, int cr,
-                                                         int cc, int hr, int hc, bool first, int u, int v, float X,
-                                                         float Y, float w, const Prune& pr, const float (&p)[4],
-                                                         int half, SearchSmem& ss, TileList<kS>& list, bool& listed) {
+__device__ __forceinline__ OwnRect bound_own(const IcpArgs& a, const Region& reg, int nr, int nc, int cr, int cc, int hr,
+                                             int hc, bool first, int u, int v, float X, float Y, float w,
+                                             const Prune& pr, const float (&p)[4], int half, SearchSmem& ss) {
     constexpr int kH = kHalves<kS>;
     const int W = a.synth_w, H = a.synth_h;
     const Packed pp{f2_pack(p[0], p[1]), f2_pack(p[2], p[3])};
@@ -647,11 +656,13 @@ __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const
     }
     if (rows <= 0 || cols <= 0) rows = cols = 0;
     const bool wraps = u + c0 + cols > W;
+    int boxes = 0;  // looked at
     if (rows * cols > kBoxArea && !wraps) {  // (blocks do not follow a window into the next row)
         // the rectangle of the blocks no further than the bound (with the roundings covered)
         const int nbx = (W + kBlockW - 1) / kBlockW;
         const int x0 = u + c0, y0 = v + r0, bx1 = (x0 + cols - 1) >> 3, by1 = (y0 + rows - 1) >> 2;
         const float far = b * 1.00001f;
+        boxes = (bx1 - (x0 >> 3) + 1) * (by1 - (y0 >> 2) + 1);
         int mx0 = bx1 + 1, mx1 = -1, my0 = by1 + 1, my1 = -1;
         for (int by = y0 >> 2; by <= by1; ++by)
             for (int bx = x0 >> 3; bx <= bx1; ++bx) {
@@ -688,10 +699,22 @@ __device__ __forceinline__ unsigned long long search_own(const IcpArgs& a, const
             atomicMax(&ss.box[3], by1);
         }
     }
+    const unsigned int cost = __reduce_add_sync(0xffffffffu, (unsigned int)(n + kBoxCost * boxes));
+    if ((threadIdx.x & 31) == 0) atomicMax(&ss.area, cost * kH);
+    return OwnRect{r0, rows, c0, cols, wraps};
+}
+template <int kS>
+__device__ __forceinline__ unsigned long long scan_own(const IcpArgs& a, const Region& reg, const OwnRect& own, int u,
+                                                       int v, const float (&p)[4], SearchSmem& ss, TileList<kS>& list,
+                                                       bool& listed) {
+    const int W = a.synth_w, H = a.synth_h;
+    const Packed pp{f2_pack(p[0], p[1]), f2_pack(p[2], p[3])};
+    const unsigned long long nz = f2_pack(a.neg_zero, a.neg_zero);
+    const int r0 = own.r0, rows = own.rows, c0 = own.c0, cols = own.cols, n = rows * cols, x0 = u + c0, y0 = v + r0;
+    const bool wraps = own.wraps;
     // (a warp's own rectangles, of vertical neighbours, read shared memory
     // without conflicts; the list's rows do not)
     const int total = (int)__reduce_add_sync(0xffffffffu, (unsigned int)n);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&ss.area, (unsigned int)total);
     const int most = max(kOwnArea, total * 3 >> 6);
     const bool in = reg.holds(x0, y0, cols, rows);
     const int number = r0 * 32 + c0;
@@ -751,7 +774,7 @@ __device__ __noinline__ void finish_step(IcpState* __restrict__ st, const FF* __
 // rows, a thread one source (two threads where kHalves is 2), a warp 32 vertically adjacent ones.  Each thread
 // back-projects and projects its source, the CTA stages the part of the
 // target that the tile's searches will mostly read in shared memory, and
-// search_own and search_items find each source's nearest candidate, the
+// bound_own, scan_own and search_items find each source's nearest candidate, the
 // reference's first strict minimum.  Target pixel (y1, x1) is linear index y1 * synth_w + x1 as
 // in the reference; indices past the buffer's end are invalid points.
 //
@@ -855,7 +878,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             ss.box[k] = ss.cbox[k] = k < 2 ? 0x7fffffff : -1;
         }
         ss.ahead_whole = guess;
-        ss.n_items = ss.count = ss.area = ss.windows = 0u;
+        ss.n_items = ss.count = ss.area = 0u;
     }
     if (threadIdx.x < kMoments) ss.acc[threadIdx.x] = FF{0.0f, 0.0f};
     __syncthreads();
@@ -900,7 +923,9 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
     for (int tile = (int)blk; tile < tiles; tile += (int)nblk) {
         const bool ahead = tile == tile0;  // its region, depths and hints were loaded above
         // the tile's scan, as it found it best in the last step
-        const bool whole = kRects ? false : kS == kWhole || first || !pr.on || tile >= kIcpMaxCtas || (ahead ? ahead_whole : st->tile[tile].whole != 0);
+        const bool whole = kRects ? false
+                                  : kS == kWhole || first || !pr.on || tile >= kIcpMaxCtas ||
+                                        (ahead ? ahead_whole : st->tile[tile].whole != 0);
         const int col = (tile % tiles_x) * kTileCols + warp, y = (tile / tiles_x) * kTileRows + lane;
         const bool mine = col < n_cols && y < a.height;
         float wp[4] = {0.f, 0.f, 0.f, 0.f};
@@ -943,13 +968,11 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             const int mv0 = (int)__reduce_min_sync(0xffffffffu, has ? (unsigned)(whole ? v : py) : 0x7fffffffu);
             const int mu1 = __reduce_max_sync(0xffffffffu, has ? (whole ? u + 21 : px + 1) : -1);
             const int mv1 = __reduce_max_sync(0xffffffffu, has ? (whole ? v + nr : py + 1) : -1);
-            const unsigned int mw = 441u * (unsigned int)__popc(__ballot_sync(0xffffffffu, has));  // (as if none were cut)
             if (lane == 0 && mu1 >= 0 && half == 0) {
                 atomicMin(&ss.cbox[0], mu0);
                 atomicMin(&ss.cbox[1], mv0);
                 atomicMax(&ss.cbox[2], mu1);
                 atomicMax(&ss.cbox[3], mv1);
-                atomicAdd(&ss.windows, mw);
             }
         }
         __syncthreads();
@@ -994,15 +1017,19 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             __syncthreads();
         } else if constexpr (kS != kWhole) {
             // the region staged ahead if it holds every projection of the tile with a
-            // margin, else the projections with as much of the windows around them as fits
-            if (ahead && !ahead_whole && pw > 0 && max(ax0 - kUseMargin, 0) >= px0 && max(ay0 - kUseMargin, 0) >= py0 &&
-                min(ax1 + kUseMargin, 640) <= px0 + pw && min(ay1 + kUseMargin, 480) <= py0 + ph) {
+            // margin, else the projections with as much of the windows around them as
+            // fits; where the target's points are off their pixels' centres, as far off
+            const int sx = __float2int_rn(0.5f * (pr.lo_x + pr.hi_x) - 0.5f);
+            const int sy = __float2int_rn(0.5f * (pr.lo_y + pr.hi_y) - 0.5f);
+            const int bx0 = ax0 - sx, by0 = ay0 + sy, bx1 = ax1 - sx, by1 = ay1 + sy;
+            if (ahead && !ahead_whole && pw > 0 && max(bx0 - kUseMargin, 0) >= px0 && max(by0 - kUseMargin, 0) >= py0 &&
+                min(bx1 + kUseMargin, 640) <= px0 + pw && min(by1 + kUseMargin, 480) <= py0 + ph) {
                 reg = Region{0, px0, py0, px0 + pw, py0 + ph, stage_pitch(pw)};
             } else {
                 for (int m = 10; m >= 0; m -= m > 4 ? 3 : 1) {
-                    const int x0 = max(ax0 - m, 0), y0 = max(ay0 - m, 0);
-                    const int w0 = min(ax1 + m, 640) - x0, h0 = min(ay1 + m, 480) - y0;
-                    if (stage_pitch(w0) * h0 > kStagePixels<kS>) continue;
+                    const int x0 = max(bx0 - m, 0), y0 = max(by0 - m, 0);
+                    const int w0 = min(bx1 + m, 640) - x0, h0 = min(by1 + m, 480) - y0;
+                    if (w0 <= 0 || h0 <= 0 || stage_pitch(w0) * h0 > kStagePixels<kS>) continue;
                     reg = Region{0, x0, y0, x0 + w0, y0 + h0, stage_pitch(w0)};
                     stage_region<kWarps>(stage_all, a.synth, n_synth, a.synth_w, x0, y0, w0, h0, reg.pitch);
                     stage_wait();
@@ -1011,11 +1038,23 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
                 }
             }
             if (kH == 2) hint = s_hint[source];
-            int hr = (int)(hint >> 16) - v, hc = (int)(hint & 0xffffu) - u;
-            if ((unsigned)hr >= (unsigned)nr || (unsigned)hc >= (unsigned)nc) hr = hc = -1;
+            // (where the window has moved past it, the window's nearest pixel)
+            const int hr = hint == ~0u ? -1 : min(max((int)(hint >> 16) - v, 0), nr - 1);
+            const int hc = hint == ~0u ? -1 : min(max((int)(hint & 0xffffu) - u, 0), nc - 1);
+            const OwnRect own = bound_own<kS>(a, reg, nr, nc, cr, cc, hr, hc, first || tile >= kIcpMaxCtas, u, v, X, Y, w,
+                                              pr, wp, half, ss);
+            if constexpr (!kRects) {  // rectangles beyond the staged region: those of all sources, if they fit
+                __syncthreads();
+                const int x0 = ss.box[0], y0 = ss.box[1], w0 = ss.box[2] - x0, h0 = ss.box[3] - y0;
+                if (ss.box[2] >= 0 && !reg.holds(x0, y0, w0, h0) && stage_pitch(w0) * h0 <= kStagePixels<kS>) {
+                    reg = Region{0, x0, y0, x0 + w0, y0 + h0, stage_pitch(w0)};
+                    stage_region<kWarps>(stage_all, a.synth, n_synth, a.synth_w, x0, y0, w0, h0, reg.pitch);
+                    stage_wait();
+                    __syncthreads();
+                }
+            }
             bool listed = false;
-            key =
-                search_own<kS>(a, reg, nr, nc, cr, cc, hr, hc, first || tile >= kIcpMaxCtas, u, v, X, Y, w, pr, wp, half, ss, list, listed);
+            key = scan_own<kS>(a, reg, own, u, v, wp, ss, list, listed);
             if (half && !listed) list.key[threadIdx.x] = key;  // for the source's first thread
             __syncthreads();
             const unsigned int n_items = ss.n_items;
@@ -1057,7 +1096,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
                 n = (unsigned int)(fminf(fmaf(2.0f * pr.kx, r, 1.5f), (float)nc) * fminf(fmaf(2.0f * pr.ky, r, 1.5f), (float)nr));
             }
             const unsigned int total = __reduce_add_sync(0xffffffffu, n);
-            if (lane == 0 && half == 0) atomicAdd(&ss.area, total);
+            if (lane == 0 && half == 0) atomicMax(&ss.area, total);
         }
         if (a.pairs && out) {
             const size_t k = (size_t)y * n_cols + col;
@@ -1085,7 +1124,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
         if (threadIdx.x == 0) {  // for the next tile
 #pragma unroll
             for (int k = 0; k < 4; ++k) ss.box[k] = ss.cbox[k] = k < 2 ? 0x7fffffff : -1;
-            ss.n_items = ss.area = ss.windows = 0u;
+            ss.n_items = ss.area = 0u;
         }
         // the tile's raw moments: each warp reduces two of the 16 over all
         // sources (lane l takes sources l, l + 32, ...), in float-float
