@@ -579,7 +579,7 @@ struct OwnRect {
     int r0, rows, c0, cols;
     bool wraps;  // reads on in the next row of the target
 };
-template <int kS>
+template <int kS, bool kRects>
 __device__ __forceinline__ OwnRect bound_own(const IcpArgs& a, const Region& reg, int nr, int nc, int cr, int cc, int hr,
                                              int hc, bool first, int u, int v, float X, float Y, float w,
                                              const Prune& pr, const float (&p)[4], int half, SearchSmem& ss) {
@@ -699,8 +699,10 @@ __device__ __forceinline__ OwnRect bound_own(const IcpArgs& a, const Region& reg
             atomicMax(&ss.box[3], by1);
         }
     }
-    const unsigned int cost = __reduce_add_sync(0xffffffffu, (unsigned int)(n + kBoxCost * boxes));
-    if ((threadIdx.x & 31) == 0) atomicMax(&ss.area, cost * kH);
+    if constexpr (!kRects) {  // for whole_next
+        const unsigned int cost = __reduce_add_sync(0xffffffffu, (unsigned int)(n + kBoxCost * boxes));
+        if ((threadIdx.x & 31) == 0) atomicMax(&ss.area, cost * kH);
+    }
     return OwnRect{r0, rows, c0, cols, wraps};
 }
 template <int kS>
@@ -810,7 +812,7 @@ __device__ __forceinline__ FF two_prod(float a, float b) {
 // One AlignStep of one frame pair; `blk` / `nblk`: this CTA's index among
 // the nblk CTAs that work on the pair (the launch's own grid, or a share of
 // a batched launch over several pairs).
-// kRects: rectangles only
+// kRects: rectangles only (a batch has tiles enough to hide a slow one).
 template <int kS, bool kRects = false>
 __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __restrict__ st, bool first,
                                               unsigned int blk, unsigned int nblk) {
@@ -1019,8 +1021,9 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             // the region staged ahead if it holds every projection of the tile with a
             // margin, else the projections with as much of the windows around them as
             // fits; where the target's points are off their pixels' centres, as far off
-            const int sx = __float2int_rn(0.5f * (pr.lo_x + pr.hi_x) - 0.5f);
-            const int sy = __float2int_rn(0.5f * (pr.lo_y + pr.hi_y) - 0.5f);
+            // (in a batch, whose 80 registers that would spill, at the projections)
+            const int sx = kRects ? 0 : __float2int_rn(0.5f * (pr.lo_x + pr.hi_x) - 0.5f);
+            const int sy = kRects ? 0 : __float2int_rn(0.5f * (pr.lo_y + pr.hi_y) - 0.5f);
             const int bx0 = ax0 - sx, by0 = ay0 + sy, bx1 = ax1 - sx, by1 = ay1 + sy;
             if (ahead && !ahead_whole && pw > 0 && max(bx0 - kUseMargin, 0) >= px0 && max(by0 - kUseMargin, 0) >= py0 &&
                 min(bx1 + kUseMargin, 640) <= px0 + pw && min(by1 + kUseMargin, 480) <= py0 + ph) {
@@ -1041,8 +1044,8 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
             // (where the window has moved past it, the window's nearest pixel)
             const int hr = hint == ~0u ? -1 : min(max((int)(hint >> 16) - v, 0), nr - 1);
             const int hc = hint == ~0u ? -1 : min(max((int)(hint & 0xffffu) - u, 0), nc - 1);
-            const OwnRect own = bound_own<kS>(a, reg, nr, nc, cr, cc, hr, hc, first || tile >= kIcpMaxCtas, u, v, X, Y, w,
-                                              pr, wp, half, ss);
+            const OwnRect own = bound_own<kS, kRects>(a, reg, nr, nc, cr, cc, hr, hc, first || tile >= kIcpMaxCtas, u, v,
+                                                      X, Y, w, pr, wp, half, ss);
             if constexpr (!kRects) {  // rectangles beyond the staged region: those of all sources, if they fit
                 __syncthreads();
                 const int x0 = ss.box[0], y0 = ss.box[1], w0 = ss.box[2] - x0, h0 = ss.box[3] - y0;
@@ -1065,7 +1068,7 @@ __device__ __forceinline__ void icp_step_body(const IcpArgs& a, IcpState* __rest
                     t.near[k] = k == 0 ? ax0 : k == 1 ? ay0 : k == 2 ? ax1 : ay1;
                     t.rect[k] = ss.box[k];
                 }
-                t.whole = whole_next(ss);
+                if constexpr (!kRects) t.whole = whole_next(ss);
             }
             if (n_items) {
                 search_items<kS>(a.synth, n_items, a.neg_zero, list);
